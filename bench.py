@@ -498,10 +498,10 @@ def autotune(lib, h, reps=5):
     assert rc == 0, lib.gbims_last_error(h)
     out = {"reduction_blocks": t.reduction_blocks}
     if t.level_mode >= 0:
-        out.update(level_mode=("sync-free" if t.level_mode == 1 else "per-level launches"),
+        out.update(level_mode=("row ranges" if t.level_mode == 1 else "per-level launches"),
                    level_ms=[round(t.level_ms[0], 4), round(t.level_ms[1], 4)],
-                   sync_free_ms_by_threads_per_row=dict(zip(
-                       ("1", "2", "4", "8", "16"),
+                   range_ms_by_rows=dict(zip(
+                       ("512", "1024", "2048", "4096", "8192"),
                        (round(t.candidate_ms[i], 4) for i in range(t.ncandidates)))))
     if t.sweep_config >= 0:
         out.update(sweep_config=t.sweep_config, sweep_config_backward=t.sweep_config_backward,
@@ -697,12 +697,12 @@ def grids_form(a, barrier) -> dict:
     """The general grids and the full-tensor formulation, one steady step to
     closure each (INNER_DVCLOSE 1e-8, INNER_RCLOSE 1e-6, OUTER_DVCLOSE 1e-8):
     a DISV hexagon grid and a DISU locally refined grid (SELL-32 product,
-    sync-free level-scheduled ILU0 sweeps, PCG), and a DIS grid with XT3D
+    ILU0 sweeps over row ranges, PCG), and a DIS grid with XT3D
     (the wider pattern, BiCGSTAB).  FP64 on the device-resident solution:
     the time step's own CUDA-event times (fill, solve, total), the median of
     3 steps from the initial heads after a warm-up step and (unless
-    --no-tune) gbims_autotune on the factored system (level-sweep form and
-    threads per row, reduction grid).  Beside each, the
+    --no-tune) gbims_autotune on the factored system (sweep form and
+    range size, reduction grid).  Beside each, the
     oracle's full solve of the same step on one core (wall clock) and the
     largest head difference."""
     from modflow6_gb300 import _lib

@@ -195,8 +195,8 @@ int gbims_time_kernels(gbims_handle *h, int reps, gbims_kernel_times *t);
 /* Autotuner (no counterpart in the reference, which has no tunable kernels):
  * on the handle's own factored system it times every wavefront tiling of
  * the structured sweeps (chunk of steps per ring buffer, ring depth,
- * neighbour-word prefetch depth, CTAs per SM), the form of the level-
- * scheduled sweeps of other patterns, and the thread-block count of the
+ * neighbour-word prefetch depth, CTAs per SM), the form and the range size
+ * of the sweeps of other patterns, and the thread-block count of the
  * dot/update reductions, and keeps the fastest for the following applies.
  * The tiling does not change any cell's arithmetic; the reduction grid only
  * changes the order in which the partial sums are added.  Batched handles
@@ -206,13 +206,12 @@ typedef struct gbims_tuning {
   int sweep_chunk, sweep_ring, sweep_prefetch;
   int sweep_occupancy;              /* 0: as many sweep CTAs per SM as fit; 2: at most two */
   int reduction_blocks;             /* chosen reduction grid (0: batched handle) */
-  int level_mode;                   /* level-scheduled sweeps (handles without wavefront
-                                       sweeps): 0 one launch per level, 1 one sync-free
-                                       launch per sweep; -1 not applicable */
+  int level_mode;                   /* general sweeps (handles without wavefront
+                                       sweeps): 0 one launch per level, 1 one launch
+                                       per sweep over ranges of rows; -1 not applicable */
   double level_ms[2];               /* one ILU0 application in each level mode */
-  int ncandidates;                  /* tilings timed (level-scheduled handles: the
-                                       sync-free form at 1, 2, 4, 8, 16 threads per
-                                       row of the widest level) */
+  int ncandidates;                  /* tilings timed (general sweeps: ranges of 512,
+                                       1024, 2048, 4096 and 8192 rows) */
   double candidate_ms[16];          /* one ILU0 application per candidate */
   double precond_ms;                /* of the chosen tilings */
   double vector_ms;                 /* dot + update at the chosen grid */

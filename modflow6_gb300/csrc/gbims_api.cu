@@ -59,7 +59,12 @@ struct gbims_handle {
   cudaGraphExec_t exec = nullptr;
   bool graph_tried = false, graph_ok = false;
   bool no_graph = false;   // GBIMS_GRAPH=0: the host drives the loop
-  LevelWords LW;           // the level-scheduled sweeps' result words (unstructured handles)
+  LevelWords LW;           // the general sweeps' result words (unstructured handles)
+  RangePlan RF, RB;        // their plans, and the range size asked for (0: the default)
+  bool planned = false;
+  int range_rows = 0;
+  long long words_nr = 0;  // the grids that the words' epochs count launches of
+  bool levels_b = false;   // B (and, for ILUT, F) holds the current factor's levels
   int G_alloc = 0;         // reduction blocks the partials were sized for
   double refine_factor = 1.0e-5;  // 1e-4 saves 3 % of the iterations but loses accuracy with BiCGSTAB
   bool factored = false;
@@ -113,20 +118,61 @@ static int fail(gbims_handle *h, int code, const std::string &msg) {
 // ---------------------------------------------------------------------------
 // graph body: one inner iteration
 // ---------------------------------------------------------------------------
-// The sync-free level sweeps' words, allocated (zeroed) before their first
-// use; a handle with wavefront sweeps never needs them.
-static int ensure_level_words(gbims_handle *h) {
-  if (h->structured || h->LW.fwd) return GBIMS_OK;
+// The level schedules that the per-level sweeps need (the ILU0 factorisation
+// keeps F from the start).
+static void ensure_levels(gbims_handle *h) {
+  if (h->levels_b) return;
+  if (h->ipc >= 3) levels_build_host(h->n, h->iapc, h->japc, true, h->F);
+  levels_build_host(h->n, h->iapc, h->japc, false, h->B);
+  h->levels_b = true;
+}
+
+// The range sweeps' plans of the current pattern and their words, zeroed
+// before their first use and whenever the grid changes (its tickets number
+// the launches); a handle with wavefront sweeps never needs them.  A pattern
+// that no range size fits is swept level by level.
+static int ensure_ranges(gbims_handle *h) {
+  if (h->structured) return GBIMS_OK;
+  if (h->LW.mode == 0) {
+    ensure_levels(h);
+    return GBIMS_OK;
+  }
+  if (!h->planned) {
+    const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
+    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed) ||
+        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed)) {
+      cudaGetLastError();
+      h->LW.mode = 0;
+      ensure_levels(h);
+      return GBIMS_OK;
+    }
+    if (h->ipc < 3) h->RF.host = h->RB.host = RangeHost();
+    h->planned = true;
+  }
   const size_t wb = (size_t)h->n * (h->mixed ? 8 : 16);
-  GB_CUDA(h, cudaMalloc(&h->LW.fwd, wb));
-  GB_CUDA(h, cudaMalloc(&h->LW.bwd, wb));
-  GB_CUDA(h, cudaMalloc((void **)&h->LW.ticket, 256));
-  GB_CUDA(h, cudaMalloc((void **)&h->LW.err, sizeof(int)));
-  GB_CUDA(h, cudaMemset(h->LW.fwd, 0, wb));
-  GB_CUDA(h, cudaMemset(h->LW.bwd, 0, wb));
-  GB_CUDA(h, cudaMemset(h->LW.ticket, 0, 256));
-  GB_CUDA(h, cudaMemset(h->LW.err, 0, sizeof(int)));
+  if (!h->LW.fwd) {
+    GB_CUDA(h, cudaMalloc(&h->LW.fwd, wb));
+    GB_CUDA(h, cudaMalloc(&h->LW.bwd, wb));
+    GB_CUDA(h, cudaMalloc((void **)&h->LW.ticket, 256));
+    GB_CUDA(h, cudaMalloc((void **)&h->LW.err, sizeof(int)));
+    GB_CUDA(h, cudaMemset(h->LW.err, 0, sizeof(int)));
+  }
+  const long long nr = (long long)h->RF.nr << 32 | h->RB.nr;
+  if (h->words_nr != nr) {
+    GB_CUDA(h, cudaMemsetAsync(h->LW.fwd, 0, wb, h->st));
+    GB_CUDA(h, cudaMemsetAsync(h->LW.bwd, 0, wb, h->st));
+    GB_CUDA(h, cudaMemsetAsync(h->LW.ticket, 0, 256, h->st));
+    h->words_nr = nr;
+  }
   return GBIMS_OK;
+}
+
+// The factor's values in the plans' order.
+static void fill_ranges(gbims_handle *h) {
+  if (h->structured || h->LW.mode == 0) return;
+  if (!h->mixed) launch_range_fill(h->RF, h->RB, h->d_apc, h->st);
+  else launch_range_fill32(h->RF, h->RB, h->d_apc32, h->st);
+  h->launches += 2;
 }
 
 // A level sweep whose wait ran out (reported by the kernels' error word).
@@ -145,7 +191,8 @@ static void precond64(gbims_handle *h, const double *r, double *z) {
     launch_dia7_apply64(h->D, h->D.d_rfull, h->D.d_zfull, h->d_ctl, h->st);
     launch_dia7_collect(h->D, h->n, h->D.d_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply64(h->D, r, z, h->d_ctl, h->st);
-  else launch_ilu_apply_levels(h->n, h->d_iapc, h->d_japc, h->d_apc, h->F, h->B, h->LW, r, z, h->d_ctl, h->st);
+  else if (h->LW.mode == 1) launch_range_apply(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else launch_ilu_apply_levels(h->n, h->d_iapc, h->d_japc, h->d_apc, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
 // The mixed form's preconditioner: FP32 factors, vectors and sweeps.
@@ -155,7 +202,8 @@ static void precond32(gbims_handle *h, const float *r, float *z) {
     launch_dia7_apply32(h->D, h->D.f_rfull, h->D.f_zfull, h->d_ctl, h->st);
     launch_dia7_collect32(h->D, h->n, h->D.f_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply32(h->D, r, z, h->d_ctl, h->st);
-  else launch_ilu_apply_levels32(h->n, h->d_iapc, h->d_japc, h->d_apc32, h->F, h->B, h->LW, r, z, h->d_ctl, h->st);
+  else if (h->LW.mode == 1) launch_range_apply32(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else launch_ilu_apply_levels32(h->n, h->d_iapc, h->d_japc, h->d_apc32, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
 // A*x and b - A*x: index-free on full DIS grids, SELL-32 otherwise.
@@ -603,9 +651,8 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, cudaMemcpy(h->S.d_src, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice));
     if (h->mixed) GB_CUDA(h, dalloc(&h->S.d_val32, col.size()));
   }
-  // level schedules of the triangular sweeps and the factorisation
-  levels_build_host(neq, h->iapc, h->japc, true, h->F);
-  levels_build_host(neq, h->iapc, h->japc, false, h->B);
+  // level schedule of the factorisation
+  if (h->ipc < 3) levels_build_host(neq, h->iapc, h->japc, true, h->F);
   // vectors (with slack after the last cell for the sweeps' aligned copies)
   size_t nn = (size_t)neq + kVecPad;
   GB_CUDA(h, dalloc(&h->d_amat, nja));
@@ -788,9 +835,11 @@ static int ilut_factor_core(gbims_handle *h) {
   GB_CUDA(h, cudaMemcpyAsync(h->d_japc, h->japc.data(), sizeof(int) * h->njapc, cudaMemcpyHostToDevice, st));
   launch_ilut_scatter(I, h->d_iapc, h->d_japc, h->d_apc, st);
   h->launches += 1;
-  levels_build_host(n, h->iapc, h->japc, true, h->F);
-  levels_build_host(n, h->iapc, h->japc, false, h->B);
-  drop_graph(h);  // the sweeps' level schedule is part of the captured loop
+  // the sweeps' schedule is that of the kept pattern, and part of the
+  // captured loop
+  h->levels_b = h->planned = false;
+  if (int rc = ensure_ranges(h)) return rc;
+  drop_graph(h);
   GB_CUDA(h, cudaStreamSynchronize(st));
   return icount;
 }
@@ -803,6 +852,8 @@ static int factor_core(gbims_handle *h) {
   if (h->dia_spmv) launch_dia7_vfill(h->D, h->d_ia, h->d_amat, st);
   else launch_sell_fill(h->S, h->d_amat, st);
   h->launches += 1;
+  if (h->ipc < 3)
+    if (int rc = ensure_ranges(h)) return rc;
   if (h->ipc >= 3) {
     int icount = ilut_factor_core(h);
     if (icount < 0) return icount;
@@ -810,6 +861,7 @@ static int factor_core(gbims_handle *h) {
       kr_f64_to_f32(h->njapc, h->d_apc, h->d_apc32, st);
       h->launches += 1;
     }
+    fill_ranges(h);
     GB_CUDA(h, cudaGetLastError());
     h->factored = true;
     return icount;
@@ -840,6 +892,7 @@ static int factor_core(gbims_handle *h) {
     if (icount > 10) break;
   }
   if (h->mixed) kr_f64_to_f32(h->nja, h->d_apc, h->d_apc32, st);
+  fill_ranges(h);
   if (h->structured) {
     const int was = h->D.ext;
     if (launch_dia7_extract(h->D, n, h->d_iapc, h->d_japc, h->d_apc, h->mixed, st) < 0)
@@ -857,7 +910,7 @@ static int factor_core(gbims_handle *h) {
 
 static int apply_core(gbims_handle *h, int kstp, int kiter, int *icnvg, int *in_iter,
                       gbims_summary *summary) {
-  if (int rc = ensure_level_words(h)) return rc;
+  if (int rc = ensure_ranges(h)) return rc;
   const int n = h->n;
   cudaStream_t st = h->st;
   (void)kiter;
@@ -1085,7 +1138,7 @@ extern "C" int gbims_matvec(gbims_handle *h, const double *x, double *y) {
 
 extern "C" int gbims_precondition(gbims_handle *h, const double *r, double *z) {
   if (!h || !r || !z) return GBIMS_ERR_ARG;
-  if (int rc = ensure_level_words(h)) return rc;
+  if (int rc = ensure_ranges(h)) return rc;
   if (!h->factored) return fail(h, GBIMS_ERR_STATE, "no factor: call gbims_factor or gbims_apply first");
   GB_CUDA(h, cudaMemcpyAsync(h->v_d, r, sizeof(double) * h->n, cudaMemcpyHostToDevice, h->st));
   // a control block with done = 0 lets the gated sweep kernels run
@@ -1125,7 +1178,7 @@ static void drop_graph(gbims_handle *h) {
 // dot-product partials are summed.
 extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
   if (!h || !out || reps <= 0) return GBIMS_ERR_ARG;
-  if (int rc = ensure_level_words(h)) return rc;
+  if (int rc = ensure_ranges(h)) return rc;
   if (!h->factored) return fail(h, GBIMS_ERR_STATE, "no factor: call gbims_factor or an apply first");
   memset(out, 0, sizeof(*out));
   out->sweep_config = -1;
@@ -1204,36 +1257,45 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
   }
   out->level_mode = -1;
   if (!h->structured) {
-    // level-scheduled sweeps: one launch per level, or one sync-free launch
-    // per sweep (the sync-free form also with 1 to 16 threads per row of
-    // the widest level, as far as the resident grid goes; level_ms[1] is its
-    // best, candidate_ms[0..4] its time at each)
+    // general sweeps: one launch per level, or one launch per sweep over row
+    // ranges of each size (level_ms[1] is the best of them, candidate_ms the
+    // time at each)
     double bt = 1e300;
-    int best = 1, best_mult = 1;
+    int best = 0, best_rows = 0;
     auto pre = [&] {
       if (!h->mixed) precond64(h, h->v_p, h->v_z);
       else precond32(h, h->f_p, h->f_z);
     };
     h->LW.mode = 0;
+    ensure_levels(h);
     out->level_ms[0] = time_it(pre);
     bt = out->level_ms[0];
-    best = 0;
     out->level_ms[1] = 1e300;
-    for (int mult : {1, 2, 4, 8, 16}) {
+    auto with_rows = [&](int rows) -> int {
       h->LW.mode = 1;
-      h->LW.sf_mult = mult;
+      h->range_rows = rows;
+      h->planned = false;
+      if (int rc = ensure_ranges(h)) return rc;
+      fill_ranges(h);
+      return GBIMS_OK;
+    };
+    for (int rows : {512, 1024, 2048, 4096, 8192}) {
+      if (int rc = with_rows(rows)) return rc;
+      if (h->LW.mode == 0) break;  // no range size fits the pattern
       const double ms = time_it(pre);
       out->candidate_ms[out->ncandidates++] = ms;
       out->level_ms[1] = std::min(out->level_ms[1], ms);
       if (ms < bt) {
         bt = ms;
         best = 1;
-        best_mult = mult;
+        best_rows = rows;
       }
     }
     if (int rc = level_words_error(h)) return rc;
+    if (best == 1) {
+      if (int rc = with_rows(best_rows)) return rc;
+    }
     h->LW.mode = best;
-    h->LW.sf_mult = best_mult;
     out->level_mode = best;
     out->precond_ms = bt;
   }
@@ -1317,6 +1379,10 @@ extern "C" int gbims_set_tuning(gbims_handle *h, int sweep_config, int reduction
     if (h->structured || level_mode > 1)
       return fail(h, GBIMS_ERR_ARG, "level mode out of range (or a structured handle)");
     h->LW.mode = level_mode;
+    if (h->factored) {  // the factor's values for the form chosen
+      if (int rc = ensure_ranges(h)) return rc;
+      fill_ranges(h);
+    }
   }
   if (sweep_config >= 0) {
     if (!h->structured || sweep_config >= dia7_num_cfgs())
@@ -1335,7 +1401,7 @@ extern "C" int gbims_set_tuning(gbims_handle *h, int sweep_config, int reduction
 
 extern "C" int gbims_time_kernels(gbims_handle *h, int reps, gbims_kernel_times *t) {
   if (!h || !t || reps <= 0) return GBIMS_ERR_ARG;
-  if (int rc = ensure_level_words(h)) return rc;
+  if (int rc = ensure_ranges(h)) return rc;
   if (!h->factored) return fail(h, GBIMS_ERR_STATE, "no factor: call gbims_factor or gbims_apply first");
   const int n = h->n;
   cudaStream_t st = h->st;
@@ -1496,6 +1562,8 @@ extern "C" int gbims_destroy(gbims_handle *h) {
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->st) cudaStreamDestroy(h->st);
+  range_free(h->RF);
+  range_free(h->RB);
   delete h;
   return GBIMS_OK;
 }
@@ -1634,7 +1702,7 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
 
 static int batch_apply_core(gbims_handle *h, int kstp, int *icnvg, int *in_iter,
                             gbims_summary *summaries) {
-  if (int rc = ensure_level_words(h)) return rc;
+  if (int rc = ensure_ranges(h)) return rc;
   const int n = h->n, nm = h->nm;
   cudaStream_t st = h->st;
   GB_CUDA(h, cudaEventRecord(h->ev0, st));

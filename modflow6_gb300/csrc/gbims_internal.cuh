@@ -120,16 +120,33 @@ struct Levels {
   int maxwidth = 0;
 };
 
-// The level-scheduled sweeps' form: mode 0 launches one kernel per level;
-// mode 1 runs each sweep as one sync-free launch over result words tagged
-// with the launch's epoch (fwd, bwd: n words each, 16 bytes in FP64, 8 in
-// FP32, zeroed once; ticket: two counters, 128 bytes apart, zeroed once).
+// The sweeps of general patterns: mode 0 launches one kernel per level; mode 1
+// runs each sweep as one launch over row ranges (k_range.cu), which hand
+// values to one another in result words tagged with the launch's epoch (fwd,
+// bwd: n words each, 16 bytes in FP64, 8 in FP32, zeroed once; ticket: two
+// counters, 128 bytes apart, zeroed once).
 struct LevelWords {
   int mode = 1;
-  int sf_mult = 8;  // sync-free sweeps: threads per row of the widest level (tuned)
   void *fwd = nullptr, *bwd = nullptr;
   unsigned long long *ticket = nullptr;
   int *err = nullptr;
+};
+
+// Plan of one range sweep (k_range.cu): rows cut into nr ranges of R; the
+// host arrays while it is built, and their device copies.
+struct RangeHost {
+  int R = 0, nr = 0, maxslots = 0, maxblock = 0, stages = 0;
+  std::vector<int> rows, off, rslice, src, dst, hptr, halo;
+  std::vector<unsigned char> blk;
+};
+struct RangePlan {
+  int n = 0, R = 0, nr = 0, maxslots = 0, maxblock = 0, stages = 0, nent = 0;
+  unsigned char *d_blk = nullptr;  // the slices' blocks (double, or float in the mixed form)
+  int *d_off = nullptr, *d_rslice = nullptr, *d_src = nullptr, *d_dst = nullptr, *d_hptr = nullptr,
+      *d_halo = nullptr;
+  // allocated elements
+  size_t c_blk = 0, c_off = 0, c_rslice = 0, c_src = 0, c_dst = 0, c_hptr = 0, c_halo = 0;
+  RangeHost host;
 };
 
 // ILUT / MILUT factorisation (k_ilut.cu).  kIlutCap bounds the working row
@@ -264,12 +281,29 @@ void launch_ilut_scatter(const IlutDev &I, const int *d_iapc, const int *d_japc,
                          cudaStream_t st);
 void launch_ilu_apply_levels(int n, const int *d_iapc, const int *d_japc,
                              const double *d_apc, const Levels &F, const Levels &B,
-                             const LevelWords &Wd, const double *r, double *d, const Ctl *ctl,
-                             cudaStream_t st);
+                             const double *r, double *d, const Ctl *ctl, cudaStream_t st);
 void launch_ilu_apply_levels32(int n, const int *d_iapc, const int *d_japc,
                                const float *d_apc32, const Levels &F, const Levels &B,
-                               const LevelWords &Wd, const float *r, float *d, const Ctl *ctl,
-                               cudaStream_t st);
+                               const float *r, float *d, const Ctl *ctl, cudaStream_t st);
+// Rows of a range without tuning.  Small ranges let more CTAs work and cost
+// more hand-overs through L2 on the way across the grid: both sweeps of a
+// hexagon grid of 90,000 cells take 354, 319, 303 and 295 us with 512, 1024,
+// 2048 and 4096 rows, a refined DISU grid of 32,000 cells 194, 172, 178 and
+// 164 us, XT3D on 15,000 cells 298, 296, 314 and 307 us (5.5, 2.9 and 2.6 ms
+// with a launch per level).
+constexpr int kRangeRows = 2048;
+// The plan of one sweep of the pattern iapc/japc in ranges of about `rows`
+// rows (fewer where a range would not fit the shared memory), uploaded; false
+// when no range size fits or device memory runs out.
+bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
+                 bool forward, int rows, bool fp32);
+void range_free(RangePlan &P);
+void launch_range_fill(const RangePlan &F, const RangePlan &B, const double *apc, cudaStream_t st);
+void launch_range_fill32(const RangePlan &F, const RangePlan &B, const float *apc, cudaStream_t st);
+void launch_range_apply(const RangePlan &F, const RangePlan &B, const LevelWords &W, const double *r,
+                        double *d, Ctl *ctl, cudaStream_t st);
+void launch_range_apply32(const RangePlan &F, const RangePlan &B, const LevelWords &W, const float *r,
+                          float *d, Ctl *ctl, cudaStream_t st);
 
 bool dia7_matches(int nlay, int nrow, int ncol, int n, const std::vector<int> &ia,
                   const std::vector<int> &ja);

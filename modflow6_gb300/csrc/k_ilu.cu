@@ -12,7 +12,6 @@
 // backward sweep D = (D - U*D) * APC(n).  Rows of a level are independent; one
 // launch per level.  Entries are summed in JAPC order with FMA.
 #include "gbims_internal.cuh"
-#include "k_llword.cuh"
 #include <algorithm>
 #include <climits>
 
@@ -184,145 +183,6 @@ __global__ void k_ilu_bwd_level(const int *__restrict__ rows, int nrows,
   d[n] = tv * apc[n];
 }
 
-// Sync-free sweeps: one launch per sweep instead of one per level.  The
-// warps walk the level-ordered row list with a grid stride, 32 consecutive
-// rows per warp; a row reads the rows it depends on as result words tagged
-// with the launch's epoch.  The polling is warp-synchronous: in each round
-// every unfinished lane loads all its dependencies' words (up to kDeps in
-// flight at once), and a lane whose words are all of this epoch finishes its
-// row; the warp repeats the round until all its lanes are done.  A lane may
-// depend on a lane of its own warp (a warp can straddle two levels): that
-// row is written in one round and seen in the next.  Rows depend only on
-// rows of lower levels, which come earlier in the list, and the grid is
-// sized so that all of its CTAs are resident: the lowest unfinished row of
-// the list can always proceed, so every wait ends (and is bounded besides).
-// Each row sums its entries in JAPC order with FMA, as the per-level kernels
-// do (bit-identical results).
-template <typename T, int DIR>
-__global__ void __launch_bounds__(256) k_ilu_sweep_sf(int n, const int *__restrict__ rows,
-                                                      const int *__restrict__ iapc,
-                                                      const int *__restrict__ japc,
-                                                      const T *__restrict__ apc,
-                                                      const T *__restrict__ r,
-                                                      const LLWord<T> *__restrict__ yin,
-                                                      LLWord<T> *out, T *d,
-                                                      unsigned long long *ticket, int *err,
-                                                      Ctl *ctl, int active) {
-  __shared__ unsigned s_ep;
-  if (threadIdx.x == 0) {
-    // every CTA takes a ticket, so launch e owns tickets [e*grid, (e+1)*grid)
-    const unsigned long long tk = atomicAdd(ticket, 1ULL);
-    s_ep = (unsigned)(tk / gridDim.x) + 1u;
-  }
-  __syncthreads();
-  if (ctl && ctl->done) return;
-  // the launch always has the same (resident) grid, so that its tickets and
-  // epochs line up with every other launch; CTAs past `active` only take
-  // their ticket
-  if ((int)blockIdx.x >= active) return;
-  const unsigned ep = s_ep;
-  const int lane = threadIdx.x & 31;
-  volatile int *vdone = ctl ? &ctl->done : nullptr;
-  constexpr int kDeps = 8;
-  const int stride = active * blockDim.x;
-  for (int q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); q0 < n; q0 += stride) {
-    const int q = q0 + lane;
-    bool done = q >= n;
-    int row = 0, j0 = 0, j1 = 0;
-    T tv0 = T(0);
-    if (!done) {
-      row = rows[q];
-      if (DIR > 0) {
-        tv0 = r[row];
-        j0 = iapc[row];
-        j1 = japc[row];
-      } else {
-        tv0 = ll_val(yin[row]);
-        j0 = japc[row];
-        j1 = iapc[row + 1];
-      }
-    }
-    const unsigned long long t0 = wclock();
-    while (true) {
-      if (!done) {
-        T tv = tv0;
-        bool ok = true;
-        for (int jb = j0; ok && jb < j1; jb += kDeps) {
-          LLRaw w[kDeps];
-          const int nd = min(kDeps, j1 - jb);
-#pragma unroll
-          for (int q2 = 0; q2 < kDeps; ++q2)
-            if (q2 < nd) ll_issue(out + japc[jb + q2], w[q2]);
-#pragma unroll
-          for (int q2 = 0; q2 < kDeps; ++q2) {
-            if (q2 >= nd || !ok) break;
-            if (!ll_ready<T>(w[q2], ep)) {
-              ok = false;
-            } else {
-              T v;
-              ll_take(w[q2], v);
-              tv = fms<T>(apc[jb + q2], v, tv);
-            }
-          }
-        }
-        if (ok) {
-          if (DIR < 0) {
-            tv = tv * apc[row];
-            d[row] = tv;
-          }
-          ll_put(out + row, tv, ep);
-          done = true;
-        }
-      }
-      if (!__any_sync(0xffffffffu, !done)) break;
-      if (__any_sync(0xffffffffu, (vdone && *vdone) || wclock() - t0 > kWaitCycles)) {
-        if (lane == 0) {
-          atomicExch(err, 1);
-          if (ctl) ctl->done = 1;
-        }
-        return;
-      }
-    }
-  }
-}
-
-// Grid of the sync-free sweeps: every CTA that can be resident (always the
-// same, see the kernel); `mult` threads per row of the widest level work,
-// the rest return after their ticket.  Threads that run several levels
-// ahead of the front have their rows' indices and operands loaded by the
-// time the front reaches them: on GB300, 8 threads per row of the widest
-// level sweep a 250k-cell hexagon grid in 2.57 ms against 3.66 ms with one
-// (the default; gbims_autotune picks among 1 to 16).
-template <typename T, int DIR>
-static int sf_grid() {
-  static int per_sm = -1;
-  if (per_sm < 0) {
-    per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilu_sweep_sf<T, DIR>, 256, 0);
-    per_sm = std::max(1, per_sm);
-  }
-  return per_sm * kNumSM;
-}
-static int sf_active(int grid, int n, int maxwidth, int mult) {
-  const long long want = ((long long)std::max(1, std::min(n, maxwidth)) * std::max(1, mult) + 255) / 256;
-  return (int)std::max<long long>(1, std::min<long long>(want, grid));
-}
-
-template <typename T>
-static void apply_sf(int n, const int *d_iapc, const int *d_japc, const T *d_apc, const Levels &F,
-                     const Levels &B, const LevelWords &Wd, const T *r, T *d, Ctl *ctl,
-                     cudaStream_t st) {
-  LLWord<T> *yf = static_cast<LLWord<T> *>(Wd.fwd);
-  LLWord<T> *zb = static_cast<LLWord<T> *>(Wd.bwd);
-  const int gf = sf_grid<T, 1>(), gb = sf_grid<T, -1>();
-  k_ilu_sweep_sf<T, 1><<<gf, 256, 0, st>>>(n, F.d_rows, d_iapc, d_japc, d_apc, r, nullptr, yf,
-                                           nullptr, Wd.ticket, Wd.err, ctl,
-                                           sf_active(gf, n, F.maxwidth, Wd.sf_mult));
-  k_ilu_sweep_sf<T, -1><<<gb, 256, 0, st>>>(n, B.d_rows, d_iapc, d_japc, d_apc, nullptr, yf, zb,
-                                            d, Wd.ticket + 16, Wd.err, ctl,
-                                            sf_active(gb, n, B.maxwidth, Wd.sf_mult));
-}
-
 template <typename T>
 static void apply_levels(const int *d_iapc, const int *d_japc, const T *d_apc,
                          const Levels &F, const Levels &B, const T *r, T *d, const Ctl *ctl,
@@ -340,22 +200,17 @@ static void apply_levels(const int *d_iapc, const int *d_japc, const T *d_apc,
 }
 
 void launch_ilu_apply_levels(int n, const int *d_iapc, const int *d_japc, const double *d_apc,
-                             const Levels &F, const Levels &B, const LevelWords &Wd,
-                             const double *r, double *d, const Ctl *ctl, cudaStream_t st) {
-  if (Wd.mode == 1)
-    apply_sf<double>(n, d_iapc, d_japc, d_apc, F, B, Wd, r, d, const_cast<Ctl *>(ctl), st);
-  else
-    apply_levels<double>(d_iapc, d_japc, d_apc, F, B, r, d, ctl, st);
+                             const Levels &F, const Levels &B, const double *r, double *d,
+                             const Ctl *ctl, cudaStream_t st) {
+  (void)n;
+  apply_levels<double>(d_iapc, d_japc, d_apc, F, B, r, d, ctl, st);
 }
 
 void launch_ilu_apply_levels32(int n, const int *d_iapc, const int *d_japc,
                                const float *d_apc32, const Levels &F, const Levels &B,
-                               const LevelWords &Wd, const float *r, float *d, const Ctl *ctl,
-                               cudaStream_t st) {
-  if (Wd.mode == 1)
-    apply_sf<float>(n, d_iapc, d_japc, d_apc32, F, B, Wd, r, d, const_cast<Ctl *>(ctl), st);
-  else
-    apply_levels<float>(d_iapc, d_japc, d_apc32, F, B, r, d, ctl, st);
+                               const float *r, float *d, const Ctl *ctl, cudaStream_t st) {
+  (void)n;
+  apply_levels<float>(d_iapc, d_japc, d_apc32, F, B, r, d, ctl, st);
 }
 
 }  // namespace gb
