@@ -59,6 +59,9 @@ extern "C" int gbmpnn_create(int nodes, int nja, const int *ia, const int *ja,
   MpnnDev &D = h->D;
   D.n = nodes;
   MP_CUDA(h, cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking));
+  MP_CUDA(h, cudaStreamCreateWithFlags(&D.side, cudaStreamNonBlocking));
+  MP_CUDA(h, cudaEventCreateWithFlags(&D.fork, cudaEventDisableTiming));
+  MP_CUDA(h, cudaEventCreateWithFlags(&D.join, cudaEventDisableTiming));
   MP_CUDA(h, alloc(&h->d_ia, n + 1));
   MP_CUDA(h, alloc(&h->d_ja, (size_t)nja));
   MP_CUDA(h, cudaMemcpy(h->d_ia, ia, sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
@@ -82,16 +85,15 @@ extern "C" int gbmpnn_create(int nodes, int nja, const int *ia, const int *ja,
     MP_CUDA(h, alloc(&D.H[l], n * H));
     MP_CUDA(h, alloc(&D.Hbf[l], n * H));
     MP_CUDA(h, alloc(&D.Abf[l], n * H));
-    MP_CUDA(h, alloc(&D.mask[l], n * H));
+    MP_CUDA(h, alloc(&D.mask[l], n * (H / 32)));
   }
-  MP_CUDA(h, alloc(&D.A, n * H));
   MP_CUDA(h, alloc(&D.y, n));
   MP_CUDA(h, alloc(&D.dy, n));
   MP_CUDA(h, alloc(&D.loss, 1));
-  MP_CUDA(h, alloc(&D.dH, n * H));
-  MP_CUDA(h, alloc(&D.dHp, n * H));
-  MP_CUDA(h, alloc(&D.dX, n * 2 * H));
-  MP_CUDA(h, alloc(&D.dZ, n * H));
+  for (int q = 0; q < 2; ++q) {
+    MP_CUDA(h, alloc(&D.T[q], n * H));
+    MP_CUDA(h, alloc(&D.A[q], n * H));
+  }
   D.nja = nja;
   MP_CUDA(h, alloc(&D.amat, (size_t)nja));
   MP_CUDA(h, cudaMemset(D.amat, 0, sizeof(double) * nja));
@@ -242,7 +244,7 @@ extern "C" int gbmpnn_destroy(gbmpnn_handle *h) {
   if (h->st) cudaStreamSynchronize(h->st);
   MpnnDev &D = h->D;
   std::vector<void *> ptrs = {h->d_ia, h->d_ja, D.w, D.deg, D.p, D.g, D.m, D.v, D.bt0, D.wbf0,
-                              D.xbf, D.A, D.y, D.dy, D.loss, D.dH, D.dHp, D.dX, D.dZ,
+                              D.xbf, D.y, D.dy, D.loss, D.T[0], D.T[1], D.A[0], D.A[1],
                               D.amat, D.ee, D.tt, D.we, D.epart};
   for (int l = 0; l < kMpnnLayers; ++l) {
     ptrs.push_back(D.bt[l]);
@@ -256,6 +258,12 @@ extern "C" int gbmpnn_destroy(gbmpnn_handle *h) {
   }
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (D.side) {
+    cudaStreamSynchronize(D.side);
+    cudaStreamDestroy(D.side);
+  }
+  if (D.fork) cudaEventDestroy(D.fork);
+  if (D.join) cudaEventDestroy(D.join);
   if (h->st) cudaStreamDestroy(h->st);
   delete h;
   return GBIMS_OK;

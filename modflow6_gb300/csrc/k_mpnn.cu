@@ -39,170 +39,447 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4],
 }
 
 
-// ---------------------------------------------------------------------------
-// Y[M x N] = [X1 | X2] (M x (K1 + K2), BF16 row-major) * B ((K1+K2) x N,
-// given transposed: Bt N x (K1+K2), BF16), + bias.  64 rows per block, each
-// of the 4 warps 16 rows x N columns.  Epilogue:
-//   EPI 0: Y = acc + bias                       (FP32 out)
-//   EPI 1: Y = relu(acc + bias), also BF16 copy, mask of acc + bias > 0
-//   EPI 2: Y = Hold + relu(acc + bias), BF16 copy, mask
-// ---------------------------------------------------------------------------
-template <int K1, int K2, int N, int EPI>
-__global__ void __launch_bounds__(128) k_gemm_rows(int M, const __nv_bfloat16 *__restrict__ X1,
-                                                   const __nv_bfloat16 *__restrict__ X2,
-                                                   const __nv_bfloat16 *__restrict__ Bt,
-                                                   const float *__restrict__ bias,
-                                                   const float *__restrict__ Hold,
-                                                   float *__restrict__ Y,
-                                                   __nv_bfloat16 *__restrict__ Ybf,
-                                                   unsigned char *__restrict__ mask) {
-  constexpr int K = K1 + K2;
-  constexpr int KP = K + 8;  // padded row (bank spread)
-  __shared__ __align__(16) __nv_bfloat16 xs[64][KP];
-  __shared__ __align__(16) __nv_bfloat16 bs[N][KP];
-  const int row0 = blockIdx.x * 64;
-  for (int e = threadIdx.x; e < N * K; e += blockDim.x) bs[e / K][e % K] = Bt[e];
-  for (int e = threadIdx.x; e < 64 * K; e += blockDim.x) {
-    const int r = e / K, c = e % K, gr = row0 + r;
-    __nv_bfloat16 v = __float2bfloat16(0.f);
-    if (gr < M) v = (c < K1) ? X1[(size_t)gr * K1 + c] : X2[(size_t)gr * K2 + (c - K1)];
-    xs[r][c] = v;
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int r0 = warp * 16;
-  float acc[N / 8][4];
-#pragma unroll
-  for (int nt = 0; nt < N / 8; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+// Rows of [X | X] operands and weights in shared memory are padded by 8
+// elements, so that the 8 rows of a fragment load fall into different banks.
+constexpr int kPad = 8;
+constexpr int kTile = 64;           // nodes per tile of the layer kernels
+constexpr int kLayerThreads = 256;  // 8 warps: 4 row groups of 16 x 2 column halves
+constexpr int kHs = kH + 8;         // padded row of the tile's FP32 residual stream
+
+// acc[NT][4] += rows r0..r0+15 of xs (row-major, K wide) times the NT*8
+// columns from c0 on of the weights ws (column-major: row c holds column c's
+// K entries), k in steps of 16 as one chain per element.
+template <int K, int NT>
+__device__ __forceinline__ void tile_mma(const __nv_bfloat16 *xs, const __nv_bfloat16 *ws, int r0,
+                                         int c0, float (&acc)[NT][4]) {
+  constexpr int KP = K + kPad;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
   for (int ks = 0; ks < K / 16; ++ks) {
     const int k0 = ks * 16 + 2 * t;
     unsigned a[4];
-    a[0] = *reinterpret_cast<const unsigned *>(&xs[r0 + g][k0]);
-    a[1] = *reinterpret_cast<const unsigned *>(&xs[r0 + g + 8][k0]);
-    a[2] = *reinterpret_cast<const unsigned *>(&xs[r0 + g][k0 + 8]);
-    a[3] = *reinterpret_cast<const unsigned *>(&xs[r0 + g + 8][k0 + 8]);
+    a[0] = *reinterpret_cast<const unsigned *>(xs + (r0 + g) * KP + k0);
+    a[1] = *reinterpret_cast<const unsigned *>(xs + (r0 + g + 8) * KP + k0);
+    a[2] = *reinterpret_cast<const unsigned *>(xs + (r0 + g) * KP + k0 + 8);
+    a[3] = *reinterpret_cast<const unsigned *>(xs + (r0 + g + 8) * KP + k0 + 8);
 #pragma unroll
-    for (int nt = 0; nt < N / 8; ++nt) {
+    for (int nt = 0; nt < NT; ++nt) {
       unsigned b[2];
-      b[0] = *reinterpret_cast<const unsigned *>(&bs[nt * 8 + g][k0]);
-      b[1] = *reinterpret_cast<const unsigned *>(&bs[nt * 8 + g][k0 + 8]);
+      b[0] = *reinterpret_cast<const unsigned *>(ws + (c0 + nt * 8 + g) * KP + k0);
+      b[1] = *reinterpret_cast<const unsigned *>(ws + (c0 + nt * 8 + g) * KP + k0 + 8);
       mma_bf16(acc[nt], a, b);
     }
   }
+}
+
+// Weights (N rows of K, BF16) into padded shared memory, 16 bytes a load.
+template <int K, int N>
+__device__ __forceinline__ void load_weights(const __nv_bfloat16 *__restrict__ W, __nv_bfloat16 *ws) {
+  for (int e = threadIdx.x; e < N * K / 8; e += kLayerThreads) {
+    const int r = e / (K / 8), c = e % (K / 8) * 8;
+    *reinterpret_cast<uint4 *>(ws + r * (K + kPad) + c) =
+        *reinterpret_cast<const uint4 *>(W + (size_t)r * K + c);
+  }
+}
+
+// Epilogue of a 64-column tile: z = acc + bias, y = max(z, 0) + hold (hold in
+// shared memory, or none).  FP32 y; for training also its BF16 copy and the
+// mask z > 0 as two 32-bit words a node (bit = column).
+template <bool HOLD, bool TRAIN>
+__device__ __forceinline__ void layer_epilogue(int n, int row0, int r0, int half,
+                                               const float (&acc)[4][4],
+                                               const float *__restrict__ bias, const float *hs,
+                                               float *__restrict__ Y,
+                                               __nv_bfloat16 *__restrict__ Ybf,
+                                               unsigned *__restrict__ mask) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int nt = 0; nt < N / 8; ++nt) {
+  for (int h = 0; h < 2; ++h) {
+    const int lr = r0 + g + 8 * h, r = row0 + lr;
+    unsigned m = 0;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+      const int c = half * 32 + nt * 8 + 2 * t;
+      const float z0 = acc[nt][2 * h] + bias[c], z1 = acc[nt][2 * h + 1] + bias[c + 1];
+      float y0 = z0 > 0.f ? z0 : 0.f, y1 = z1 > 0.f ? z1 : 0.f;
+      if (HOLD) {
+        const float2 o = *reinterpret_cast<const float2 *>(hs + lr * kHs + c);
+        y0 += o.x;
+        y1 += o.y;
+      }
+      if (TRAIN) m |= (z0 > 0.f ? 1u : 0u) << (nt * 8 + 2 * t) | (z1 > 0.f ? 2u : 0u) << (nt * 8 + 2 * t);
+      if (r < n) {
+        const size_t o = (size_t)r * kH + c;
+        *reinterpret_cast<float2 *>(Y + o) = make_float2(y0, y1);
+        if (TRAIN) *reinterpret_cast<__nv_bfloat162 *>(Ybf + o) = __floats2bfloat162_rn(y0, y1);
+      }
+    }
+    if (TRAIN) {
+      m |= __shfl_xor_sync(0xffffffffu, m, 1);
+      m |= __shfl_xor_sync(0xffffffffu, m, 2);
+      if (t == 0 && r < n) mask[(size_t)r * 2 + half] = m;
+    }
+  }
+}
+
+// H0 = relu(X W0 + b0).
+template <bool TRAIN>
+__global__ void __launch_bounds__(kLayerThreads) k_layer0(int n, const __nv_bfloat16 *__restrict__ X,
+                                                          const __nv_bfloat16 *__restrict__ Bt,
+                                                          const float *__restrict__ bias,
+                                                          float *__restrict__ Y,
+                                                          __nv_bfloat16 *__restrict__ Ybf,
+                                                          unsigned *__restrict__ mask) {
+  __shared__ __align__(16) __nv_bfloat16 xs[kTile * (kIn + kPad)];
+  __shared__ __align__(16) __nv_bfloat16 ws[kH * (kIn + kPad)];
+  load_weights<kIn, kH>(Bt, ws);
+  const int warp = threadIdx.x >> 5, r0 = (warp & 3) * 16, half = warp >> 2;
+  const int ntile = (n + kTile - 1) / kTile;
+  for (int tl = blockIdx.x; tl < ntile; tl += gridDim.x) {
+    const int row0 = tl * kTile;
+    __syncthreads();
+    if (threadIdx.x < kTile * kIn / 8) {
+      const int r = threadIdx.x / (kIn / 8), c = threadIdx.x % (kIn / 8) * 8;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (row0 + r < n) v = *reinterpret_cast<const uint4 *>(X + (size_t)(row0 + r) * kIn + c);
+      *reinterpret_cast<uint4 *>(xs + r * (kIn + kPad) + c) = v;
+    }
+    __syncthreads();
+    float acc[4][4] = {};
+    tile_mma<kIn, 4>(xs, ws, r0, half * 32, acc);
+    layer_epilogue<false, TRAIN>(n, row0, r0, half, acc, bias, nullptr, Y, Ybf, mask);
+  }
+}
+
+// Sums over the off-diagonal entries of kQ nodes of w * row (FP32, entry
+// order): a half-warp a node, a lane 4 of the 64 features.  The nodes' row
+// pointers are loaded together, then their first 8 entries, then each node's
+// 8 rows at once: the latencies of a tile's nodes overlap.
+constexpr int kQ = kTile / 16;  // nodes of a half-warp in a tile
+struct Gather {
+  int p0[kQ], p1[kQ], j[kQ];
+  float w[kQ];
+  __device__ __forceinline__ void load(int row0, int n, const int *__restrict__ ia,
+                                       const int *__restrict__ ja, const float *__restrict__ wt) {
+    const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int node = row0 + q * 16 + hw;
+      p0[q] = p1[q] = 0;
+      if (node < n) {
+        p0[q] = ia[node] + 1;
+        p1[q] = ia[node + 1];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      j[q] = 0;
+      w[q] = 0.f;
+      if (l16 < 8 && p0[q] + l16 < p1[q]) {
+        j[q] = ja[p0[q] + l16];
+        w[q] = wt[p0[q] + l16];
+      }
+    }
+  }
+  __device__ __forceinline__ float4 sum(int q, const int *__restrict__ ja,
+                                        const float *__restrict__ wt, const float *__restrict__ X) {
+    const int l16 = threadIdx.x & 15;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    int p = p0[q], jv = j[q];
+    float wv = w[q];
+    while (true) {
+      const int m = p1[q] - p;
+      float4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int jk = __shfl_sync(0xffffffffu, jv, k, 16);
+        if (k < m) v[k] = reinterpret_cast<const float4 *>(X + (size_t)jk * kH)[l16];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float wk = __shfl_sync(0xffffffffu, wv, k, 16);
+        if (k < m) {
+          a.x = fmaf(wk, v[k].x, a.x);
+          a.y = fmaf(wk, v[k].y, a.y);
+          a.z = fmaf(wk, v[k].z, a.z);
+          a.w = fmaf(wk, v[k].w, a.w);
+        }
+      }
+      p += 8;
+      if (!__any_sync(0xffffffffu, p < p1[q])) return a;
+      // a node with more than 8 neighbours
+      jv = 0;
+      wv = 0.f;
+      if (l16 < 8 && p + l16 < p1[q]) {
+        jv = ja[p + l16];
+        wv = wt[p + l16];
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ uint2 pack_bf16(float4 v) {
+  union {
+    __nv_bfloat162 b[2];
+    uint2 u;
+  } x;
+  x.b[0] = __floats2bfloat162_rn(v.x, v.y);
+  x.b[1] = __floats2bfloat162_rn(v.z, v.w);
+  return x.u;
+}
+
+// One message-passing layer, H_l = H_{l-1} + relu([H_{l-1}, S H_{l-1}] W + b),
+// in one pass over the nodes.  Bound by memory: 512 bytes a node to and from
+// HBM and seven gathered rows of 256 bytes from L2, against 16 kFLOP a node
+// of products.  So a tile's aggregation, both halves of its BF16 operand and
+// its residual rows stay in shared memory (they used to pass through global
+// memory between two kernels), the weights stay there for all of a block's
+// tiles, and every access is 8 or 16 bytes.  196,608 nodes of a 7-point graph:
+// 251 us a layer as an aggregation and a product kernel, 93 us now (80 us
+// without the copies for training); the gathers alone move 350 MB from L2.
+template <bool TRAIN>
+__global__ void __launch_bounds__(kLayerThreads, 4)
+    k_layer(int n, const int *__restrict__ ia, const int *__restrict__ ja, const float *__restrict__ w,
+            const float *__restrict__ H, const __nv_bfloat16 *__restrict__ Bt,
+            const float *__restrict__ bias, float *__restrict__ Y, __nv_bfloat16 *__restrict__ Abf,
+            __nv_bfloat16 *__restrict__ Ybf, unsigned *__restrict__ mask) {
+  constexpr int KP = kCat + kPad;
+  extern __shared__ __align__(16) unsigned char smem_layer[];
+  __nv_bfloat16 *ws = reinterpret_cast<__nv_bfloat16 *>(smem_layer);
+  __nv_bfloat16 *xs = ws + kH * KP;
+  float *hs = reinterpret_cast<float *>(xs + kTile * KP);
+  load_weights<kCat, kH>(Bt, ws);
+  const int warp = threadIdx.x >> 5, r0 = (warp & 3) * 16, half = warp >> 2;
+  const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
+  const int ntile = (n + kTile - 1) / kTile;
+  for (int tl = blockIdx.x; tl < ntile; tl += gridDim.x) {
+    const int row0 = tl * kTile;
+    __syncthreads();  // the last tile's operands are read
+    Gather gt;
+    gt.load(row0, n, ia, ja, w);
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int r = q * 16 + hw, node = row0 + r;
+      float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (node < n) own = reinterpret_cast<const float4 *>(H + (size_t)node * kH)[l16];
+      const uint2 a = pack_bf16(gt.sum(q, ja, w, H));
+      *reinterpret_cast<float4 *>(hs + r * kHs + 4 * l16) = own;
+      *reinterpret_cast<uint2 *>(xs + r * KP + 4 * l16) = pack_bf16(own);
+      *reinterpret_cast<uint2 *>(xs + r * KP + kH + 4 * l16) = a;
+      if (TRAIN && node < n) *reinterpret_cast<uint2 *>(Abf + (size_t)node * kH + 4 * l16) = a;
+    }
+    __syncthreads();
+    float acc[4][4] = {};
+    tile_mma<kCat, 4>(xs, ws, r0, half * 32, acc);
+    layer_epilogue<true, TRAIN>(n, row0, r0, half, acc, bias, hs, Y, Ybf, mask);
+  }
+}
+
+// Four 8x8 BF16 matrices from shared memory, transposed.
+__device__ __forceinline__ void ldsm_t4(unsigned (&r)[4], const __nv_bfloat16 *p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
+// The gradient that reaches a layer's output, of the tile's nodes: T + S D
+// (T the residual and own-row part, D the aggregated part of the layer
+// above, both from its kernel), or dy wout^T below the read-out.  Masked by
+// the layer's relu it goes into zs as BF16; the bias gradient's sums are kept
+// in db; the unmasked gradient in hs if given.
+template <bool TOP>
+__device__ __forceinline__ void tile_dz(int n, int row0, const int *__restrict__ ia,
+                                        const int *__restrict__ ja, const float *__restrict__ w,
+                                        const float *__restrict__ T, const float *__restrict__ D,
+                                        const float *__restrict__ dy, const float *__restrict__ wout,
+                                        const unsigned *__restrict__ mask, __nv_bfloat16 *zs,
+                                        float *hs, float4 &db) {
+  const int hw = threadIdx.x >> 4, l16 = threadIdx.x & 15;
+  Gather gt;
+  if (!TOP) gt.load(row0, n, ia, ja, w);
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) {
+    const int r = q * 16 + hw, node = row0 + r;
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned m = 0;
+    if (node < n) {
+      m = mask[(size_t)node * 2 + (l16 >> 3)] >> (4 * (l16 & 7));
+      if (TOP) {
+        const float e = dy[node];
+        d = make_float4(e * wout[4 * l16], e * wout[4 * l16 + 1], e * wout[4 * l16 + 2],
+                        e * wout[4 * l16 + 3]);
+      } else {
+        d = reinterpret_cast<const float4 *>(T + (size_t)node * kH)[l16];
+      }
+    }
+    if (!TOP) {
+      const float4 a = gt.sum(q, ja, w, D);
+      d = make_float4(d.x + a.x, d.y + a.y, d.z + a.z, d.w + a.w);
+    }
+    if (hs) *reinterpret_cast<float4 *>(hs + r * kHs + 4 * l16) = d;
+    const float4 z = make_float4(m & 1u ? d.x : 0.f, m & 2u ? d.y : 0.f, m & 4u ? d.z : 0.f,
+                                 m & 8u ? d.w : 0.f);
+    *reinterpret_cast<uint2 *>(zs + r * (kH + kPad) + 4 * l16) = pack_bf16(z);
+    db.x += z.x;
+    db.y += z.y;
+    db.z += z.z;
+    db.w += z.w;
+  }
+}
+
+// The block's bias-gradient sums into the gradient.
+__device__ __forceinline__ void flush_db(float *sb, float4 db, float *__restrict__ g) {
+  const int l16 = threadIdx.x & 15;
+  __syncthreads();
+  if (threadIdx.x < kH) sb[threadIdx.x] = 0.f;
+  __syncthreads();
+  atomicAdd(sb + 4 * l16, db.x);
+  atomicAdd(sb + 4 * l16 + 1, db.y);
+  atomicAdd(sb + 4 * l16 + 2, db.z);
+  atomicAdd(sb + 4 * l16 + 3, db.w);
+  __syncthreads();
+  if (threadIdx.x < kH) atomicAdd(g + threadIdx.x, sb[threadIdx.x]);
+}
+
+// Backward of one message-passing layer, in one pass over the nodes:
+//   dH = T + S D (or dy wout^T), dZ = mask * dH, dW += [H, A]^T dZ, db += dZ,
+//   [dX1, dX2] = dZ W^T, Tout = dH + dX1, Dout = dX2
+// where the layer below then takes Tout + S Dout as its dH.  Bound by memory
+// like the forward layer (1.3 kB a node and seven gathered rows): dZ and dH
+// stay in shared memory, and dW is summed in the tensor cores' FP32
+// accumulators over all of a block's tiles, a block's sums going out once
+// (a reduction per 64 nodes, 8192 atomics each, took 240 of 390 us).
+// 196,608 nodes: 392 us a layer in four kernels before, 161 us now.
+constexpr int kBwdSmem = (kCat * (kH + kPad) + kTile * (kH + kPad) + kTile * (kCat + kPad)) * 2 +
+                         kTile * kHs * 4;
+template <bool TOP>
+__global__ void __launch_bounds__(kLayerThreads, 2)
+    k_layer_bwd(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+                const float *__restrict__ w, const float *__restrict__ T, const float *__restrict__ D,
+                const float *__restrict__ dy, const float *__restrict__ wout,
+                const unsigned *__restrict__ mask, const __nv_bfloat16 *__restrict__ Hbf,
+                const __nv_bfloat16 *__restrict__ Abf, const __nv_bfloat16 *__restrict__ W,
+                float *__restrict__ Tout, float *__restrict__ Dout, float *__restrict__ gW,
+                float *__restrict__ gb) {
+  constexpr int KP = kH + kPad, XP = kCat + kPad;
+  extern __shared__ __align__(16) unsigned char smem_layer[];
+  __shared__ float sb[kH];
+  __nv_bfloat16 *ws = reinterpret_cast<__nv_bfloat16 *>(smem_layer);
+  __nv_bfloat16 *zs = ws + kCat * KP;
+  __nv_bfloat16 *xs = zs + kTile * KP;
+  float *hs = reinterpret_cast<float *>(xs + kTile * XP);
+  load_weights<kH, kCat>(W, ws);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int r0 = (warp & 3) * 16, half = warp >> 2;
+  const int ntile = (n + kTile - 1) / kTile;
+  float4 db = make_float4(0.f, 0.f, 0.f, 0.f);
+  float dw[8][4] = {};  // rows 16*warp.. of dW, all 64 columns
+  for (int tl = blockIdx.x; tl < ntile; tl += gridDim.x) {
+    const int row0 = tl * kTile;
+    __syncthreads();  // the last tile's operands are read
+    for (int e = threadIdx.x; e < kTile * kCat / 8; e += kLayerThreads) {
+      const int r = e / (kCat / 8), c = e % (kCat / 8) * 8, node = row0 + r;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (node < n)
+        v = *reinterpret_cast<const uint4 *>(c < kH ? Hbf + (size_t)node * kH + c
+                                                    : Abf + (size_t)node * kH + (c - kH));
+      *reinterpret_cast<uint4 *>(xs + r * XP + c) = v;
+    }
+    tile_dz<TOP>(n, row0, ia, ja, w, T, D, dy, wout, mask, zs, hs, db);
+    __syncthreads();
+    // dW += X^T dZ
+#pragma unroll
+    for (int ks = 0; ks < kTile / 16; ++ks) {
+      unsigned a[4];
+      ldsm_t4(a, xs + (ks * 16 + (lane & 7) + (lane >> 4) * 8) * XP + warp * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        unsigned b[4];
+        ldsm_t4(b, zs + (ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * KP + np * 16 + (lane >> 4) * 8);
+        const unsigned b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+        mma_bf16(dw[2 * np], a, b0);
+        mma_bf16(dw[2 * np + 1], a, b1);
+      }
+    }
+    // dX = dZ W^T: warps 0-3 the own-row half, 4-7 the aggregated half
+    float acc[8][4] = {};
+    tile_mma<kH, 8>(zs, ws, r0, half * kH, acc);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int r = row0 + r0 + g + 8 * h;
-      if (r >= M) continue;
+      const int lr = r0 + g + 8 * h, r = row0 + lr;
+      if (r >= n) continue;
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int c = nt * 8 + 2 * t + q;
-        const size_t o = (size_t)r * N + c;
-        float z = acc[nt][2 * h + q] + (bias ? bias[c] : 0.f);
-        if (EPI == 0) {
-          Y[o] = z;
+      for (int nt = 0; nt < 8; ++nt) {
+        const int c = nt * 8 + 2 * t;
+        float2 v = make_float2(acc[nt][2 * h], acc[nt][2 * h + 1]);
+        if (half == 0) {
+          const float2 o = *reinterpret_cast<const float2 *>(hs + lr * kHs + c);
+          v = make_float2(o.x + v.x, o.y + v.y);
+          *reinterpret_cast<float2 *>(Tout + (size_t)r * kH + c) = v;
         } else {
-          const bool pos = z > 0.f;
-          float yv = pos ? z : 0.f;
-          if (EPI == 2) yv += Hold[o];
-          Y[o] = yv;
-          Ybf[o] = __float2bfloat16(yv);
-          mask[o] = pos ? 1 : 0;
+          *reinterpret_cast<float2 *>(Dout + (size_t)r * kH + c) = v;
         }
       }
     }
   }
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float *o = gW + (warp * 16 + g + 8 * h) * kH + nt * 8 + 2 * t;
+      atomicAdd(o, dw[nt][2 * h]);
+      atomicAdd(o + 1, dw[nt][2 * h + 1]);
+    }
+  flush_db(sb, db, gb);
 }
 
-// ---------------------------------------------------------------------------
-// G[K x N] += X^T dZ over a chunk of 64 rows: X (M x K, BF16), dZ (M x N,
-// BF16); the block's partial sums go to G with atomicAdd.  Each warp owns
-// K/4 rows of G.
-// ---------------------------------------------------------------------------
-template <int K1, int K2, int N>
-__global__ void __launch_bounds__(128) k_gemm_xtdz(int M, const __nv_bfloat16 *__restrict__ X1,
-                                                   const __nv_bfloat16 *__restrict__ X2,
-                                                   const __nv_bfloat16 *__restrict__ dZ,
-                                                   float *__restrict__ G) {
-  constexpr int K = K1 + K2;
-  constexpr int MC = 64, MP = MC + 8;
-  __shared__ __align__(16) __nv_bfloat16 xt[K][MP];   // X^T chunk
-  __shared__ __align__(16) __nv_bfloat16 dzt[N][MP];  // dZ^T chunk
-  const int m0 = blockIdx.x * MC;
-  for (int e = threadIdx.x; e < MC * K; e += blockDim.x) {
-    const int m = e / K, c = e % K, gm = m0 + m;
-    __nv_bfloat16 v = __float2bfloat16(0.f);
-    if (gm < M) v = (c < K1) ? X1[(size_t)gm * K1 + c] : X2[(size_t)gm * K2 + (c - K1)];
-    xt[c][m] = v;
-  }
-  for (int e = threadIdx.x; e < MC * N; e += blockDim.x) {
-    const int m = e / N, c = e % N, gm = m0 + m;
-    dzt[c][m] = (gm < M) ? dZ[(size_t)gm * N + c] : __float2bfloat16(0.f);
-  }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  constexpr int FT = K / 16 / 4 > 0 ? K / 16 / 4 : 1;  // m16 tiles of G rows per warp
-  if (warp * FT * 16 >= K) return;
-  float acc[FT][N / 8][4];
-#pragma unroll
-  for (int f = 0; f < FT; ++f)
-#pragma unroll
-    for (int nt = 0; nt < N / 8; ++nt) acc[f][nt][0] = acc[f][nt][1] = acc[f][nt][2] = acc[f][nt][3] = 0.f;
-#pragma unroll
-  for (int ks = 0; ks < MC / 16; ++ks) {
-    const int k0 = ks * 16 + 2 * t;
-    unsigned b[N / 8][2];
-#pragma unroll
-    for (int nt = 0; nt < N / 8; ++nt) {
-      b[nt][0] = *reinterpret_cast<const unsigned *>(&dzt[nt * 8 + g][k0]);
-      b[nt][1] = *reinterpret_cast<const unsigned *>(&dzt[nt * 8 + g][k0 + 8]);
+// Backward of the input layer: dZ as above, dW0 += X^T dZ, db0 += dZ.
+__global__ void __launch_bounds__(kLayerThreads, 4)
+    k_layer0_bwd(int n, const int *__restrict__ ia, const int *__restrict__ ja,
+                 const float *__restrict__ w, const float *__restrict__ T, const float *__restrict__ D,
+                 const unsigned *__restrict__ mask, const __nv_bfloat16 *__restrict__ X,
+                 float *__restrict__ gW, float *__restrict__ gb) {
+  constexpr int KP = kH + kPad, XP = kIn + kPad;
+  __shared__ __align__(16) __nv_bfloat16 zs[kTile * KP];
+  __shared__ __align__(16) __nv_bfloat16 xs[kTile * XP];
+  __shared__ float sb[kH];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int ntile = (n + kTile - 1) / kTile;
+  float4 db = make_float4(0.f, 0.f, 0.f, 0.f);
+  float dw[4] = {};  // the 16 rows of dW0, columns 8*warp..
+  for (int tl = blockIdx.x; tl < ntile; tl += gridDim.x) {
+    const int row0 = tl * kTile;
+    __syncthreads();
+    if (threadIdx.x < kTile * kIn / 8) {
+      const int r = threadIdx.x / (kIn / 8), c = threadIdx.x % (kIn / 8) * 8;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (row0 + r < n) v = *reinterpret_cast<const uint4 *>(X + (size_t)(row0 + r) * kIn + c);
+      *reinterpret_cast<uint4 *>(xs + r * XP + c) = v;
     }
+    tile_dz<false>(n, row0, ia, ja, w, T, D, nullptr, nullptr, mask, zs, nullptr, db);
+    __syncthreads();
 #pragma unroll
-    for (int f = 0; f < FT; ++f) {
-      const int fr = (warp * FT + f) * 16;
-      unsigned a[4];
-      a[0] = *reinterpret_cast<const unsigned *>(&xt[fr + g][k0]);
-      a[1] = *reinterpret_cast<const unsigned *>(&xt[fr + g + 8][k0]);
-      a[2] = *reinterpret_cast<const unsigned *>(&xt[fr + g][k0 + 8]);
-      a[3] = *reinterpret_cast<const unsigned *>(&xt[fr + g + 8][k0 + 8]);
+    for (int kp = 0; kp < kTile / 32; ++kp) {
+      // the B fragments of two k-steps of this warp's 8 columns
+      unsigned b[4];
+      ldsm_t4(b, zs + (kp * 32 + lane) * KP + warp * 8);
 #pragma unroll
-      for (int nt = 0; nt < N / 8; ++nt) mma_bf16(acc[f][nt], a, b[nt]);
+      for (int s = 0; s < 2; ++s) {
+        unsigned a[4];
+        ldsm_t4(a, xs + (kp * 32 + s * 16 + (lane & 7) + (lane >> 4) * 8) * XP + ((lane >> 3) & 1) * 8);
+        const unsigned bb[2] = {b[2 * s], b[2 * s + 1]};
+        mma_bf16(dw, a, bb);
+      }
     }
   }
 #pragma unroll
-  for (int f = 0; f < FT; ++f)
-#pragma unroll
-    for (int nt = 0; nt < N / 8; ++nt)
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const int r = (warp * FT + f) * 16 + g + 8 * h, c = nt * 8 + 2 * t + q;
-          atomicAdd(&G[r * N + c], acc[f][nt][2 * h + q]);
-        }
-}
-
-// A = S H over the CSR pattern (off-diagonals), FP32 in, BF16 and FP32 out.
-__global__ void k_aggregate(int n, const int *__restrict__ ia, const int *__restrict__ ja,
-                            const float *__restrict__ w, const float *__restrict__ H,
-                            float *__restrict__ A, __nv_bfloat16 *__restrict__ Abf) {
-  // one warp per node, 2 features per lane
-  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (node >= n) return;
-  float a0 = 0.f, a1 = 0.f;
-  for (int p = ia[node] + 1; p < ia[node + 1]; ++p) {
-    const float wv = w[p];
-    const float2 h = reinterpret_cast<const float2 *>(H + (size_t)ja[p] * kH)[lane];
-    a0 = fmaf(wv, h.x, a0);
-    a1 = fmaf(wv, h.y, a1);
+  for (int h = 0; h < 2; ++h) {
+    float *o = gW + (g + 8 * h) * kH + warp * 8 + 2 * t;
+    atomicAdd(o, dw[2 * h]);
+    atomicAdd(o + 1, dw[2 * h + 1]);
   }
-  reinterpret_cast<float2 *>(A + (size_t)node * kH)[lane] = make_float2(a0, a1);
-  if (Abf) reinterpret_cast<__nv_bfloat162 *>(Abf + (size_t)node * kH)[lane] = __floats2bfloat162_rn(a0, a1);
+  flush_db(sb, db, gb);
 }
 
 // Edge weights S_ij = c_ij / sqrt(d_i d_j) from the assembled matrix.
@@ -233,33 +510,69 @@ __global__ void k_f32_to_bf16(long long n, const float *__restrict__ s, __nv_bfl
     d[i] = __float2bfloat16(s[i]);
 }
 
-// y = H wout + bout (one warp per node); optional loss and dy.
-__global__ void k_readout(int n, const float *__restrict__ H, const float *__restrict__ wout,
-                          const float *__restrict__ bout, float *__restrict__ y,
-                          const float *__restrict__ target, const float *__restrict__ mask,
-                          float inv_count, float *__restrict__ dy, float *__restrict__ loss) {
-  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// y = H wout + bout (one warp per node at a time); with a target also dy.
+__global__ void __launch_bounds__(256) k_readout(int n, const float *__restrict__ H,
+                                                 const float *__restrict__ wout,
+                                                 const float *__restrict__ bout,
+                                                 float *__restrict__ y,
+                                                 const float *__restrict__ target,
+                                                 const float *__restrict__ mask, float inv_count,
+                                                 float *__restrict__ dy) {
   const int lane = threadIdx.x & 31;
-  if (node >= n) return;
-  const float2 h = reinterpret_cast<const float2 *>(H + (size_t)node * kH)[lane];
-  float s = h.x * wout[2 * lane] + h.y * wout[2 * lane + 1];
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  const float w0 = wout[2 * lane], w1 = wout[2 * lane + 1], b = bout[0];
+  for (int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; node < n; node += warps) {
+    const float2 h = reinterpret_cast<const float2 *>(H + (size_t)node * kH)[lane];
+    float s = h.x * w0 + h.y * w1;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) {
-    const float yv = s + bout[0];
-    y[node] = yv;
-    if (target) {
-      const float m = mask[node];
-      const float e = (yv - target[node]) * m;
-      dy[node] = 2.f * e * inv_count;
-      atomicAdd(loss, e * e * inv_count);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      const float yv = s + b;
+      y[node] = yv;
+      if (target) dy[node] = 2.f * ((yv - target[node]) * mask[node]) * inv_count;
     }
   }
 }
 
-// Readout backward: dH = dy wout^T (overwrites dH), dwout += H^T dy, dbout += sum dy.
-__global__ void k_readout_bwd(int n, const float *__restrict__ H, const float *__restrict__ wout,
-                              const float *__restrict__ dy, float *__restrict__ dH,
+// loss += sum of the masked squared errors, one FP32 addition a node in node
+// order (so that the loss is the same from run to run): 4 cycles a node on
+// one thread, 0.4 ms at 200,000 nodes, while the backward pass runs on the
+// main stream.  One atomic a node, in any order, took 0.31 ms of the forward
+// pass.  The other threads prepare the next 2048 terms meanwhile.
+__global__ void __launch_bounds__(256) k_loss(int n, const float *__restrict__ y,
+                                              const float *__restrict__ target,
+                                              const float *__restrict__ mask, float inv_count,
+                                              float *__restrict__ loss) {
+  constexpr int kChunk = 2048;
+  __shared__ __align__(16) float term[2][kChunk];
+  const int nch = (n + kChunk - 1) / kChunk;
+  float sum = 0.f;
+  for (int c = 0; c <= nch; ++c) {
+    if (c < nch && threadIdx.x >= 32)
+      for (int k = threadIdx.x - 32; k < kChunk; k += 224) {
+        const int i = c * kChunk + k;
+        float v = 0.f;
+        if (i < n) {
+          const float e = (y[i] - target[i]) * mask[i];
+          v = e * e * inv_count;
+        }
+        term[c & 1][k] = v;
+      }
+    if (c > 0 && threadIdx.x == 0) {
+      const float4 *t = reinterpret_cast<const float4 *>(term[(c - 1) & 1]);
+#pragma unroll 8
+      for (int k = 0; k < kChunk / 4; ++k) {
+        const float4 v = t[k];
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) atomicAdd(loss, sum);
+}
+
+// Read-out backward: dwout += H^T dy, dbout += sum dy.
+__global__ void k_readout_bwd(int n, const float *__restrict__ H, const float *__restrict__ dy,
                               float *__restrict__ dwout, float *__restrict__ dbout) {
   __shared__ float sw[kH];
   __shared__ float sb;
@@ -272,8 +585,6 @@ __global__ void k_readout_bwd(int n, const float *__restrict__ H, const float *_
   for (int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; node < n; node += warps) {
     const float d = dy[node];
     const float2 h = reinterpret_cast<const float2 *>(H + (size_t)node * kH)[lane];
-    reinterpret_cast<float2 *>(dH + (size_t)node * kH)[lane] =
-        make_float2(d * wout[2 * lane], d * wout[2 * lane + 1]);
     g0 = fmaf(d, h.x, g0);
     g1 = fmaf(d, h.y, g1);
     if (lane == 0) gb += d;
@@ -284,49 +595,6 @@ __global__ void k_readout_bwd(int n, const float *__restrict__ H, const float *_
   __syncthreads();
   if (threadIdx.x < kH) atomicAdd(&dwout[threadIdx.x], sw[threadIdx.x]);
   if (threadIdx.x == 0) atomicAdd(dbout, sb);
-}
-
-// dZ = dH (x) mask, as BF16 for the GEMMs, and the bias gradient db += sum dZ.
-__global__ void k_relu_bwd(int n, const float *__restrict__ dH,
-                           const unsigned char *__restrict__ mask, __nv_bfloat16 *__restrict__ dZ,
-                           float *__restrict__ db) {
-  __shared__ float sb[kH];
-  if (threadIdx.x < kH) sb[threadIdx.x] = 0.f;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  float b0 = 0.f, b1 = 0.f;
-  for (int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; node < n; node += warps) {
-    const size_t o = (size_t)node * kH + 2 * lane;
-    const float d0 = mask[o] ? dH[o] : 0.f, d1 = mask[o + 1] ? dH[o + 1] : 0.f;
-    reinterpret_cast<__nv_bfloat162 *>(dZ)[o / 2] = __floats2bfloat162_rn(d0, d1);
-    b0 += d0;
-    b1 += d1;
-  }
-  atomicAdd(&sb[2 * lane], b0);
-  atomicAdd(&sb[2 * lane + 1], b1);
-  __syncthreads();
-  if (threadIdx.x < kH) atomicAdd(&db[threadIdx.x], sb[threadIdx.x]);
-}
-
-// dH_prev = dH (residual) + dXcat[:, :64] + S dXcat[:, 64:]
-__global__ void k_layer_bwd_combine(int n, const int *__restrict__ ia, const int *__restrict__ ja,
-                                    const float *__restrict__ w, const float *__restrict__ dH,
-                                    const float *__restrict__ dX, float *__restrict__ dHprev) {
-  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (node >= n) return;
-  float a0 = 0.f, a1 = 0.f;
-  for (int p = ia[node] + 1; p < ia[node + 1]; ++p) {
-    const float wv = w[p];
-    const float2 d = reinterpret_cast<const float2 *>(dX + (size_t)ja[p] * kCat + kH)[lane];
-    a0 = fmaf(wv, d.x, a0);
-    a1 = fmaf(wv, d.y, a1);
-  }
-  const float2 r = reinterpret_cast<const float2 *>(dH + (size_t)node * kH)[lane];
-  const float2 x = reinterpret_cast<const float2 *>(dX + (size_t)node * kCat)[lane];
-  reinterpret_cast<float2 *>(dHprev + (size_t)node * kH)[lane] =
-      make_float2(r.x + x.x + a0, r.y + x.y + a1);
 }
 
 // Adam (bias-corrected), FP32 master weights.
@@ -531,24 +799,60 @@ void mpnn_forward(MpnnDev &D, const float *d_x, const float *target, const float
   forward_from_xbf(D, target, mask, inv_count, st);
 }
 
+// Blocks of the layer kernel: as many as are resident, each with the weights
+// in shared memory and a stride of tiles.
+constexpr size_t kLayerSmem = (kH + kTile) * (kCat + kPad) * 2 + kTile * kHs * 4;
+template <bool TRAIN>
+static int layer_grid(int tiles) {
+  static int per_sm = 0;
+  if (per_sm == 0) {
+    cudaFuncSetAttribute(k_layer<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLayerSmem);
+    int occ = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_layer<TRAIN>, kLayerThreads, kLayerSmem);
+    per_sm = std::max(1, occ);
+  }
+  return std::min(per_sm * kNumSM, tiles);
+}
+
+// The layers, H[0] to H[kL].  Without a target nothing is kept for a backward
+// pass: no BF16 copies, no masks, and the residual stream alternates between
+// two buffers (100 MB at 200,000 nodes, which stay in L2).
+template <bool TRAIN>
+static void forward_layers(MpnnDev &D, cudaStream_t st) {
+  using P = MpnnLayout;
+  const int n = D.n;
+  const int tiles = (n + kTile - 1) / kTile;
+  k_layer0<TRAIN><<<std::min(tiles, 8 * kNumSM), kLayerThreads, 0, st>>>(
+      n, D.xbf, D.bt0, D.p + P::b0, D.H[0], D.Hbf[0], D.mask[0]);
+  const int grid = layer_grid<TRAIN>(tiles);
+  for (int l = 1; l <= kL; ++l) {
+    float *in = D.H[TRAIN ? l - 1 : (l - 1) & 1], *out = D.H[TRAIN ? l : l & 1];
+    k_layer<TRAIN><<<grid, kLayerThreads, kLayerSmem, st>>>(n, D.ia, D.ja, D.w, in, D.bt[l - 1],
+                                                      D.p + P::B(l), out, D.Abf[l], D.Hbf[l],
+                                                      D.mask[l]);
+  }
+}
+
 static void forward_from_xbf(MpnnDev &D, const float *target, const float *mask, float inv_count,
                              cudaStream_t st) {
   using P = MpnnLayout;
   const int n = D.n;
-  const int gb = (n + 63) / 64;
-  k_gemm_rows<kIn, 0, kH, 1><<<gb, 128, 0, st>>>(n, D.xbf, nullptr, D.bt0, D.p + P::b0, nullptr,
-                                                  D.H[0], D.Hbf[0], D.mask[0]);
-  const int ga = (int)(((long long)n * 32 + 255) / 256);
-  for (int l = 1; l <= kL; ++l) {
-    k_aggregate<<<ga, 256, 0, st>>>(n, D.ia, D.ja, D.w, D.H[l - 1], D.A, D.Abf[l]);
-    k_gemm_rows<kH, kH, kH, 2><<<gb, 128, 0, st>>>(n, D.Hbf[l - 1], D.Abf[l], D.bt[l - 1],
-                                                    D.p + P::B(l), D.H[l - 1], D.H[l], D.Hbf[l],
-                                                    D.mask[l]);
-  }
+  static_assert(kL % 2 == 0, "the last layer's output in H[0] without a target");
+  const float *top = target ? D.H[kL] : D.H[0];
+  if (target) forward_layers<true>(D, st);
+  else forward_layers<false>(D, st);
   if (target) cudaMemsetAsync(D.loss, 0, sizeof(float), st);
   const bool energy = target && D.energy;
-  k_readout<<<ga, 256, 0, st>>>(n, D.H[kL], D.p + P::wout, D.p + P::bout, D.y, target, mask,
-                                energy ? inv_count * D.mse_w : inv_count, D.dy, D.loss);
+  const float inv_loss = energy ? inv_count * D.mse_w : inv_count;
+  k_readout<<<ngrid((long long)n * 32, 256), 256, 0, st>>>(
+      n, top, D.p + P::wout, D.p + P::bout, D.y, target, mask, inv_loss, D.dy);
+  if (target) {
+    // on a stream of its own beside what follows; mpnn_backward waits for it
+    cudaEventRecord(D.fork, st);
+    cudaStreamWaitEvent(D.side, D.fork, 0);
+    k_loss<<<1, 256, 0, D.side>>>(n, D.y, target, mask, inv_loss, D.loss);
+    cudaEventRecord(D.join, D.side);
+  }
   if (energy) {
     const int G = std::min(kMpnnRedBlocks, (n + 255) / 256);
     k_energy_err<<<ngrid(n, 256), 256, 0, st>>>(n, D.y, target, mask, D.dh_soft, D.dh_scale, D.ee, D.tt);
@@ -562,25 +866,34 @@ static void forward_from_xbf(MpnnDev &D, const float *target, const float *mask,
 void mpnn_backward(MpnnDev &D, cudaStream_t st) {
   using P = MpnnLayout;
   const int n = D.n;
-  const int ga = (int)(((long long)n * 32 + 255) / 256);
-  const int gr = ngrid((long long)n * 32, 256);
-  const int gb = (n + 63) / 64;
-  const int gc = (n + 63) / 64;
   cudaMemsetAsync(D.g, 0, sizeof(float) * P::total, st);
-  k_readout_bwd<<<gr, 256, 0, st>>>(n, D.H[kL], D.p + P::wout, D.dy, D.dH, D.g + P::wout,
-                                    D.g + P::bout);
-  for (int l = kL; l >= 1; --l) {
-    k_relu_bwd<<<gr, 256, 0, st>>>(n, D.dH, D.mask[l], D.dZ, D.g + P::B(l));
-    // dW_l = [H_{l-1}, A_l]^T dZ
-    k_gemm_xtdz<kH, kH, kH><<<gc, 128, 0, st>>>(n, D.Hbf[l - 1], D.Abf[l], D.dZ, D.g + P::W(l));
-    // d[H_{l-1}, A_l] = dZ W_l^T  (W_l as BF16, kCat x kH; transposed use: Bt = W_l)
-    k_gemm_rows<kH, 0, kCat, 0><<<gb, 128, 0, st>>>(n, D.dZ, nullptr, D.wbf[l - 1], nullptr,
-                                                     nullptr, D.dX, nullptr, nullptr);
-    k_layer_bwd_combine<<<ga, 256, 0, st>>>(n, D.ia, D.ja, D.w, D.dH, D.dX, D.dHp);
-    std::swap(D.dH, D.dHp);
+  k_readout_bwd<<<ngrid((long long)n * 32, 256), 256, 0, st>>>(n, D.H[kL], D.dy, D.g + P::wout,
+                                                               D.g + P::bout);
+  const int tiles = (n + kTile - 1) / kTile;
+  static bool opted = false;
+  if (!opted) {
+    cudaFuncSetAttribute(k_layer_bwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+    cudaFuncSetAttribute(k_layer_bwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+    opted = true;
   }
-  k_relu_bwd<<<gr, 256, 0, st>>>(n, D.dH, D.mask[0], D.dZ, D.g + P::b0);
-  k_gemm_xtdz<kIn, 0, kH><<<gc, 128, 0, st>>>(n, D.xbf, nullptr, D.dZ, D.g + P::w0);
+  // two blocks an SM fill the register files; one place is left for the loss
+  // kernel beside them (a block without a place would run after all others
+  // and double the layer's time)
+  const int grid = std::min(tiles, 2 * kNumSM - 1);
+  for (int l = kL; l >= 1; --l) {
+    const int in = l & 1, out = in ^ 1;
+    if (l == kL)
+      k_layer_bwd<true><<<grid, kLayerThreads, kBwdSmem, st>>>(
+          n, D.ia, D.ja, D.w, nullptr, nullptr, D.dy, D.p + P::wout, D.mask[l], D.Hbf[l - 1],
+          D.Abf[l], D.wbf[l - 1], D.T[out], D.A[out], D.g + P::W(l), D.g + P::B(l));
+    else
+      k_layer_bwd<false><<<grid, kLayerThreads, kBwdSmem, st>>>(
+          n, D.ia, D.ja, D.w, D.T[in], D.A[in], nullptr, nullptr, D.mask[l], D.Hbf[l - 1],
+          D.Abf[l], D.wbf[l - 1], D.T[out], D.A[out], D.g + P::W(l), D.g + P::B(l));
+  }
+  k_layer0_bwd<<<std::min(tiles, 4 * kNumSM - 1), kLayerThreads, 0, st>>>(
+      n, D.ia, D.ja, D.w, D.T[0], D.A[0], D.mask[0], D.xbf, D.g + P::w0, D.g + P::b0);
+  cudaStreamWaitEvent(st, D.join, 0);  // the loss of the forward pass
 }
 
 void mpnn_adam(MpnnDev &D, float lr, cudaStream_t st) {

@@ -22,12 +22,14 @@ struct MpnnDev {
   __nv_bfloat16 *xbf = nullptr;                                     // features, BF16
   float *H[kMpnnLayers + 1] = {};             // residual stream per layer (FP32)
   __nv_bfloat16 *Hbf[kMpnnLayers + 1] = {};
-  float *A = nullptr;                         // aggregation scratch (FP32)
   __nv_bfloat16 *Abf[kMpnnLayers + 1] = {};   // aggregations (BF16, for dW)
-  unsigned char *mask[kMpnnLayers + 1] = {};  // relu masks
+  unsigned *mask[kMpnnLayers + 1] = {};       // relu masks, two 32-bit words a node
   float *y = nullptr, *dy = nullptr, *loss = nullptr;
-  float *dH = nullptr, *dHp = nullptr, *dX = nullptr;
-  __nv_bfloat16 *dZ = nullptr;
+  // backward, alternating by layer: the gradient's residual and own-row part
+  // and its aggregated part before the aggregation
+  float *T[2] = {}, *A[2] = {};
+  cudaStream_t side = nullptr;                // the loss, beside the backward pass
+  cudaEvent_t fork = nullptr, join = nullptr;
   int steps = 0;                              // Adam steps taken
   // energy loss (mode 1): the matrix of the last set_graph, the errors and
   // true changes in head units, W*e, and per-block partials of e'We, t'Wt
