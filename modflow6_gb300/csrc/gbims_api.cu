@@ -427,10 +427,12 @@ static int setup_structured(gbims_handle *h, const std::vector<int> &shapes,
   GB_CUDA(h, cudaMemset(h->D.d_flags, 0, sizeof(int) * h->D.nflags));
   GB_CUDA(h, dalloc(&h->D.d_err, 4));
   GB_CUDA(h, cudaMemset(h->D.d_err, 0, sizeof(int) * 4));
-  // default tiling: the fastest on the 10M-cell case in both precisions
-  // (chunk 8, ring 4, prefetch 2, two CTAs per SM); gbims_autotune picks
-  // per system
-  h->D.cfg = 7;
+  // default tiling: chunk 8, ring 4, prefetch 1, as many CTAs per SM as fit,
+  // within 5 % of the best of the twelve on eight shapes from 1 x 20 x 30 to
+  // 10 x 600 x 600 cells in both precisions (10 x 600 x 600: 331 us an FP64
+  // application, 347 with prefetch 2, 377 with chunk 16, 382 with chunk 4);
+  // gbims_autotune picks per system
+  h->D.cfg = 0;
   if (const char *nv = std::getenv("GBIMS_SWEEP_NATIVE")) h->D.ext_allowed = (nv[0] == '0');
   h->structured = true;
   return GBIMS_OK;

@@ -20,26 +20,38 @@
 //
 // Hand-over.  Every result goes to global memory as a word tagged with the
 // epoch of its launch (k_llword.cuh): a consumer that reads the current
-// epoch has the value, with no fence or progress counter in between.  Four
-// warps per CTA, so that no wait stalls the dependent chain:
+// epoch has the value, with no fence or progress counter in between.  Five
+// warps per CTA (seven backward), so that no wait stalls the dependent chain:
 //  * copy: streams the block's own factor tiles (and, backward, its forward
 //    result) into a ring of NS shared-memory buffers with bulk copies
-//    (cp.async.bulk), one "full" mbarrier per buffer; it also writes each
-//    chunk's own right-hand side (forward r read in natural order and split
-//    into df64 pairs, backward dinv*y) into the buffer ("rdy" mbarrier): in
-//    the layers with a layer neighbour the pre-compute warp was the slowest
-//    warp with that work, and this warp idles between its copies;
+//    (cp.async.bulk), one "full" mbarrier per buffer;
+//  * rhs: writes each chunk's own right-hand side (forward r, read in natural
+//    order and split into df64 pairs, backward dinv*y) into the buffer, "rdy"
+//    mbarrier: with that work too the pre-compute warp, and then the copy
+//    warp, was the slowest warp of its CTA;
 //  * pre-compute: loads the layer neighbour's words (PF chunks ahead) and
 //    folds the layer term into the right-hand side (forward r - Lz*zn,
 //    backward dinv*y - Uz'*zn), released through a "prep" mbarrier;
 //  * edge: loads the neighbour block's last line (PF chunks ahead) for the
 //    first lane;
 //  * compute: per step one shuffle and the two FMAs of the row and column
-//    neighbours; writes each result word, and backward also the result in
-//    natural order, then frees the buffer through its "empty" mbarrier.
+//    neighbours; writes each result word, then frees the buffer through its
+//    "empty" mbarrier;
+//  * out (backward, two more warps, a chunk each in turn): write the results
+//    in natural order from a pair of chunk buffers the compute warp leaves
+//    them in.  There they cost the chain's warp one shared-memory store a
+//    step; done by the compute warp itself, the widening, the FP64 add and a
+//    store to 32 cache lines a step doubled the backward sweep's step.  One
+//    out warp is slower than the chain: a chunk's eight FP64 adds alone hold
+//    its pipe for 512 cycles.
+// One application in df64 with the extra warps, against four warps a CTA (and
+// prefetch 2): 65.5 -> 44.9 us on 1 x 100 x 100 cells, 70 -> 50 on 5 x 90 x 90,
+// 150 -> 104 on 10 x 200 x 200, 457 -> 327 on 10 x 600 x 600; in FP32 41 -> 35,
+// 49 -> 40, 105 -> 81 and 290 -> 259.
+//
 // The compute and pre-compute warps sit on different SM sub-partitions, so
 // that their FP64 instructions do not share a pipe.  Every wait is bounded
-// by the global timer; a wait that runs out sets an error flag and
+// by the SM's cycle counter; a wait that runs out sets an error flag and
 // Ctl::done, the copies in flight are drained, and the CTA returns.  CTAs
 // take a ticket in launch order and depend only on smaller tickets, so the
 // chain of waits always ends.
@@ -55,9 +67,8 @@
 // (pairs of floats, k_df64.cuh) when every factor tile lies in the float
 // exponent range, because GB300 issues a warp's FP64 FMA only every 64 cycles
 // or so and a step carries two of them; otherwise, or when GBIMS_SWEEP_NATIVE
-// is set, it sweeps in native FP64.  The df64 backward sweep converts its
-// result to FP64 (one FP64 add per cell) in the compute warp, off the chain,
-// on the FP64 pipe that the df64 chain leaves idle.
+// is set, it sweeps in native FP64.  The df64 backward sweep's out warp
+// converts the results to FP64 (one FP64 add per cell).
 #include <algorithm>
 #include <cstdlib>
 
@@ -194,12 +205,18 @@ struct alignas(16) Stage<T, C, -1> {
   T rv[C * 32];
   T yn[C];
 };
+// The backward results of two chunks on their way to natural order.
+template <typename T, int C>
+struct alignas(16) OutBuf {
+  T r[2][C * 32];
+};
+constexpr int sweep_threads(int dir) { return dir > 0 ? 160 : 224; }
 
 // Warp roles of a sweep CTA.
 // (numbered so that, with two CTAs on an SM, each compute warp shares its
 // sub-partition with the other CTA's edge warp, the lightest role, and each
 // pre-compute warp with the other CTA's copy warp; see the placement below)
-enum { kRoleCompute = 0, kRolePre = 1, kRoleEdge = 2, kRoleCopy = 3 };
+enum { kRoleCompute = 0, kRolePre = 1, kRoleEdge = 2, kRoleCopy = 3, kRoleRhs = 4, kRoleOut = 5 };
 
 // Poll result words of the current epoch, bounded; warp-uniform result.
 // `want` marks the lanes' words still missing (bit t = word t).  A round
@@ -229,7 +246,7 @@ __device__ __forceinline__ bool ll_poll(const LLWord<T> *q, long long stride, un
 // DIR = +1 forward, -1 backward.  A CTA is one block: 32 lines of one layer.
 // PF: chunks of neighbour words whose loads are in flight ahead of use.
 template <typename T, int S, int C, int NS, int DIR, int PF>
-__global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
+__global__ void __launch_bounds__(sweep_threads(DIR)) k_dia7_sweep(SweepArgs<T> p) {
   constexpr int W = 32;
   using St = Stage<T, C, DIR>;
   using E = Elem<T>;
@@ -240,6 +257,9 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
   unsigned long long *empty = full + NS;
   unsigned long long *prep = full + 2 * NS;
   unsigned long long *rdy = full + 3 * NS;  // rv written (edge warp)
+  unsigned long long *ofull = full + 4 * NS, *oempty = ofull + 2;  // backward: the out warp's buffers
+  OutBuf<T, C> *ob = reinterpret_cast<OutBuf<T, C> *>(smem_raw + NS * sizeof(St) +
+                                                      (4 * NS + 4) * sizeof(unsigned long long));
   __shared__ int s_id, s_abort, s_rot, s_m;
   __shared__ unsigned s_ep;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -276,6 +296,11 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
       mbar_init(&prep[s], 2);  // pre-compute warp + edge warp
       mbar_init(&rdy[s], 1);   // edge warp
     }
+    if (DIR < 0)
+      for (int q = 0; q < 2; ++q) {
+        mbar_init(&ofull[q], 1);
+        mbar_init(&oempty[q], 1);
+      }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -283,7 +308,7 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
   // a member of a batch that has reached its closure is not swept; its CTAs
   // only depend on one another, so none of them waits for it
   if (p.mctl && p.mctl[s_m].done) return;
-  const int role = (warp - s_rot) & 3;
+  const int role = warp == 4 ? kRoleRhs : warp > 4 ? kRoleOut : (warp - s_rot) & 3;
   const int id = s_id;
   const unsigned ep = s_ep;
   const Dia7Geo geo = p.geo[s_m];
@@ -430,57 +455,78 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
   const int i = (DIR > 0) ? (b * W + lane) : (b * W + (W - 1 - lane));
   const bool line_ok = i >= 0 && i < nrow;
   const int ncol = geo.ncol;
-  V *zrow = (DIR < 0 && line_ok) ? p.znat + geo.row0 + ((long long)k * nrow + i) * ncol : nullptr;
 
-  if (role == kRoleCopy) {
-    // ---------------- copy warp ----------------
-    // The block's own tiles have no producer in this launch: they stream
-    // into the ring as fast as buffers free up.
-    int issued = 0;
-    bool ok = true;
-    const unsigned tileb = C * W * sizeof(T);
-    // It also writes each chunk's own right-hand side for the pre-compute
-    // warp: forward r
-    // from natural order (lane l walks line b*W + l; step g is column
-    // g - S*l), kept as loaded until it is used (a conversion right after
-    // the load would wait for it and the prefetch would hide nothing);
-    // backward dinv*y from the stage's tiles
-    const int ri = b * W + lane;
-    const bool rline = (DIR > 0) && ri < nrow;
-    const V *rrow = rline ? p.rnat + geo.row0 + ((long long)k * nrow + ri) * geo.ncol : nullptr;
-    auto rload = [&](int c, V (&dst)[C]) {
+  if (DIR < 0 && role == kRoleOut) {
+    // ---------------- out warps ----------------
+    V *zrow = line_ok ? p.znat + geo.row0 + ((long long)k * nrow + i) * ncol : nullptr;
+    const int q = warp - 5;
+    for (int c = q; c < nch; c += 2) {
+      const bool got = mbar_wait(&ofull[q], (c >> 1) & 1, v_abort);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (lane == 0) *v_abort = 1;
+        return;
+      }
+      T v[C];
+#pragma unroll
+      for (int t = 0; t < C; ++t) v[t] = ob->r[q][t * W + lane];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&oempty[q]);
 #pragma unroll
       for (int t = 0; t < C; ++t) {
         const int jj = c * C + t - S * lane;
-        dst[t] = (rline && (unsigned)jj < (unsigned)geo.ncol) ? __ldg(rrow + jj) : V(0);
+        if (line_ok && (unsigned)jj < (unsigned)ncol) zrow[ncol - 1 - jj] = E::to_vec(v[t]);
       }
-    };
-    // r is loaded PR chunks ahead of its chunk (at least four: under the
-    // load of a full grid its latency reaches several chunks)
-    constexpr int PR = (PF < 4) ? 4 : PF;
-    V rr[PR][C];
+    }
+    return;
+  }
+
+  if (role == kRoleRhs) {
+    // ---------------- rhs warp ----------------
     if constexpr (DIR > 0) {
+      // r from natural order (lane l walks line b*W + l; step g is column
+      // g - S*l), loaded PR chunks ahead of its chunk (at least four: under
+      // the load of a full grid its latency reaches several chunks) and kept
+      // as loaded until it is used (a conversion right after the load would
+      // wait for it and the prefetch would hide nothing)
+      const V *rrow = line_ok ? p.rnat + geo.row0 + ((long long)k * nrow + i) * ncol : nullptr;
+      auto rload = [&](int c, V (&dst)[C]) {
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+          const int jj = c * C + t - S * lane;
+          dst[t] = (line_ok && (unsigned)jj < (unsigned)ncol) ? __ldg(rrow + jj) : V(0);
+        }
+      };
+      constexpr int PR = (PF < 4) ? 4 : PF;
+      V rr[PR][C];
 #pragma unroll
       for (int j = 0; j < PR; ++j)
         if (j < nch) rload(j, rr[j]);
-    }
-    // chunk q's rv: forward right after its tiles are issued (r has no
-    // producer in the launch), backward once its tiles have landed, LB
-    // chunks behind the copies (half the ring: the copies of LB chunks stay
-    // in flight, and a chunk's tiles have had LB chunks' time to land).
-    // LB <= NS - 1 keeps the waits acyclic: rv of chunk q is made after the
-    // copy of q + LB, which waits for the compute warp's chunk q + LB - NS,
-    // whose rv came LB chunks earlier still.
-    constexpr int LB = (NS / 2 > 1) ? NS / 2 : 1;
-    auto make_rv = [&](int q, int j) -> bool {
-      St &st = stg[q % NS];
-      if constexpr (DIR > 0) {
+      for (int c0 = 0; c0 < nch; c0 += PR) {
 #pragma unroll
-        for (int t = 0; t < C; ++t) st.rv[t * W + lane] = E::from_vec(rr[j][t]);
-        if (q + PR < nch) rload(q + PR, rr[j]);
-      } else {
-        (void)j;
-        if (!__all_sync(0xffffffffu, mbar_wait(&full[q % NS], (q / NS) & 1, v_abort))) return false;
+        for (int j = 0; j < PR; ++j) {
+          const int c = c0 + j;
+          if (c >= nch) break;
+          const int s = c % NS;
+          if (c >= NS && !__all_sync(0xffffffffu, mbar_wait(&empty[s], ((c / NS) - 1) & 1, v_abort))) {
+            if (lane == 0) *v_abort = 1;
+            return;
+          }
+          St &st = stg[s];
+#pragma unroll
+          for (int t = 0; t < C; ++t) st.rv[t * W + lane] = E::from_vec(rr[j][t]);
+          if (c + PR < nch) rload(c + PR, rr[j]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&rdy[s]);
+        }
+      }
+    } else {
+      for (int c = 0; c < nch; ++c) {
+        const int s = c % NS;
+        if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (c / NS) & 1, v_abort))) {
+          if (lane == 0) *v_abort = 1;
+          return;
+        }
+        St &st = stg[s];
 #pragma unroll
         for (int t = 0; t < C; ++t) {
           const int e = t * W + lane;
@@ -489,16 +535,21 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
           const T dv = st.d[e];
           st.rv[e] = dinv_zero(dv) ? E::zero() : E::mul(dv, ll_val(st.y[C * W - 1 - e]));
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&rdy[s]);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&rdy[q % NS]);
-      return true;
-    };
-    for (int c0 = 0; ok && c0 < nch; c0 += PR) {
-#pragma unroll
-    for (int j = 0; j < PR; ++j) {
-      const int c = c0 + j;
-      if (c >= nch) break;
+    }
+    return;
+  }
+
+  if (role == kRoleCopy) {
+    // ---------------- copy warp ----------------
+    // The block's own tiles have no producer in this launch: they stream
+    // into the ring as fast as buffers free up.
+    int issued = 0;
+    bool ok = true;
+    const unsigned tileb = C * W * sizeof(T);
+    for (int c = 0; c < nch; ++c) {
       const int s = c % NS;
       if (c >= NS) {
         const bool got = mbar_wait(&empty[s], ((c / NS) - 1) & 1, v_abort);
@@ -530,16 +581,6 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
       }
       issued = c + 1;
       __syncwarp();
-      if constexpr (DIR > 0) {
-        ok = make_rv(c, j);
-      } else {
-        if (c >= LB) ok = make_rv(c - LB, 0);
-      }
-      if (!ok) break;
-    }
-    }
-    if constexpr (DIR < 0) {
-      for (int q = max(0, nch - LB); ok && q < nch; ++q) ok = make_rv(q, 0);
     }
     if (!ok) fail();
     if (lane == 0) {
@@ -562,15 +603,21 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
   T h1 = E::zero(), h2 = E::zero();
   for (int c = 0; c < nch; ++c) {
     const int s = c % NS;
-    const bool got = mbar_wait(&full[s], (c / NS) & 1, v_abort) &&
-                     mbar_wait(&prep[s], (c / NS) & 1, v_abort);
+    // (the pre-compute warp has seen the chunk's tiles land before it arrives)
+    const bool got = mbar_wait(&prep[s], (c / NS) & 1, v_abort);
     if (!__all_sync(0xffffffffu, got)) {
       if (lane == 0) *v_abort = 1;
       return;
     }
+    if (DIR < 0 && c >= 2) {
+      const bool free2 = mbar_wait(&oempty[c & 1], ((c >> 1) - 1) & 1, v_abort);
+      if (!__all_sync(0xffffffffu, free2)) {
+        if (lane == 0) *v_abort = 1;
+        return;
+      }
+    }
     St &st = stg[s];
     const int g0 = c * C;
-    const int jc = g0 - S * lane;
     T ra[C], rb[C], rx[C], ryn[C];
 #pragma unroll
     for (int t = 0; t < C; ++t) {
@@ -590,18 +637,16 @@ __global__ void __launch_bounds__(128) k_dia7_sweep(SweepArgs<T> p) {
       T tv = E::fms(rx[t], h1, ra[t]);
       tv = E::fms(rb[t], yv, tv);
       ll_put(outt + (long long)(g0 + t) * W, tv, ep);
-      if constexpr (DIR < 0) {
-        // the result in natural order (df64: widened and added in FP64, off
-        // the chain, on this sub-partition's otherwise idle FP64 pipe)
-        const int jj = jc + t;
-        if (line_ok && (unsigned)jj < (unsigned)ncol) zrow[ncol - 1 - jj] = E::to_vec(tv);
-      }
+      if constexpr (DIR < 0) ob->r[c & 1][t * W + lane] = tv;
       h2 = h1;
       h1 = tv;
     }
     // the input buffer goes back to the copy and edge warps
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[s]);
+    if (lane == 0) {
+      mbar_arrive(&empty[s]);
+      if (DIR < 0) mbar_arrive(&ofull[c & 1]);
+    }
   }
 }
 
@@ -727,7 +772,8 @@ constexpr int kNumSweepCfgs = sizeof(kSweepCfgs) / sizeof(kSweepCfgs[0]);
 
 template <typename T, int C, int NS, int DIR>
 constexpr size_t stage_bytes() {
-  return NS * sizeof(Stage<T, C, DIR>) + 4 * NS * sizeof(unsigned long long);
+  return NS * sizeof(Stage<T, C, DIR>) + (4 * NS + (DIR < 0 ? 4 : 0)) * sizeof(unsigned long long) +
+         (DIR < 0 ? sizeof(OutBuf<T, C>) : 0);
 }
 static_assert(stage_bytes<double, 16, 2, -1>() <= 72 * 1024 && stage_bytes<double, 4, 8, -1>() <= 72 * 1024 &&
                   stage_bytes<double, 8, 4, -1>() <= 72 * 1024,
@@ -960,7 +1006,7 @@ static void sweep_one(const SweepArgs<T> &a, const Dia7 &D, int occ, cudaStream_
     opted = true;
   }
   const size_t sm = (occ == 2) ? std::max(bytes, kOcc2Smem) : bytes;
-  k_dia7_sweep<T, kSOf<T>, C, NS, DIR, PF><<<D.ntickets, 128, sm, st>>>(a);
+  k_dia7_sweep<T, kSOf<T>, C, NS, DIR, PF><<<D.ntickets, sweep_threads(DIR), sm, st>>>(a);
 }
 
 template <typename T, int DIR>
