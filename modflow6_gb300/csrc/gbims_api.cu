@@ -37,9 +37,10 @@ struct gbims_handle {
   double *d_amat = nullptr, *d_rhs = nullptr, *d_x = nullptr;
   double *v_d = nullptr, *v_p = nullptr, *v_q = nullptr, *v_z = nullptr, *v_t = nullptr,
          *v_v = nullptr, *v_dhat = nullptr, *v_phat = nullptr, *v_qhat = nullptr;
+  double *v_p1 = nullptr;  // where the product makes P: its odd iterations' buffer
   // FP32 inner vectors (mixed)
   float *f_d = nullptr, *f_p = nullptr, *f_q = nullptr, *f_z = nullptr, *f_t = nullptr,
-        *f_v = nullptr, *f_dhat = nullptr, *f_phat = nullptr, *f_qhat = nullptr;
+        *f_v = nullptr, *f_dhat = nullptr, *f_phat = nullptr, *f_qhat = nullptr, *f_p1 = nullptr;
   // SCALING_METHOD: DSCALE, DSCALE2 and the column position map (L2NORM)
   double *d_dscale = nullptr, *d_dscale2 = nullptr;
   int *d_cptr = nullptr, *d_cpos = nullptr;
@@ -223,117 +224,148 @@ static void residual64(gbims_handle *h, const Ctl *c, int only_if_north_due) {
   else launch_residual64(h->S, h->d_x, h->d_rhs, h->v_d, c, only_if_north_due, h->st);
 }
 
+// Whether the products are fused with the Krylov steps around them: on
+// systems up to kFuseRows rows whose reductions have a block per 256 rows (no
+// tuned grid), and not where the records' kernel reads P between them.
+static bool fused(const gbims_handle *h) {
+  return h->nm == 0 && h->n <= kFuseRows && h->G == (h->n + kRedBlock - 1) / kRedBlock &&
+         !(h->rec_cap > 0 && h->rec_nmod > 1);
+}
+
+static void spmv_fin(gbims_handle *h, int op, const void *x, const void *w, void *p0, void *p1, void *y) {
+  SpmvFin f;
+  f.op = op;
+  f.x = x;
+  f.w = w;
+  f.p0 = p0;
+  f.p1 = p1;
+  f.y = y;
+  f.part = h->d_part;
+  f.ctl = h->d_ctl;
+  launch_spmv_fin(h->dia_spmv ? &h->D : nullptr, h->dia_spmv ? nullptr : &h->S, h->mixed, f, h->st);
+}
+
 static void enqueue_iteration(gbims_handle *h, unsigned long long cond, int use_cond) {
   const int n = h->n, G = h->G;
   Ctl *c = h->d_ctl;
   cudaStream_t st = h->st;
   double *part = h->d_part;
+  const bool l2 = h->s.icnvgopt >= 2;
+  const bool fuse = fused(h);
   if (h->nm > 0 && h->mixed) {
     // batched ensemble, mixed form: every member's FP32 PCG iteration and,
     // where due, its FP64 refinement, in the same launches
     const BatchDev &B = h->bd;
     precond32(h, h->f_d, h->f_z);
-    kb_dot32(B, h->f_d, h->f_z, part, st);
-    kb_ctl_cg_rho(B, part, st);
+    kb_dot32(B, h->f_d, h->f_z, part, kFinCgRho, st);
     kb_cg_pupdate32(B, h->f_z, h->f_p, st);
     spmv32(h, h->f_p, h->f_q, c);
-    kb_dot32(B, h->f_p, h->f_q, part, st);
-    kb_ctl_alpha(B, part, st);
-    kb_cg_update_mixed(B, h->d_x, h->f_d, h->f_p, h->f_q, part, st);
-    kb_ctl_mixed_inner(B, part, h->refine_factor, st);
+    kb_dot32(B, h->f_p, h->f_q, part, kFinAlpha, st);
+    kb_cg_update_mixed(B, h->d_x, h->f_d, h->f_p, h->f_q, part, h->refine_factor, st);
     kb_any_due(B, c, st);
     residual64(h, c, 1);
-    kb_true_resid_stats(B, h->v_d, h->f_d, part, st);
-    kb_ctl_refine(B, part, st);
-    kb_all_done(B, c, cond, use_cond, 1, st);
+    kb_true_resid_stats(B, h->v_d, h->f_d, part, c, cond, use_cond, st);
     return;
   }
   if (h->nm > 0) {
     // batched ensemble, PCG: every member's iteration in the same launches
     const BatchDev &B = h->bd;
     precond64(h, h->v_d, h->v_z);
-    kb_dot64(B, h->v_d, h->v_z, part, st);
-    kb_ctl_cg_rho(B, part, st);
+    kb_dot64(B, h->v_d, h->v_z, part, kFinCgRho, st);
     kb_cg_pupdate64(B, h->v_z, h->v_p, st);
     spmv64(h, h->v_p, h->v_q, c);
-    kb_dot64(B, h->v_p, h->v_q, part, st);
-    kb_ctl_alpha(B, part, st);
-    kb_cg_update64(B, h->d_x, h->v_d, h->v_p, h->v_q, part, st);
-    kb_ctl_cg_cnvg(B, part, st);
-    kb_all_done(B, c, cond, use_cond, 1, st);
+    kb_dot64(B, h->v_p, h->v_q, part, kFinAlpha, st);
+    kb_cg_update64(B, h->d_x, h->v_d, h->v_p, h->v_q, part, c, cond, use_cond, st, l2);
     return;
   }
+  const bool rec_models = h->rec_cap > 0 && h->rec_nmod > 1;
   if (!h->mixed && !h->bcgs) {
     // ims_base_cg, ImsLinearBase.f90:100-236
     precond64(h, h->v_d, h->v_z);
-    kr_dot64(n, h->v_d, h->v_z, part, G, c, st);
-    kr_ctl_cg_rho(c, part, G, st);
-    kr_cg_pupdate64(n, h->v_z, h->v_p, c, st);
-    spmv64(h, h->v_p, h->v_q, c);
-    kr_dot64(n, h->v_p, h->v_q, part, G, c, st);
-    kr_ctl_alpha(c, part, G, st);
-    kr_cg_update64(n, h->d_x, h->v_d, h->v_p, h->v_q, part, G, c, st, h->s.icnvgopt >= 2);
-    if (h->rec_cap > 0 && h->rec_nmod > 1)
+    kr_dot64(n, h->v_d, h->v_z, part, G, c, kFinCgRho, st);
+    if (fuse) {
+      spmv_fin(h, 0, h->v_z, nullptr, h->v_p, h->v_p1, h->v_q);
+    } else {
+      kr_cg_pupdate64(n, h->v_z, h->v_p, c, st);
+      spmv64(h, h->v_p, h->v_q, c);
+      kr_dot64(n, h->v_p, h->v_q, part, G, c, kFinAlpha, st);
+    }
+    kr_cg_update64(n, h->d_x, h->v_d, h->v_p, fuse ? h->v_p1 : nullptr, h->v_q, part, G, c,
+                   !rec_models, cond, use_cond, st, l2);
+    if (rec_models) {
       kr_rec_models(false, h->rec_nmod, h->d_modstart, h->v_p, nullptr, h->v_d, nullptr,
                     h->d_rec_part, h->rec_G, c, st);
-    kr_ctl_cg_cnvg(c, part, G, cond, use_cond, st);
+      kr_ctl_cg_cnvg(c, part, G, cond, use_cond, st, l2);
+    }
     if (h->s.north > 0) residual64(h, c, 1);  // the NORTH residual refresh
   } else if (!h->mixed && h->bcgs) {
     // ims_base_bcgs, ImsLinearBase.f90:338-545
-    kr_dot64(n, h->v_dhat, h->v_d, part, G, c, st);
-    kr_ctl_bcgs_rho(c, part, G, st);
+    kr_dot64(n, h->v_dhat, h->v_d, part, G, c, kFinBcgsRho, st);
     kr_bcgs_p64(n, h->v_d, h->v_p, h->v_v, c, st);
     precond64(h, h->v_p, h->v_phat);
-    spmv64(h, h->v_phat, h->v_v, c);
-    kr_dot64(n, h->v_dhat, h->v_v, part, G, c, st);
-    kr_ctl_alpha(c, part, G, st);
+    if (fuse) {
+      spmv_fin(h, 1, h->v_phat, h->v_dhat, nullptr, nullptr, h->v_v);
+    } else {
+      spmv64(h, h->v_phat, h->v_v, c);
+      kr_dot64(n, h->v_dhat, h->v_v, part, G, c, kFinAlpha, st);
+    }
     kr_bcgs_q64(n, h->v_d, h->v_v, h->v_q, c, st);
     precond64(h, h->v_q, h->v_qhat);
-    spmv64(h, h->v_qhat, h->v_t, c);
-    kr_dot_tq_tt64(n, h->v_t, h->v_q, part, G, c, st);
-    kr_ctl_omega(c, part, G, st);
-    kr_bcgs_update64(n, h->d_x, h->v_d, h->v_phat, h->v_qhat, h->v_q, h->v_t, h->d_dscale, part, G, c, st,
-                     h->s.icnvgopt >= 2);
-    if (h->rec_cap > 0 && h->rec_nmod > 1)
+    if (fuse) {
+      spmv_fin(h, 2, h->v_qhat, h->v_q, nullptr, nullptr, h->v_t);
+    } else {
+      spmv64(h, h->v_qhat, h->v_t, c);
+      kr_dot_tq_tt64(n, h->v_t, h->v_q, part, G, c, st);
+    }
+    kr_bcgs_update64(n, h->d_x, h->v_d, h->v_phat, h->v_qhat, h->v_q, h->v_t, h->d_dscale, part, G,
+                     c, !rec_models, cond, use_cond, st, l2);
+    if (rec_models) {
       kr_rec_models(true, h->rec_nmod, h->d_modstart, h->v_phat, h->v_qhat, h->v_d, h->d_dscale,
                     h->d_rec_part, h->rec_G, c, st);
-    kr_ctl_bcgs_cnvg(c, part, G, cond, use_cond, st);
+      kr_ctl_bcgs_cnvg(c, part, G, cond, use_cond, st, l2);
+    }
     if (h->s.north > 0) residual64(h, c, 1);  // the NORTH residual refresh
   } else if (h->mixed && !h->bcgs) {
     // PCG on the FP32 matrix with FP32 vectors and preconditioner, FP64
     // scalars and heads; the FP64 true residual restarts the recurrence at
     // each refinement
     precond32(h, h->f_d, h->f_z);
-    kr_dot32(n, h->f_d, h->f_z, part, G, c, st);
-    kr_ctl_cg_rho(c, part, G, st);
-    kr_cg_pupdate32(n, h->f_z, h->f_p, c, st);
-    spmv32(h, h->f_p, h->f_q, c);
-    kr_dot32(n, h->f_p, h->f_q, part, G, c, st);
-    kr_ctl_alpha(c, part, G, st);
-    kr_cg_update_mixed(n, h->d_x, h->f_d, h->f_p, h->f_q, part, G, c, st);
-    kr_ctl_mixed_inner(c, part, G, 0, h->refine_factor, st);
+    kr_dot32(n, h->f_d, h->f_z, part, G, c, kFinCgRho, st);
+    if (fuse) {
+      spmv_fin(h, 0, h->f_z, nullptr, h->f_p, h->f_p1, h->f_q);
+    } else {
+      kr_cg_pupdate32(n, h->f_z, h->f_p, c, st);
+      spmv32(h, h->f_p, h->f_q, c);
+      kr_dot32(n, h->f_p, h->f_q, part, G, c, kFinAlpha, st);
+    }
+    kr_cg_update_mixed(n, h->d_x, h->f_d, h->f_p, fuse ? h->f_p1 : nullptr, h->f_q, part, G, c, true,
+                       h->refine_factor, st);
     residual64(h, c, 1);
-    kr_true_resid_stats(n, h->v_d, h->f_d, nullptr, nullptr, nullptr, part, G, c, st);
-    kr_ctl_refine(c, part, G, cond, use_cond, st);
+    kr_true_resid_stats(n, h->v_d, h->f_d, nullptr, nullptr, nullptr, part, G, c, cond, use_cond, st);
   } else {
     // BiCGSTAB, same precision split
-    kr_dot32(n, h->f_dhat, h->f_d, part, G, c, st);
-    kr_ctl_bcgs_rho(c, part, G, st);
+    kr_dot32(n, h->f_dhat, h->f_d, part, G, c, kFinBcgsRho, st);
     kr_bcgs_p32(n, h->f_d, h->f_p, h->f_v, c, st);
     precond32(h, h->f_p, h->f_phat);
-    spmv32(h, h->f_phat, h->f_v, c);
-    kr_dot32(n, h->f_dhat, h->f_v, part, G, c, st);
-    kr_ctl_alpha(c, part, G, st);
+    if (fuse) {
+      spmv_fin(h, 1, h->f_phat, h->f_dhat, nullptr, nullptr, h->f_v);
+    } else {
+      spmv32(h, h->f_phat, h->f_v, c);
+      kr_dot32(n, h->f_dhat, h->f_v, part, G, c, kFinAlpha, st);
+    }
     kr_bcgs_q32(n, h->f_d, h->f_v, h->f_q, c, st);
     precond32(h, h->f_q, h->f_qhat);
-    spmv32(h, h->f_qhat, h->f_t, c);
-    kr_dot_tq_tt32(n, h->f_t, h->f_q, part, G, c, st);
-    kr_ctl_omega(c, part, G, st);
-    kr_bcgs_update32(n, h->d_x, h->f_d, h->f_phat, h->f_qhat, h->f_q, h->f_t, h->d_dscale, part, G, c, st);
-    kr_ctl_mixed_inner(c, part, G, 1, h->refine_factor, st);
+    if (fuse) {
+      spmv_fin(h, 2, h->f_qhat, h->f_q, nullptr, nullptr, h->f_t);
+    } else {
+      spmv32(h, h->f_qhat, h->f_t, c);
+      kr_dot_tq_tt32(n, h->f_t, h->f_q, part, G, c, st);
+    }
+    kr_bcgs_update32(n, h->d_x, h->f_d, h->f_phat, h->f_qhat, h->f_q, h->f_t, h->d_dscale, part, G, c,
+                     h->refine_factor, st);
     residual64(h, c, 1);
-    kr_true_resid_stats(n, h->v_d, h->f_d, h->f_dhat, nullptr, h->d_dscale, part, G, c, st);
-    kr_ctl_refine(c, part, G, cond, use_cond, st);
+    kr_true_resid_stats(n, h->v_d, h->f_d, h->f_dhat, nullptr, h->d_dscale, part, G, c, cond, use_cond,
+                        st);
   }
 }
 
@@ -665,6 +697,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, dalloc(&h->v_p, nn));
     GB_CUDA(h, dalloc(&h->v_q, nn));
     GB_CUDA(h, dalloc(&h->v_z, nn));
+    if (!h->bcgs && neq <= kFuseRows) GB_CUDA(h, dalloc(&h->v_p1, nn));
     if (h->bcgs) {
       GB_CUDA(h, dalloc(&h->v_t, nn)); GB_CUDA(h, dalloc(&h->v_v, nn));
       GB_CUDA(h, dalloc(&h->v_dhat, nn)); GB_CUDA(h, dalloc(&h->v_phat, nn));
@@ -675,6 +708,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, dalloc(&h->d_apc32, npc));
     GB_CUDA(h, dalloc(&h->f_d, nn)); GB_CUDA(h, dalloc(&h->f_p, nn));
     GB_CUDA(h, dalloc(&h->f_q, nn)); GB_CUDA(h, dalloc(&h->f_z, nn));
+    if (!h->bcgs && neq <= kFuseRows) GB_CUDA(h, dalloc(&h->f_p1, nn));
     if (h->bcgs) {
       GB_CUDA(h, dalloc(&h->f_t, nn)); GB_CUDA(h, dalloc(&h->f_v, nn));
       GB_CUDA(h, dalloc(&h->f_dhat, nn)); GB_CUDA(h, dalloc(&h->f_phat, nn));
@@ -1311,11 +1345,11 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     for (int g : cand) {
       const double ms = time_it([&] {
         if (!h->mixed) {
-          kr_dot64(n, h->v_p, h->v_q, h->d_part, g, h->d_ctl, st);
-          kr_cg_update64(n, h->v_z, h->v_d, h->v_p, h->v_q, h->d_part, g, h->d_ctl, st, h->s.icnvgopt >= 2);
+          kr_dot64(n, h->v_p, h->v_q, h->d_part, g, h->d_ctl, kFinNone, st);
+          kr_cg_update64(n, h->v_z, h->v_d, h->v_p, nullptr, h->v_q, h->d_part, g, h->d_ctl, false, 0ULL, 0, st, h->s.icnvgopt >= 2);
         } else {
-          kr_dot32(n, h->f_p, h->f_q, h->d_part, g, h->d_ctl, st);
-          kr_cg_update_mixed(n, h->v_d, h->f_d, h->f_p, h->f_q, h->d_part, g, h->d_ctl, st);
+          kr_dot32(n, h->f_p, h->f_q, h->d_part, g, h->d_ctl, kFinNone, st);
+          kr_cg_update_mixed(n, h->v_d, h->f_d, h->f_p, nullptr, h->f_q, h->d_part, g, h->d_ctl, false, h->refine_factor, st);
         }
       });
       if (ms < bt) {
@@ -1436,13 +1470,13 @@ extern "C" int gbims_time_kernels(gbims_handle *h, int reps, gbims_kernel_times 
   if (!h->mixed) {
     t->spmv_ms = time_it([&] { spmv64(h, h->v_p, h->v_q, h->d_ctl); });
     t->precond_ms = time_it([&] { precond64(h, h->v_p, h->v_z); });
-    t->dot_ms = time_it([&] { kr_dot64(n, h->v_p, h->v_q, h->d_part, h->G, h->d_ctl, st); });
-    t->update_ms = time_it([&] { kr_cg_update64(n, h->v_z, h->v_d, h->v_p, h->v_q, h->d_part, h->G, h->d_ctl, st, h->s.icnvgopt >= 2); });
+    t->dot_ms = time_it([&] { kr_dot64(n, h->v_p, h->v_q, h->d_part, h->G, h->d_ctl, kFinNone, st); });
+    t->update_ms = time_it([&] { kr_cg_update64(n, h->v_z, h->v_d, h->v_p, nullptr, h->v_q, h->d_part, h->G, h->d_ctl, false, 0ULL, 0, st, h->s.icnvgopt >= 2); });
   } else {
     t->spmv_ms = time_it([&] { spmv32(h, h->f_p, h->f_q, h->d_ctl); });
     t->precond_ms = time_it([&] { precond32(h, h->f_p, h->f_z); });
-    t->dot_ms = time_it([&] { kr_dot32(n, h->f_p, h->f_q, h->d_part, h->G, h->d_ctl, st); });
-    t->update_ms = time_it([&] { kr_cg_update_mixed(n, h->v_d, h->f_d, h->f_p, h->f_q, h->d_part, h->G, h->d_ctl, st); });
+    t->dot_ms = time_it([&] { kr_dot32(n, h->f_p, h->f_q, h->d_part, h->G, h->d_ctl, kFinNone, st); });
+    t->update_ms = time_it([&] { kr_cg_update_mixed(n, h->v_d, h->f_d, h->f_p, nullptr, h->f_q, h->d_part, h->G, h->d_ctl, false, h->refine_factor, st); });
   }
   GB_CUDA(h, cudaGetLastError());
   // algorithmic bytes: CSR values + column indices + row pointers, x read
@@ -1546,7 +1580,7 @@ extern "C" int gbims_destroy(gbims_handle *h) {
                   h->D.f_lz, h->D.f_ly, h->D.f_lx, h->D.f_ux, h->D.f_uy, h->D.f_uz, h->D.f_dinv,
                   h->D.ll_y, h->D.ll_z,
                   h->D.d_flags, h->D.d_err, h->d_amat, h->d_rhs, h->d_x, h->v_d, h->v_p, h->v_q,
-                  h->v_z, h->v_t, h->v_v, h->v_dhat, h->v_phat, h->v_qhat, h->f_d, h->f_p,
+                  h->v_z, h->v_t, h->v_v, h->v_p1, h->f_p1, h->v_dhat, h->v_phat, h->v_qhat, h->f_d, h->f_p,
                   h->f_q, h->f_z, h->f_t, h->f_v, h->f_dhat, h->f_phat, h->f_qhat, h->d_part,
                   h->d_dscale, h->d_dscale2, h->d_cptr, h->d_cpos, h->D.d_sv, h->D.f_sv,
                   h->d_bcm, h->d_bcr, h->d_bmc, h->d_bmr, h->d_ctls, h->D.d_geo, h->S.d_slm,
@@ -1733,7 +1767,7 @@ static int batch_apply_core(gbims_handle *h, int kstp, int *icnvg, int *in_iter,
   residual64(h, nullptr, 0);
   kb_sumsq64(h->bd, h->v_d, h->d_part, st);
   kb_ctl_set_l2norm0(h->bd, h->d_part, st);
-  kb_all_done(h->bd, h->d_ctl, 0ULL, 0, 0, st);
+  kb_all_done(h->bd, h->d_ctl, st);
   if (h->mixed) {
     // the FP32 recurrence starts from the FP64 residual
     kr_f64_to_f32(n, h->v_d, h->f_d, st);
@@ -1754,6 +1788,12 @@ static int batch_apply_core(gbims_handle *h, int kstp, int *icnvg, int *in_iter,
       batch = std::min(batch * 2, 32);
     }
   }
+  // the L2 norms of the final residuals, as in a single solve
+  const bool l2_after = !h->mixed && h->s.icnvgopt < 2;
+  if (l2_after) {
+    kb_sumsq64(h->bd, h->v_d, h->d_part, st);
+    kb_ctl_set_l2norm(h->bd, h->d_part, st);
+  }
   if (h->s.iscl != 0) {
     launch_unscale_x(n, h->d_x, h->d_dscale2, st);
     h->launches += 1;
@@ -1763,7 +1803,7 @@ static int batch_apply_core(gbims_handle *h, int kstp, int *icnvg, int *in_iter,
   GB_CUDA(h, cudaMemcpyAsync(h->h_ctls, h->d_ctls, sizeof(Ctl) * nm, cudaMemcpyDeviceToHost, st));
   GB_CUDA(h, cudaStreamSynchronize(st));
   GB_CUDA(h, cudaGetLastError());
-  h->launches += 4 + (h->mixed ? 1 : 0) + (long long)h->body_kernels * h->h_ctl->bodies;
+  h->launches += 4 + (h->mixed ? 1 : 0) + (l2_after ? 2 : 0) + (long long)h->body_kernels * h->h_ctl->bodies;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   bool nonfinite = false;

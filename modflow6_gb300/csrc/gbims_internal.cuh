@@ -14,6 +14,9 @@ namespace gb {
 constexpr int kNumSM = 152;       // GB300: 2 dies x 76 SMs
 constexpr int kRedBlock = 256;    // threads per reduction block
 constexpr int kMaxRedBlocks = 8 * kNumSM;  // grid of reduction kernels: 8 x 256 threads per SM
+// Systems up to this size run their products fused with the Krylov steps
+// around them (k_sparse.cu)
+constexpr int kFuseRows = kMaxRedBlocks * kRedBlock;
 constexpr int kSell = 32;         // SELL slice height (one warp)
 constexpr int kMaxRowLen = 64;    // ILU0 factor: longest supported CSR row
 
@@ -43,6 +46,7 @@ struct Ctl {
   int bodies;         // loop bodies executed in this solve
   int guard_tripped;  // the body limit ended the loop
   int restart_due;    // mixed form: the pending true-residual check restarts the recurrence
+  unsigned fin;       // blocks of the current reduction kernel that have finished
   // Per-inner-iteration records (gbims_set_inner_records; rec == nullptr:
   // off).  Row r of rec (stride 3 + 4*rec_nmod): iteration, alpha, omega,
   // then per model dvmax, locdv, rmax, locr.  rec_part holds the per-model

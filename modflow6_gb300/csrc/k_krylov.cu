@@ -5,132 +5,29 @@
 // BiCGSTAB: ims_base_bcgs (:249-549).  Convergence: ims_base_testcnvg
 // (:1101-1146) and is_close (src/Utilities/MathUtil.f90:45-86).
 //
-// Each reduction kernel writes one partial per block; a single-block control
-// kernel sums the partials in a fixed order (so results are reproducible run
-// to run), then runs the scalar logic of the reference on the device: beta,
+// Each reduction kernel writes one partial per block; its last block to finish
+// sums the partials in a fixed order (so results are reproducible run to
+// run), then runs the scalar logic of the reference on the device: beta,
 // alpha, omega with the +SIGN(DPREC, denominator) guard, the closure test,
 // the stagnation exits and the NORTH residual schedule.  It sets Ctl::done,
 // which every kernel of the loop checks first, and the WHILE condition of the
 // CUDA graph, so the whole inner loop runs without a host round trip.
 #include "gbims_internal.cuh"
 #include "k_krylov.cuh"
-#include <cfloat>
+#include "k_reduce.cuh"
 
 namespace gb {
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__device__ __forceinline__ MaxLoc warp_maxloc(MaxLoc m) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    MaxLoc b;
-    b.val = __shfl_xor_sync(0xffffffffu, m.val, o);
-    b.idx = __shfl_xor_sync(0xffffffffu, m.idx, o);
-    maxloc_merge(m, b);
-  }
-  return m;
-}
-
-// Sum NV values over the block; thread 0 gets the results (fixed order).
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV]) {
-  __shared__ double sh[NV][kRedBlock / 32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double s = warp_sum(v[k]);
-    if (lane == 0) sh[k][wid] = s;
-  }
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double s = (lane < (int)(blockDim.x >> 5)) ? sh[k][lane] : 0.0;
-      v[k] = warp_sum(s);
-    }
-  }
-  __syncthreads();
-}
-
-template <int NM>
-__device__ __forceinline__ void block_maxloc(MaxLoc (&m)[NM]) {
-  __shared__ double shv[NM][kRedBlock / 32];
-  __shared__ long long shi[NM][kRedBlock / 32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NM; ++k) {
-    MaxLoc r = warp_maxloc(m[k]);
-    if (lane == 0) {
-      shv[k][wid] = r.val;
-      shi[k][wid] = r.idx;
-    }
-  }
-  __syncthreads();
-  if (wid == 0) {
-#pragma unroll
-    for (int k = 0; k < NM; ++k) {
-      MaxLoc r;
-      r.val = 0.0;
-      r.idx = -1;
-      if (lane < (int)(blockDim.x >> 5)) {
-        r.val = shv[k][lane];
-        r.idx = shi[k][lane];
-      }
-      m[k] = warp_maxloc(r);
-    }
-  }
-  __syncthreads();
-}
 
 __device__ __forceinline__ double to_d(double v) { return v; }
 __device__ __forceinline__ double to_d(float v) { return (double)v; }
 
-// 1 if v is Inf or NaN, tested on the exponent bits with integer
-// instructions: on GB300 every FP64 instruction (a compare included) goes
-// through the narrow FP64 pipe, which bounds the vector updates otherwise.
-__device__ __forceinline__ unsigned nonfinite(double v) {
-  return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
-}
-__device__ __forceinline__ unsigned nonfinite(float v) {
-  return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u;
-}
-
-// Sums of FP32 products with FP64-like accuracy and no FP64 instruction per
-// element (on GB300 those run on a narrow pipe): each product is split
-// exactly into p + e (p = x*y rounded, e = fma(x, y, -p)), and the p are
-// added with Neumaier's compensated summation, their rounding errors and
-// the e collected in c.  The pair enters the FP64 reductions as
-// (double)s + (double)c.  Explicit _rn operations keep the compiler from
-// contracting the splitting steps.
-struct CSum {
-  float s, c;
-};
-__device__ __forceinline__ void csum_add(CSum &a, float p) {
-  const float t = __fadd_rn(a.s, p);
-  const float bp = __fsub_rn(t, a.s);
-  a.c = __fadd_rn(a.c, __fadd_rn(__fsub_rn(a.s, __fsub_rn(t, bp)), __fsub_rn(p, bp)));
-  a.s = t;
-}
-__device__ __forceinline__ void csum_prod(CSum &a, float x, float y) {
-  const float p = __fmul_rn(x, y);
-  const float e = __fmaf_rn(x, y, -p);
-  csum_add(a, p);
-  a.c = __fadd_rn(a.c, e);
-}
-__device__ __forceinline__ double csum_value(const CSum &a) { return (double)a.s + (double)a.c; }
-
 // ---------------------------------------------------------------------------
 // dot products: partial[b] (and partial[G+b])
 // ---------------------------------------------------------------------------
-template <typename TA, typename TB>
+template <typename TA, typename TB, int FIN>
 __global__ void __launch_bounds__(kRedBlock) k_dot(int n, const TA *__restrict__ a,
-                                                    const TB *__restrict__ b,
-                                                    double *__restrict__ part,
-                                                    const Ctl *__restrict__ ctl) {
+                                                    const TB *__restrict__ b, double *part,
+                                                    Ctl *ctl) {
   if (ctl->done) return;
   double v[1] = {0.0};
   // four rows per trip, loads first: the same summation order as one row
@@ -151,13 +48,14 @@ __global__ void __launch_bounds__(kRedBlock) k_dot(int n, const TA *__restrict__
   for (; i < n; i += stride) v[0] = fma(to_d(a[i]), to_d(b[i]), v[0]);
   block_sum<1>(v);
   if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  if (FIN && last_block(&ctl->fin, gridDim.x)) finish_dot<FIN>(ctl, part, gridDim.x);
 }
 
 // The mixed form's FP32 dot products, summed as above.
+template <int FIN>
 __global__ void __launch_bounds__(kRedBlock) k_dot32c(int n, const float *__restrict__ a,
-                                                       const float *__restrict__ b,
-                                                       double *__restrict__ part,
-                                                       const Ctl *__restrict__ ctl) {
+                                                       const float *__restrict__ b, double *part,
+                                                       Ctl *ctl) {
   if (ctl->done) return;
   CSum acc{0.f, 0.f};
   const int stride = gridDim.x * blockDim.x;
@@ -171,12 +69,12 @@ __global__ void __launch_bounds__(kRedBlock) k_dot32c(int n, const float *__rest
   double v[1] = {csum_value(acc)};
   block_sum<1>(v);
   if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  if (FIN && last_block(&ctl->fin, gridDim.x)) finish_dot<FIN>(ctl, part, gridDim.x);
 }
 
 __global__ void __launch_bounds__(kRedBlock) k_dot_tq_tt32c(int n, const float *__restrict__ t,
                                                              const float *__restrict__ q,
-                                                             double *__restrict__ part,
-                                                             const Ctl *__restrict__ ctl) {
+                                                             double *part, Ctl *ctl) {
   if (ctl->done) return;
   CSum tq{0.f, 0.f}, tt{0.f, 0.f};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -190,14 +88,14 @@ __global__ void __launch_bounds__(kRedBlock) k_dot_tq_tt32c(int n, const float *
     part[blockIdx.x] = v[0];
     part[gridDim.x + blockIdx.x] = v[1];
   }
+  if (last_block(&ctl->fin, gridDim.x)) finish_dot<kFinOmega>(ctl, part, gridDim.x);
 }
 
 // t.q and t.t in one pass (BiCGSTAB omega)
 template <typename T>
 __global__ void __launch_bounds__(kRedBlock) k_dot_tq_tt(int n, const T *__restrict__ t,
-                                                          const T *__restrict__ q,
-                                                          double *__restrict__ part,
-                                                          const Ctl *__restrict__ ctl) {
+                                                          const T *__restrict__ q, double *part,
+                                                          Ctl *ctl) {
   if (ctl->done) return;
   double v[2] = {0.0, 0.0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -210,6 +108,7 @@ __global__ void __launch_bounds__(kRedBlock) k_dot_tq_tt(int n, const T *__restr
     part[blockIdx.x] = v[0];
     part[gridDim.x + blockIdx.x] = v[1];
   }
+  if (last_block(&ctl->fin, gridDim.x)) finish_dot<kFinOmega>(ctl, part, gridDim.x);
 }
 
 // sum of squares (L2NORM0)
@@ -226,97 +125,8 @@ __global__ void __launch_bounds__(kRedBlock) k_sumsq(int n, const T *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-// partial-sum finalisation inside the single-block control kernels
-// ---------------------------------------------------------------------------
-__device__ double ctl_reduce_sum(const double *part, int G) {
-  double v[1] = {0.0};
-  for (int i = threadIdx.x; i < G; i += blockDim.x) v[0] += part[i];
-  block_sum<1>(v);
-  return v[0];  // valid in thread 0
-}
-
-__device__ MaxLoc ctl_reduce_maxloc(const double *pv, const double *pi, int G) {
-  MaxLoc m[1];
-  m[0].val = 0.0;
-  m[0].idx = -1;
-  for (int i = threadIdx.x; i < G; i += blockDim.x) {
-    MaxLoc b;
-    b.val = pv[i];
-    b.idx = (long long)pi[i];
-    maxloc_merge(m[0], b);
-  }
-  block_maxloc<1>(m);
-  return m[0];
-}
-
-__device__ __forceinline__ bool d_is_close(double a, double b) {
-  if (a == b) return true;
-  double tol = 100.0 * DBL_EPSILON * fmax(fabs(a), fabs(b));
-  if (tol < 0.0) tol = 0.0;
-  return fabs(a - b) <= tol;
-}
-
-__device__ __forceinline__ void d_testcnvg(int icnvgopt, int &icnvg, int iiter, double dvmax,
-                                           double rmax, double rmax0, double epfact,
-                                           double dvclose, double rclose) {
-  if (icnvgopt == 0) {
-    if (fabs(dvmax) <= dvclose && fabs(rmax) <= rclose) icnvg = 1;
-  } else if (icnvgopt == 1) {
-    if (fabs(dvmax) <= dvclose && fabs(rmax) <= rclose) icnvg = (iiter == 1) ? 1 : -1;
-  } else if (icnvgopt == 2) {
-    if (fabs(dvmax) <= dvclose || rmax <= rclose) icnvg = 1;
-    else if (rmax <= rmax0 * epfact) icnvg = -1;
-  } else if (icnvgopt == 3) {
-    if (fabs(dvmax) <= dvclose) icnvg = 1;
-    else if (rmax <= rmax0 * rclose) icnvg = -1;
-  } else if (icnvgopt == 4) {
-    if (fabs(dvmax) <= dvclose && rmax <= rclose) icnvg = 1;
-    else if (rmax <= rmax0 * epfact) icnvg = -1;
-  }
-}
-
-__device__ __forceinline__ double sign_dprec(double den) { return copysign(DBL_EPSILON, den); }
-
-// Sets the WHILE condition of the graph.  Independently of the IMS exit logic,
-// the loop is cut after 2*itmax + 16 bodies, so no input can keep the device
-// looping.
-__device__ __forceinline__ void set_loop(Ctl *ctl, unsigned long long cond, int use_cond) {
-  ctl->bodies += 1;
-  if (ctl->bodies > 2 * ctl->itmax + 16 && !ctl->done) {
-    ctl->done = 1;
-    ctl->guard_tripped = 1;
-  }
-  if (use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, ctl->done ? 0u : 1u);
-}
-
-// ---------------------------------------------------------------------------
 // PCG
 // ---------------------------------------------------------------------------
-__device__ void ctl_cg_rho(Ctl *ctl, const double *part, int G) {
-  if (ctl->done) return;
-  double s = ctl_reduce_sum(part, G);
-  if (threadIdx.x == 0) {
-    ctl->rho = s;
-    ctl->beta = ctl->first ? 0.0 : s / ctl->rho0;
-  }
-}
-__global__ void k_ctl_cg_rho(Ctl *ctl, const double *part, int G) {
-  ctl_cg_rho(ctl, part, G);
-}
-
-__device__ void ctl_alpha(Ctl *ctl, const double *part, int G) {
-  if (ctl->done) return;
-  double s = ctl_reduce_sum(part, G);
-  if (threadIdx.x == 0) {
-    double den = s + sign_dprec(s);
-    ctl->alpha = ctl->rho / den;
-  }
-}
-__global__ void k_ctl_alpha(Ctl *ctl, const double *part, int G) {
-  ctl_alpha(ctl, part, G);
-}
-
-
 __global__ void __launch_bounds__(256) k_cg_pupdate64(int n, const double *__restrict__ z,
                                                       double *__restrict__ p,
                                                       const Ctl *__restrict__ ctl) {
@@ -336,184 +146,51 @@ __global__ void __launch_bounds__(256) k_cg_pupdate32(int n, const float *__rest
   p[i] = ctl->first ? z[i] : fmaf((float)ctl->beta, p[i], z[i]);
 }
 
-// x += alpha*p ; d -= alpha*q ; max|alpha p|, max|d|, sum d^2 (FP64 path).
-// partial slots: [0]=l2, [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite
-// The sum of squares is taken only when the closure test reads it (L2 =
-// true: RCLOSE options L2NORM_RCLOSE and RELATIVE_RCLOSE, ICNVGOPT 2-4); with
-// the infinity-norm tests the reference computes it but never reads it
-// inside the loop, and on GB300 it is a quarter of the kernel's FP64 work.
+// A block's share of an update into its partial slots: [0]=l2 (when taken),
+// [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite.
 template <bool L2>
-__global__ void __launch_bounds__(kRedBlock) k_cg_update64(int n, double *__restrict__ x,
-                                                            double *__restrict__ d,
-                                                            const double *__restrict__ p,
-                                                            const double *__restrict__ q,
-                                                            double *__restrict__ part,
-                                                            const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  const double alpha = ctl->alpha;
-  double v[2] = {0.0, 0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  auto row = [&](int i, double pi, double xi, double qi, double dI) {
-    double tv = alpha * pi;
-    x[i] = xi + tv;
-    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
-    double di = fma(-alpha, qi, dI);
-    d[i] = di;
-    if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i; }
-    if (L2) v[0] = fma(di, di, v[0]);
-    nf |= nonfinite(di) | nonfinite(tv);
-  };
-  // four rows per trip, their 16 loads issued before any row is used (the
-  // same order of rows per thread as one row per trip, so the same sums and
-  // maxima): the loads of a trip cover the latency of the FP64 work of the
-  // trip before
-  constexpr int R = 4;
-  const int stride = gridDim.x * blockDim.x;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + (R - 1) * stride < n; i += R * stride) {
-    double pr[R], xr[R], qr[R], dr[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int j = i + r * stride;
-      pr[r] = __ldcs(p + j);
-      xr[r] = __ldcs(x + j);
-      qr[r] = __ldcs(q + j);
-      dr[r] = __ldcs(d + j);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) row(i + r * stride, pr[r], xr[r], qr[r], dr[r]);
-  }
-  for (; i < n; i += stride) row(i, p[i], x[i], q[i], d[i]);
-  v[1] = (double)nf;
-  block_sum<2>(v);
+__device__ __forceinline__ void update_partials(double l2, unsigned nf, MaxLoc (&m)[2], double *part,
+                                                int G, int b) {
+  const int any = __syncthreads_or((int)nf);
+  double v[1] = {l2};
+  if (L2) block_sum<1>(v);
   block_maxloc<2>(m);
   if (threadIdx.x == 0) {
-    int G = gridDim.x, b = blockIdx.x;
-    part[b] = v[0];
+    part[b] = L2 ? v[0] : 0.0;
     part[G + b] = m[0].val; part[2 * G + b] = (double)m[0].idx;
     part[3 * G + b] = m[1].val; part[4 * G + b] = (double)m[1].idx;
-    part[5 * G + b] = v[1];
-  }
-}
-
-
-// Mixed inner update: the step alpha*p in FP32, added to the FP64 heads;
-// d32 -= alpha*q32; the maxima on FP32 magnitudes (integer compares of the
-// bit patterns) and the L2 sum compensated in FP32, so that the only FP64
-// instructions per row are the conversion of the step and the head update.
-__global__ void __launch_bounds__(kRedBlock) k_cg_update_mixed(int n, double *__restrict__ x,
-                                                                float *__restrict__ d,
-                                                                const float *__restrict__ p,
-                                                                const float *__restrict__ q,
-                                                                double *__restrict__ part,
-                                                                const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  const float alphaf = (float)ctl->alpha;
-  CSum l2{0.f, 0.f};
-  unsigned nf = 0;
-  unsigned bdx = 0, brr = 0;  // largest magnitudes so far (bit patterns)
-  float vdx = 0.f, vrr = 0.f;
-  int idx_dx = -1, idx_rr = -1;
-  auto row = [&](int i, float pi, double xi, float qi, float dI) {
-    const float tv = __fmul_rn(alphaf, pi);
-    x[i] = xi + (double)tv;
-    const unsigned at = __float_as_uint(tv) & 0x7fffffffu;
-    if (at > bdx) { bdx = at; vdx = tv; idx_dx = i; }
-    const float di = __fmaf_rn(-alphaf, qi, dI);
-    d[i] = di;
-    const unsigned ad = __float_as_uint(di) & 0x7fffffffu;
-    if (ad > brr) { brr = ad; vrr = di; idx_rr = i; }
-    csum_prod(l2, di, di);
-    nf |= nonfinite(di) | nonfinite(tv);
-  };
-  const int stride = gridDim.x * blockDim.x;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + stride < n; i += 2 * stride) {
-    const int j = i + stride;
-    const float p0 = p[i], q0 = q[i], d0 = d[i];
-    const double x0 = x[i];
-    const float p1 = p[j], q1 = q[j], d1 = d[j];
-    const double x1 = x[j];
-    row(i, p0, x0, q0, d0);
-    row(j, p1, x1, q1, d1);
-  }
-  if (i < n) row(i, p[i], x[i], q[i], d[i]);
-  double v[2] = {csum_value(l2), (double)nf};
-  MaxLoc m[2];
-  m[0].val = (double)vdx; m[0].idx = idx_dx;
-  m[1].val = (double)vrr; m[1].idx = idx_rr;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
-    int G = gridDim.x, b = blockIdx.x;
-    part[b] = v[0];
-    part[G + b] = m[0].val; part[2 * G + b] = (double)m[0].idx;
-    part[3 * G + b] = m[1].val; part[4 * G + b] = (double)m[1].idx;
-    part[5 * G + b] = v[1];
+    part[5 * G + b] = any ? 1.0 : 0.0;
   }
 }
 
 // Finalise an update reduction into ctl (deltax, rmax, l2norm, nonfinite).
-__device__ void ctl_finish_update(Ctl *ctl, const double *part, int G) {
-  double l2 = ctl_reduce_sum(part, G);
-  MaxLoc dx = ctl_reduce_maxloc(part + G, part + 2 * G, G);
-  MaxLoc rm = ctl_reduce_maxloc(part + 3 * G, part + 4 * G, G);
-  double nf = ctl_reduce_sum(part + 5 * G, G);
-  if (threadIdx.x == 0) {
-    ctl->l2norm = sqrt(l2);
-    ctl->deltax = dx.val;
-    ctl->xloc = dx.idx;
-    ctl->rmax = rm.val;
-    ctl->rloc = rm.idx;
-    if (nf != 0.0) ctl->nonfinite = 1;
+template <bool L2>
+__device__ __forceinline__ void ctl_finish_update(Ctl *ctl, const double *part, int G) {
+  double l2[1] = {0.0};
+  MaxLoc m[2];
+  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  int nf = 0;
+  for (int i = threadIdx.x; i < G; i += blockDim.x) {
+    MaxLoc a, b;
+    if (L2) l2[0] += __ldcg(part + i);
+    a.val = __ldcg(part + G + i);
+    a.idx = (long long)__ldcg(part + 2 * G + i);
+    b.val = __ldcg(part + 3 * G + i);
+    b.idx = (long long)__ldcg(part + 4 * G + i);
+    nf |= __ldcg(part + 5 * G + i) != 0.0;
+    maxloc_merge(m[0], a);
+    maxloc_merge(m[1], b);
   }
-}
-
-// Per-model maxima of one iteration for the inner records, when the solution
-// has more than one model (CONVNMOD > 1; ImsLinearBase.f90:141-182 for PCG,
-// :431-480 for BiCGSTAB): for each model's rows, the largest head change
-// (the step the update kernel added: PCG alpha*p, BiCGSTAB alpha*phat +
-// omega*qhat, times DSCALE when scaled) and the largest residual (divided by
-// DSCALE when scaled), signed, with its row.  The step is recomputed with the
-// update kernel's own expression, so the values are the ones the update
-// compared.  Partial slots per model im: [4im] dx value, [4im+1] its row,
-// [4im+2] r value, [4im+3] its row (G blocks each).
-template <bool BCGS>
-__global__ void __launch_bounds__(kRedBlock) k_rec_models(int nm, const int *__restrict__ modstart,
-                                                          const double *__restrict__ p,
-                                                          const double *__restrict__ q,
-                                                          const double *__restrict__ d,
-                                                          const double *__restrict__ dscale,
-                                                          double *__restrict__ part,
-                                                          const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  const double alpha = ctl->alpha, omega = ctl->omega;
-  const int G = gridDim.x, b = blockIdx.x;
-  for (int im = 0; im < nm; ++im) {
-    MaxLoc m[2];
-    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-    const int r0 = modstart[im], r1 = modstart[im + 1];
-    for (int i = r0 + b * blockDim.x + threadIdx.x; i < r1; i += G * blockDim.x) {
-      double tv;
-      if (BCGS) tv = fma(alpha, p[i], omega * q[i]);
-      else tv = alpha * p[i];
-      double rv = d[i];
-      if (BCGS && dscale) {
-        tv = tv * dscale[i];
-        rv = rv / dscale[i];
-      }
-      if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
-      if (absgt(rv, m[1].val)) { m[1].val = rv; m[1].idx = i; }
-    }
-    block_maxloc<2>(m);
-    if (threadIdx.x == 0) {
-      part[(4 * im) * G + b] = m[0].val;
-      part[(4 * im + 1) * G + b] = (double)m[0].idx;
-      part[(4 * im + 2) * G + b] = m[1].val;
-      part[(4 * im + 3) * G + b] = (double)m[1].idx;
-    }
+  nf = __syncthreads_or(nf);
+  if (L2) block_sum<1>(l2);
+  block_maxloc<2>(m);
+  if (threadIdx.x == 0) {
+    ctl->l2norm = L2 ? sqrt(l2[0]) : 0.0;
+    ctl->deltax = m[0].val;
+    ctl->xloc = m[0].idx;
+    ctl->rmax = m[1].val;
+    ctl->rloc = m[1].idx;
+    if (nf) ctl->nonfinite = 1;
   }
 }
 
@@ -564,13 +241,14 @@ __device__ void ctl_record(Ctl *ctl, bool bcgs) {
 }
 
 // End of a PCG iteration: closure test and loop control (ImsLinearBase.f90:196-236).
-__device__ void ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
+template <bool L2>
+__device__ __forceinline__ void ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
                               int use_cond) {
   if (ctl->done) {
     if (threadIdx.x == 0) set_loop(ctl, cond, use_cond);
     return;
   }
-  ctl_finish_update(ctl, part, G);
+  ctl_finish_update<L2>(ctl, part, G);
   if (ctl->rec) ctl_record(ctl, false);
   if (threadIdx.x != 0) return;
   double rcnvg = (ctl->icnvgopt == 2 || ctl->icnvgopt == 3 || ctl->icnvgopt == 4) ? ctl->l2norm
@@ -608,116 +286,15 @@ __device__ void ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long l
   if (ctl->done && ctl->icnvg < 0) ctl->icnvg = 0;
   set_loop(ctl, cond, use_cond);
 }
-__global__ void k_ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
-                              int use_cond) {
-  ctl_cg_cnvg(ctl, part, G, cond, use_cond);
-}
-
-// ---------------------------------------------------------------------------
-// BiCGSTAB
-// ---------------------------------------------------------------------------
-__device__ void ctl_bcgs_rho(Ctl *ctl, const double *part, int G) {
-  if (ctl->done) return;
-  double s = ctl_reduce_sum(part, G);
-  if (threadIdx.x == 0) {
-    ctl->rho = s;
-    if (!ctl->first) ctl->beta = (s / ctl->rho0) * (ctl->alpha0 / ctl->omega0);
-  }
-}
-__global__ void k_ctl_bcgs_rho(Ctl *ctl, const double *part, int G) {
-  ctl_bcgs_rho(ctl, part, G);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_bcgs_p(int n, const T *__restrict__ d, T *__restrict__ p,
-                                                const T *__restrict__ v,
-                                                const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (ctl->first) {
-    p[i] = d[i];
-  } else {
-    T beta = (T)ctl->beta, om = (T)ctl->omega0;
-    T inner = fma(-om, v[i], p[i]);
-    p[i] = fma(beta, inner, d[i]);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_bcgs_q(int n, const T *__restrict__ d, const T *__restrict__ v,
-                                                T *__restrict__ q, const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  q[i] = fma(-(T)ctl->alpha, v[i], d[i]);
-}
-
-__device__ void ctl_omega(Ctl *ctl, const double *part, int G) {
-  if (ctl->done) return;
-  double num = ctl_reduce_sum(part, G);
-  double den = ctl_reduce_sum(part + G, G);
-  if (threadIdx.x == 0) {
-    den = den + sign_dprec(den);
-    ctl->omega = num / den;
-  }
-}
-__global__ void k_ctl_omega(Ctl *ctl, const double *part, int G) {
-  ctl_omega(ctl, part, G);
-}
-
-// x += alpha*phat + omega*qhat ; d = q - omega*t (ImsLinearBase.f90:428-480).
-// L2 as in k_cg_update64.
-template <typename T, bool L2>
-__global__ void __launch_bounds__(kRedBlock) k_bcgs_update(int n, double *__restrict__ x,
-                                                            T *__restrict__ d,
-                                                            const T *__restrict__ phat,
-                                                            const T *__restrict__ qhat,
-                                                            const T *__restrict__ q,
-                                                            const T *__restrict__ t,
-                                                            const double *__restrict__ dscale,
-                                                            double *__restrict__ part,
-                                                            const Ctl *__restrict__ ctl) {
-  if (ctl->done) return;
-  const double alpha = ctl->alpha, omega = ctl->omega;
-  const T omegat = (T)omega;
-  double v[2] = {0.0, 0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double tv = fma(alpha, to_d(phat[i]), omega * to_d(qhat[i]));
-    x[i] = x[i] + tv;
-    if (dscale) tv = tv * dscale[i];
-    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
-    T di = fma(-omegat, t[i], q[i]);
-    d[i] = di;
-    double rv = to_d(di);
-    if (dscale) rv = rv / dscale[i];
-    if (absgt(rv, m[1].val)) { m[1].val = rv; m[1].idx = i; }
-    if (L2) v[0] = fma(rv, rv, v[0]);
-    nf |= nonfinite(rv) | nonfinite(tv);
-  }
-  v[1] = (double)nf;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
-    int G = gridDim.x, b = blockIdx.x;
-    part[b] = v[0];
-    part[G + b] = m[0].val; part[2 * G + b] = (double)m[0].idx;
-    part[3 * G + b] = m[1].val; part[4 * G + b] = (double)m[1].idx;
-    part[5 * G + b] = v[1];
-  }
-}
-
 // End of a BiCGSTAB iteration (ImsLinearBase.f90:498-545).
-__device__ void ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
+template <bool L2>
+__device__ __forceinline__ void ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
                                 int use_cond) {
   if (ctl->done) {
     if (threadIdx.x == 0) set_loop(ctl, cond, use_cond);
     return;
   }
-  ctl_finish_update(ctl, part, G);
+  ctl_finish_update<L2>(ctl, part, G);
   if (ctl->rec) ctl_record(ctl, true);
   if (threadIdx.x != 0) return;
   double rcnvg = (ctl->icnvgopt == 2 || ctl->icnvgopt == 3 || ctl->icnvgopt == 4) ? ctl->l2norm
@@ -758,23 +335,14 @@ __device__ void ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long
   if (ctl->done && ctl->icnvg < 0) ctl->icnvg = 0;
   set_loop(ctl, cond, use_cond);
 }
-__global__ void k_ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
-                                int use_cond) {
-  ctl_bcgs_cnvg(ctl, part, G, cond, use_cond);
-}
-
-// ---------------------------------------------------------------------------
-// Mixed precision: FP64 iterative refinement around the FP32 inner loop
-// ---------------------------------------------------------------------------
-
 // End of a mixed inner iteration.  The IMS test runs on the recursive FP32
 // residual; when it passes, or the recursive residual has dropped by
 // refine_factor since the last refinement, the next true-residual check is
 // requested (Ctl::north_due = 2) instead of stopping.
-__device__ void ctl_mixed_inner(Ctl *ctl, const double *part, int G, int bcgs,
+__device__ __forceinline__ void ctl_mixed_inner(Ctl *ctl, const double *part, int G, int bcgs,
                                   double refine_factor) {
   if (ctl->done) return;
-  ctl_finish_update(ctl, part, G);
+  ctl_finish_update<true>(ctl, part, G);
   if (threadIdx.x != 0) return;
   double rcnvg = (ctl->icnvgopt == 2 || ctl->icnvgopt == 3 || ctl->icnvgopt == 4) ? ctl->l2norm
                                                                                 : ctl->rmax;
@@ -816,51 +384,8 @@ __device__ void ctl_mixed_inner(Ctl *ctl, const double *part, int G, int bcgs,
     }
   }
 }
-__global__ void k_ctl_mixed_inner(Ctl *ctl, const double *part, int G, int bcgs,
-                                  double refine_factor) {
-  ctl_mixed_inner(ctl, part, G, bcgs, refine_factor);
-}
-
-// True residual r = b - A x in FP64 with its max|r| and L2, only when
-// requested; the FP32 residual is reset from it.
-__global__ void __launch_bounds__(kRedBlock) k_true_resid_stats(int n, const double *__restrict__ r,
-                                                                 float *__restrict__ d32,
-                                                                 float *__restrict__ dhat32,
-                                                                 double *__restrict__ dhat64,
-                                                                 const double *__restrict__ dscale,
-                                                                 double *__restrict__ part,
-                                                                 const Ctl *__restrict__ ctl) {
-  if (ctl->done || ctl->north_due != 2) return;
-  double v[2] = {0.0, 0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double ri = r[i];
-    if (d32) d32[i] = (float)ri;
-    if (ctl->restart_due) {  // BiCGSTAB shadow residual, on a restart
-      if (dhat32) dhat32[i] = (float)ri;
-      if (dhat64) dhat64[i] = ri;
-    }
-    if (dscale) ri = ri / dscale[i];    // BiCGSTAB reports the unscaled residual
-    if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i; }
-    v[0] = fma(ri, ri, v[0]);
-    nf |= nonfinite(ri);
-  }
-  v[1] = (double)nf;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
-    int G = gridDim.x, b = blockIdx.x;
-    part[b] = v[0];
-    part[G + b] = 0.0; part[2 * G + b] = -1.0;
-    part[3 * G + b] = m[1].val; part[4 * G + b] = (double)m[1].idx;
-    part[5 * G + b] = v[1];
-  }
-}
-
 // Closure test on the FP64 true residual; restart the inner loop if needed.
-__device__ void ctl_refine(Ctl *ctl, const double *part, int G, unsigned long long cond,
+__device__ __forceinline__ void ctl_refine(Ctl *ctl, const double *part, int G, unsigned long long cond,
                              int use_cond) {
   if (ctl->done || ctl->north_due != 2) {
     if (threadIdx.x == 0) set_loop(ctl, cond, use_cond);
@@ -868,7 +393,7 @@ __device__ void ctl_refine(Ctl *ctl, const double *part, int G, unsigned long lo
   }
   double dsave = ctl->scratch[1];
   long long lsave = (long long)ctl->scratch[2];
-  ctl_finish_update(ctl, part, G);
+  ctl_finish_update<true>(ctl, part, G);
   if (threadIdx.x != 0) return;
   ctl->deltax = dsave;
   ctl->xloc = lsave;
@@ -908,9 +433,286 @@ __device__ void ctl_refine(Ctl *ctl, const double *part, int G, unsigned long lo
   }
   set_loop(ctl, cond, use_cond);
 }
-__global__ void k_ctl_refine(Ctl *ctl, const double *part, int G, unsigned long long cond,
-                             int use_cond) {
-  ctl_refine(ctl, part, G, cond, use_cond);
+// The closure tests as kernels of their own, behind the per-model records.
+template <bool L2>
+__global__ void k_ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
+                              int use_cond) {
+  ctl_cg_cnvg<L2>(ctl, part, G, cond, use_cond);
+}
+
+template <bool L2>
+__global__ void k_ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond,
+                                int use_cond) {
+  ctl_bcgs_cnvg<L2>(ctl, part, G, cond, use_cond);
+}
+
+// x += alpha*p ; d -= alpha*q ; max|alpha p|, max|d|, sum d^2 (FP64 path).
+// partial slots: [0]=l2, [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite
+// The sum of squares is taken only when the closure test reads it (L2 =
+// true: RCLOSE options L2NORM_RCLOSE and RELATIVE_RCLOSE, ICNVGOPT 2-4); with
+// the infinity-norm tests the reference computes it but never reads it
+// inside the loop, and on GB300 it is a quarter of the kernel's FP64 work.
+// p1: P alternates between p (even iterations) and p1 (odd ones), or null.
+// FIN: the last block runs the closure test.
+template <bool L2, bool FIN>
+__global__ void __launch_bounds__(kRedBlock) k_cg_update64(int n, double *__restrict__ x,
+                                                            double *__restrict__ d, const double *p,
+                                                            const double *p1,
+                                                            const double *__restrict__ q,
+                                                            double *part, Ctl *ctl,
+                                                            unsigned long long cond, int use_cond) {
+  if (ctl->done) {
+    if (FIN && blockIdx.x == 0 && threadIdx.x == 0) set_loop(ctl, cond, use_cond);
+    return;
+  }
+  const double alpha = ctl->alpha;
+  if (p1 && (ctl->iter & 1)) p = p1;
+  double v[1] = {0.0};
+  unsigned nf = 0;
+  MaxLoc m[2];
+  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  auto row = [&](int i, double pi, double xi, double qi, double dI) {
+    double tv = alpha * pi;
+    x[i] = xi + tv;
+    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
+    double di = fma(-alpha, qi, dI);
+    d[i] = di;
+    if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i; }
+    if (L2) v[0] = fma(di, di, v[0]);
+    nf |= nonfinite(di) | nonfinite(tv);
+  };
+  // four rows per trip, their 16 loads issued before any row is used (the
+  // same order of rows per thread as one row per trip, so the same sums and
+  // maxima): the loads of a trip cover the latency of the FP64 work of the
+  // trip before
+  constexpr int R = 4;
+  const int stride = gridDim.x * blockDim.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + (R - 1) * stride < n; i += R * stride) {
+    double pr[R], xr[R], qr[R], dr[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = i + r * stride;
+      pr[r] = __ldcs(p + j);
+      xr[r] = __ldcs(x + j);
+      qr[r] = __ldcs(q + j);
+      dr[r] = __ldcs(d + j);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) row(i + r * stride, pr[r], xr[r], qr[r], dr[r]);
+  }
+  for (; i < n; i += stride) row(i, p[i], x[i], q[i], d[i]);
+  update_partials<L2>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_cg_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
+}
+
+
+// Mixed inner update: the step alpha*p in FP32, added to the FP64 heads;
+// d32 -= alpha*q32; the maxima on FP32 magnitudes (integer compares of the
+// bit patterns) and the L2 sum compensated in FP32, so that the only FP64
+// instructions per row are the conversion of the step and the head update.
+template <bool FIN>
+__global__ void __launch_bounds__(kRedBlock) k_cg_update_mixed(int n, double *__restrict__ x,
+                                                                float *__restrict__ d, const float *p,
+                                                                const float *p1,
+                                                                const float *__restrict__ q,
+                                                                double *part, Ctl *ctl,
+                                                                double refine_factor) {
+  if (ctl->done) return;
+  const float alphaf = (float)ctl->alpha;
+  if (p1 && (ctl->iter & 1)) p = p1;
+  CSum l2{0.f, 0.f};
+  unsigned nf = 0;
+  unsigned bdx = 0, brr = 0;  // largest magnitudes so far (bit patterns)
+  float vdx = 0.f, vrr = 0.f;
+  int idx_dx = -1, idx_rr = -1;
+  auto row = [&](int i, float pi, double xi, float qi, float dI) {
+    const float tv = __fmul_rn(alphaf, pi);
+    x[i] = xi + (double)tv;
+    const unsigned at = __float_as_uint(tv) & 0x7fffffffu;
+    if (at > bdx) { bdx = at; vdx = tv; idx_dx = i; }
+    const float di = __fmaf_rn(-alphaf, qi, dI);
+    d[i] = di;
+    const unsigned ad = __float_as_uint(di) & 0x7fffffffu;
+    if (ad > brr) { brr = ad; vrr = di; idx_rr = i; }
+    csum_prod(l2, di, di);
+    nf |= nonfinite(di) | nonfinite(tv);
+  };
+  const int stride = gridDim.x * blockDim.x;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (; i + stride < n; i += 2 * stride) {
+    const int j = i + stride;
+    const float p0 = p[i], q0 = q[i], d0 = d[i];
+    const double x0 = x[i];
+    const float p1 = p[j], q1 = q[j], d1 = d[j];
+    const double x1 = x[j];
+    row(i, p0, x0, q0, d0);
+    row(j, p1, x1, q1, d1);
+  }
+  if (i < n) row(i, p[i], x[i], q[i], d[i]);
+  MaxLoc m[2];
+  m[0].val = (double)vdx; m[0].idx = idx_dx;
+  m[1].val = (double)vrr; m[1].idx = idx_rr;
+  update_partials<true>(csum_value(l2), nf, m, part, gridDim.x, blockIdx.x);
+  if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_mixed_inner(ctl, part, gridDim.x, 0, refine_factor);
+}
+
+// Per-model maxima of one iteration for the inner records, when the solution
+// has more than one model (CONVNMOD > 1; ImsLinearBase.f90:141-182 for PCG,
+// :431-480 for BiCGSTAB): for each model's rows, the largest head change
+// (the step the update kernel added: PCG alpha*p, BiCGSTAB alpha*phat +
+// omega*qhat, times DSCALE when scaled) and the largest residual (divided by
+// DSCALE when scaled), signed, with its row.  The step is recomputed with the
+// update kernel's own expression, so the values are the ones the update
+// compared.  Partial slots per model im: [4im] dx value, [4im+1] its row,
+// [4im+2] r value, [4im+3] its row (G blocks each).
+template <bool BCGS>
+__global__ void __launch_bounds__(kRedBlock) k_rec_models(int nm, const int *__restrict__ modstart,
+                                                          const double *__restrict__ p,
+                                                          const double *__restrict__ q,
+                                                          const double *__restrict__ d,
+                                                          const double *__restrict__ dscale,
+                                                          double *__restrict__ part,
+                                                          const Ctl *__restrict__ ctl) {
+  if (ctl->done) return;
+  const double alpha = ctl->alpha, omega = ctl->omega;
+  const int G = gridDim.x, b = blockIdx.x;
+  for (int im = 0; im < nm; ++im) {
+    MaxLoc m[2];
+    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+    const int r0 = modstart[im], r1 = modstart[im + 1];
+    for (int i = r0 + b * blockDim.x + threadIdx.x; i < r1; i += G * blockDim.x) {
+      double tv;
+      if (BCGS) tv = fma(alpha, p[i], omega * q[i]);
+      else tv = alpha * p[i];
+      double rv = d[i];
+      if (BCGS && dscale) {
+        tv = tv * dscale[i];
+        rv = rv / dscale[i];
+      }
+      if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
+      if (absgt(rv, m[1].val)) { m[1].val = rv; m[1].idx = i; }
+    }
+    block_maxloc<2>(m);
+    if (threadIdx.x == 0) {
+      part[(4 * im) * G + b] = m[0].val;
+      part[(4 * im + 1) * G + b] = (double)m[0].idx;
+      part[(4 * im + 2) * G + b] = m[1].val;
+      part[(4 * im + 3) * G + b] = (double)m[1].idx;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// BiCGSTAB
+// ---------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(256) k_bcgs_p(int n, const T *__restrict__ d, T *__restrict__ p,
+                                                const T *__restrict__ v,
+                                                const Ctl *__restrict__ ctl) {
+  if (ctl->done) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  if (ctl->first) {
+    p[i] = d[i];
+  } else {
+    T beta = (T)ctl->beta, om = (T)ctl->omega0;
+    T inner = fma(-om, v[i], p[i]);
+    p[i] = fma(beta, inner, d[i]);
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_bcgs_q(int n, const T *__restrict__ d, const T *__restrict__ v,
+                                                T *__restrict__ q, const Ctl *__restrict__ ctl) {
+  if (ctl->done) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  q[i] = fma(-(T)ctl->alpha, v[i], d[i]);
+}
+
+// x += alpha*phat + omega*qhat ; d = q - omega*t (ImsLinearBase.f90:428-480).
+// L2 as in k_cg_update64.
+// FIN 1: the last block runs the closure test; 2: the end of a mixed inner
+// iteration.
+template <typename T, bool L2, int FIN>
+__global__ void __launch_bounds__(kRedBlock) k_bcgs_update(int n, double *__restrict__ x,
+                                                            T *__restrict__ d,
+                                                            const T *__restrict__ phat,
+                                                            const T *__restrict__ qhat,
+                                                            const T *__restrict__ q,
+                                                            const T *__restrict__ t,
+                                                            const double *__restrict__ dscale,
+                                                            double *part, Ctl *ctl,
+                                                            unsigned long long cond, int use_cond,
+                                                            double refine_factor) {
+  if (ctl->done) {
+    if (FIN == 1 && blockIdx.x == 0 && threadIdx.x == 0) set_loop(ctl, cond, use_cond);
+    return;
+  }
+  const double alpha = ctl->alpha, omega = ctl->omega;
+  const T omegat = (T)omega;
+  double v[1] = {0.0};
+  unsigned nf = 0;
+  MaxLoc m[2];
+  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double tv = fma(alpha, to_d(phat[i]), omega * to_d(qhat[i]));
+    x[i] = x[i] + tv;
+    if (dscale) tv = tv * dscale[i];
+    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
+    T di = fma(-omegat, t[i], q[i]);
+    d[i] = di;
+    double rv = to_d(di);
+    if (dscale) rv = rv / dscale[i];
+    if (absgt(rv, m[1].val)) { m[1].val = rv; m[1].idx = i; }
+    if (L2) v[0] = fma(rv, rv, v[0]);
+    nf |= nonfinite(rv) | nonfinite(tv);
+  }
+  update_partials<L2>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  if (FIN && last_block(&ctl->fin, gridDim.x)) {
+    if (FIN == 1) ctl_bcgs_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
+    else ctl_mixed_inner(ctl, part, gridDim.x, 1, refine_factor);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Mixed precision: FP64 iterative refinement around the FP32 inner loop
+// ---------------------------------------------------------------------------
+
+// True residual r = b - A x in FP64 with its max|r| and L2, only when
+// requested; the FP32 residual is reset from it.
+__global__ void __launch_bounds__(kRedBlock) k_true_resid_stats(int n, const double *__restrict__ r,
+                                                                 float *__restrict__ d32,
+                                                                 float *__restrict__ dhat32,
+                                                                 double *__restrict__ dhat64,
+                                                                 const double *__restrict__ dscale,
+                                                                 double *part, Ctl *ctl,
+                                                                 unsigned long long cond,
+                                                                 int use_cond) {
+  if (ctl->done || ctl->north_due != 2) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) set_loop(ctl, cond, use_cond);
+    return;
+  }
+  double v[1] = {0.0};
+  unsigned nf = 0;
+  MaxLoc m[2];
+  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    double ri = r[i];
+    if (d32) d32[i] = (float)ri;
+    if (ctl->restart_due) {  // BiCGSTAB shadow residual, on a restart
+      if (dhat32) dhat32[i] = (float)ri;
+      if (dhat64) dhat64[i] = ri;
+    }
+    if (dscale) ri = ri / dscale[i];    // BiCGSTAB reports the unscaled residual
+    if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i; }
+    v[0] = fma(ri, ri, v[0]);
+    nf |= nonfinite(ri);
+  }
+  m[0].idx = -1;
+  update_partials<true>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  if (last_block(&ctl->fin, gridDim.x)) ctl_refine(ctl, part, gridDim.x, cond, use_cond);
 }
 
 // ---------------------------------------------------------------------------
@@ -978,16 +780,32 @@ __device__ __forceinline__ double *member_part(double *part, const BatchDev &B, 
   return part + 8LL * B.mc[m];
 }
 
-template <typename TA, typename TB>
-__global__ void __launch_bounds__(kRedBlock) k_b_dot(BatchDev B, const TA *__restrict__ a,
-                                                     const TB *__restrict__ b,
-                                                     double *__restrict__ part) {
+// Rows a thread of a chunk's block handles: its loads are issued before any
+// row is used.
+constexpr int kChunkTrips = kChunkRows / kRedBlock;
+
+template <int FIN>
+__global__ void __launch_bounds__(kRedBlock) k_b_dot(BatchDev B, const double *__restrict__ a,
+                                                     const double *__restrict__ b, double *part) {
   const ChunkRef c = chunk_of(B, blockIdx.x);
-  if (B.ctls[c.m].done) return;
+  Ctl *ctl = B.ctls + c.m;
+  if (ctl->done) return;
   double v[1] = {0.0};
-  for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) v[0] = fma(to_d(a[i]), to_d(b[i]), v[0]);
+  double ar[kChunkTrips], br[kChunkTrips];
+  const int i0 = c.r0 + threadIdx.x;
+#pragma unroll
+  for (int t = 0; t < kChunkTrips; ++t)
+    if (i0 + t * kRedBlock < c.r1) {
+      ar[t] = a[i0 + t * kRedBlock];
+      br[t] = b[i0 + t * kRedBlock];
+    }
+#pragma unroll
+  for (int t = 0; t < kChunkTrips; ++t)
+    if (i0 + t * kRedBlock < c.r1) v[0] = fma(ar[t], br[t], v[0]);
   block_sum<1>(v);
-  if (threadIdx.x == 0) member_part(part, B, c.m)[c.b] = v[0];
+  double *pm = member_part(part, B, c.m);
+  if (threadIdx.x == 0) pm[c.b] = v[0];
+  if (last_block(&ctl->fin, c.G)) finish_dot<FIN>(ctl, pm, c.G);
 }
 
 __global__ void __launch_bounds__(kRedBlock) k_b_sumsq(BatchDev B, const double *__restrict__ a,
@@ -1007,96 +825,125 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_pupdate(BatchDev B, const T 
   if (ctl.done) return;
   const bool first = ctl.first;
   const double beta = ctl.beta;
-  for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x)
-    p[i] = first ? z[i] : (T)fma((double)(T)beta, (double)p[i], (double)z[i]);
+  T zr[kChunkTrips], pr[kChunkTrips];
+  const int i0 = c.r0 + threadIdx.x;
+#pragma unroll
+  for (int t = 0; t < kChunkTrips; ++t)
+    if (i0 + t * kRedBlock < c.r1) {
+      zr[t] = z[i0 + t * kRedBlock];
+      pr[t] = p[i0 + t * kRedBlock];
+    }
+#pragma unroll
+  for (int t = 0; t < kChunkTrips; ++t)
+    if (i0 + t * kRedBlock < c.r1)
+      p[i0 + t * kRedBlock] = first ? zr[t] : (T)fma((double)(T)beta, (double)pr[t], (double)zr[t]);
 }
 
-// x += alpha*p ; d -= alpha*q with the same partial slots as k_cg_update64.
+// The batch's own control block gets done = every member done; it gates the
+// shared kernels (SpMV, preconditioner) and drives the WHILE condition.  By
+// one block, after every member's control step.
+__device__ __forceinline__ void batch_all_done(const BatchDev &B, Ctl *gctl, unsigned long long cond,
+                                               int use_cond, int count_body) {
+  int any = 0;
+  for (int m = threadIdx.x; m < B.nm; m += blockDim.x) any |= !((volatile Ctl *)B.ctls)[m].done;
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) {
+    if (!any) gctl->done = 1;
+    if (count_body) set_loop(gctl, cond, use_cond);
+  }
+}
+
+// x += alpha*p ; d -= alpha*q with the same partial slots as k_cg_update64
+// (L2 as there); a member's last block runs its closure test, the launch's
+// last block decides whether the batch goes on.  With a thread's eight rows
+// one at a time the loads' latency and the FP64 work took turns (61 us on 1.7
+// million rows).
+template <bool L2>
 __global__ void __launch_bounds__(kRedBlock) k_b_cg_update64(BatchDev B, double *__restrict__ x,
                                                              double *__restrict__ d,
                                                              const double *__restrict__ p,
                                                              const double *__restrict__ q,
-                                                             double *__restrict__ part) {
+                                                             double *part, Ctl *gctl,
+                                                             unsigned long long cond, int use_cond) {
   const ChunkRef c = chunk_of(B, blockIdx.x);
-  const Ctl &ctl = B.ctls[c.m];
-  if (ctl.done) return;
-  const double alpha = ctl.alpha;
-  double v[2] = {0.0, 0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  const int row0 = B.mr[c.m];  // member-local row numbers for the maxima
-  for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
-    double tv = alpha * p[i];
-    x[i] = x[i] + tv;
-    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i - row0; }
-    double di = fma(-alpha, q[i], d[i]);
-    d[i] = di;
-    if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i - row0; }
-    v[0] = fma(di, di, v[0]);
-    nf |= nonfinite(di) | nonfinite(tv);
-  }
-  v[1] = (double)nf;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
+  Ctl *ctl = B.ctls + c.m;
+  if (!ctl->done) {
+    const double alpha = ctl->alpha;
+    double v[1] = {0.0};
+    unsigned nf = 0;
+    MaxLoc m[2];
+    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+    const int row0 = B.mr[c.m];  // member-local row numbers for the maxima
+    constexpr int R = 4;
+#pragma unroll
+    for (int h = 0; h < kChunkTrips / R; ++h) {
+      double pr[R], xr[R], qr[R], dr[R];
+      const int i0 = c.r0 + threadIdx.x + h * R * kRedBlock;
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int i = i0 + t * kRedBlock;
+        if (i < c.r1) {
+          pr[t] = p[i];
+          xr[t] = x[i];
+          qr[t] = q[i];
+          dr[t] = d[i];
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int i = i0 + t * kRedBlock;
+        if (i < c.r1) {
+          const double tv = alpha * pr[t];
+          x[i] = xr[t] + tv;
+          if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i - row0; }
+          const double di = fma(-alpha, qr[t], dr[t]);
+          d[i] = di;
+          if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i - row0; }
+          if (L2) v[0] = fma(di, di, v[0]);
+          nf |= nonfinite(di) | nonfinite(tv);
+        }
+      }
+    }
     double *pm = member_part(part, B, c.m);
-    const int G = c.G, b = c.b;
-    pm[b] = v[0];
-    pm[G + b] = m[0].val; pm[2 * G + b] = (double)m[0].idx;
-    pm[3 * G + b] = m[1].val; pm[4 * G + b] = (double)m[1].idx;
-    pm[5 * G + b] = v[1];
+    update_partials<L2>(v[0], nf, m, pm, c.G, c.b);
+    if (last_block(&ctl->fin, c.G)) ctl_cg_cnvg<L2>(ctl, pm, c.G, 0ULL, 0);
   }
+  __syncthreads();
+  if (last_block(&gctl->fin, gridDim.x)) batch_all_done(B, gctl, cond, use_cond, 1);
 }
 
 __global__ void k_b_ctl_set_l2norm0(BatchDev B, const double *part) {
   const int m = blockIdx.x;
   ctl_set_l2norm0(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m]);
 }
-__global__ void k_b_ctl_cg_rho(BatchDev B, const double *part) {
+// The L2 norm of a member's final residual, for a loop that did not take it.
+__global__ void k_b_ctl_set_l2norm(BatchDev B, const double *part) {
   const int m = blockIdx.x;
-  ctl_cg_rho(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m]);
-}
-__global__ void k_b_ctl_alpha(BatchDev B, const double *part) {
-  const int m = blockIdx.x;
-  ctl_alpha(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m]);
-}
-__global__ void k_b_ctl_cg_cnvg(BatchDev B, const double *part) {
-  const int m = blockIdx.x;
-  ctl_cg_cnvg(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m], 0ULL, 0);
+  Ctl *ctl = B.ctls + m;
+  const double s = ctl_reduce_sum(part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m]);
+  if (threadIdx.x == 0 && ctl->l2norm0 != 0.0) ctl->l2norm = sqrt(s);
 }
 
-// The batch's own control block gets done = every member done; it gates the
-// shared kernels (SpMV, preconditioner) and drives the WHILE condition.
-__global__ void k_b_all_done(BatchDev B, Ctl *gctl, unsigned long long cond, int use_cond,
-                            int count_body) {
-  __shared__ int s_any;
-  if (threadIdx.x == 0) s_any = 0;
-  __syncthreads();
-  for (int m = threadIdx.x; m < B.nm; m += blockDim.x)
-    if (!B.ctls[m].done) atomicOr(&s_any, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (!s_any) gctl->done = 1;
-    if (count_body) set_loop(gctl, cond, use_cond);
-  }
-}
+__global__ void k_b_all_done(BatchDev B, Ctl *gctl) { batch_all_done(B, gctl, 0ULL, 0, 0); }
 
 // ---------------------------------------------------------------------------
 // Batched mixed form: the single solve's FP32 inner loop and FP64
 // refinement (k_dot32c, k_cg_pupdate32, k_cg_update_mixed,
 // ctl_mixed_inner, k_true_resid_stats, ctl_refine) per member.
 // ---------------------------------------------------------------------------
+template <int FIN>
 __global__ void __launch_bounds__(kRedBlock) k_b_dot32c(BatchDev B, const float *__restrict__ a,
-                                                         const float *__restrict__ b,
-                                                         double *__restrict__ part) {
+                                                         const float *__restrict__ b, double *part) {
   const ChunkRef c = chunk_of(B, blockIdx.x);
-  if (B.ctls[c.m].done) return;
+  Ctl *ctl = B.ctls + c.m;
+  if (ctl->done) return;
   CSum acc{0.f, 0.f};
   for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) csum_prod(acc, a[i], b[i]);
   double v[1] = {csum_value(acc)};
   block_sum<1>(v);
-  if (threadIdx.x == 0) member_part(part, B, c.m)[c.b] = v[0];
+  double *pm = member_part(part, B, c.m);
+  if (threadIdx.x == 0) pm[c.b] = v[0];
+  if (last_block(&ctl->fin, c.G)) finish_dot<FIN>(ctl, pm, c.G);
 }
 
 __global__ void __launch_bounds__(kRedBlock) k_b_cg_pupdate32(BatchDev B, const float *__restrict__ z,
@@ -1113,11 +960,11 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update_mixed(BatchDev B, dou
                                                                   float *__restrict__ d,
                                                                   const float *__restrict__ p,
                                                                   const float *__restrict__ q,
-                                                                  double *__restrict__ part) {
+                                                                  double *part, double refine_factor) {
   const ChunkRef c = chunk_of(B, blockIdx.x);
-  const Ctl &ctl = B.ctls[c.m];
-  if (ctl.done) return;
-  const float alphaf = (float)ctl.alpha;
+  Ctl *ctl = B.ctls + c.m;
+  if (ctl->done) return;
+  const float alphaf = (float)ctl->alpha;
   const int row0 = B.mr[c.m];  // member-local row numbers for the maxima
   CSum l2{0.f, 0.f};
   unsigned nf = 0, bdx = 0, brr = 0;
@@ -1135,25 +982,12 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update_mixed(BatchDev B, dou
     csum_prod(l2, di, di);
     nf |= nonfinite(di) | nonfinite(tv);
   }
-  double v[2] = {csum_value(l2), (double)nf};
   MaxLoc m[2];
   m[0].val = (double)vdx; m[0].idx = idx_dx;
   m[1].val = (double)vrr; m[1].idx = idx_rr;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
-    double *pm = member_part(part, B, c.m);
-    const int G = c.G, b = c.b;
-    pm[b] = v[0];
-    pm[G + b] = m[0].val; pm[2 * G + b] = (double)m[0].idx;
-    pm[3 * G + b] = m[1].val; pm[4 * G + b] = (double)m[1].idx;
-    pm[5 * G + b] = v[1];
-  }
-}
-
-__global__ void k_b_ctl_mixed_inner(BatchDev B, const double *part, double refine_factor) {
-  const int m = blockIdx.x;
-  ctl_mixed_inner(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m], 0, refine_factor);
+  double *pm = member_part(part, B, c.m);
+  update_partials<true>(csum_value(l2), nf, m, pm, c.G, c.b);
+  if (last_block(&ctl->fin, c.G)) ctl_mixed_inner(ctl, pm, c.G, 0, refine_factor);
 }
 
 // The batch's own block asks for the FP64 true residual when any member
@@ -1172,38 +1006,30 @@ __global__ void k_b_any_due(BatchDev B, Ctl *gctl) {
 __global__ void __launch_bounds__(kRedBlock) k_b_true_resid_stats(BatchDev B,
                                                                    const double *__restrict__ r,
                                                                    float *__restrict__ d32,
-                                                                   double *__restrict__ part) {
+                                                                   double *part, Ctl *gctl,
+                                                                   unsigned long long cond,
+                                                                   int use_cond) {
   const ChunkRef c = chunk_of(B, blockIdx.x);
-  const Ctl &ctl = B.ctls[c.m];
-  if (ctl.done || ctl.north_due != 2) return;
-  const int row0 = B.mr[c.m];
-  double v[2] = {0.0, 0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
-    const double ri = r[i];
-    d32[i] = (float)ri;
-    if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i - row0; }
-    v[0] = fma(ri, ri, v[0]);
-    nf |= nonfinite(ri);
-  }
-  v[1] = (double)nf;
-  block_sum<2>(v);
-  block_maxloc<2>(m);
-  if (threadIdx.x == 0) {
+  Ctl *ctl = B.ctls + c.m;
+  if (!ctl->done && ctl->north_due == 2) {
+    const int row0 = B.mr[c.m];
+    double v[1] = {0.0};
+    unsigned nf = 0;
+    MaxLoc m[2];
+    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+    for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
+      const double ri = r[i];
+      d32[i] = (float)ri;
+      if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i - row0; }
+      v[0] = fma(ri, ri, v[0]);
+      nf |= nonfinite(ri);
+    }
     double *pm = member_part(part, B, c.m);
-    const int G = c.G, b = c.b;
-    pm[b] = v[0];
-    pm[G + b] = 0.0; pm[2 * G + b] = -1.0;
-    pm[3 * G + b] = m[1].val; pm[4 * G + b] = (double)m[1].idx;
-    pm[5 * G + b] = v[1];
+    update_partials<true>(v[0], nf, m, pm, c.G, c.b);
+    if (last_block(&ctl->fin, c.G)) ctl_refine(ctl, pm, c.G, 0ULL, 0);
   }
-}
-
-__global__ void k_b_ctl_refine(BatchDev B, const double *part) {
-  const int m = blockIdx.x;
-  ctl_refine(B.ctls + m, part + 8LL * B.mc[m], B.mc[m + 1] - B.mc[m], 0ULL, 0);
+  __syncthreads();
+  if (last_block(&gctl->fin, gridDim.x)) batch_all_done(B, gctl, cond, use_cond, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1267,16 +1093,22 @@ void kr_residual_rows(int n, const int *ia, const int *ja, int base, const doubl
 }
 static inline int egrid(int n) { return std::max(1, (n + 255) / 256); }
 
-void kr_dot64(int n, const double *a, const double *b, double *part, int G, const Ctl *ctl, cudaStream_t st) {
-  k_dot<double, double><<<G, kRedBlock, 0, st>>>(n, a, b, part, ctl);
+void kr_dot64(int n, const double *a, const double *b, double *part, int G, Ctl *ctl, Fin fin, cudaStream_t st) {
+  auto *k = fin == kFinCgRho ? k_dot<double, double, kFinCgRho>
+            : fin == kFinAlpha ? k_dot<double, double, kFinAlpha>
+            : fin == kFinBcgsRho ? k_dot<double, double, kFinBcgsRho> : k_dot<double, double, kFinNone>;
+  k<<<G, kRedBlock, 0, st>>>(n, a, b, part, ctl);
 }
-void kr_dot_tq_tt64(int n, const double *t, const double *q, double *part, int G, const Ctl *ctl, cudaStream_t st) {
+void kr_dot_tq_tt64(int n, const double *t, const double *q, double *part, int G, Ctl *ctl, cudaStream_t st) {
   k_dot_tq_tt<double><<<G, kRedBlock, 0, st>>>(n, t, q, part, ctl);
 }
-void kr_dot32(int n, const float *a, const float *b, double *part, int G, const Ctl *ctl, cudaStream_t st) {
-  k_dot32c<<<G, kRedBlock, 0, st>>>(n, a, b, part, ctl);
+void kr_dot32(int n, const float *a, const float *b, double *part, int G, Ctl *ctl, Fin fin, cudaStream_t st) {
+  auto *k = fin == kFinCgRho ? k_dot32c<kFinCgRho>
+            : fin == kFinAlpha ? k_dot32c<kFinAlpha>
+            : fin == kFinBcgsRho ? k_dot32c<kFinBcgsRho> : k_dot32c<kFinNone>;
+  k<<<G, kRedBlock, 0, st>>>(n, a, b, part, ctl);
 }
-void kr_dot_tq_tt32(int n, const float *t, const float *q, double *part, int G, const Ctl *ctl, cudaStream_t st) {
+void kr_dot_tq_tt32(int n, const float *t, const float *q, double *part, int G, Ctl *ctl, cudaStream_t st) {
   k_dot_tq_tt32c<<<G, kRedBlock, 0, st>>>(n, t, q, part, ctl);
 }
 void kr_sumsq64(int n, const double *a, double *part, int G, cudaStream_t st) {
@@ -1288,19 +1120,15 @@ void kr_ctl_set_l2norm0(Ctl *ctl, const double *part, int G, cudaStream_t st) {
 void kr_ctl_set_l2norm(Ctl *ctl, const double *part, int G, cudaStream_t st) {
   k_ctl_set_l2norm<<<1, kRedBlock, 0, st>>>(ctl, part, G);
 }
-void kr_ctl_cg_rho(Ctl *ctl, const double *part, int G, cudaStream_t st) {
-  k_ctl_cg_rho<<<1, kRedBlock, 0, st>>>(ctl, part, G);
-}
-void kr_ctl_alpha(Ctl *ctl, const double *part, int G, cudaStream_t st) {
-  k_ctl_alpha<<<1, kRedBlock, 0, st>>>(ctl, part, G);
-}
 void kr_cg_pupdate64(int n, const double *z, double *p, const Ctl *ctl, cudaStream_t st) {
   k_cg_pupdate64<<<egrid(n), 256, 0, st>>>(n, z, p, ctl);
 }
-void kr_cg_update64(int n, double *x, double *d, const double *p, const double *q, double *part,
-                    int G, const Ctl *ctl, cudaStream_t st, bool l2) {
-  if (l2) k_cg_update64<true><<<G, kRedBlock, 0, st>>>(n, x, d, p, q, part, ctl);
-  else k_cg_update64<false><<<G, kRedBlock, 0, st>>>(n, x, d, p, q, part, ctl);
+void kr_cg_update64(int n, double *x, double *d, const double *p, const double *p1, const double *q,
+                    double *part, int G, Ctl *ctl, bool fin, unsigned long long cond, int use_cond,
+                    cudaStream_t st, bool l2) {
+  auto *k = l2 ? (fin ? k_cg_update64<true, true> : k_cg_update64<true, false>)
+               : (fin ? k_cg_update64<false, true> : k_cg_update64<false, false>);
+  k<<<G, kRedBlock, 0, st>>>(n, x, d, p, p1, q, part, ctl, cond, use_cond);
 }
 void kr_rec_models(bool bcgs, int nm, const int *modstart, const double *p, const double *q,
                    const double *d, const double *dscale, double *part, int G, const Ctl *ctl,
@@ -1311,16 +1139,15 @@ void kr_rec_models(bool bcgs, int nm, const int *modstart, const double *p, cons
 void kr_cg_pupdate32(int n, const float *z, float *p, const Ctl *ctl, cudaStream_t st) {
   k_cg_pupdate32<<<egrid(n), 256, 0, st>>>(n, z, p, ctl);
 }
-void kr_cg_update_mixed(int n, double *x, float *d, const float *p, const float *q, double *part,
-                        int G, const Ctl *ctl, cudaStream_t st) {
-  k_cg_update_mixed<<<G, kRedBlock, 0, st>>>(n, x, d, p, q, part, ctl);
+void kr_cg_update_mixed(int n, double *x, float *d, const float *p, const float *p1, const float *q,
+                        double *part, int G, Ctl *ctl, bool fin, double refine_factor, cudaStream_t st) {
+  auto *k = fin ? k_cg_update_mixed<true> : k_cg_update_mixed<false>;
+  k<<<G, kRedBlock, 0, st>>>(n, x, d, p, p1, q, part, ctl, refine_factor);
 }
 void kr_ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond, int use_cond,
-                    cudaStream_t st) {
-  k_ctl_cg_cnvg<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
-}
-void kr_ctl_bcgs_rho(Ctl *ctl, const double *part, int G, cudaStream_t st) {
-  k_ctl_bcgs_rho<<<1, kRedBlock, 0, st>>>(ctl, part, G);
+                    cudaStream_t st, bool l2) {
+  auto *k = l2 ? k_ctl_cg_cnvg<true> : k_ctl_cg_cnvg<false>;
+  k<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
 }
 void kr_bcgs_p64(int n, const double *d, double *p, const double *v, const Ctl *ctl, cudaStream_t st) {
   k_bcgs_p<double><<<egrid(n), 256, 0, st>>>(n, d, p, v, ctl);
@@ -1334,36 +1161,29 @@ void kr_bcgs_p32(int n, const float *d, float *p, const float *v, const Ctl *ctl
 void kr_bcgs_q32(int n, const float *d, const float *v, float *q, const Ctl *ctl, cudaStream_t st) {
   k_bcgs_q<float><<<egrid(n), 256, 0, st>>>(n, d, v, q, ctl);
 }
-void kr_ctl_omega(Ctl *ctl, const double *part, int G, cudaStream_t st) {
-  k_ctl_omega<<<1, kRedBlock, 0, st>>>(ctl, part, G);
-}
 void kr_bcgs_update64(int n, double *x, double *d, const double *phat, const double *qhat,
                       const double *q, const double *t, const double *dscale, double *part, int G,
-                      const Ctl *ctl, cudaStream_t st, bool l2) {
-  if (l2) k_bcgs_update<double, true><<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl);
-  else k_bcgs_update<double, false><<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl);
+                      Ctl *ctl, bool fin, unsigned long long cond, int use_cond, cudaStream_t st, bool l2) {
+  auto *k = l2 ? (fin ? k_bcgs_update<double, true, 1> : k_bcgs_update<double, true, 0>)
+               : (fin ? k_bcgs_update<double, false, 1> : k_bcgs_update<double, false, 0>);
+  k<<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl, cond, use_cond, 0.0);
 }
 void kr_bcgs_update32(int n, double *x, float *d, const float *phat, const float *qhat,
                       const float *q, const float *t, const double *dscale, double *part, int G,
-                      const Ctl *ctl, cudaStream_t st) {
-  k_bcgs_update<float, true><<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl);
+                      Ctl *ctl, double refine_factor, cudaStream_t st) {
+  k_bcgs_update<float, true, 2><<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl,
+                                                         0ULL, 0, refine_factor);
 }
 void kr_ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond, int use_cond,
-                      cudaStream_t st) {
-  k_ctl_bcgs_cnvg<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
-}
-void kr_ctl_mixed_inner(Ctl *ctl, const double *part, int G, int bcgs, double refine_factor,
-                        cudaStream_t st) {
-  k_ctl_mixed_inner<<<1, kRedBlock, 0, st>>>(ctl, part, G, bcgs, refine_factor);
+                      cudaStream_t st, bool l2) {
+  auto *k = l2 ? k_ctl_bcgs_cnvg<true> : k_ctl_bcgs_cnvg<false>;
+  k<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
 }
 void kr_true_resid_stats(int n, const double *r, float *d32, float *dhat32, double *dhat64,
-                         const double *dscale, double *part, int G, const Ctl *ctl,
-                         cudaStream_t st) {
-  k_true_resid_stats<<<G, kRedBlock, 0, st>>>(n, r, d32, dhat32, dhat64, dscale, part, ctl);
-}
-void kr_ctl_refine(Ctl *ctl, const double *part, int G, unsigned long long cond, int use_cond,
-                   cudaStream_t st) {
-  k_ctl_refine<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
+                         const double *dscale, double *part, int G, Ctl *ctl,
+                         unsigned long long cond, int use_cond, cudaStream_t st) {
+  k_true_resid_stats<<<G, kRedBlock, 0, st>>>(n, r, d32, dhat32, dhat64, dscale, part, ctl, cond,
+                                              use_cond);
 }
 void kr_f64_to_f32(int n, const double *s, float *d, cudaStream_t st) {
   k_convert<float, double><<<std::min(egrid(n), 4 * kNumSM), 256, 0, st>>>(n, s, d);
@@ -1374,8 +1194,9 @@ void kr_f32_to_f64(int n, const float *s, double *d, cudaStream_t st) {
 
 
 // batched ensemble launchers
-void kb_dot64(const BatchDev &B, const double *a, const double *b, double *part, cudaStream_t st) {
-  k_b_dot<double, double><<<B.nchunks, kRedBlock, 0, st>>>(B, a, b, part);
+void kb_dot64(const BatchDev &B, const double *a, const double *b, double *part, Fin fin, cudaStream_t st) {
+  auto *k = fin == kFinCgRho ? k_b_dot<kFinCgRho> : k_b_dot<kFinAlpha>;
+  k<<<B.nchunks, kRedBlock, 0, st>>>(B, a, b, part);
 }
 void kb_sumsq64(const BatchDev &B, const double *a, double *part, cudaStream_t st) {
   k_b_sumsq<<<B.nchunks, kRedBlock, 0, st>>>(B, a, part);
@@ -1384,48 +1205,37 @@ void kb_cg_pupdate64(const BatchDev &B, const double *z, double *p, cudaStream_t
   k_b_cg_pupdate<double><<<B.nchunks, kRedBlock, 0, st>>>(B, z, p);
 }
 void kb_cg_update64(const BatchDev &B, double *x, double *d, const double *p, const double *q,
-                    double *part, cudaStream_t st) {
-  k_b_cg_update64<<<B.nchunks, kRedBlock, 0, st>>>(B, x, d, p, q, part);
+                    double *part, Ctl *gctl, unsigned long long cond, int use_cond, cudaStream_t st,
+                    bool l2) {
+  auto *k = l2 ? k_b_cg_update64<true> : k_b_cg_update64<false>;
+  k<<<B.nchunks, kRedBlock, 0, st>>>(B, x, d, p, q, part, gctl, cond, use_cond);
 }
 void kb_ctl_set_l2norm0(const BatchDev &B, const double *part, cudaStream_t st) {
   k_b_ctl_set_l2norm0<<<B.nm, kRedBlock, 0, st>>>(B, part);
 }
-void kb_ctl_cg_rho(const BatchDev &B, const double *part, cudaStream_t st) {
-  k_b_ctl_cg_rho<<<B.nm, kRedBlock, 0, st>>>(B, part);
+void kb_ctl_set_l2norm(const BatchDev &B, const double *part, cudaStream_t st) {
+  k_b_ctl_set_l2norm<<<B.nm, kRedBlock, 0, st>>>(B, part);
 }
-void kb_ctl_alpha(const BatchDev &B, const double *part, cudaStream_t st) {
-  k_b_ctl_alpha<<<B.nm, kRedBlock, 0, st>>>(B, part);
+void kb_all_done(const BatchDev &B, Ctl *gctl, cudaStream_t st) {
+  k_b_all_done<<<1, kRedBlock, 0, st>>>(B, gctl);
 }
-void kb_ctl_cg_cnvg(const BatchDev &B, const double *part, cudaStream_t st) {
-  k_b_ctl_cg_cnvg<<<B.nm, kRedBlock, 0, st>>>(B, part);
-}
-void kb_all_done(const BatchDev &B, Ctl *gctl, unsigned long long cond, int use_cond,
-                 int count_body, cudaStream_t st) {
-  k_b_all_done<<<1, kRedBlock, 0, st>>>(B, gctl, cond, use_cond, count_body);
-}
-void kb_dot32(const BatchDev &B, const float *a, const float *b, double *part, cudaStream_t st) {
-  k_b_dot32c<<<B.nchunks, kRedBlock, 0, st>>>(B, a, b, part);
+void kb_dot32(const BatchDev &B, const float *a, const float *b, double *part, Fin fin, cudaStream_t st) {
+  auto *k = fin == kFinCgRho ? k_b_dot32c<kFinCgRho> : k_b_dot32c<kFinAlpha>;
+  k<<<B.nchunks, kRedBlock, 0, st>>>(B, a, b, part);
 }
 void kb_cg_pupdate32(const BatchDev &B, const float *z, float *p, cudaStream_t st) {
   k_b_cg_pupdate32<<<B.nchunks, kRedBlock, 0, st>>>(B, z, p);
 }
 void kb_cg_update_mixed(const BatchDev &B, double *x, float *d, const float *p, const float *q,
-                        double *part, cudaStream_t st) {
-  k_b_cg_update_mixed<<<B.nchunks, kRedBlock, 0, st>>>(B, x, d, p, q, part);
-}
-void kb_ctl_mixed_inner(const BatchDev &B, const double *part, double refine_factor,
-                        cudaStream_t st) {
-  k_b_ctl_mixed_inner<<<B.nm, kRedBlock, 0, st>>>(B, part, refine_factor);
+                        double *part, double refine_factor, cudaStream_t st) {
+  k_b_cg_update_mixed<<<B.nchunks, kRedBlock, 0, st>>>(B, x, d, p, q, part, refine_factor);
 }
 void kb_any_due(const BatchDev &B, Ctl *gctl, cudaStream_t st) {
   k_b_any_due<<<1, kRedBlock, 0, st>>>(B, gctl);
 }
-void kb_true_resid_stats(const BatchDev &B, const double *r, float *d32, double *part,
-                         cudaStream_t st) {
-  k_b_true_resid_stats<<<B.nchunks, kRedBlock, 0, st>>>(B, r, d32, part);
-}
-void kb_ctl_refine(const BatchDev &B, const double *part, cudaStream_t st) {
-  k_b_ctl_refine<<<B.nm, kRedBlock, 0, st>>>(B, part);
+void kb_true_resid_stats(const BatchDev &B, const double *r, float *d32, double *part, Ctl *gctl,
+                         unsigned long long cond, int use_cond, cudaStream_t st) {
+  k_b_true_resid_stats<<<B.nchunks, kRedBlock, 0, st>>>(B, r, d32, part, gctl, cond, use_cond);
 }
 
 }  // namespace gb

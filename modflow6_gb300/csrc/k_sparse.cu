@@ -8,6 +8,8 @@
 // (JA) order with fused multiply-adds, t = fma(a, x, t) from t = 0, the order
 // of amux with FMA contraction.
 #include "gbims_internal.cuh"
+#include "k_krylov.cuh"
+#include "k_reduce.cuh"
 
 namespace gb {
 
@@ -247,6 +249,185 @@ void launch_residual64(const Sell &S, const double *x, const double *b, double *
   k_sell_spmv<double, 1><<<rows_grid(S.n), 256, 0, st>>>(S.n, S.d_ptr, S.d_col, S.d_val, x, b,
                                                           d, ctl, only_if_north_due, S.d_slm,
                                                           S.d_mrow, S.nm, S.mctl);
+}
+
+// ---------------------------------------------------------------------------
+// Products fused with the Krylov steps around them (SpmvFin), for systems
+// where launches and the gaps between them are what an iteration costs: the
+// search direction's update, the product, its dot product and the scalar are
+// one kernel instead of four.  The direction is recomputed at each row's
+// neighbours, which doubles the product's FP64 instructions: on large systems,
+// where those bound it, the kernels stay apart.  One row a thread, 256 rows a
+// block: the rows, and so the partial sums, of k_dot's blocks.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double prod_sum(double a, double b) { return fma(a, b, 0.0); }
+__device__ __forceinline__ double prod_sum(float a, float b) {
+  CSum s{0.f, 0.f};
+  csum_prod(s, a, b);
+  return csum_value(s);
+}
+
+template <typename T>
+struct FinArgs {
+  const T *x, *w;
+  T *p0, *p1, *y;
+  double *part;
+  Ctl *ctl;
+};
+
+// The vector a product multiplies: x, or P of this iteration from z = x and
+// the last P.
+template <typename T, int OP>
+struct Operand {
+  const T *x, *old = nullptr;
+  T *now = nullptr;
+  T beta = T(0);
+  bool first = false;
+  __device__ __forceinline__ explicit Operand(const FinArgs<T> &a) : x(a.x) {
+    if (OP == 0) {
+      const bool odd = a.ctl->iter & 1;
+      now = odd ? a.p1 : a.p0;
+      old = odd ? a.p0 : a.p1;
+      beta = (T)a.ctl->beta;
+      first = a.ctl->first != 0;
+    }
+  }
+  struct Raw {
+    T a, b;
+  };
+  __device__ __forceinline__ void load(int i, Raw &r) const {
+    r.a = __ldg(x + i);
+    if (OP == 0 && !first) r.b = old[i];
+  }
+  __device__ __forceinline__ T value(const Raw &r) const {
+    if (OP == 0) return first ? r.a : mac<T>(beta, r.b, r.a);
+    return r.a;
+  }
+};
+
+// What a block does with its rows' products.
+template <typename T, int OP>
+__device__ __forceinline__ void finish_rows(const FinArgs<T> &a, int row, bool ok, T own, T t,
+                                            const Operand<T, OP> &x) {
+  constexpr int NV = OP == 2 ? 2 : 1;
+  double v[NV] = {};
+  if (ok) {
+    a.y[row] = t;
+    if (OP == 0) {
+      x.now[row] = own;
+      v[0] = prod_sum(own, t);
+    } else {
+      v[0] = OP == 1 ? prod_sum(a.w[row], t) : prod_sum(t, a.w[row]);
+      if (OP == 2) v[NV - 1] = prod_sum(t, t);
+    }
+  }
+  block_sum<NV>(v);
+  if (threadIdx.x == 0) {
+    a.part[blockIdx.x] = v[0];
+    if (OP == 2) a.part[gridDim.x + blockIdx.x] = v[NV - 1];
+  }
+  if (last_block(&a.ctl->fin, gridDim.x))
+    finish_dot<OP == 2 ? kFinOmega : kFinAlpha>(a.ctl, a.part, gridDim.x);
+}
+
+template <typename T, int OP>
+__global__ void __launch_bounds__(kRedBlock) k_dia7_spmv_fin(int nlay, int nrow, int ncol,
+                                                             const T *__restrict__ v, FinArgs<T> a) {
+  if (a.ctl->done) return;
+  const int nrc = nrow * ncol, n = nrc * nlay;
+  const int r = blockIdx.x * kRedBlock + threadIdx.x;
+  const Operand<T, OP> x(a);
+  T t = T(0), own = T(0);
+  if (r < n) {
+    const int k = r / nrc;
+    const int rem = r - k * nrc;
+    const int i = rem / ncol, j = rem - i * ncol;
+    const bool has[7] = {true, k > 0, i > 0, j > 0, j < ncol - 1, i < nrow - 1, k < nlay - 1};
+    const int off[7] = {0, -nrc, -ncol, -1, 1, ncol, nrc};
+    T vv[7];
+    typename Operand<T, OP>::Raw xx[7];
+#pragma unroll
+    for (int s = 0; s < 7; ++s)
+      if (has[s]) {
+        vv[s] = v[(size_t)s * n + r];
+        x.load(r + off[s], xx[s]);
+      }
+    own = x.value(xx[0]);
+    t = mac<T>(vv[0], own, t);
+#pragma unroll
+    for (int s = 1; s < 7; ++s)
+      if (has[s]) t = mac<T>(vv[s], x.value(xx[s]), t);
+  }
+  finish_rows<T, OP>(a, r, r < n, own, t, x);
+}
+
+template <typename T, int OP>
+__global__ void __launch_bounds__(kRedBlock) k_sell_spmv_fin(int n, const int *__restrict__ ptr,
+                                                             const int *__restrict__ col,
+                                                             const T *__restrict__ val, FinArgs<T> a) {
+  if (a.ctl->done) return;
+  const int r = blockIdx.x * kRedBlock + threadIdx.x;
+  const Operand<T, OP> x(a);
+  T t = T(0), own = T(0);
+  if (r < n) {
+    const int s = r / kSell, lane = r % kSell;
+    const int p0 = ptr[s], w = (ptr[s + 1] - p0) / kSell;
+    const int *c = col + p0 + lane;
+    const T *v = val + p0 + lane;
+    for (int b = 0; b < w; b += 8) {
+      int cc[8];
+      T vv[8];
+      typename Operand<T, OP>::Raw xx[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (b + k < w) {
+          cc[k] = c[(b + k) * kSell];
+          vv[k] = v[(b + k) * kSell];
+        }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (b + k < w) x.load(cc[k], xx[k]);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (b + k < w) {
+          const T xv = x.value(xx[k]);
+          if (b + k == 0) own = xv;  // the diagonal comes first
+          t = mac<T>(vv[k], xv, t);
+        }
+    }
+  }
+  finish_rows<T, OP>(a, r, r < n, own, t, x);
+}
+
+template <typename T, int OP>
+static void spmv_fin_t(const Dia7 *D, const Sell *S, const T *val, const SpmvFin &f, cudaStream_t st) {
+  FinArgs<T> a;
+  a.x = static_cast<const T *>(f.x);
+  a.w = static_cast<const T *>(f.w);
+  a.p0 = static_cast<T *>(f.p0);
+  a.p1 = static_cast<T *>(f.p1);
+  a.y = static_cast<T *>(f.y);
+  a.part = f.part;
+  a.ctl = f.ctl;
+  if (D)
+    k_dia7_spmv_fin<T, OP><<<rows_grid(D->nlay * D->nrow * D->ncol), kRedBlock, 0, st>>>(
+        D->nlay, D->nrow, D->ncol, val, a);
+  else
+    k_sell_spmv_fin<T, OP><<<rows_grid(S->n), kRedBlock, 0, st>>>(S->n, S->d_ptr, S->d_col, val, a);
+}
+
+void launch_spmv_fin(const Dia7 *D, const Sell *S, bool fp32, const SpmvFin &f, cudaStream_t st) {
+  if (!fp32) {
+    const double *val = D ? D->d_sv : S->d_val;
+    if (f.op == 0) spmv_fin_t<double, 0>(D, S, val, f, st);
+    else if (f.op == 1) spmv_fin_t<double, 1>(D, S, val, f, st);
+    else spmv_fin_t<double, 2>(D, S, val, f, st);
+  } else {
+    const float *val = D ? D->f_sv : S->d_val32;
+    if (f.op == 0) spmv_fin_t<float, 0>(D, S, val, f, st);
+    else if (f.op == 1) spmv_fin_t<float, 1>(D, S, val, f, st);
+    else spmv_fin_t<float, 2>(D, S, val, f, st);
+  }
 }
 
 }  // namespace gb
