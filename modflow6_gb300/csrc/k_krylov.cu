@@ -146,6 +146,41 @@ __global__ void __launch_bounds__(256) k_cg_pupdate32(int n, const float *__rest
   p[i] = ctl->first ? z[i] : fmaf((float)ctl->beta, p[i], z[i]);
 }
 
+// The element of largest magnitude a thread has seen, kept as its bits: for
+// finite doubles the order of the magnitudes' bit patterns is the order of the
+// magnitudes, Inf and NaN come above all of them.  Integer instructions and
+// selects only, in inline PTX: from the plain comparison the compiler made a
+// branch per row, behind which the rows' FP64 instructions waited for one
+// another (the update of 3.6 million rows took 68 us, without the maxima 35).
+struct MaxBits {
+  unsigned long long s = 0;
+  int i = -1;
+  __device__ __forceinline__ void take(double v, int row) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    asm("{\n .reg .pred p;\n .reg .b64 a, b;\n"
+        " and.b64 a, %2, 0x7fffffffffffffff;\n and.b64 b, %0, 0x7fffffffffffffff;\n"
+        " setp.gt.u64 p, a, b;\n selp.b64 %0, %2, %0, p;\n selp.b32 %1, %3, %1, p;\n}"
+        : "+l"(s), "+r"(i)
+        : "l"(u), "r"(row));
+  }
+  __device__ __forceinline__ MaxLoc loc() const { return MaxLoc{__longlong_as_double((long long)s), (long long)i}; }
+  __device__ __forceinline__ unsigned nonfinite() const { return ((unsigned)(s >> 32) & 0x7ff00000u) == 0x7ff00000u; }
+};
+
+struct MaxBits32 {
+  unsigned s = 0;
+  int i = -1;
+  __device__ __forceinline__ void take(float v, int row) {
+    asm("{\n .reg .pred p;\n .reg .b32 a, b;\n"
+        " and.b32 a, %2, 0x7fffffff;\n and.b32 b, %0, 0x7fffffff;\n"
+        " setp.gt.u32 p, a, b;\n selp.b32 %0, %2, %0, p;\n selp.b32 %1, %3, %1, p;\n}"
+        : "+r"(s), "+r"(i)
+        : "r"(__float_as_uint(v)), "r"(row));
+  }
+  __device__ __forceinline__ MaxLoc loc() const { return MaxLoc{(double)__uint_as_float(s), (long long)i}; }
+  __device__ __forceinline__ unsigned nonfinite() const { return (s & 0x7f800000u) == 0x7f800000u; }
+};
+
 // A block's share of an update into its partial slots: [0]=l2 (when taken),
 // [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite.
 template <bool L2>
@@ -468,19 +503,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update64(int n, double *__rest
   const double alpha = ctl->alpha;
   if (p1 && (ctl->iter & 1)) p = p1;
   double v[1] = {0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
-  auto row = [&](int i, double pi, double xi, double qi, double dI) {
-    double tv = alpha * pi;
-    x[i] = xi + tv;
-    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
-    double di = fma(-alpha, qi, dI);
-    d[i] = di;
-    if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i; }
-    if (L2) v[0] = fma(di, di, v[0]);
-    nf |= nonfinite(di) | nonfinite(tv);
-  };
+  MaxBits mx, mr;
   // four rows per trip, their 16 loads issued before any row is used (the
   // same order of rows per thread as one row per trip, so the same sums and
   // maxima): the loads of a trip cover the latency of the FP64 work of the
@@ -499,10 +522,30 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update64(int n, double *__rest
       dr[r] = __ldcs(d + j);
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) row(i + r * stride, pr[r], xr[r], qr[r], dr[r]);
+    for (int r = 0; r < R; ++r) {
+      const int j = i + r * stride;
+      pr[r] = alpha * pr[r];
+      x[j] = xr[r] + pr[r];
+      dr[r] = fma(-alpha, qr[r], dr[r]);
+      d[j] = dr[r];
+      if (L2) v[0] = fma(dr[r], dr[r], v[0]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      mx.take(pr[r], i + r * stride);
+      mr.take(dr[r], i + r * stride);
+    }
   }
-  for (; i < n; i += stride) row(i, p[i], x[i], q[i], d[i]);
-  update_partials<L2>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  for (; i < n; i += stride) {
+    const double tv = alpha * p[i], di = fma(-alpha, q[i], d[i]);
+    x[i] = x[i] + tv;
+    d[i] = di;
+    if (L2) v[0] = fma(di, di, v[0]);
+    mx.take(tv, i);
+    mr.take(di, i);
+  }
+  MaxLoc m[2] = {mx.loc(), mr.loc()};
+  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_cg_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
 }
 
@@ -522,38 +565,47 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update_mixed(int n, double *__
   const float alphaf = (float)ctl->alpha;
   if (p1 && (ctl->iter & 1)) p = p1;
   CSum l2{0.f, 0.f};
-  unsigned nf = 0;
-  unsigned bdx = 0, brr = 0;  // largest magnitudes so far (bit patterns)
-  float vdx = 0.f, vrr = 0.f;
-  int idx_dx = -1, idx_rr = -1;
-  auto row = [&](int i, float pi, double xi, float qi, float dI) {
-    const float tv = __fmul_rn(alphaf, pi);
-    x[i] = xi + (double)tv;
-    const unsigned at = __float_as_uint(tv) & 0x7fffffffu;
-    if (at > bdx) { bdx = at; vdx = tv; idx_dx = i; }
-    const float di = __fmaf_rn(-alphaf, qi, dI);
-    d[i] = di;
-    const unsigned ad = __float_as_uint(di) & 0x7fffffffu;
-    if (ad > brr) { brr = ad; vrr = di; idx_rr = i; }
-    csum_prod(l2, di, di);
-    nf |= nonfinite(di) | nonfinite(tv);
-  };
+  MaxBits32 mx, mr;
+  // four rows per trip, as in k_cg_update64
+  constexpr int R = 4;
   const int stride = gridDim.x * blockDim.x;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (; i + stride < n; i += 2 * stride) {
-    const int j = i + stride;
-    const float p0 = p[i], q0 = q[i], d0 = d[i];
-    const double x0 = x[i];
-    const float p1 = p[j], q1 = q[j], d1 = d[j];
-    const double x1 = x[j];
-    row(i, p0, x0, q0, d0);
-    row(j, p1, x1, q1, d1);
+  for (; i + (R - 1) * stride < n; i += R * stride) {
+    float pr[R], qr[R], dr[R];
+    double xr[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = i + r * stride;
+      pr[r] = p[j];
+      xr[r] = x[j];
+      qr[r] = q[j];
+      dr[r] = d[j];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int j = i + r * stride;
+      pr[r] = __fmul_rn(alphaf, pr[r]);
+      x[j] = xr[r] + (double)pr[r];
+      dr[r] = __fmaf_rn(-alphaf, qr[r], dr[r]);
+      d[j] = dr[r];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      mx.take(pr[r], i + r * stride);
+      mr.take(dr[r], i + r * stride);
+      csum_prod(l2, dr[r], dr[r]);
+    }
   }
-  if (i < n) row(i, p[i], x[i], q[i], d[i]);
-  MaxLoc m[2];
-  m[0].val = (double)vdx; m[0].idx = idx_dx;
-  m[1].val = (double)vrr; m[1].idx = idx_rr;
-  update_partials<true>(csum_value(l2), nf, m, part, gridDim.x, blockIdx.x);
+  for (; i < n; i += stride) {
+    const float tv = __fmul_rn(alphaf, p[i]), di = __fmaf_rn(-alphaf, q[i], d[i]);
+    x[i] = x[i] + (double)tv;
+    d[i] = di;
+    mx.take(tv, i);
+    mr.take(di, i);
+    csum_prod(l2, di, di);
+  }
+  MaxLoc m[2] = {mx.loc(), mr.loc()};
+  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_mixed_inner(ctl, part, gridDim.x, 0, refine_factor);
 }
 
@@ -653,23 +705,21 @@ __global__ void __launch_bounds__(kRedBlock) k_bcgs_update(int n, double *__rest
   const double alpha = ctl->alpha, omega = ctl->omega;
   const T omegat = (T)omega;
   double v[1] = {0.0};
-  unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  MaxBits mx, mr;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double tv = fma(alpha, to_d(phat[i]), omega * to_d(qhat[i]));
     x[i] = x[i] + tv;
     if (dscale) tv = tv * dscale[i];
-    if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i; }
+    mx.take(tv, i);
     T di = fma(-omegat, t[i], q[i]);
     d[i] = di;
     double rv = to_d(di);
     if (dscale) rv = rv / dscale[i];
-    if (absgt(rv, m[1].val)) { m[1].val = rv; m[1].idx = i; }
+    mr.take(rv, i);
     if (L2) v[0] = fma(rv, rv, v[0]);
-    nf |= nonfinite(rv) | nonfinite(tv);
   }
-  update_partials<L2>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  MaxLoc m[2] = {mx.loc(), mr.loc()};
+  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) {
     if (FIN == 1) ctl_bcgs_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
     else ctl_mixed_inner(ctl, part, gridDim.x, 1, refine_factor);
@@ -870,9 +920,7 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update64(BatchDev B, double 
   if (!ctl->done) {
     const double alpha = ctl->alpha;
     double v[1] = {0.0};
-    unsigned nf = 0;
-    MaxLoc m[2];
-    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+    MaxBits mx, mr;
     const int row0 = B.mr[c.m];  // member-local row numbers for the maxima
     constexpr int R = 4;
 #pragma unroll
@@ -893,19 +941,25 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update64(BatchDev B, double 
       for (int t = 0; t < R; ++t) {
         const int i = i0 + t * kRedBlock;
         if (i < c.r1) {
-          const double tv = alpha * pr[t];
-          x[i] = xr[t] + tv;
-          if (absgt(tv, m[0].val)) { m[0].val = tv; m[0].idx = i - row0; }
-          const double di = fma(-alpha, qr[t], dr[t]);
-          d[i] = di;
-          if (absgt(di, m[1].val)) { m[1].val = di; m[1].idx = i - row0; }
-          if (L2) v[0] = fma(di, di, v[0]);
-          nf |= nonfinite(di) | nonfinite(tv);
+          pr[t] = alpha * pr[t];
+          x[i] = xr[t] + pr[t];
+          dr[t] = fma(-alpha, qr[t], dr[t]);
+          d[i] = dr[t];
+          if (L2) v[0] = fma(dr[t], dr[t], v[0]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int i = i0 + t * kRedBlock;
+        if (i < c.r1) {
+          mx.take(pr[t], i - row0);
+          mr.take(dr[t], i - row0);
         }
       }
     }
+    MaxLoc m[2] = {mx.loc(), mr.loc()};
     double *pm = member_part(part, B, c.m);
-    update_partials<L2>(v[0], nf, m, pm, c.G, c.b);
+    update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, pm, c.G, c.b);
     if (last_block(&ctl->fin, c.G)) ctl_cg_cnvg<L2>(ctl, pm, c.G, 0ULL, 0);
   }
   __syncthreads();
@@ -967,26 +1021,18 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update_mixed(BatchDev B, dou
   const float alphaf = (float)ctl->alpha;
   const int row0 = B.mr[c.m];  // member-local row numbers for the maxima
   CSum l2{0.f, 0.f};
-  unsigned nf = 0, bdx = 0, brr = 0;
-  float vdx = 0.f, vrr = 0.f;
-  int idx_dx = -1, idx_rr = -1;
+  MaxBits32 mx, mr;
   for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
-    const float tv = __fmul_rn(alphaf, p[i]);
+    const float tv = __fmul_rn(alphaf, p[i]), di = __fmaf_rn(-alphaf, q[i], d[i]);
     x[i] = x[i] + (double)tv;
-    const unsigned at = __float_as_uint(tv) & 0x7fffffffu;
-    if (at > bdx) { bdx = at; vdx = tv; idx_dx = i - row0; }
-    const float di = __fmaf_rn(-alphaf, q[i], d[i]);
     d[i] = di;
-    const unsigned ad = __float_as_uint(di) & 0x7fffffffu;
-    if (ad > brr) { brr = ad; vrr = di; idx_rr = i - row0; }
+    mx.take(tv, i - row0);
+    mr.take(di, i - row0);
     csum_prod(l2, di, di);
-    nf |= nonfinite(di) | nonfinite(tv);
   }
-  MaxLoc m[2];
-  m[0].val = (double)vdx; m[0].idx = idx_dx;
-  m[1].val = (double)vrr; m[1].idx = idx_rr;
+  MaxLoc m[2] = {mx.loc(), mr.loc()};
   double *pm = member_part(part, B, c.m);
-  update_partials<true>(csum_value(l2), nf, m, pm, c.G, c.b);
+  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), m, pm, c.G, c.b);
   if (last_block(&ctl->fin, c.G)) ctl_mixed_inner(ctl, pm, c.G, 0, refine_factor);
 }
 
@@ -1123,11 +1169,16 @@ void kr_ctl_set_l2norm(Ctl *ctl, const double *part, int G, cudaStream_t st) {
 void kr_cg_pupdate64(int n, const double *z, double *p, const Ctl *ctl, cudaStream_t st) {
   k_cg_pupdate64<<<egrid(n), 256, 0, st>>>(n, z, p, ctl);
 }
+// Blocks of an update that only takes maxima, which come out the same from any
+// grid: what is resident at once.
+constexpr int kUpdateBlocks = 4 * kNumSM;
+
 void kr_cg_update64(int n, double *x, double *d, const double *p, const double *p1, const double *q,
                     double *part, int G, Ctl *ctl, bool fin, unsigned long long cond, int use_cond,
                     cudaStream_t st, bool l2) {
   auto *k = l2 ? (fin ? k_cg_update64<true, true> : k_cg_update64<true, false>)
                : (fin ? k_cg_update64<false, true> : k_cg_update64<false, false>);
+  if (!l2) G = std::min(G, kUpdateBlocks);
   k<<<G, kRedBlock, 0, st>>>(n, x, d, p, p1, q, part, ctl, cond, use_cond);
 }
 void kr_rec_models(bool bcgs, int nm, const int *modstart, const double *p, const double *q,
@@ -1146,6 +1197,7 @@ void kr_cg_update_mixed(int n, double *x, float *d, const float *p, const float 
 }
 void kr_ctl_cg_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond, int use_cond,
                     cudaStream_t st, bool l2) {
+  if (!l2) G = std::min(G, kUpdateBlocks);
   auto *k = l2 ? k_ctl_cg_cnvg<true> : k_ctl_cg_cnvg<false>;
   k<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
 }
@@ -1166,6 +1218,7 @@ void kr_bcgs_update64(int n, double *x, double *d, const double *phat, const dou
                       Ctl *ctl, bool fin, unsigned long long cond, int use_cond, cudaStream_t st, bool l2) {
   auto *k = l2 ? (fin ? k_bcgs_update<double, true, 1> : k_bcgs_update<double, true, 0>)
                : (fin ? k_bcgs_update<double, false, 1> : k_bcgs_update<double, false, 0>);
+  if (!l2) G = std::min(G, kUpdateBlocks);
   k<<<G, kRedBlock, 0, st>>>(n, x, d, phat, qhat, q, t, dscale, part, ctl, cond, use_cond, 0.0);
 }
 void kr_bcgs_update32(int n, double *x, float *d, const float *phat, const float *qhat,
@@ -1176,6 +1229,7 @@ void kr_bcgs_update32(int n, double *x, float *d, const float *phat, const float
 }
 void kr_ctl_bcgs_cnvg(Ctl *ctl, const double *part, int G, unsigned long long cond, int use_cond,
                       cudaStream_t st, bool l2) {
+  if (!l2) G = std::min(G, kUpdateBlocks);
   auto *k = l2 ? k_ctl_bcgs_cnvg<true> : k_ctl_bcgs_cnvg<false>;
   k<<<1, kRedBlock, 0, st>>>(ctl, part, G, cond, use_cond);
 }

@@ -16,15 +16,25 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// The entry of largest magnitude of a warp, the smallest row among equals (as
+// maxloc_merge; {0, -1} when all are zero), in every lane.  Three integer
+// warp reductions and a shuffle: merging pairs over five shuffle steps took
+// some 400 instructions a warp, a good part of an update kernel on the sizes
+// where a thread has one or two rows.
 __device__ __forceinline__ MaxLoc warp_maxloc(MaxLoc m) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    MaxLoc b;
-    b.val = __shfl_xor_sync(0xffffffffu, m.val, o);
-    b.idx = __shfl_xor_sync(0xffffffffu, m.idx, o);
-    maxloc_merge(m, b);
-  }
-  return m;
+  const unsigned all = 0xffffffffu;
+  const unsigned hi = (unsigned)__double2hiint(m.val) & 0x7fffffffu, lo = (unsigned)__double2loint(m.val);
+  const unsigned mh = __reduce_max_sync(all, hi);
+  const unsigned ml = __reduce_max_sync(all, hi == mh ? lo : 0u);
+  const bool best = hi == mh && lo == ml && (mh | ml) != 0u;
+  const unsigned row = best ? (unsigned)m.idx : all;
+  const unsigned mr = __reduce_min_sync(all, row);
+  const unsigned who = __ballot_sync(all, best && row == mr);
+  const int sh = __shfl_sync(all, __double2hiint(m.val), who ? __ffs((int)who) - 1 : 0);
+  MaxLoc r;
+  r.val = who ? __hiloint2double(sh, (int)ml) : 0.0;
+  r.idx = mr == all ? -1 : (long long)mr;
+  return r;
 }
 
 // Sum NV values over the block; thread 0 gets the results (fixed order).
