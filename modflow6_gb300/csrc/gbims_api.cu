@@ -30,6 +30,7 @@ struct gbims_handle {
   float *d_apc32 = nullptr;
   Sell S;
   Levels F, B;
+  FactorWords FW;
   Dia7 D;
   bool structured = false;  // wavefront sweeps (one or more full DIS grids)
   bool dia_spmv = false;    // index-free SpMV (a single full DIS grid)
@@ -686,7 +687,14 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     if (h->mixed) GB_CUDA(h, dalloc(&h->S.d_val32, col.size()));
   }
   // level schedule of the factorisation
-  if (h->ipc < 3) levels_build_host(neq, h->iapc, h->japc, true, h->F);
+  if (h->ipc < 3) {
+    levels_build_host(neq, h->iapc, h->japc, true, h->F);
+    h->FW.short_rows = ilu_short_rows(neq, h->iapc, h->japc);
+    h->FW.count = (size_t)nja;
+    GB_CUDA(h, cudaMalloc(&h->FW.words, 16 * h->FW.count));
+    GB_CUDA(h, cudaMemset(h->FW.words, 0, 16 * h->FW.count));
+    GB_CUDA(h, cudaMalloc((void **)&h->FW.claim, sizeof(int)));
+  }
   // vectors (with slack after the last cell for the sweeps' aligned copies)
   size_t nn = (size_t)neq + kVecPad;
   GB_CUDA(h, dalloc(&h->d_amat, nja));
@@ -910,12 +918,14 @@ static int factor_core(gbims_handle *h) {
     init.pivot_fail = INT_MAX;
     *h->h_ctl = init;
     GB_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, st));
-    launch_ilu_factor(n, h->d_ia, h->d_ja, h->d_amat, h->d_iapc, h->d_japc, h->d_apc, h->F,
-                      h->s.relax, delta, ipcflag, h->d_ctl, st);
-    h->launches += h->F.nlev;
+    if (launch_ilu_factor(n, h->d_ia, h->d_ja, h->d_amat, h->d_iapc, h->d_japc, h->d_apc, h->F,
+                          h->FW, h->s.relax, delta, ipcflag, h->d_ctl, st) != 0)
+      return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation launch failed");
+    h->launches += 1;
     GB_CUDA(h, cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     GB_CUDA(h, cudaStreamSynchronize(st));
     GB_CUDA(h, cudaGetLastError());
+    if (h->h_ctl->scratch_err) return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation wait limit reached");
     ipcflag = (h->h_ctl->pivot_fail != INT_MAX) ? 1 : 0;
     if (ipcflag < 1) break;
     delta = 1.5 * delta + 1.0e-3;
@@ -1575,7 +1585,8 @@ extern "C" int gbims_destroy(gbims_handle *h) {
   if (h->exec) cudaGraphExecDestroy(h->exec);
   if (h->graph) cudaGraphDestroy(h->graph);
   void *ptrs[] = {h->d_ia, h->d_ja, h->d_iapc, h->d_japc, h->d_apc, h->d_apc32, h->S.d_ptr,
-                  h->S.d_col, h->S.d_src, h->S.d_val, h->S.d_val32, h->F.d_rows, h->B.d_rows,
+                  h->S.d_col, h->S.d_src, h->S.d_val, h->S.d_val32, h->F.d_rows, h->B.d_rows, h->F.d_slices,
+                  h->B.d_slices, h->FW.words, h->FW.claim,
                   h->D.d_lz, h->D.d_ly, h->D.d_lx, h->D.d_ux, h->D.d_uy, h->D.d_uz, h->D.d_dinv,
                   h->D.f_lz, h->D.f_ly, h->D.f_lx, h->D.f_ux, h->D.f_uy, h->D.f_uz, h->D.f_dinv,
                   h->D.ll_y, h->D.ll_z,

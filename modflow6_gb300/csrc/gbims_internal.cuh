@@ -47,6 +47,7 @@ struct Ctl {
   int guard_tripped;  // the body limit ended the loop
   int restart_due;    // mixed form: the pending true-residual check restarts the recurrence
   unsigned fin;       // blocks of the current reduction kernel that have finished
+  int scratch_err;    // factorisation: a wait ran out
   // Per-inner-iteration records (gbims_set_inner_records; rec == nullptr:
   // off).  Row r of rec (stride 3 + 4*rec_nmod): iteration, alpha, omega,
   // then per model dvmax, locdv, rmax, locr.  rec_part holds the per-model
@@ -122,7 +123,23 @@ struct Levels {
   std::vector<int> ptr;   // nlev+1
   int *d_rows = nullptr;  // n
   int maxwidth = 0;
+  // the factorisation's slices: position in rows and count, up to 32 rows of
+  // one level each
+  int2 *d_slices = nullptr;
+  int nslices = 0;
 };
+
+// The ILU0 factorisation's result words (one per APC position, 16 bytes,
+// zeroed once), their epoch, and the counter its warps claim slices from.
+struct FactorWords {
+  void *words = nullptr;
+  size_t count = 0;
+  int *claim = nullptr;
+  unsigned epoch = 0;
+  bool short_rows = false;
+};
+// Warps per 32 rows of the widest level (see launch_ilu_factor).
+constexpr int kFactorAhead = 4;
 
 // The sweeps of general patterns: mode 0 launches one kernel per level; mode 1
 // runs each sweep as one launch over row ranges (k_range.cu), which hand
@@ -275,10 +292,11 @@ void rcm_order(int n, const std::vector<int> &ia, const std::vector<int> &ja,
 // the Yale minimum-degree ordering; returns odrv's flag (0 on success).
 int md_order(int n, const std::vector<int> &ia, const std::vector<int> &ja,
              std::vector<int> &lorder);
-void launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_amat,
-                       const int *d_iapc, const int *d_japc, double *d_apc,
-                       const Levels &L, double relax, double delta, int ipcflag,
-                       Ctl *ctl, cudaStream_t st);
+bool ilu_short_rows(int n, const std::vector<int> &iapc, const std::vector<int> &japc);
+int launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_amat,
+                      const int *d_iapc, const int *d_japc, double *d_apc, const Levels &L,
+                      FactorWords &W, double relax, double delta, int ipcflag, Ctl *ctl,
+                      cudaStream_t st);
 void launch_ilut_factor(const IlutDev &I, const int *d_ia, const int *d_ja, const double *d_amat,
                         double droptol, double relax, double delta, int izero, cudaStream_t st);
 void launch_ilut_scatter(const IlutDev &I, const int *d_iapc, const int *d_japc, double *d_apc,

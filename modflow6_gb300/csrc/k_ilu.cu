@@ -1,17 +1,17 @@
 // k_ilu.cu -- ILU0 / MILU0 factorisation and level-scheduled triangular sweeps.
 //
 // Factorisation: ims_base_pcilu0 (src/Solution/LinearMethods/ImsLinearBase.f90:928-1042)
-// restated per row, one thread per row, rows of one dependency level in one
-// launch.  The row's work vector W lives in registers, indexed by the row's
-// sorted pattern (IAPC/JAPC from ims_base_pccrs); every update to a W slot and
-// to the dropped-fill sum rs happens in the reference's order, and every
-// operation is rounded separately (no FMA), so APC is bit-for-bit the
-// reference's.
+// restated per row, one thread per row, in one launch (see k_ilu0_factor).
+// The row's work vector W is indexed by the row's sorted pattern (IAPC/JAPC
+// from ims_base_pccrs); every update to a W slot and to the dropped-fill sum
+// rs happens in the reference's order, and every operation is rounded
+// separately (no FMA), so APC is bit-for-bit the reference's.
 //
 // Apply: ims_base_ilu0a (:1049-1092).  Forward sweep D = R - L*D (unit lower),
 // backward sweep D = (D - U*D) * APC(n).  Rows of a level are independent; one
 // launch per level.  Entries are summed in JAPC order with FMA.
 #include "gbims_internal.cuh"
+#include "k_llword.cuh"
 #include <algorithm>
 #include <climits>
 
@@ -44,11 +44,21 @@ void levels_build_host(int n, const std::vector<int> &iapc, const std::vector<in
   for (int r = 0; r < n; ++r) rows[fill[lev[r]]++] = r;
   L.maxwidth = 0;
   for (int l = 0; l < nlev; ++l) L.maxwidth = std::max(L.maxwidth, L.ptr[l + 1] - L.ptr[l]);
+  // slices: up to 32 rows of one level
+  std::vector<int2> sl;
+  for (int l = 0; l < nlev; ++l)
+    for (int q = L.ptr[l]; q < L.ptr[l + 1]; q += 32)
+      sl.push_back(make_int2(q, std::min(32, L.ptr[l + 1] - q)));
+  L.nslices = (int)sl.size();
   if (L.d_rows) cudaFree(L.d_rows);
+  if (L.d_slices) cudaFree(L.d_slices);
   L.d_rows = nullptr;
+  L.d_slices = nullptr;
   if (n > 0) {
     cudaMalloc(&L.d_rows, sizeof(int) * n);
     cudaMemcpy(L.d_rows, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    cudaMalloc(&L.d_slices, sizeof(int2) * sl.size());
+    cudaMemcpy(L.d_slices, sl.data(), sizeof(int2) * sl.size(), cudaMemcpyHostToDevice);
   }
 }
 
@@ -65,87 +75,276 @@ __device__ __forceinline__ int find_sorted(const int *__restrict__ japc, int i0,
   return -1;
 }
 
-__global__ void k_ilu0_factor_level(const int *__restrict__ rows, int nrows,
-                                    const int *__restrict__ ia, const int *__restrict__ ja,
-                                    const double *__restrict__ amat,
-                                    const int *__restrict__ iapc,
-                                    const int *__restrict__ japc, double *apc,
-                                    double relax, double delta, int ipcflag, Ctl *ctl) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nrows) return;
-  if (ctl->pivot_fail != INT_MAX) return;  // a lower row failed: the attempt is void
-  int n = rows[t];
-  int ic0 = iapc[n], ic1 = iapc[n + 1], iu = japc[n];
-  int len = ic1 - ic0;
-  // w[0..len) : off-diagonal slots in JAPC order; wd : the diagonal slot
-  double w[kMaxRowLen];
-#pragma unroll 8
-  for (int k = 0; k < kMaxRowLen; ++k)
-    if (k < len) w[k] = 0.0;
-  double wd = 0.0;
-  // W(jcol) = W(jcol) + AMAT(j) over the CSR row (ImsLinearBase.f90:985-989)
-  for (int j = ia[n]; j < ia[n + 1]; ++j) {
-    int c = ja[j];
-    if (c == n) {
-      wd = __dadd_rn(wd, amat[j]);
-    } else {
-      int k = find_sorted(japc, ic0, ic1, c);
-      if (k >= 0) w[k] = __dadd_rn(w[k], amat[j]);
-    }
-  }
-  double rs = 0.0;
-  // LOWER loop (:993-1007)
-  for (int j = ic0; j < iu; ++j) {
-    int jcol = japc[j];
-    int kj = j - ic0;
-    int iic1 = iapc[jcol + 1];
-    int iiu = japc[jcol];
-    double tl = __dmul_rn(w[kj], apc[jcol]);
-    w[kj] = tl;
-    for (int jj = iiu; jj < iic1; ++jj) {
-      int jjcol = japc[jj];
-      double prod = __dmul_rn(tl, apc[jj]);
-      if (jjcol == n) {
-        wd = __dsub_rn(wd, prod);
-      } else {
-        int k = find_sorted(japc, ic0, ic1, jjcol);
-        if (k >= 0) w[k] = __dsub_rn(w[k], prod);
-        else rs = __dadd_rn(rs, prod);
-      }
-    }
-  }
-  // DIAGONAL (:1010-1037)
-  double d = wd;
-  double tl = __dsub_rn(__dmul_rn(__dadd_rn(1.0, delta), d), __dmul_rn(relax, rs));
-  double sd1 = copysign(fabs(d), tl);
-  if (sd1 != d) {
-    if (ipcflag > 1) tl = copysign(1.0e-6, d);
-    else {
-      atomicMin(&ctl->pivot_fail, n);
-      return;
-    }
-  }
-  if (fabs(tl) == 0.0) {
-    if (ipcflag > 1) tl = copysign(1.0e-6, d);
-    else {
-      atomicMin(&ctl->pivot_fail, n);
-      return;
-    }
-  }
-  apc[n] = __drcp_rn(tl);
-  for (int k = 0; k < len; ++k) apc[ic0 + k] = w[k];
+// Where an elimination product goes: an off-diagonal slot of the row (its
+// position), the diagonal, or the dropped-fill sum.
+constexpr int kToDiag = 14, kDropped = 15;
+constexpr int kShort = 6;  // lower and upper entries of a row of the short form (a target fits 4 bits)
+
+// A product whose exponents are so large that it, or a sum of a row's
+// products, could overflow.
+__device__ __forceinline__ bool may_overflow(double a, double b) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+  return ea == 0x7ff || eb == 0x7ff || ea + eb - 1023 > 2000;
 }
 
-void launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_amat,
-                       const int *d_iapc, const int *d_japc, double *d_apc, const Levels &L,
-                       double relax, double delta, int ipcflag, Ctl *ctl, cudaStream_t st) {
-  for (int l = 0; l < L.nlev; ++l) {
-    int nr = L.ptr[l + 1] - L.ptr[l];
-    k_ilu0_factor_level<<<(nr + 127) / 128, 128, 0, st>>>(L.d_rows + L.ptr[l], nr, d_ia, d_ja,
-                                                          d_amat, d_iapc, d_japc, d_apc, relax,
-                                                          delta, ipcflag, ctl);
+// The whole factorisation in one launch.  Bound by its chain: a level hands
+// its inverse pivots and upper entries to the next through L2 (0.7 us) and a
+// row has about 25 dependent FP64 instructions of 64 cycles.  A launch per
+// level added a launch, its ten dependent index loads and the gap between
+// kernels to each: a factorisation of 1 x 100 x 100 cells (199 levels) took 2.1
+// ms and takes 0.55, of 10 x 200 x 200 (408) 8.5 and 2.0, of 10 x 400 x 400
+// (808) 18.4 and 4.1.
+//
+// Warps claim slices (up to 32 rows of one level) in level order.  A warp
+// waits for the row a lane eliminates next by polling the words that row's
+// owner writes: its inverse pivot and upper entries, each tagged with the
+// epoch of the launch (k_llword.cuh), so that no fence stands between them.
+// All lanes of a warp take their e-th lower entry together: an FP64
+// instruction costs the same for one lane as for 32.  Slices are claimed in
+// order, so the lowest unfinished one can always proceed, however many warps
+// are resident; every wait is bounded, and ends when a pivot has failed (the
+// attempt is void and retried).
+//
+// SHORT: rows of at most kShort lower and upper entries; their index work is
+// done before the waits.  MILU: the dropped-fill sum is needed (relax > 0);
+// without it only products that might overflow are summed, because then
+// 0 * rs is not zero.
+template <bool SHORT, bool MILU>
+__global__ void __launch_bounds__(128) k_ilu0_factor(
+    int nslices, const int2 *__restrict__ slices, const int *__restrict__ rows,
+    const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ amat,
+    const int *__restrict__ iapc, const int *__restrict__ japc, double *apc,
+    LLWord<double> *words, unsigned ep, int *claim, double relax, double delta, int ipcflag, Ctl *ctl) {
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  volatile int *failed = &ctl->pivot_fail;
+  // false when a wait runs out or the attempt is void
+  auto keep_waiting = [&](unsigned &turns) -> bool {
+    if ((++turns & 63u) != 0) return true;
+    if (turns > (1u << 23)) {  // L2 round trips: seconds
+      if (lane == 0) atomicExch(&ctl->scratch_err, 1);
+      return false;
+    }
+    return __all_sync(all, *failed == INT_MAX && *(volatile int *)&ctl->scratch_err == 0);
+  };
+  while (true) {
+    int s = 0;
+    if (lane == 0) s = atomicAdd(claim, 1);
+    s = __shfl_sync(all, s, 0);
+    if (s >= nslices) return;
+    if (!__all_sync(all, *failed == INT_MAX)) return;  // a row failed: the attempt is void
+    const int2 sl = slices[s];
+    const bool mine = lane < sl.y;
+    const int n = rows[sl.x + min(lane, sl.y - 1)];
+    const int ic0 = iapc[n], ic1 = iapc[n + 1], iu = japc[n];
+    const int len = ic1 - ic0, nlow = iu - ic0;
+    // w[0..len): off-diagonal slots in JAPC order; wd: the diagonal slot
+    double w[SHORT ? 2 * kShort : kMaxRowLen];
+    if (!SHORT) {
+#pragma unroll 8
+      for (int k = 0; k < kMaxRowLen; ++k)
+        if (k < len) w[k] = 0.0;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 2 * kShort; ++k) w[k] = 0.0;
+    }
+    double wd = 0.0;
+    // W(jcol) = W(jcol) + AMAT(j) over the CSR row (ImsLinearBase.f90:985-989)
+    for (int j = ia[n]; j < ia[n + 1]; ++j) {
+      const int c = ja[j];
+      if (c == n) {
+        wd = __dadd_rn(wd, amat[j]);
+      } else {
+        const int k = find_sorted(japc, ic0, ic1, c);
+        if (k >= 0) w[k] = __dadd_rn(w[k], amat[j]);
+      }
+    }
+    // the index work of a short row: per lower entry its row, where that
+    // row's upper entries start, how many there are, and their targets
+    int col[kShort], u0[kShort], nu[kShort];
+    unsigned tgt[kShort];
+    if (SHORT) {
+#pragma unroll
+      for (int e = 0; e < kShort; ++e) {
+        col[e] = u0[e] = nu[e] = 0;
+        tgt[e] = 0;
+        if (e < nlow) {
+          col[e] = japc[ic0 + e];
+          u0[e] = japc[col[e]];
+          nu[e] = iapc[col[e] + 1] - u0[e];
+#pragma unroll
+          for (int u = 0; u < kShort; ++u)
+            if (u < nu[e]) {
+              const int c = japc[u0[e] + u];
+              int t = kToDiag;
+              if (c != n) {
+                t = find_sorted(japc, ic0, ic1, c);
+                if (t < 0) t = kDropped;
+              }
+              tgt[e] |= (unsigned)t << (4 * u);
+            }
+        }
+      }
+    }
+    double nrs = 0.0;  // minus the dropped-fill sum
+    // LOWER loop (:993-1007): one product into its target
+    auto eliminate = [&](double tl, double uval, int t) {
+      if (t == kDropped && !MILU && !may_overflow(tl, uval)) return;
+      const double prod = __dmul_rn(tl, uval);
+      double x = t == kToDiag ? wd : t == kDropped ? nrs : w[t];
+      x = __dsub_rn(x, prod);
+      if (t == kToDiag) wd = x;
+      else if (t == kDropped) nrs = x;
+      else w[t] = x;
+    };
+    const int maxlow = __reduce_max_sync(all, mine ? nlow : 0);
+    unsigned turns = 0;
+    if (SHORT) {
+#pragma unroll
+      for (int e = 0; e < kShort; ++e) {
+        if (e >= maxlow) break;
+        const bool act = mine && e < nlow;
+        LLRaw rd, ru[kShort];
+        while (true) {
+          bool ok = true;
+          if (act) {
+            ll_issue(words + col[e], rd);
+#pragma unroll
+            for (int u = 0; u < kShort; ++u)
+              if (u < nu[e]) ll_issue(words + u0[e] + u, ru[u]);
+            ok = ll_ready<double>(rd, ep);
+#pragma unroll
+            for (int u = 0; u < kShort; ++u)
+              if (u < nu[e]) ok = ok && ll_ready<double>(ru[u], ep);
+          }
+          if (__all_sync(all, ok)) break;
+          if (!keep_waiting(turns)) return;
+        }
+        if (act) {
+          double dv;
+          ll_take(rd, dv);
+          const double tl = __dmul_rn(w[e], dv);
+          w[e] = tl;
+#pragma unroll
+          for (int u = 0; u < kShort; ++u)
+            if (u < nu[e]) {
+              double uv;
+              ll_take(ru[u], uv);
+              eliminate(tl, uv, (int)((tgt[e] >> (4 * u)) & 15u));
+            }
+        }
+      }
+    } else {
+      for (int e = 0; e < maxlow; ++e) {
+        const bool act = mine && e < nlow;
+        int jcol = 0, uu0 = 0, uu1 = 0;
+        if (act) {
+          jcol = japc[ic0 + e];
+          uu0 = japc[jcol];
+          uu1 = iapc[jcol + 1];
+        }
+        double tl = 0.0;
+        const int most = __reduce_max_sync(all, uu1 - uu0);
+        for (int ub = 0; ub == 0 || ub < most; ub += 4) {
+          // the inverse pivot with the first four upper entries
+          LLRaw rd, ru[4];
+          while (true) {
+            bool ok = true;
+            if (act) {
+              if (ub == 0) ll_issue(words + jcol, rd);
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (uu0 + ub + u < uu1) ll_issue(words + uu0 + ub + u, ru[u]);
+              if (ub == 0) ok = ll_ready<double>(rd, ep);
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (uu0 + ub + u < uu1) ok = ok && ll_ready<double>(ru[u], ep);
+            }
+            if (__all_sync(all, ok)) break;
+            if (!keep_waiting(turns)) return;
+          }
+          if (act) {
+            if (ub == 0) {
+              double dv;
+              ll_take(rd, dv);
+              tl = __dmul_rn(w[e], dv);
+              w[e] = tl;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (uu0 + ub + u < uu1) {
+                const int c = japc[uu0 + ub + u];
+                double uv;
+                ll_take(ru[u], uv);
+                const int k = c == n ? -2 : find_sorted(japc, ic0, ic1, c);
+                if (k == -1 && !MILU && !may_overflow(tl, uv)) continue;
+                const double prod = __dmul_rn(tl, uv);
+                const double x = __dsub_rn(k == -2 ? wd : k == -1 ? nrs : w[k], prod);
+                if (k == -2) wd = x;
+                else if (k == -1) nrs = x;
+                else w[k] = x;
+              }
+          }
+        }
+      }
+    }
+    if (!mine) continue;
+    // the upper entries are final
+    for (int k = nlow; k < len; ++k) ll_put(words + ic0 + k, w[k], ep);
+    // DIAGONAL (:1010-1037)
+    const double d = wd;
+    double tl = __dsub_rn(__dmul_rn(__dadd_rn(1.0, delta), d), __dmul_rn(relax, -nrs));
+    const double sd1 = copysign(fabs(d), tl);
+    bool bad = false;
+    if (sd1 != d) {
+      if (ipcflag > 1) tl = copysign(1.0e-6, d);
+      else bad = true;
+    }
+    if (!bad && fabs(tl) == 0.0) {
+      if (ipcflag > 1) tl = copysign(1.0e-6, d);
+      else bad = true;
+    }
+    if (bad) {
+      atomicMin(&ctl->pivot_fail, n);
+      continue;
+    }
+    const double inv = __drcp_rn(tl);
+    ll_put(words + n, inv, ep);
+    apc[n] = inv;
+    for (int k = 0; k < len; ++k) apc[ic0 + k] = w[k];
   }
+}
+
+// True when every row has at most kShort lower and upper entries.
+bool ilu_short_rows(int n, const std::vector<int> &iapc, const std::vector<int> &japc) {
+  for (int r = 0; r < n; ++r)
+    if (japc[r] - iapc[r] > kShort || iapc[r + 1] - japc[r] > kShort) return false;
+  return true;
+}
+
+// Warps at work: enough that those ahead of the front have their rows' index
+// work done when it arrives, few enough that their polls do not slow it
+// (kFactorAhead 2, 4, 8, 16 and 64 on 10 x 400 x 400 cells: 5.3, 4.4, 4.8, 6.1
+// and 50 ms).
+int launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_amat,
+                      const int *d_iapc, const int *d_japc, double *d_apc, const Levels &L,
+                      FactorWords &W, double relax, double delta, int ipcflag, Ctl *ctl,
+                      cudaStream_t st) {
   (void)n;
+  W.epoch += 1;
+  if (W.epoch == 0) {  // the epochs wrapped: clear the words
+    if (cudaMemsetAsync(W.words, 0, 16 * W.count, st) != cudaSuccess) return -1;
+    W.epoch = 1;
+  }
+  if (cudaMemsetAsync(W.claim, 0, sizeof(int), st) != cudaSuccess) return -1;
+  const long long warps = std::min<long long>((long long)(L.maxwidth + 31) / 32 * kFactorAhead, L.nslices);
+  const int grid = (int)std::max<long long>(1, std::min<long long>((warps + 3) / 4, 8LL * kNumSM));
+  auto *k = W.short_rows ? (relax > 0.0 ? k_ilu0_factor<true, true> : k_ilu0_factor<true, false>)
+                         : (relax > 0.0 ? k_ilu0_factor<false, true> : k_ilu0_factor<false, false>);
+  k<<<grid, 128, 0, st>>>(L.nslices, L.d_slices, L.d_rows, d_ia, d_ja, d_amat, d_iapc, d_japc, d_apc,
+                          static_cast<LLWord<double> *>(W.words), W.epoch, W.claim, relax, delta,
+                          ipcflag, ctl);
+  return 0;
 }
 
 template <typename T>

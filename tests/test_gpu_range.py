@@ -72,3 +72,23 @@ def test_range_sweeps_bitexact(gblib, name):
     assert gblib.gbims_factor(m32._h, _lib.dptr(amat), None) == 0
     assert gblib.gbims_precondition(m32._h, _lib.dptr(v), _lib.dptr(z)) == 0
     assert np.max(np.abs(z - zo)) <= 1e-5 * np.max(np.abs(zo))
+
+
+@pytest.mark.parametrize("relax", [0.0, 0.97])
+@pytest.mark.parametrize("name,n,offsets", [
+    ("six", 700, [1, 2, 3, 30, 31, 32]), ("seven", 700, [1, 2, 3, 30, 31, 32, 33]),
+    ("one-row", 1, []), ("chain", 200, [1]), ("wide-levels", 5000, [2500, 2501]),
+    ("thirty", 400, list(range(1, 31)))])
+def test_one_launch_factor_bitexact(gblib, name, n, offsets, relax):
+    """The ILU0/MILU0 factor against the oracle's, bit for bit, at the edge
+    between its short rows (six lower and upper entries) and long ones, for
+    the narrowest and the widest levels, with and without the dropped fill."""
+    ia, ja, amat = banded_pattern(n, offsets, seed=3 * n + len(offsets))
+    o = oracle.Ims(oracle.settings(relax=relax), ia, ja)
+    o.apply(amat.copy(), np.ones(n), np.zeros(n))
+    ims = ImsLinear(ImsLinearSettings(structure=GENERAL, relax=relax)).imslinear_allocate(n, ia, ja)
+    apc = np.zeros(ja.size)
+    for _ in range(2):
+        assert gblib.gbims_factor(ims._h, _lib.dptr(amat), None) >= 0
+        assert gblib.gbims_get_apc(ims._h, _lib.dptr(apc)) == 0
+        np.testing.assert_array_equal(apc, o.apc())
