@@ -397,7 +397,8 @@ static bool build_graph(gbims_handle *h) {
     cudaGetLastError();
     return false;
   }
-  enqueue_iteration(h, (unsigned long long)cond, 1);
+  const int per_body = fused(h) ? kBodyIterations : 1;
+  for (int i = 0; i < per_body; ++i) enqueue_iteration(h, (unsigned long long)cond, 1);
   cudaGraph_t captured = nullptr;
   cudaError_t e = cudaStreamEndCapture(h->st, &captured);
   if (e != cudaSuccess) {
@@ -415,6 +416,7 @@ static bool build_graph(gbims_handle *h) {
     cudaGraphNodeType ty;
     if (cudaGraphNodeGetType(nd, &ty) == cudaSuccess && ty == cudaGraphNodeTypeKernel) h->body_kernels++;
   }
+  h->body_kernels /= per_body;  // the loop counts iterations
   cudaGraphExec_t exec = nullptr;
   if (cudaGraphInstantiate(&exec, g, 0) != cudaSuccess) {
     cudaGraphDestroy(g);

@@ -17,6 +17,12 @@ constexpr int kMaxRedBlocks = 8 * kNumSM;  // grid of reduction kernels: 8 x 256
 // Systems up to this size run their products fused with the Krylov steps
 // around them (k_sparse.cu)
 constexpr int kFuseRows = kMaxRedBlocks * kRedBlock;
+// Iterations in one body of the inner loop's graph on those systems: a turn of
+// the WHILE node costs 3 us, an iteration's kernels after the end of the loop
+// about 6.  1x20x30 2.45 -> 2.33 ms a step at 4 and 2.34 at 8, 1x100x100 11.42
+// -> 10.90 and 10.87; larger systems would wait for more idle blocks and gain
+// under 1 %, so they keep one.
+constexpr int kBodyIterations = 4;
 constexpr int kSell = 32;         // SELL slice height (one warp)
 constexpr int kMaxRowLen = 64;    // ILU0 factor: longest supported CSR row
 
