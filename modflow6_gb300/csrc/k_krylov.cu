@@ -163,8 +163,23 @@ struct MaxBits {
         : "+l"(s), "+r"(i)
         : "l"(u), "r"(row));
   }
-  __device__ __forceinline__ MaxLoc loc() const { return MaxLoc{__longlong_as_double((long long)s), (long long)i}; }
   __device__ __forceinline__ unsigned nonfinite() const { return ((unsigned)(s >> 32) & 0x7ff00000u) == 0x7ff00000u; }
+  __device__ __forceinline__ double value() const { return __longlong_as_double((long long)s); }
+  // of the block's partials, in any order of their rows
+  __device__ __forceinline__ void merge(double v, int row) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    const unsigned long long a = u & 0x7fffffffffffffffull, b = s & 0x7fffffffffffffffull;
+    if (a > b || (a == b && (unsigned)row < (unsigned)i)) {
+      s = u;
+      i = row;
+    }
+  }
+  // the largest of the warp, the smallest row among equals, in every lane
+  __device__ __forceinline__ void warp() {
+    const MaxLoc m = warp_maxloc(MaxLoc{value(), (long long)i});
+    s = (unsigned long long)__double_as_longlong(m.val);
+    i = (int)m.idx;
+  }
 };
 
 struct MaxBits32 {
@@ -177,24 +192,57 @@ struct MaxBits32 {
         : "+r"(s), "+r"(i)
         : "r"(__float_as_uint(v)), "r"(row));
   }
-  __device__ __forceinline__ MaxLoc loc() const { return MaxLoc{(double)__uint_as_float(s), (long long)i}; }
   __device__ __forceinline__ unsigned nonfinite() const { return (s & 0x7f800000u) == 0x7f800000u; }
+  __device__ __forceinline__ double value() const { return widen(__uint_as_float(s)); }
+  __device__ __forceinline__ void warp() {
+    const unsigned all = 0xffffffffu, a = s & 0x7fffffffu;
+    const unsigned top = __reduce_max_sync(all, a);
+    const unsigned row = a == top ? (unsigned)i : all;  // -1 while nothing is above zero
+    const unsigned first = __reduce_min_sync(all, row);
+    const unsigned who = __ballot_sync(all, a == top && row == first);
+    s = __shfl_sync(all, s, __ffs((int)who) - 1);
+    i = (int)first;
+  }
 };
 
 // A block's share of an update into its partial slots: [0]=l2 (when taken),
-// [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite.
-template <bool L2>
-__device__ __forceinline__ void update_partials(double l2, unsigned nf, MaxLoc (&m)[2], double *part,
-                                                int G, int b) {
+// [1]=dx val, [2]=dx idx, [3]=r val, [4]=r idx, [5]=nonfinite; the rows and
+// the flag as integers.
+template <bool L2, class M>
+__device__ __forceinline__ void update_partials(double l2, unsigned nf, M mx, M mr, double *part, int G, int b) {
+  __shared__ decltype(M::s) sv[2][kRedBlock / 32];
+  __shared__ int si[2][kRedBlock / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  mx.warp();
+  mr.warp();
+  if (lane == 0) {
+    sv[0][wid] = mx.s;
+    si[0][wid] = mx.i;
+    sv[1][wid] = mr.s;
+    si[1][wid] = mr.i;
+  }
   const int any = __syncthreads_or((int)nf);
+  if (wid == 0) {
+    mx = M();
+    mr = M();
+    if (lane < kRedBlock / 32) {
+      mx.s = sv[0][lane];
+      mx.i = si[0][lane];
+      mr.s = sv[1][lane];
+      mr.i = si[1][lane];
+    }
+    mx.warp();
+    mr.warp();
+  }
   double v[1] = {l2};
   if (L2) block_sum<1>(v);
-  block_maxloc<2>(m);
   if (threadIdx.x == 0) {
     part[b] = L2 ? v[0] : 0.0;
-    part[G + b] = m[0].val; part[2 * G + b] = (double)m[0].idx;
-    part[3 * G + b] = m[1].val; part[4 * G + b] = (double)m[1].idx;
-    part[5 * G + b] = any ? 1.0 : 0.0;
+    part[G + b] = mx.value();
+    part[2 * G + b] = __longlong_as_double(mx.i);
+    part[3 * G + b] = mr.value();
+    part[4 * G + b] = __longlong_as_double(mr.i);
+    part[5 * G + b] = __longlong_as_double(any ? 1 : 0);
   }
 }
 
@@ -202,22 +250,34 @@ __device__ __forceinline__ void update_partials(double l2, unsigned nf, MaxLoc (
 template <bool L2>
 __device__ __forceinline__ void ctl_finish_update(Ctl *ctl, const double *part, int G) {
   double l2[1] = {0.0};
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  MaxBits mx, mr;
   int nf = 0;
-  for (int i = threadIdx.x; i < G; i += blockDim.x) {
-    MaxLoc a, b;
-    if (L2) l2[0] += __ldcg(part + i);
-    a.val = __ldcg(part + G + i);
-    a.idx = (long long)__ldcg(part + 2 * G + i);
-    b.val = __ldcg(part + 3 * G + i);
-    b.idx = (long long)__ldcg(part + 4 * G + i);
-    nf |= __ldcg(part + 5 * G + i) != 0.0;
-    maxloc_merge(m[0], a);
-    maxloc_merge(m[1], b);
+  for (int i0 = threadIdx.x; i0 < G; i0 += kPartTrips * kRedBlock) {
+    double l[kPartTrips], xv[kPartTrips], rv[kPartTrips];
+    int xi[kPartTrips], ri[kPartTrips];
+#pragma unroll
+    for (int t = 0; t < kPartTrips; ++t) {
+      const int i = i0 + t * kRedBlock;
+      if (i < G) {
+        if (L2) l[t] = __ldcg(part + i);
+        xv[t] = __ldcg(part + G + i);
+        xi[t] = __double2loint(__ldcg(part + 2 * G + i));
+        rv[t] = __ldcg(part + 3 * G + i);
+        ri[t] = __double2loint(__ldcg(part + 4 * G + i));
+        nf |= __double2loint(__ldcg(part + 5 * G + i));
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < kPartTrips; ++t)
+      if (i0 + t * kRedBlock < G) {
+        if (L2) l2[0] += l[t];
+        mx.merge(xv[t], xi[t]);
+        mr.merge(rv[t], ri[t]);
+      }
   }
   nf = __syncthreads_or(nf);
   if (L2) block_sum<1>(l2);
+  MaxLoc m[2] = {{mx.value(), mx.i}, {mr.value(), mr.i}};
   block_maxloc<2>(m);
   if (threadIdx.x == 0) {
     ctl->l2norm = L2 ? sqrt(l2[0]) : 0.0;
@@ -544,8 +604,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update64(int n, double *__rest
     mx.take(tv, i);
     mr.take(di, i);
   }
-  MaxLoc m[2] = {mx.loc(), mr.loc()};
-  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
+  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), mx, mr, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_cg_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
 }
 
@@ -585,7 +644,7 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update_mixed(int n, double *__
     for (int r = 0; r < R; ++r) {
       const int j = i + r * stride;
       pr[r] = __fmul_rn(alphaf, pr[r]);
-      x[j] = xr[r] + (double)pr[r];
+      x[j] = xr[r] + widen(pr[r]);
       dr[r] = __fmaf_rn(-alphaf, qr[r], dr[r]);
       d[j] = dr[r];
     }
@@ -598,14 +657,13 @@ __global__ void __launch_bounds__(kRedBlock) k_cg_update_mixed(int n, double *__
   }
   for (; i < n; i += stride) {
     const float tv = __fmul_rn(alphaf, p[i]), di = __fmaf_rn(-alphaf, q[i], d[i]);
-    x[i] = x[i] + (double)tv;
+    x[i] = x[i] + widen(tv);
     d[i] = di;
     mx.take(tv, i);
     mr.take(di, i);
     csum_prod(l2, di, di);
   }
-  MaxLoc m[2] = {mx.loc(), mr.loc()};
-  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
+  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), mx, mr, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) ctl_mixed_inner(ctl, part, gridDim.x, 0, refine_factor);
 }
 
@@ -718,8 +776,7 @@ __global__ void __launch_bounds__(kRedBlock) k_bcgs_update(int n, double *__rest
     mr.take(rv, i);
     if (L2) v[0] = fma(rv, rv, v[0]);
   }
-  MaxLoc m[2] = {mx.loc(), mr.loc()};
-  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, part, gridDim.x, blockIdx.x);
+  update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), mx, mr, part, gridDim.x, blockIdx.x);
   if (FIN && last_block(&ctl->fin, gridDim.x)) {
     if (FIN == 1) ctl_bcgs_cnvg<L2>(ctl, part, gridDim.x, cond, use_cond);
     else ctl_mixed_inner(ctl, part, gridDim.x, 1, refine_factor);
@@ -746,8 +803,7 @@ __global__ void __launch_bounds__(kRedBlock) k_true_resid_stats(int n, const dou
   }
   double v[1] = {0.0};
   unsigned nf = 0;
-  MaxLoc m[2];
-  m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+  MaxBits none, mr;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double ri = r[i];
     if (d32) d32[i] = (float)ri;
@@ -756,12 +812,11 @@ __global__ void __launch_bounds__(kRedBlock) k_true_resid_stats(int n, const dou
       if (dhat64) dhat64[i] = ri;
     }
     if (dscale) ri = ri / dscale[i];    // BiCGSTAB reports the unscaled residual
-    if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i; }
+    mr.take(ri, i);
     v[0] = fma(ri, ri, v[0]);
     nf |= nonfinite(ri);
   }
-  m[0].idx = -1;
-  update_partials<true>(v[0], nf, m, part, gridDim.x, blockIdx.x);
+  update_partials<true>(v[0], nf, none, mr, part, gridDim.x, blockIdx.x);
   if (last_block(&ctl->fin, gridDim.x)) ctl_refine(ctl, part, gridDim.x, cond, use_cond);
 }
 
@@ -957,9 +1012,8 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update64(BatchDev B, double 
         }
       }
     }
-    MaxLoc m[2] = {mx.loc(), mr.loc()};
     double *pm = member_part(part, B, c.m);
-    update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), m, pm, c.G, c.b);
+    update_partials<L2>(v[0], mx.nonfinite() | mr.nonfinite(), mx, mr, pm, c.G, c.b);
     if (last_block(&ctl->fin, c.G)) ctl_cg_cnvg<L2>(ctl, pm, c.G, 0ULL, 0);
   }
   __syncthreads();
@@ -1024,15 +1078,14 @@ __global__ void __launch_bounds__(kRedBlock) k_b_cg_update_mixed(BatchDev B, dou
   MaxBits32 mx, mr;
   for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
     const float tv = __fmul_rn(alphaf, p[i]), di = __fmaf_rn(-alphaf, q[i], d[i]);
-    x[i] = x[i] + (double)tv;
+    x[i] = x[i] + widen(tv);
     d[i] = di;
     mx.take(tv, i - row0);
     mr.take(di, i - row0);
     csum_prod(l2, di, di);
   }
-  MaxLoc m[2] = {mx.loc(), mr.loc()};
   double *pm = member_part(part, B, c.m);
-  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), m, pm, c.G, c.b);
+  update_partials<true>(csum_value(l2), mx.nonfinite() | mr.nonfinite(), mx, mr, pm, c.G, c.b);
   if (last_block(&ctl->fin, c.G)) ctl_mixed_inner(ctl, pm, c.G, 0, refine_factor);
 }
 
@@ -1061,17 +1114,16 @@ __global__ void __launch_bounds__(kRedBlock) k_b_true_resid_stats(BatchDev B,
     const int row0 = B.mr[c.m];
     double v[1] = {0.0};
     unsigned nf = 0;
-    MaxLoc m[2];
-    m[0].val = 0.0; m[0].idx = -1; m[1].val = 0.0; m[1].idx = -1;
+    MaxBits none, mr;
     for (int i = c.r0 + threadIdx.x; i < c.r1; i += blockDim.x) {
       const double ri = r[i];
       d32[i] = (float)ri;
-      if (absgt(ri, m[1].val)) { m[1].val = ri; m[1].idx = i - row0; }
+      mr.take(ri, i - row0);
       v[0] = fma(ri, ri, v[0]);
       nf |= nonfinite(ri);
     }
     double *pm = member_part(part, B, c.m);
-    update_partials<true>(v[0], nf, m, pm, c.G, c.b);
+    update_partials<true>(v[0], nf, none, mr, pm, c.G, c.b);
     if (last_block(&ctl->fin, c.G)) ctl_refine(ctl, pm, c.G, 0ULL, 0);
   }
   __syncthreads();
