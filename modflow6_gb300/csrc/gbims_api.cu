@@ -33,7 +33,7 @@ struct gbims_handle {
   FactorWords FW;
   Dia7 D;
   bool structured = false;  // wavefront sweeps (one or more full DIS grids)
-  bool dia_spmv = false;    // index-free SpMV (a single full DIS grid)
+  bool dia_spmv = false;    // index-free SpMV (full DIS grids)
   // owned FP64 buffers
   double *d_amat = nullptr, *d_rhs = nullptr, *d_x = nullptr;
   double *v_d = nullptr, *v_p = nullptr, *v_q = nullptr, *v_z = nullptr, *v_t = nullptr,
@@ -1707,23 +1707,8 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
   h->bd.mc = h->d_bmc;
   h->bd.mr = h->d_bmr;
   h->bd.ctls = h->d_ctls;
-  // the products skip the rows of members that are done: per SELL slice its
-  // member, or -1 where a member boundary falls inside the slice
-  if (h->S.nslices > 0) {
-    std::vector<int> slm(h->S.nslices);
-    for (int sl = 0, m = 0; sl < h->S.nslices; ++sl) {
-      const int r0 = sl * kSell, r1 = std::min(neq, r0 + kSell) - 1;
-      while (mrow[m + 1] <= r0) ++m;
-      slm[sl] = (r1 < mrow[m + 1]) ? m : -1;
-    }
-    GB_CUDA(h, dalloc(&h->S.d_slm, slm.size()));
-    GB_CUDA(h, cudaMemcpy(h->S.d_slm, slm.data(), sizeof(int) * slm.size(), cudaMemcpyHostToDevice));
-    h->S.d_mrow = h->d_bmr;
-    h->S.nm = nmembers;
-    h->S.mctl = h->d_ctls;
-  }
   // full DIS grids: the wavefront sweeps run every member's layers and
-  // blocks as the CTAs of one launch
+  // blocks as the CTAs of one launch, and the products need no index arrays
   if (shapes) {
     std::vector<int> sh(shapes, shapes + 3 * nmembers);
     std::vector<long long> row0(nmembers);
@@ -1745,6 +1730,35 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
     int rc2 = setup_structured(h, sh, row0);
     if (rc2 != GBIMS_OK) return rc2;
     h->D.mctl = h->d_ctls;
+    for (void *p : {(void *)h->S.d_ptr, (void *)h->S.d_col, (void *)h->S.d_src, (void *)h->S.d_val,
+                    (void *)h->S.d_val32})
+      cudaFree(p);
+    h->S = Sell();
+    GB_CUDA(h, dalloc(&h->D.d_sv, (size_t)7 * neq));
+    if (h->mixed) GB_CUDA(h, dalloc(&h->D.f_sv, (size_t)7 * neq));
+    h->D.rows.nchunks = nchunks;
+    h->D.rows.n = neq;
+    h->D.rows.cm = h->d_bcm;
+    h->D.rows.cr = h->d_bcr;
+    h->D.rows.geo = h->D.d_geo;
+    h->D.rows.mctl = h->d_ctls;
+    h->dia_spmv = true;
+    return GBIMS_OK;
+  }
+  // the products skip the rows of members that are done: per SELL slice its
+  // member, or -1 where a member boundary falls inside the slice
+  if (h->S.nslices > 0) {
+    std::vector<int> slm(h->S.nslices);
+    for (int sl = 0, m = 0; sl < h->S.nslices; ++sl) {
+      const int r0 = sl * kSell, r1 = std::min(neq, r0 + kSell) - 1;
+      while (mrow[m + 1] <= r0) ++m;
+      slm[sl] = (r1 < mrow[m + 1]) ? m : -1;
+    }
+    GB_CUDA(h, dalloc(&h->S.d_slm, slm.size()));
+    GB_CUDA(h, cudaMemcpy(h->S.d_slm, slm.data(), sizeof(int) * slm.size(), cudaMemcpyHostToDevice));
+    h->S.d_mrow = h->d_bmr;
+    h->S.nm = nmembers;
+    h->S.mctl = h->d_ctls;
   }
   return GBIMS_OK;
 }

@@ -213,10 +213,20 @@ struct Dia7Geo {
   long long row0;     // first row of the member in the natural-order vectors
 };
 
+// The rows of a batch of such grids for the index-free products: chunks of at
+// most kChunkRows rows of one member (nchunks 0: a single grid).
+struct Dia7Rows {
+  int nchunks = 0, n = 0;
+  const int *cm = nullptr, *cr = nullptr;  // BatchDev's
+  const Dia7Geo *geo = nullptr;
+  const Ctl *mctl = nullptr;
+};
+
 // Structured 7-point DIS layout of the ILU0 factors for the wavefront sweeps:
 // per block of lines, G x W tiles (row = wavefront step, column = lane).
 struct Dia7 {
   int nlay = 0, nrow = 0, ncol = 0;  // single model: its shape (index-free SpMV)
+  Dia7Rows rows;                     // batch: its rows (index-free SpMV)
   int nb = 0, G = 0;       // single model: blocks per layer, padded steps per block
   long long slots = 0;     // total elements per skewed array (all members)
   int nm = 0;              // members
