@@ -692,7 +692,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
   if (h->ipc < 3) {
     levels_build_host(neq, h->iapc, h->japc, true, h->F);
     h->FW.short_rows = ilu_short_rows(neq, h->iapc, h->japc);
-    h->FW.count = (size_t)nja;
+    h->FW.count = std::max((size_t)nja, (size_t)h->D.slots);
     GB_CUDA(h, cudaMalloc(&h->FW.words, 16 * h->FW.count));
     GB_CUDA(h, cudaMemset(h->FW.words, 0, 16 * h->FW.count));
     GB_CUDA(h, cudaMalloc((void **)&h->FW.claim, sizeof(int)));
@@ -914,19 +914,27 @@ static int factor_core(gbims_handle *h) {
   }
   int ipcflag = 0, icount = 0;
   double delta = 0.0;
+  bool dropped = h->s.relax > 0.0;  // the wavefront form: with the dropped-fill sum
   for (;;) {
     Ctl init;
     memset(&init, 0, sizeof(init));
     init.pivot_fail = INT_MAX;
     *h->h_ctl = init;
     GB_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, st));
-    if (launch_ilu_factor(n, h->d_ia, h->d_ja, h->d_amat, h->d_iapc, h->d_japc, h->d_apc, h->F,
-                          h->FW, h->s.relax, delta, ipcflag, h->d_ctl, st) != 0)
-      return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation launch failed");
-    h->launches += 1;
+    const int rc = h->dia_spmv
+                       ? launch_dia7_factor(h->D, n, h->d_iapc, h->d_apc, h->FW, h->s.relax, delta, ipcflag,
+                                            dropped, h->d_ctl, st)
+                       : launch_ilu_factor(n, h->d_ia, h->d_ja, h->d_amat, h->d_iapc, h->d_japc, h->d_apc, h->F,
+                                           h->FW, h->s.relax, delta, ipcflag, h->d_ctl, st);
+    if (rc != 0) return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation launch failed");
+    h->launches += h->dia_spmv ? 2 : 1;
     GB_CUDA(h, cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     GB_CUDA(h, cudaStreamSynchronize(st));
     GB_CUDA(h, cudaGetLastError());
+    if (!dropped && h->h_ctl->scratch_err == 2) {
+      dropped = true;  // it might overflow: it counts then
+      continue;
+    }
     if (h->h_ctl->scratch_err) return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation wait limit reached");
     ipcflag = (h->h_ctl->pivot_fail != INT_MAX) ? 1 : 0;
     if (ipcflag < 1) break;
@@ -1736,6 +1744,13 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
     h->S = Sell();
     GB_CUDA(h, dalloc(&h->D.d_sv, (size_t)7 * neq));
     if (h->mixed) GB_CUDA(h, dalloc(&h->D.f_sv, (size_t)7 * neq));
+    if ((size_t)h->D.slots > h->FW.count) {
+      cudaFree(h->FW.words);
+      h->FW.words = nullptr;
+      h->FW.count = (size_t)h->D.slots;
+      GB_CUDA(h, cudaMalloc(&h->FW.words, 16 * h->FW.count));
+      GB_CUDA(h, cudaMemset(h->FW.words, 0, 16 * h->FW.count));
+    }
     h->D.rows.nchunks = nchunks;
     h->D.rows.n = neq;
     h->D.rows.cm = h->d_bcm;

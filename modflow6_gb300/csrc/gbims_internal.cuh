@@ -94,6 +94,13 @@ __device__ __forceinline__ bool absgt(double a, double b) {
   return ua > ub;
 }
 
+// A product whose exponents are so large that it, or a sum of a row's
+// products, could overflow.
+__device__ __forceinline__ bool may_overflow(double a, double b) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+  return ea == 0x7ff || eb == 0x7ff || ea + eb - 1023 > 2000;
+}
+
 __device__ __forceinline__ void maxloc_merge(MaxLoc &a, const MaxLoc &b) {
   unsigned long long ua = __double_as_longlong(a.val) & 0x7fffffffffffffffULL;
   unsigned long long ub = __double_as_longlong(b.val) & 0x7fffffffffffffffULL;
@@ -309,6 +316,10 @@ void rcm_order(int n, const std::vector<int> &ia, const std::vector<int> &ja,
 int md_order(int n, const std::vector<int> &ia, const std::vector<int> &ja,
              std::vector<int> &lorder);
 bool ilu_short_rows(int n, const std::vector<int> &iapc, const std::vector<int> &japc);
+int factor_words_next(FactorWords &W, cudaStream_t st);
+// ctl->scratch_err afterwards: 1 a wait ran out, 2 to be repeated with dropped = true
+int launch_dia7_factor(const Dia7 &D, int n, const int *d_iapc, double *d_apc, FactorWords &W, double relax,
+                       double delta, int ipcflag, bool dropped, Ctl *ctl, cudaStream_t st);
 int launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_amat,
                       const int *d_iapc, const int *d_japc, double *d_apc, const Levels &L,
                       FactorWords &W, double relax, double delta, int ipcflag, Ctl *ctl,

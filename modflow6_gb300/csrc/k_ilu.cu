@@ -1,4 +1,5 @@
-// k_ilu.cu -- ILU0 / MILU0 factorisation and level-scheduled triangular sweeps.
+// k_ilu.cu -- ILU0 / MILU0 factorisation of general patterns and the triangular sweeps
+// a level at a time.
 //
 // Factorisation: ims_base_pcilu0 (src/Solution/LinearMethods/ImsLinearBase.f90:928-1042)
 // restated per row, one thread per row, in one launch (see k_ilu0_factor).
@@ -79,13 +80,6 @@ __device__ __forceinline__ int find_sorted(const int *__restrict__ japc, int i0,
 // position), the diagonal, or the dropped-fill sum.
 constexpr int kToDiag = 14, kDropped = 15;
 constexpr int kShort = 6;  // lower and upper entries of a row of the short form (a target fits 4 bits)
-
-// A product whose exponents are so large that it, or a sum of a row's
-// products, could overflow.
-__device__ __forceinline__ bool may_overflow(double a, double b) {
-  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
-  return ea == 0x7ff || eb == 0x7ff || ea + eb - 1023 > 2000;
-}
 
 // The whole factorisation in one launch.  Bound by its chain: a level hands
 // its inverse pivots and upper entries to the next through L2 (0.7 us) and a
@@ -322,6 +316,16 @@ bool ilu_short_rows(int n, const std::vector<int> &iapc, const std::vector<int> 
   return true;
 }
 
+// A new epoch for the words of the next launch, and its claims from zero.
+int factor_words_next(FactorWords &W, cudaStream_t st) {
+  W.epoch += 1;
+  if (W.epoch == 0) {  // the epochs wrapped: clear the words
+    if (cudaMemsetAsync(W.words, 0, 16 * W.count, st) != cudaSuccess) return -1;
+    W.epoch = 1;
+  }
+  return cudaMemsetAsync(W.claim, 0, sizeof(int), st) == cudaSuccess ? 0 : -1;
+}
+
 // Warps at work: enough that those ahead of the front have their rows' index
 // work done when it arrives, few enough that their polls do not slow it
 // (kFactorAhead 2, 4, 8, 16 and 64 on 10 x 400 x 400 cells: 5.3, 4.4, 4.8, 6.1
@@ -331,12 +335,7 @@ int launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_a
                       FactorWords &W, double relax, double delta, int ipcflag, Ctl *ctl,
                       cudaStream_t st) {
   (void)n;
-  W.epoch += 1;
-  if (W.epoch == 0) {  // the epochs wrapped: clear the words
-    if (cudaMemsetAsync(W.words, 0, 16 * W.count, st) != cudaSuccess) return -1;
-    W.epoch = 1;
-  }
-  if (cudaMemsetAsync(W.claim, 0, sizeof(int), st) != cudaSuccess) return -1;
+  if (factor_words_next(W, st) != 0) return -1;
   const long long warps = std::min<long long>((long long)(L.maxwidth + 31) / 32 * kFactorAhead, L.nslices);
   const int grid = (int)std::max<long long>(1, std::min<long long>((warps + 3) / 4, 8LL * kNumSM));
   auto *k = W.short_rows ? (relax > 0.0 ? k_ilu0_factor<true, true> : k_ilu0_factor<true, false>)
