@@ -816,7 +816,7 @@ def kernels_arm(a):
     amat, rhs = sln_ls_fixups(con["ia"], con["ja"], m.ibound, amat, rhs, x0, isymmetric=True)
     out = {"workload": workload_config(a, m)["workload"], "reps": a.steps}
     # the full-grid (index-free SpMV, wavefront sweeps) forms, then the
-    # general-pattern form (SELL-32 SpMV, level-scheduled sweeps) in FP64
+    # general-pattern form (SELL-32 SpMV, range sweeps) in FP64
     for name, prec, st in (("fp64", _lib.GBIMS_FP64, shape), ("mixed", _lib.GBIMS_MIXED, shape),
                            ("fp64_general", _lib.GBIMS_FP64, GENERAL)):
         ims = ImsLinear(ImsLinearSettings(precision=prec, structure=st, **C2_IMS))

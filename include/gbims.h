@@ -68,7 +68,7 @@ typedef struct gbims_settings {
                            nrow*ncol, then every row checked), so a caller
                            that passes only IA/JA, as imslinear_ar does,
                            reaches the structured path.  nlay < 0: never (the
-                           level-scheduled sweeps on the general pattern). */
+                           sweeps of general patterns). */
 } gbims_settings;
 
 /* Convergence summary of the last apply (ConvergenceSummary.f90 fields for a
@@ -394,7 +394,7 @@ int gbsln_create(const gbsln_model *model, const gbnpf_options *npf,
  * stencil (Xt3dInterface.f90, Xt3dAlgorithm.f90; without ANGLE2 the
  * horizontal connections have no z component, as in the reference), whose
  * matrix has the wider pattern (each row: the cell, its neighbours and
- * theirs) and is solved on the level-scheduled path; 2: XT3D RHS, the
+ * theirs) and is solved on the general-pattern path; 2: XT3D RHS, the
  * neighbours' terms on the right-hand side at the current heads and the
  * model's own pattern (:478-490). */
 typedef struct gbsln_ktensor {
@@ -431,7 +431,7 @@ typedef struct gbsln_grid {
 /* gbsln_create on a grid given by its connectivity.  The model's K,
  * ICELLTYPE, storage and boundaries are read from `model` (its nlay, nrow,
  * ncol, delr, delc, top and botm are not read).  The solve takes the
- * general-pattern path (SELL-32 product, level-scheduled ILU0) unless the
+ * general-pattern path (SELL-32 product, ILU0 swept by row ranges) unless the
  * pattern is that of a full DIS grid, which is found from IA/JA.  The checks
  * of con_finalize are made (diagonal first, ascending rows, every
  * connection with its counterpart, ihc in 0..2): GBIMS_ERR_ARG with the

@@ -808,7 +808,7 @@ int sln_setup(gbsln_handle *h, const gbsln_model *m, const gbnpf_options *npf, c
     int rc = xt3d_host(m, xt, geom, c, ibound, xh, h->err);
     if (rc < 0) return rc;
     h->nja = (int)xh.sja.size();
-    h->ims_s.nlay = -1;  // the wider pattern: the level-scheduled sweeps
+    h->ims_s.nlay = -1;  // the wider pattern: the general patterns' sweeps
   }
   cudaError_t e = cudaSuccess;
   auto chk = [&](cudaError_t x) { if (x != cudaSuccess && e == cudaSuccess) e = x; };

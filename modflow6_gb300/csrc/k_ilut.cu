@@ -24,7 +24,7 @@
 // Output: per row, in padded slots (lfil L entries, lfil - 1 U entries), the
 // kept columns and values, their counts and the inverse pivot.  The host
 // turns the counts into the IAPC/JAPC layout of the ILU0 preconditioner and
-// k_ilut_scatter moves the values there, so the level-scheduled sweeps apply
+// k_ilut_scatter moves the values there, so the general patterns' sweeps apply
 // ILUT unchanged (lusol, :465-516, is the ilu0a pair of sweeps).
 #include "gbims_internal.cuh"
 #include "k_llword.cuh"

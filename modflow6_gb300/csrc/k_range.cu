@@ -47,9 +47,9 @@
 // rows, backward: higher rows), which are resident or finished: the lowest
 // unfinished slice can always proceed, and every wait is bounded besides.
 //
-// Both sweeps, FP64 (one sync-free launch per sweep over words in L2 before):
-// DISV hexagons 4 x 150 x 150 1885 -> 303 us, XT3D 3 x 70 x 70 1668 -> 314 us,
-// ILUT (5, 1e-4) on 6 x 60 x 60 cells 1538 -> 255 us.
+// Both sweeps, FP64 (before: one launch per sweep, every row's values handed
+// over through L2): DISV hexagons 4 x 150 x 150 1885 -> 288 us, XT3D 3 x 70 x 70
+// 1668 -> 283 us, ILUT (5, 1e-4) on 6 x 60 x 60 cells 1538 -> 242 us.
 #include <algorithm>
 #include <climits>
 

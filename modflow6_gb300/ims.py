@@ -16,7 +16,7 @@ import numpy as np
 from . import _lib
 
 CG_METHOD = 1
-# `structure` value that keeps the level-scheduled sweeps on a DIS pattern
+# `structure` value that keeps the general patterns' sweeps on a DIS pattern
 GENERAL = (-1, 0, 0)
 BCGS_METHOD = 2
 
@@ -40,7 +40,7 @@ class ImsLinearSettings:
     droptol: float = 0.0         # PRECONDITIONER_DROP_TOLERANCE
     precision: int = _lib.GBIMS_FP64
     # (nlay, nrow, ncol) of a DIS grid for the wavefront sweeps; (0, 0, 0):
-    # found from the pattern; GENERAL: the level-scheduled sweeps always
+    # found from the pattern; GENERAL: the general patterns' sweeps always
     structure: tuple = field(default=(0, 0, 0))
 
     @classmethod
