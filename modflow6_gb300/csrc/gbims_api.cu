@@ -688,11 +688,13 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, cudaMemcpy(h->S.d_src, src.data(), sizeof(int) * src.size(), cudaMemcpyHostToDevice));
     if (h->mixed) GB_CUDA(h, dalloc(&h->S.d_val32, col.size()));
   }
-  // level schedule of the factorisation
+  // level schedule of the factorisation (full DIS grids: the wavefront's order)
   if (h->ipc < 3) {
-    levels_build_host(neq, h->iapc, h->japc, true, h->F);
-    h->FW.short_rows = ilu_short_rows(neq, h->iapc, h->japc);
-    h->FW.count = std::max((size_t)nja, (size_t)h->D.slots);
+    if (!h->dia_spmv) {
+      levels_build_host(neq, h->iapc, h->japc, true, h->F);
+      h->FW.short_rows = ilu_short_rows(neq, h->iapc, h->japc);
+    }
+    h->FW.count = h->dia_spmv ? (size_t)h->D.slots : (size_t)nja;
     GB_CUDA(h, cudaMalloc(&h->FW.words, 16 * h->FW.count));
     GB_CUDA(h, cudaMemset(h->FW.words, 0, 16 * h->FW.count));
     GB_CUDA(h, cudaMalloc((void **)&h->FW.claim, sizeof(int)));
