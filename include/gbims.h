@@ -152,7 +152,7 @@ int gbims_get_inner_records(gbims_handle *h, int cap, int *nrec, int *itinner, d
  * rows.  shapes (3 * nmembers: nlay, nrow, ncol per member) may be NULL;
  * when given, every member must be a full DIS grid of that shape and the
  * preconditioner runs as one wavefront launch over all members (otherwise the
- * level schedule of the whole batch).  FP64 PCG only (GBIMS_ERR_UNSUPPORTED
+ * whole batch as one general pattern).  FP64 PCG only (GBIMS_ERR_UNSUPPORTED
  * otherwise); the handle is released with gbims_destroy. */
 int gbims_batch_create(const gbims_settings *settings, int nmembers, const int *member_rows,
                        int neq, int nja, const int *ia, const int *ja, const int *shapes,

@@ -1665,7 +1665,7 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
   for (int m = 0; m < nmembers; ++m)
     if (mrow[m + 1] <= mrow[m]) return GBIMS_ERR_ARG;
   gbims_settings s = *settings;
-  s.nlay = -1;  // members are swept by the level schedule of the whole batch
+  s.nlay = -1;  // without shapes the members are swept as one general pattern
   s.nrow = s.ncol = 0;
   int rc = gbims_create(&s, neq, nja, ia, ja, out);
   gbims_handle *h = *out;
