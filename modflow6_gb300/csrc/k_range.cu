@@ -52,6 +52,7 @@
 // 1668 -> 283 us, ILUT (5, 1e-4) on 6 x 60 x 60 cells 1538 -> 242 us.
 #include <algorithm>
 #include <climits>
+#include <cstring>
 
 #include "gbims_internal.cuh"
 #include "k_llword.cuh"
@@ -69,11 +70,10 @@ constexpr int kRangeThreads = 32 * (kComputeWarps + kFetchWarps + 1);  // and th
 constexpr int kMinStages = 6, kMaxStages = 16;
 constexpr size_t kRingBytes = 48 * 1024, kSmemBytes = 216 * 1024;
 
-// A slice's block: a 16-byte header (rows + 256 * entries of the longest row +
-// 65536 * first slot, the starts of the parts after the row numbers), the row
-// numbers (~row when another range reads it), the slot numbers (entry e
-// of row l at e*rows + l), the factor values in the same order, the inverse
-// pivots; every part starts on 16 bytes.  Shorter rows are padded with zero
+// A slice's block: a 16-byte header (SliceHead), the row numbers (~row when
+// another range reads it), the slot numbers (entry e of row l at e*rows + l),
+// the factor values in the same order, the inverse pivots; every part starts
+// on 16 bytes.  Shorter rows are padded with zero
 // values and the slot that always holds zero: fma(-0, 0, t) is t.
 struct BlockLayout {
   int rows, slots, vals, dinv, bytes;
@@ -85,6 +85,23 @@ struct BlockLayout {
     bytes = dinv + ((tsize * nl + 15) & ~15);
   }
 };
+
+// The header: rows and the first row's slot, the start of the slot numbers and
+// the entries of the longest row (ILUT keeps up to kIlutCap of them, one more
+// than eight bits hold), the starts of the values and the pivots.
+struct SliceHead {
+  int x, y, vals, dinv;
+  static SliceHead pack(int nl, int entries, int first, const BlockLayout &L) {
+    return {(int)((unsigned)nl | (unsigned)first << 16), (int)((unsigned)L.slots | (unsigned)entries << 16),
+            L.vals, L.dinv};
+  }
+  __host__ __device__ int rows() const { return x & 0xffff; }
+  __host__ __device__ unsigned first() const { return (unsigned)x >> 16; }
+  __host__ __device__ int entries() const { return (int)((unsigned)y >> 16); }
+  __host__ __device__ int slots() const { return y & 0xffff; }
+};
+static_assert(sizeof(SliceHead) == 16 && kIlutCap < 65536 && kMaxRowLen < 65536,
+              "a slice's header is 16 bytes and counts a row's entries in 16 bits");
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -346,7 +363,7 @@ __global__ void __launch_bounds__(kRangeThreads, 1) k_range_sweep(RangeArgs<T> p
   // row and store nothing, so that no step of the chain is conditional.
   int n_code = 0;
   T n_rhs = T(0);
-  int4 n_head = make_int4(0, 0, 0, 0);
+  SliceHead n_head = {0, 0, 0, 0};
   int q = warp < ns ? warp : 0, nq = q;  // ring buffers of this slice and the next
   unsigned parity = 0;                   // of the next slice's
   auto ahead = [&]() -> bool {
@@ -354,8 +371,9 @@ __global__ void __launch_bounds__(kRangeThreads, 1) k_range_sweep(RangeArgs<T> p
     while (!__all_sync(0xffffffffu, bar_test(full + nq, parity)))
       if (--turns == 0) return false;
     const unsigned char *bl = ring + (unsigned)nq * (unsigned)p.stage_bytes;
-    n_head = *reinterpret_cast<const int4 *>(bl);
-    const int l = min(lane, (n_head.x & 255) - 1);
+    const int4 word = *reinterpret_cast<const int4 *>(bl);
+    n_head = {word.x, word.y, word.z, word.w};
+    const int l = min(lane, n_head.rows() - 1);
     n_code = reinterpret_cast<const int *>(bl + 16)[l];
     n_rhs = p.rhs[n_code < 0 ? ~n_code : n_code];
     return true;
@@ -363,9 +381,9 @@ __global__ void __launch_bounds__(kRangeThreads, 1) k_range_sweep(RangeArgs<T> p
   bool ok = warp >= ns || ahead();
   for (int s = warp; ok && s < ns; s += kComputeWarps) {
     const unsigned char *bl = ring + (unsigned)q * (unsigned)p.stage_bytes;
-    const int4 head = n_head;
-    const int nl = head.x & 255, w = (head.x >> 8) & 255, l = min(lane, nl - 1);
-    const unsigned own = slots_at + (unsigned)sizeof(T) * (((unsigned)head.x >> 16) + lane);
+    const SliceHead head = n_head;
+    const int nl = head.rows(), w = head.entries(), l = min(lane, nl - 1);
+    const unsigned own = slots_at + (unsigned)sizeof(T) * (head.first() + lane);
     const int code = n_code, row = code < 0 ? ~code : code;
     T tv = n_rhs;
     nq = q + kComputeWarps;
@@ -374,9 +392,9 @@ __global__ void __launch_bounds__(kRangeThreads, 1) k_range_sweep(RangeArgs<T> p
       parity ^= 1u;
     }
     ok = s + kComputeWarps >= ns || ahead();
-    const unsigned short *sls = reinterpret_cast<const unsigned short *>(bl + head.y) + l;
-    const T *vals = reinterpret_cast<const T *>(bl + head.z) + l;
-    const T dinv = (DIR < 0) ? reinterpret_cast<const T *>(bl + head.w)[l] : T(0);
+    const unsigned short *sls = reinterpret_cast<const unsigned short *>(bl + head.slots()) + l;
+    const T *vals = reinterpret_cast<const T *>(bl + head.vals) + l;
+    const T dinv = (DIR < 0) ? reinterpret_cast<const T *>(bl + head.dinv)[l] : T(0);
     int left = w;
     for (; ok && left > 8; left -= 8) {
       ok = take_entries<T, 8>(slots_at, sls, vals, nl, tv);
@@ -473,17 +491,15 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
         const int r = P.rows[q1];
         w = std::max(w, forward ? japc[r] - iapc[r] : iapc[r + 1] - japc[r]);
       }
+      if (w > 65535) return false;
       const int nl = q1 - q0;
       const BlockLayout L(nl, w, (int)tsize);
       const size_t at = P.blk.size();
       if ((at + L.bytes) / 16 > (size_t)INT_MAX || (at + L.bytes) / tsize > (size_t)INT_MAX) return false;
       P.blk.resize(at + L.bytes, 0);
-      int *head = reinterpret_cast<int *>(&P.blk[at]);
-      head[0] = (int)((unsigned)nl + 256u * (unsigned)w + 65536u * (unsigned)(q0 - r0));
-      head[1] = L.slots;
-      head[2] = L.vals;
-      head[3] = L.dinv;
-      for (int l = 0; l < nl; ++l) head[4 + l] = P.rows[q0 + l];
+      const SliceHead head = SliceHead::pack(nl, w, q0 - r0, L);
+      memcpy(&P.blk[at], &head, sizeof(head));
+      memcpy(&P.blk[at + L.rows], &P.rows[q0], sizeof(int) * nl);
       for (int l = 0; l < nl; ++l) {
         const int r = P.rows[q0 + l];
         const int j0 = forward ? iapc[r] : japc[r], j1 = forward ? japc[r] : iapc[r + 1];
@@ -530,9 +546,11 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
   if (P.src.size() > (size_t)INT_MAX) return false;
   // which rows other ranges read is known now
   for (size_t s = 0; s + 1 < P.off.size(); ++s) {
-    int *head = reinterpret_cast<int *>(&P.blk[16 * (size_t)P.off[s]]);
-    for (int l = 0; l < (head[0] & 255); ++l)
-      if (read[head[4 + l]]) head[4 + l] = ~head[4 + l];
+    unsigned char *block = &P.blk[16 * (size_t)P.off[s]];
+    const int nl = reinterpret_cast<const SliceHead *>(block)->rows();
+    int *rows = reinterpret_cast<int *>(block + sizeof(SliceHead));
+    for (int l = 0; l < nl; ++l)
+      if (read[rows[l]]) rows[l] = ~rows[l];
   }
   return true;
 }
