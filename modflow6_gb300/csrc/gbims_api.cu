@@ -63,7 +63,7 @@ struct gbims_handle {
   bool no_graph = false;   // GBIMS_GRAPH=0: the host drives the loop
   LevelWords LW;           // the general sweeps' result words (unstructured handles)
   RangePlan RF, RB;        // their plans, and the range size asked for (0: the default)
-  bool planned = false;
+  int plan = 0;            // the current pattern: not planned yet, planned (1), no plan (-1)
   int range_rows = 0;
   long long words_nr = 0;  // the grids that the words' epochs count launches of
   bool levels_b = false;   // B (and, for ILUT, F) holds the current factor's levels
@@ -133,23 +133,24 @@ static void ensure_levels(gbims_handle *h) {
 // before their first use and whenever the grid changes (its tickets number
 // the launches); a handle with wavefront sweeps never needs them.  A pattern
 // that no range size fits is swept level by level.
+static bool by_ranges(const gbims_handle *h) { return h->LW.mode == 1 && h->plan == 1; }
+
 static int ensure_ranges(gbims_handle *h) {
   if (h->structured) return GBIMS_OK;
-  if (h->LW.mode == 0) {
-    ensure_levels(h);
-    return GBIMS_OK;
-  }
-  if (!h->planned) {
+  if (h->LW.mode == 1 && h->plan == 0) {
     const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
     if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed) ||
         !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed)) {
       cudaGetLastError();
-      h->LW.mode = 0;
-      ensure_levels(h);
-      return GBIMS_OK;
+      h->plan = -1;
+    } else {
+      h->plan = 1;
     }
     if (h->ipc < 3) h->RF.host = h->RB.host = RangeHost();
-    h->planned = true;
+  }
+  if (!by_ranges(h)) {
+    ensure_levels(h);
+    return GBIMS_OK;
   }
   const size_t wb = (size_t)h->n * (h->mixed ? 8 : 16);
   if (!h->LW.fwd) {
@@ -171,7 +172,7 @@ static int ensure_ranges(gbims_handle *h) {
 
 // The factor's values in the plans' order.
 static void fill_ranges(gbims_handle *h) {
-  if (h->structured || h->LW.mode == 0) return;
+  if (h->structured || !by_ranges(h)) return;
   if (!h->mixed) launch_range_fill(h->RF, h->RB, h->d_apc, h->st);
   else launch_range_fill32(h->RF, h->RB, h->d_apc32, h->st);
   h->launches += 2;
@@ -193,7 +194,7 @@ static void precond64(gbims_handle *h, const double *r, double *z) {
     launch_dia7_apply64(h->D, h->D.d_rfull, h->D.d_zfull, h->d_ctl, h->st);
     launch_dia7_collect(h->D, h->n, h->D.d_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply64(h->D, r, z, h->d_ctl, h->st);
-  else if (h->LW.mode == 1) launch_range_apply(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else if (by_ranges(h)) launch_range_apply(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
   else launch_ilu_apply_levels(h->n, h->d_iapc, h->d_japc, h->d_apc, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
@@ -204,7 +205,7 @@ static void precond32(gbims_handle *h, const float *r, float *z) {
     launch_dia7_apply32(h->D, h->D.f_rfull, h->D.f_zfull, h->d_ctl, h->st);
     launch_dia7_collect32(h->D, h->n, h->D.f_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply32(h->D, r, z, h->d_ctl, h->st);
-  else if (h->LW.mode == 1) launch_range_apply32(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else if (by_ranges(h)) launch_range_apply32(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
   else launch_ilu_apply_levels32(h->n, h->d_iapc, h->d_japc, h->d_apc32, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
@@ -885,7 +886,8 @@ static int ilut_factor_core(gbims_handle *h) {
   h->launches += 1;
   // the sweeps' schedule is that of the kept pattern, and part of the
   // captured loop
-  h->levels_b = h->planned = false;
+  h->levels_b = false;
+  h->plan = 0;
   if (int rc = ensure_ranges(h)) return rc;
   drop_graph(h);
   GB_CUDA(h, cudaStreamSynchronize(st));
@@ -1332,14 +1334,14 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     auto with_rows = [&](int rows) -> int {
       h->LW.mode = 1;
       h->range_rows = rows;
-      h->planned = false;
+      h->plan = 0;
       if (int rc = ensure_ranges(h)) return rc;
       fill_ranges(h);
       return GBIMS_OK;
     };
     for (int rows : {512, 1024, 2048, 4096, 8192}) {
       if (int rc = with_rows(rows)) return rc;
-      if (h->LW.mode == 0) break;  // no range size fits the pattern
+      if (!by_ranges(h)) break;  // no range size fits the pattern
       const double ms = time_it(pre);
       out->candidate_ms[out->ncandidates++] = ms;
       out->level_ms[1] = std::min(out->level_ms[1], ms);

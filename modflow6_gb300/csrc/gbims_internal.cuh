@@ -342,8 +342,8 @@ void launch_ilu_apply_levels32(int n, const int *d_iapc, const int *d_japc,
 // with a launch per level).
 constexpr int kRangeRows = 2048;
 // The plan of one sweep of the pattern iapc/japc in ranges of about `rows`
-// rows (fewer where a range would not fit the shared memory), uploaded; false
-// when no range size fits or device memory runs out.
+// rows (fewer, and slices of fewer rows, where a range would not fit the shared
+// memory), uploaded; false when no range size fits or device memory runs out.
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
                  bool forward, int rows, bool fp32);
 void range_free(RangePlan &P);

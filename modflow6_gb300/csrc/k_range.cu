@@ -69,6 +69,10 @@ constexpr int kRangeThreads = 32 * (kComputeWarps + kFetchWarps + 1);  // and th
 // looks kComputeWarps slices ahead, so the ring must hold more than that.
 constexpr int kMinStages = 6, kMaxStages = 16;
 constexpr size_t kRingBytes = 48 * 1024, kSmemBytes = 216 * 1024;
+// Largest block of a plan whose full slices' ring does not fit, which starts
+// at about 107 FP64 entries for 32 rows: wide levels of long rows are then cut
+// into slices of fewer rows (6 of 256 entries).
+constexpr int kNarrowBlock = 16 * 1024;
 
 // A slice's block: a 16-byte header (SliceHead), the row numbers (~row when
 // another range reads it), the slot numbers (entry e of row l at e*rows + l),
@@ -451,11 +455,13 @@ bool upload(std::vector<V> &h, V **d, size_t *cap) {
 
 }  // namespace
 
-// The plan of one sweep for ranges of R rows; false when a range's slots
-// exceed the shared memory.  `order`: all rows by level, `lev` their levels.
+// The plan of one sweep for ranges of R rows, its slices' blocks of at most
+// `block` bytes where they have more than one row; false when a range's slots
+// and the ring exceed the shared memory.  `order`: all rows by level, `lev`
+// their levels.
 static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<int> &japc,
                          bool forward, const std::vector<int> &order, const std::vector<int> &lev,
-                         int R, size_t tsize, RangeHost &P) {
+                         int R, int block, size_t tsize, RangeHost &P) {
   const int nr = (n + R - 1) / R;
   P.R = R;
   P.nr = nr;
@@ -489,7 +495,9 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
       const int l0 = lev[P.rows[q0]];
       for (; q1 < r0 + nloc && q1 < q0 + 32 && lev[P.rows[q1]] == l0; ++q1) {
         const int r = P.rows[q1];
-        w = std::max(w, forward ? japc[r] - iapc[r] : iapc[r + 1] - japc[r]);
+        const int wide = std::max(w, forward ? japc[r] - iapc[r] : iapc[r + 1] - japc[r]);
+        if (q1 > q0 && BlockLayout(q1 + 1 - q0, wide, (int)tsize).bytes > block) break;
+        w = wide;
       }
       if (w > 65535) return false;
       const int nl = q1 - q0;
@@ -580,11 +588,17 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
   RangeHost &H = P.host;
   std::vector<int> order, lev;
   level_order(n, iapc, japc, forward, order, lev);
-  int R = std::max(32, (rows + 31) / 32 * 32);
-  while (!range_layout(n, iapc, japc, forward, order, lev, R, fp32 ? 4 : 8, H)) {
-    if (R <= 256) return false;
-    R = std::max(256, R / 2);
+  // full slices in ranges of at least 256 rows, else narrow ones in any
+  const int R0 = std::max(32, (rows + 31) / 32 * 32);
+  bool fits = false;
+  for (int block : {INT_MAX, kNarrowBlock}) {
+    const int least = block == INT_MAX ? 256 : 32;
+    for (int R = R0; !fits; R = std::max(least, R / 2)) {
+      fits = range_layout(n, iapc, japc, forward, order, lev, R, block, fp32 ? 4 : 8, H);
+      if (R <= least) break;
+    }
   }
+  if (!fits) return false;
   P.n = n;
   P.R = H.R;
   P.nr = H.nr;

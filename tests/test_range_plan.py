@@ -105,3 +105,25 @@ def test_wide_rows_bitexact(plans, w):
         # each row sums w products of at most max|z| / w: a few FP32 roundings
         # of the result's scale a row, which the 1/w factors damp
         assert np.max(np.abs(z32 - z)) <= 1e-4 * np.max(np.abs(z))
+
+
+def test_cut_slices_and_halved_ranges(plans):
+    """Levels of 32 rows and 128 entries, whose ring of full slices does not
+    fit, in narrower slices; halos that only fit smaller ranges; and a plan
+    that fits as it is, which stays with full slices."""
+    v = np.random.default_rng(3).standard_normal(8192)
+    iapc, japc, apc = factor_pattern(8192, lambda r: range(r - 32 * 128, r, 32), seed=1)
+    z, info = walk(plans, iapc, japc, apc, v, 2048)
+    np.testing.assert_array_equal(z, oracle.ilu0a(apc, iapc, japc, v, fma=True))
+    for i in info:
+        assert i["maxblock"] <= 16 * 1024 and i["slices"] > 8192 // 32
+    n = 40000
+    u = np.random.default_rng(4).standard_normal(n)
+    iapc, japc, apc = factor_pattern(n, lambda r: [r - 1, r - 8200, r - 16400, r - 24600], seed=2)
+    z, info = walk(plans, iapc, japc, apc, u, 8192)
+    np.testing.assert_array_equal(z, oracle.ilu0a(apc, iapc, japc, u, fma=True))
+    assert all(i["R"] == 4096 for i in info)
+    iapc, japc, apc = factor_pattern(3200, lambda r: range(r - 32 * 60, r, 32), seed=1)
+    z, info = walk(plans, iapc, japc, apc, v[:3200], 2048)
+    np.testing.assert_array_equal(z, oracle.ilu0a(apc, iapc, japc, v[:3200], fma=True))
+    assert all(i["slices"] == 100 for i in info)
