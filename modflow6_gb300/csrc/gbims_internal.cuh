@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -25,6 +26,24 @@ constexpr int kFuseRows = kMaxRedBlocks * kRedBlock;
 constexpr int kBodyIterations = 4;
 constexpr int kSell = 32;         // SELL slice height (one warp)
 constexpr int kMaxRowLen = 64;    // ILU0 factor: longest supported CSR row
+
+// A kernel's dynamic shared memory above 48 KB, asked for once on each device of
+// the process (the attribute is the device's) by whichever thread comes first;
+// a failure is left to the launch that follows.
+class SharedOptIn {
+  std::atomic<unsigned long long> asked{0};  // a bit a device
+
+ public:
+  template <class K>
+  void operator()(K *kernel, size_t bytes) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    const unsigned long long bit = dev < 64 ? 1ULL << dev : 0ULL;
+    if (bit && (asked.load(std::memory_order_acquire) & bit)) return;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess)
+      asked.fetch_or(bit, std::memory_order_release);
+  }
+};
 
 // Exit reasons reported in gbims_summary.exit_reason.
 enum ExitReason { kExitNone = 0, kExitClosure = 1, kExitStagnation = 2, kExitItmax = 3,

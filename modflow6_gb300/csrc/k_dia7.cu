@@ -999,12 +999,8 @@ int launch_dia7_extract(Dia7 &D, int n, const int *d_iapc, const int *d_japc,
 template <typename T, int C, int NS, int PF, int DIR>
 static void sweep_one(const SweepArgs<T> &a, const Dia7 &D, int occ, cudaStream_t st) {
   constexpr size_t bytes = stage_bytes<T, C, NS, DIR>();
-  static bool opted = false;
-  if (!opted) {  // allow up to the two-per-SM request
-    cudaFuncSetAttribute(k_dia7_sweep<T, kSOf<T>, C, NS, DIR, PF>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(bytes, kOcc2Smem));
-    opted = true;
-  }
+  static SharedOptIn opt_in;  // up to the two-per-SM request
+  opt_in(k_dia7_sweep<T, kSOf<T>, C, NS, DIR, PF>, std::max(bytes, kOcc2Smem));
   const size_t sm = (occ == 2) ? std::max(bytes, kOcc2Smem) : bytes;
   k_dia7_sweep<T, kSOf<T>, C, NS, DIR, PF><<<D.ntickets, sweep_threads(DIR), sm, st>>>(a);
 }

@@ -381,17 +381,15 @@ __global__ void k_ilut_scatter(IlutDev I, const int *__restrict__ iapc,
 
 }  // namespace
 
+static_assert(kIlutWarps * sizeof(IlutRow) <= 48 * 1024, "no opt-in needed");
 static int ilut_grid() {
-  static int blocks = -1;
-  if (blocks < 0) {
-    int per_sm = 1;
-    cudaFuncSetAttribute(k_ilut_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(kIlutWarps * sizeof(IlutRow)));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ilut_factor, 32 * kIlutWarps,
+  static const int per_sm = [] {  // every device is a GB300
+    int occ = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ilut_factor, 32 * kIlutWarps,
                                                   kIlutWarps * sizeof(IlutRow));
-    blocks = std::max(1, per_sm) * kNumSM;
-  }
-  return blocks;
+    return std::max(1, occ);
+  }();
+  return per_sm * kNumSM;
 }
 
 void launch_ilut_factor(const IlutDev &I, const int *d_ia, const int *d_ja, const double *d_amat,

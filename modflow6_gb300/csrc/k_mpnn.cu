@@ -804,13 +804,13 @@ void mpnn_forward(MpnnDev &D, const float *d_x, const float *target, const float
 constexpr size_t kLayerSmem = (kH + kTile) * (kCat + kPad) * 2 + kTile * kHs * 4;
 template <bool TRAIN>
 static int layer_grid(int tiles) {
-  static int per_sm = 0;
-  if (per_sm == 0) {
-    cudaFuncSetAttribute(k_layer<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLayerSmem);
+  static SharedOptIn opt_in;
+  opt_in(k_layer<TRAIN>, kLayerSmem);
+  static const int per_sm = [] {  // every device is a GB300
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_layer<TRAIN>, kLayerThreads, kLayerSmem);
-    per_sm = std::max(1, occ);
-  }
+    return std::max(1, occ);
+  }();
   return std::min(per_sm * kNumSM, tiles);
 }
 
@@ -870,12 +870,9 @@ void mpnn_backward(MpnnDev &D, cudaStream_t st) {
   k_readout_bwd<<<ngrid((long long)n * 32, 256), 256, 0, st>>>(n, D.H[kL], D.dy, D.g + P::wout,
                                                                D.g + P::bout);
   const int tiles = (n + kTile - 1) / kTile;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(k_layer_bwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-    cudaFuncSetAttribute(k_layer_bwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
-    opted = true;
-  }
+  static SharedOptIn opt_in[2];
+  opt_in[0](k_layer_bwd<true>, kBwdSmem);
+  opt_in[1](k_layer_bwd<false>, kBwdSmem);
   // two blocks an SM fill the register files; one place is left for the loss
   // kernel beside them (a block without a place would run after all others
   // and double the layer's time)

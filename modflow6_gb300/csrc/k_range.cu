@@ -654,12 +654,8 @@ static void sweep_t(const RangePlan &P, const T *rhs, T *d, void *words, unsigne
   a.recip = ~0ULL / (unsigned long long)P.nr;
   a.err = err;
   a.ctl = ctl;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(k_range_sweep<T, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSmemBytes);
-    opted = true;
-  }
+  static SharedOptIn opt_in;
+  opt_in(k_range_sweep<T, DIR>, kSmemBytes);
   const size_t sm = (size_t)P.stages * P.maxblock + ((sizeof(T) * (size_t)P.maxslots + 15) & ~(size_t)15);
   k_range_sweep<T, DIR><<<P.nr, kRangeThreads, sm, st>>>(a);
 }

@@ -1,0 +1,109 @@
+"""What the library allocates, copies and launches, and where, on a stand-in for
+the CUDA runtime that writes it down (c_abi/host_cudart.cpp): no GPU."""
+import ctypes as C
+import re
+import shutil
+import subprocess
+from pathlib import Path
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from modflow6_gb300 import _lib
+from modflow6_gb300.ims import GENERAL, ImsLinear, ImsLinearSettings
+from test_gpu_batch_products import grid
+
+ROOT = Path(__file__).resolve().parents[1]
+
+
+@pytest.fixture(scope="module")
+def hostlib(tmp_path_factory):
+    """The library's own objects, linked with the stand-in."""
+    if shutil.which("nvcc") is None or shutil.which("g++") is None:
+        pytest.skip("nvcc or g++ not available")
+    from modflow6_gb300 import build
+    build.build()
+    out = tmp_path_factory.mktemp("host") / "libhost.so"
+    cuda = Path(shutil.which("nvcc")).resolve().parents[1]
+    objs = [str(build.OBJ / (s.stem + ".o")) for s in build.sources()]
+    cmd = ["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", str(cuda / "include"), "-o", str(out),
+           str(ROOT / "tests" / "c_abi" / "host_cudart.cpp"), *objs, "-Wl,-Bsymbolic", "-Wl,-z,defs"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    lib = C.CDLL(str(out))
+    for name, (res, args) in _lib._SIGS.items():
+        fn = getattr(lib, name)
+        fn.restype = res
+        fn.argtypes = args
+    lib.host_trace.restype = C.c_char_p
+    lib.host_bytes.restype = C.c_longlong
+    return lib
+
+
+@pytest.fixture
+def host(hostlib, monkeypatch):
+    monkeypatch.setattr(_lib, "_lib", hostlib)
+    hostlib.host_set_device(0)
+    hostlib.host_trace_clear()
+    yield hostlib
+    hostlib.host_set_device(0)
+
+
+def trace(host):
+    """The calls so far, kernels by their plain names; and a fresh trace."""
+    lines = host.host_trace().decode().splitlines()
+    host.host_trace_clear()
+    return [re.sub(r"_ZN\S*?(\d+)(k_[a-z0-9_]+)\S*", lambda m: m.group(2)[:int(m.group(1))], l) for l in lines]
+
+
+def launches(lines):
+    return [l.split()[2] for l in lines if l.startswith("launch ")]
+
+
+def band_pattern(n, offsets):
+    """A symmetric matrix of the given band offsets, diagonal first."""
+    ia, ja, a = np.zeros(n + 1, np.int32), [], []
+    for r in range(n):
+        row = sorted(c for o in offsets for c in (r - o, r + o) if 0 <= c < n)
+        ja += [r] + row
+        a += [-(len(row) + 1.0)] + [1.0] * len(row)
+        ia[r + 1] = len(ja)
+    return ia, np.array(ja, np.int32), np.array(a)
+
+
+def optins(lines, device):
+    return {l.split()[2]: int(l.split()[3]) for l in lines if l.startswith(f"optin {device} ")}
+
+
+def test_shared_memory_is_asked_for_on_each_device(host):
+    """A kernel's dynamic shared memory above 48 KB is a setting of the device
+    it runs on: handles on two devices of a process each ask for theirs."""
+    n = 6000
+    ia, ja, a = band_pattern(n, list(range(100, 109)) + list(range(2000, 2009)))
+    di, dj, da = band_pattern(n, [1, 50])
+    asked = {}
+    for device in (0, 1, 0):
+        host.host_set_device(device)
+        net = C.c_void_p()
+        assert host.gbmpnn_create(n, dj.size, _lib.iptr(di), _lib.iptr(dj), 1, C.byref(net)) == 0
+        x = np.zeros(n * 16, np.float32).ctypes.data_as(C.c_void_p)
+        y = np.zeros(n, np.float32).ctypes.data_as(C.c_void_p)
+        assert host.gbmpnn_forward(net, x, y) == 0
+        assert host.gbmpnn_gradients(net, x, y, y, 1.0, None, None) == 0
+        host.gbmpnn_destroy(net)
+        z = np.zeros(n)
+        ims = ImsLinear(ImsLinearSettings(structure=GENERAL)).imslinear_allocate(n, ia, ja)
+        assert host.gbims_factor(ims._h, _lib.dptr(a), None) == 0
+        assert host.gbims_precondition(ims._h, _lib.dptr(z), _lib.dptr(z)) == 0
+        gi, gj, ga = grid(2, 40, 75, np.random.default_rng(0))
+        ims = ImsLinear(ImsLinearSettings(structure=(2, 40, 75))).imslinear_allocate(n, gi, gj)
+        assert host.gbims_factor(ims._h, _lib.dptr(ga), None) == 0
+        assert host.gbims_set_tuning(ims._h, 6, 0, -1) == 0  # the tiling of two blocks an SM
+        assert host.gbims_precondition(ims._h, _lib.dptr(z), _lib.dptr(z)) == 0
+        lines = trace(host)
+        ran = {l.split()[2]: int(l.split()[4]) for l in lines if l.startswith("launch ")}
+        big = {k: b for k, b in ran.items() if b > 48 * 1024}
+        assert {"k_layer", "k_layer_bwd", "k_range_sweep", "k_dia7_sweep"} <= set(big)
+        asked.setdefault(device, {}).update(optins(lines, device))
+        assert all(asked[device].get(k, 0) >= b for k, b in big.items()), (device, big, asked)
