@@ -187,6 +187,12 @@ static int level_words_error(gbims_handle *h) {
   return GBIMS_OK;
 }
 
+// The members' control blocks gate a batch's products and sweeps.  Before a
+// call outside a solve they are cleared: a solve leaves them done.
+static cudaError_t clear_members(gbims_handle *h) {
+  return h->nm > 0 ? cudaMemsetAsync(h->d_ctls, 0, sizeof(Ctl) * h->nm, h->st) : cudaSuccess;
+}
+
 static void precond64(gbims_handle *h, const double *r, double *z) {
   if (h->structured && h->D.mapped) {
     // an IDOMAIN-reduced grid: the sweeps on the full grid
@@ -1189,6 +1195,7 @@ extern "C" int gbims_matvec(gbims_handle *h, const double *x, double *y) {
   if (!h || !x || !y) return GBIMS_ERR_ARG;
   if (!h->factored) return fail(h, GBIMS_ERR_STATE, "no matrix: call gbims_factor or gbims_apply first");
   GB_CUDA(h, cudaMemcpyAsync(h->v_d, x, sizeof(double) * h->n, cudaMemcpyHostToDevice, h->st));
+  GB_CUDA(h, clear_members(h));
   spmv64(h, h->v_d, h->d_rhs, nullptr);
   GB_CUDA(h, cudaGetLastError());
   GB_CUDA(h, cudaMemcpyAsync(y, h->d_rhs, sizeof(double) * h->n, cudaMemcpyDeviceToHost, h->st));
@@ -1207,6 +1214,7 @@ extern "C" int gbims_precondition(gbims_handle *h, const double *r, double *z) {
   c.pivot_fail = INT_MAX;
   *h->h_ctl = c;
   GB_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, h->st));
+  GB_CUDA(h, clear_members(h));
   if (!h->mixed) {
     precond64(h, h->v_d, h->d_rhs);
   } else {
@@ -1251,7 +1259,7 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
   c.alpha = 1.0e-30;  // keeps x unchanged to rounding in the update timing
   *h->h_ctl = c;
   GB_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, st));
-  if (h->nm > 0) GB_CUDA(h, cudaMemsetAsync(h->d_ctls, 0, sizeof(Ctl) * h->nm, st));
+  GB_CUDA(h, clear_members(h));
   const int eg = std::min(4 * kNumSM, (n + 255) / 256);
   if (!h->mixed) {
     k_zero_vec<<<eg, 256, 0, st>>>(n, h->v_p, h->v_q, h->v_z, nullptr);
@@ -1471,6 +1479,7 @@ extern "C" int gbims_time_kernels(gbims_handle *h, int reps, gbims_kernel_times 
   c.alpha = 1.0e-30;  // keeps x unchanged to rounding in the update timing
   *h->h_ctl = c;
   GB_CUDA(h, cudaMemcpyAsync(h->d_ctl, h->h_ctl, sizeof(Ctl), cudaMemcpyHostToDevice, st));
+  GB_CUDA(h, clear_members(h));
   int eg = std::min(4 * kNumSM, (n + 255) / 256);
   // deterministic, finite operands
   if (!h->mixed) {
@@ -1701,6 +1710,7 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
   GB_CUDA(h, dalloc(&h->d_bmc, mc.size()));
   GB_CUDA(h, dalloc(&h->d_bmr, mrow.size()));
   GB_CUDA(h, dalloc(&h->d_ctls, (size_t)nmembers));
+  GB_CUDA(h, cudaMemset(h->d_ctls, 0, sizeof(Ctl) * nmembers));
   GB_CUDA(h, cudaMallocHost((void **)&h->h_ctls, sizeof(Ctl) * nmembers));
   GB_CUDA(h, cudaMemcpy(h->d_bcm, cm.data(), sizeof(int) * cm.size(), cudaMemcpyHostToDevice));
   GB_CUDA(h, cudaMemcpy(h->d_bcr, cr.data(), sizeof(int) * cr.size(), cudaMemcpyHostToDevice));

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 from modflow6_gb300 import _lib
+from modflow6_gb300.ensemble import EnsembleLinear
 from modflow6_gb300.ims import GENERAL, ImsLinear, ImsLinearSettings
 from test_gpu_batch_products import grid
 
@@ -107,3 +108,25 @@ def test_shared_memory_is_asked_for_on_each_device(host):
         assert {"k_layer", "k_layer_bwd", "k_range_sweep", "k_dia7_sweep"} <= set(big)
         asked.setdefault(device, {}).update(optins(lines, device))
         assert all(asked[device].get(k, 0) >= b for k, b in big.items()), (device, big, asked)
+
+
+@pytest.mark.parametrize("shapes", [None, [(1, 5, 6)] * 3], ids=["general", "grids"])
+def test_batch_calls_clear_the_control_blocks(host, shapes):
+    """The members' control blocks gate a batch's products and sweeps: they are
+    cleared when the handle is made and before a call outside a solve."""
+    members = [grid(1, 5, 6, np.random.default_rng(0))] * 3
+    ia = np.concatenate([[0]] + [i[1:] + k * i[-1] for k, (i, _, _) in enumerate(members)]).astype(np.int32)
+    ja = np.concatenate([j + 30 * k for k, (_, j, _) in enumerate(members)]).astype(np.int32)
+    a = np.concatenate([m[2] for m in members])
+    v, t = np.zeros(90), _lib.GbimsKernelTimes()
+    ens = EnsembleLinear(ImsLinearSettings()).allocate(np.array([0, 30, 60, 90], np.int32), ia, ja, shapes)
+    assert host.gbims_factor(ens._h, _lib.dptr(a), None) == 0
+    trace(host)
+    for call in (lambda: host.gbims_matvec(ens._h, _lib.dptr(v), _lib.dptr(v)),
+                 lambda: host.gbims_precondition(ens._h, _lib.dptr(v), _lib.dptr(v)),
+                 lambda: host.gbims_time_kernels(ens._h, 1, C.byref(t))):
+        assert call() == 0
+        lines = trace(host)
+        first = next(i for i, l in enumerate(lines) if "spmv" in l or "sweep" in l)
+        assert any(l.startswith("memset") for l in lines[:first]), lines
+    ens.close()
