@@ -937,7 +937,7 @@ static int factor_core(gbims_handle *h) {
                        : launch_ilu_factor(n, h->d_ia, h->d_ja, h->d_amat, h->d_iapc, h->d_japc, h->d_apc, h->F,
                                            h->FW, h->s.relax, delta, ipcflag, h->d_ctl, st);
     if (rc != 0) return fail(h, GBIMS_ERR_CUDA, "ILU0 factorisation launch failed");
-    h->launches += h->dia_spmv ? 2 : 1;
+    h->launches += 2;
     GB_CUDA(h, cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     GB_CUDA(h, cudaStreamSynchronize(st));
     GB_CUDA(h, cudaGetLastError());

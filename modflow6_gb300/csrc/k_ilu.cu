@@ -96,8 +96,13 @@ constexpr int kShort = 6;  // lower and upper entries of a row of the short form
 // All lanes of a warp take their e-th lower entry together: an FP64
 // instruction costs the same for one lane as for 32.  Slices are claimed in
 // order, so the lowest unfinished one can always proceed, however many warps
-// are resident; every wait is bounded, and ends when a pivot has failed (the
-// attempt is void and retried).
+// are resident; every wait is bounded.
+//
+// Where a pivot fails, the attempt is void, and the last attempt's rows before
+// the first failure are the factor's (ImsLinearBase.f90:1010-1042).  So the
+// rows after a failed one are left out as soon as it is known, the rows before
+// it are all made, and the values go to APC from the words, by
+// k_ilu0_commit, up to the first failure.
 //
 // SHORT: rows of at most kShort lower and upper entries; their index work is
 // done before the waits.  MILU: the dropped-fill sum is needed (relax > 0);
@@ -107,29 +112,30 @@ template <bool SHORT, bool MILU>
 __global__ void __launch_bounds__(128) k_ilu0_factor(
     int nslices, const int2 *__restrict__ slices, const int *__restrict__ rows,
     const int *__restrict__ ia, const int *__restrict__ ja, const double *__restrict__ amat,
-    const int *__restrict__ iapc, const int *__restrict__ japc, double *apc,
-    LLWord<double> *words, unsigned ep, int *claim, double relax, double delta, int ipcflag, Ctl *ctl) {
+    const int *__restrict__ iapc, const int *__restrict__ japc, LLWord<double> *words, unsigned ep, int *claim, double relax, double delta, int ipcflag, Ctl *ctl) {
   const unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   volatile int *failed = &ctl->pivot_fail;
-  // false when a wait runs out or the attempt is void
-  auto keep_waiting = [&](unsigned &turns) -> bool {
-    if ((++turns & 63u) != 0) return true;
-    if (turns > (1u << 23)) {  // L2 round trips: seconds
-      if (lane == 0) atomicExch(&ctl->scratch_err, 1);
-      return false;
-    }
-    return __all_sync(all, *failed == INT_MAX && *(volatile int *)&ctl->scratch_err == 0);
-  };
   while (true) {
     int s = 0;
     if (lane == 0) s = atomicAdd(claim, 1);
     s = __shfl_sync(all, s, 0);
     if (s >= nslices) return;
-    if (!__all_sync(all, *failed == INT_MAX)) return;  // a row failed: the attempt is void
     const int2 sl = slices[s];
-    const bool mine = lane < sl.y;
     const int n = rows[sl.x + min(lane, sl.y - 1)];
+    bool mine = lane < sl.y && n < *failed;  // not behind a row that failed
+    if (!__any_sync(all, mine)) continue;
+    // false when a wait runs out
+    unsigned turns = 0;
+    auto keep_waiting = [&]() -> bool {
+      if ((++turns & 63u) != 0) return true;
+      if (turns > (1u << 23)) {  // L2 round trips: seconds
+        if (lane == 0) atomicExch(&ctl->scratch_err, 1);
+        return false;
+      }
+      mine = mine && n < *failed;
+      return __all_sync(all, *(volatile int *)&ctl->scratch_err == 0);
+    };
     const int ic0 = iapc[n], ic1 = iapc[n + 1], iu = japc[n];
     const int len = ic1 - ic0, nlow = iu - ic0;
     // w[0..len): off-diagonal slots in JAPC order; wd: the diagonal slot
@@ -192,15 +198,15 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
       else w[t] = x;
     };
     const int maxlow = __reduce_max_sync(all, mine ? nlow : 0);
-    unsigned turns = 0;
     if (SHORT) {
 #pragma unroll
       for (int e = 0; e < kShort; ++e) {
         if (e >= maxlow) break;
-        const bool act = mine && e < nlow;
+        bool act;
         LLRaw rd, ru[kShort];
         while (true) {
           bool ok = true;
+          act = mine && e < nlow;
           if (act) {
             ll_issue(words + col[e], rd);
 #pragma unroll
@@ -212,7 +218,7 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
               if (u < nu[e]) ok = ok && ll_ready<double>(ru[u], ep);
           }
           if (__all_sync(all, ok)) break;
-          if (!keep_waiting(turns)) return;
+          if (!keep_waiting()) return;
         }
         if (act) {
           double dv;
@@ -230,9 +236,8 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
       }
     } else {
       for (int e = 0; e < maxlow; ++e) {
-        const bool act = mine && e < nlow;
         int jcol = 0, uu0 = 0, uu1 = 0;
-        if (act) {
+        if (mine && e < nlow) {
           jcol = japc[ic0 + e];
           uu0 = japc[jcol];
           uu1 = iapc[jcol + 1];
@@ -241,9 +246,11 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
         const int most = __reduce_max_sync(all, uu1 - uu0);
         for (int ub = 0; ub == 0 || ub < most; ub += 4) {
           // the inverse pivot with the first four upper entries
+          bool act;
           LLRaw rd, ru[4];
           while (true) {
             bool ok = true;
+            act = mine && e < nlow;
             if (act) {
               if (ub == 0) ll_issue(words + jcol, rd);
 #pragma unroll
@@ -255,7 +262,7 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
                 if (uu0 + ub + u < uu1) ok = ok && ll_ready<double>(ru[u], ep);
             }
             if (__all_sync(all, ok)) break;
-            if (!keep_waiting(turns)) return;
+            if (!keep_waiting()) return;
           }
           if (act) {
             if (ub == 0) {
@@ -283,8 +290,9 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
       }
     }
     if (!mine) continue;
-    // the upper entries are final
+    // the upper entries are final (the lower ones go to APC from their words)
     for (int k = nlow; k < len; ++k) ll_put(words + ic0 + k, w[k], ep);
+    for (int k = 0; k < nlow; ++k) ll_put(words + ic0 + k, w[k], ep);
     // DIAGONAL (:1010-1037)
     const double d = wd;
     double tl = __dsub_rn(__dmul_rn(__dadd_rn(1.0, delta), d), __dmul_rn(relax, -nrs));
@@ -302,11 +310,18 @@ __global__ void __launch_bounds__(128) k_ilu0_factor(
       atomicMin(&ctl->pivot_fail, n);
       continue;
     }
-    const double inv = __drcp_rn(tl);
-    ll_put(words + n, inv, ep);
-    apc[n] = inv;
-    for (int k = 0; k < len; ++k) apc[ic0 + k] = w[k];
+    ll_put(words + n, __drcp_rn(tl), ep);
   }
+}
+
+// The rows before the first failure into APC; the others keep what they held.
+__global__ void __launch_bounds__(256) k_ilu0_commit(int n, const int *__restrict__ iapc,
+                                                     const LLWord<double> *__restrict__ words,
+                                                     double *__restrict__ apc, const Ctl *ctl) {
+  if (ctl->scratch_err) return;
+  const int rows = min(n, ctl->pivot_fail), end = iapc[rows];
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < end; p += gridDim.x * blockDim.x)
+    if (p < rows || p >= n) apc[p] = ll_val(words[p]);
 }
 
 // True when every row has at most kShort lower and upper entries.
@@ -334,15 +349,16 @@ int launch_ilu_factor(int n, const int *d_ia, const int *d_ja, const double *d_a
                       const int *d_iapc, const int *d_japc, double *d_apc, const Levels &L,
                       FactorWords &W, double relax, double delta, int ipcflag, Ctl *ctl,
                       cudaStream_t st) {
-  (void)n;
   if (factor_words_next(W, st) != 0) return -1;
   const long long warps = std::min<long long>((long long)(L.maxwidth + 31) / 32 * kFactorAhead, L.nslices);
   const int grid = (int)std::max<long long>(1, std::min<long long>((warps + 3) / 4, 8LL * kNumSM));
   auto *k = W.short_rows ? (relax > 0.0 ? k_ilu0_factor<true, true> : k_ilu0_factor<true, false>)
                          : (relax > 0.0 ? k_ilu0_factor<false, true> : k_ilu0_factor<false, false>);
-  k<<<grid, 128, 0, st>>>(L.nslices, L.d_slices, L.d_rows, d_ia, d_ja, d_amat, d_iapc, d_japc, d_apc,
-                          static_cast<LLWord<double> *>(W.words), W.epoch, W.claim, relax, delta,
-                          ipcflag, ctl);
+  LLWord<double> *words = static_cast<LLWord<double> *>(W.words);
+  k<<<grid, 128, 0, st>>>(L.nslices, L.d_slices, L.d_rows, d_ia, d_ja, d_amat, d_iapc, d_japc, words, W.epoch,
+                          W.claim, relax, delta, ipcflag, ctl);
+  k_ilu0_commit<<<std::min<int>((int)((W.count + 255) / 256), 8 * kNumSM), 256, 0, st>>>(n, d_iapc, words, d_apc,
+                                                                                        ctl);
   return 0;
 }
 
