@@ -124,8 +124,8 @@ static int fail(gbims_handle *h, int code, const std::string &msg) {
 // keeps F from the start).
 static void ensure_levels(gbims_handle *h) {
   if (h->levels_b) return;
-  if (h->ipc >= 3) levels_build_host(h->n, h->iapc, h->japc, true, h->F);
-  levels_build_host(h->n, h->iapc, h->japc, false, h->B);
+  if (h->ipc >= 3) levels_build_host(h->n, h->iapc, h->japc, true, h->F, h->st);
+  levels_build_host(h->n, h->iapc, h->japc, false, h->B, h->st);
   h->levels_b = true;
 }
 
@@ -139,8 +139,8 @@ static int ensure_ranges(gbims_handle *h) {
   if (h->structured) return GBIMS_OK;
   if (h->LW.mode == 1 && h->plan == 0) {
     const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
-    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed) ||
-        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed)) {
+    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, h->st) ||
+        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, h->st)) {
       cudaGetLastError();
       h->plan = -1;
     } else {
@@ -158,7 +158,7 @@ static int ensure_ranges(gbims_handle *h) {
     GB_CUDA(h, cudaMalloc(&h->LW.bwd, wb));
     GB_CUDA(h, cudaMalloc((void **)&h->LW.ticket, 256));
     GB_CUDA(h, cudaMalloc((void **)&h->LW.err, sizeof(int)));
-    GB_CUDA(h, cudaMemset(h->LW.err, 0, sizeof(int)));
+    GB_CUDA(h, cudaMemsetAsync(h->LW.err, 0, sizeof(int), h->st));
   }
   const long long nr = (long long)h->RF.nr << 32 | h->RB.nr;
   if (h->words_nr != nr) {
@@ -698,7 +698,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
   // level schedule of the factorisation (full DIS grids: the wavefront's order)
   if (h->ipc < 3) {
     if (!h->dia_spmv) {
-      levels_build_host(neq, h->iapc, h->japc, true, h->F);
+      levels_build_host(neq, h->iapc, h->japc, true, h->F, h->st);
       h->FW.short_rows = ilu_short_rows(neq, h->iapc, h->japc);
     }
     h->FW.count = h->dia_spmv ? (size_t)h->D.slots : (size_t)nja;

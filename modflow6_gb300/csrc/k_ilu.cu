@@ -19,7 +19,7 @@
 namespace gb {
 
 void levels_build_host(int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                       bool forward, Levels &L) {
+                       bool forward, Levels &L, cudaStream_t st) {
   std::vector<int> lev(n, 0);
   int nlev = 0;
   if (forward) {
@@ -57,9 +57,10 @@ void levels_build_host(int n, const std::vector<int> &iapc, const std::vector<in
   L.d_slices = nullptr;
   if (n > 0) {
     cudaMalloc(&L.d_rows, sizeof(int) * n);
-    cudaMemcpy(L.d_rows, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(L.d_rows, rows.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
     cudaMalloc(&L.d_slices, sizeof(int2) * sl.size());
-    cudaMemcpy(L.d_slices, sl.data(), sizeof(int2) * sl.size(), cudaMemcpyHostToDevice);
+    cudaMemcpyAsync(L.d_slices, sl.data(), sizeof(int2) * sl.size(), cudaMemcpyHostToDevice, st);
+    cudaStreamSynchronize(st);
   }
 }
 

@@ -440,8 +440,10 @@ __global__ void k_range_fill(int nent, const int *__restrict__ src, const int *_
     blk[dst[q]] = apc[src[q]];
 }
 
+// On the stream of the kernels that read it: work on a non-blocking stream does
+// not wait for copies on the legacy stream.
 template <typename V>
-bool upload(std::vector<V> &h, V **d, size_t *cap) {
+bool upload(const std::vector<V> &h, V **d, size_t *cap, cudaStream_t st) {
   if (h.size() > *cap || !*d) {
     if (*d) cudaFree(*d);
     *d = nullptr;
@@ -450,7 +452,7 @@ bool upload(std::vector<V> &h, V **d, size_t *cap) {
     if (cudaMalloc((void **)d, sizeof(V) * want) != cudaSuccess) return false;
     *cap = want;
   }
-  return h.empty() || cudaMemcpy(*d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+  return h.empty() || cudaMemcpyAsync(*d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st) == cudaSuccess;
 }
 
 }  // namespace
@@ -584,7 +586,7 @@ static void level_order(int n, const std::vector<int> &iapc, const std::vector<i
 }
 
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                 bool forward, int rows, bool fp32) {
+                 bool forward, int rows, bool fp32, cudaStream_t st) {
   RangeHost &H = P.host;
   std::vector<int> order, lev;
   level_order(n, iapc, japc, forward, order, lev);
@@ -606,10 +608,13 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
   P.stages = H.stages;
   P.maxblock = H.maxblock;
   P.nent = (int)H.src.size();
-  return upload(H.blk, &P.d_blk, &P.c_blk) && upload(H.off, &P.d_off, &P.c_off) &&
-         upload(H.rslice, &P.d_rslice, &P.c_rslice) && upload(H.src, &P.d_src, &P.c_src) &&
-         upload(H.dst, &P.d_dst, &P.c_dst) && upload(H.hptr, &P.d_hptr, &P.c_hptr) &&
-         upload(H.halo, &P.d_halo, &P.c_halo);
+  const bool sent =
+      upload(H.blk, &P.d_blk, &P.c_blk, st) && upload(H.off, &P.d_off, &P.c_off, st) &&
+      upload(H.rslice, &P.d_rslice, &P.c_rslice, st) && upload(H.src, &P.d_src, &P.c_src, st) &&
+      upload(H.dst, &P.d_dst, &P.c_dst, st) && upload(H.hptr, &P.d_hptr, &P.c_hptr, st) &&
+      upload(H.halo, &P.d_halo, &P.c_halo, st);
+  // the host arrays may go when this returns
+  return cudaStreamSynchronize(st) == cudaSuccess && sent;
 }
 
 void range_free(RangePlan &P) {

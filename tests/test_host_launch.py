@@ -130,3 +130,19 @@ def test_batch_calls_clear_the_control_blocks(host, shapes):
         first = next(i for i, l in enumerate(lines) if "spmv" in l or "sweep" in l)
         assert any(l.startswith("memset") for l in lines[:first]), lines
     ens.close()
+
+
+@pytest.mark.parametrize("level", [0, 3], ids=["ilu0", "ilut"])
+def test_plans_are_sent_on_the_handles_stream(host, level):
+    """Work on the handle's stream, which does not wait for the legacy stream,
+    reads the sweeps' plans and level schedules: their copies go on it too."""
+    ia, ja, a = band_pattern(3000, [1, 50])
+    ims = ImsLinear(ImsLinearSettings(structure=GENERAL, level=level)).imslinear_allocate(3000, ia, ja)
+    trace(host)
+    assert host.gbims_factor(ims._h, _lib.dptr(a), None) == 0
+    assert host.gbims_set_tuning(ims._h, -1, 0, 0) == 0
+    assert host.gbims_set_tuning(ims._h, -1, 0, 1) == 0
+    assert host.gbims_factor(ims._h, _lib.dptr(a), None) == 0
+    lines = trace(host)
+    assert "k_range_fill" in launches(lines)
+    assert not [l for l in lines if re.match(r"(memcpy|memset) 0 ", l)]
