@@ -1250,6 +1250,9 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
   if (!h->factored) return fail(h, GBIMS_ERR_STATE, "no factor: call gbims_factor or an apply first");
   memset(out, 0, sizeof(*out));
   out->sweep_config = -1;
+  // the captured loop's kernels read plans that are replaced below, whatever
+  // becomes of this call
+  drop_graph(h);
   const int n = h->n;
   cudaStream_t st = h->st;
   // control blocks that let every kernel run (batch members included)
@@ -1394,7 +1397,6 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     out->vector_ms = bt;
   }
   GB_CUDA(h, cudaGetLastError());
-  drop_graph(h);
   return GBIMS_OK;
 }
 
@@ -1443,9 +1445,15 @@ extern "C" int gbims_set_dis_nodes(gbims_handle *h, const int *nodeuser) {
 extern "C" int gbims_set_tuning(gbims_handle *h, int sweep_config, int reduction_blocks,
                                 int level_mode) {
   if (!h) return GBIMS_ERR_ARG;
+  // all of it is checked before any of it changes
+  if (level_mode >= 0 && (h->structured || level_mode > 1))
+    return fail(h, GBIMS_ERR_ARG, "level mode out of range (or a structured handle)");
+  if (sweep_config >= 0 && (!h->structured || sweep_config >= dia7_num_cfgs()))
+    return fail(h, GBIMS_ERR_ARG, "sweep configuration out of range (or not a structured handle)");
+  if (reduction_blocks > 0 && (h->nm > 0 || reduction_blocks > h->G_alloc))
+    return fail(h, GBIMS_ERR_ARG, "reduction blocks out of range (or a batch handle)");
+  drop_graph(h);
   if (level_mode >= 0) {
-    if (h->structured || level_mode > 1)
-      return fail(h, GBIMS_ERR_ARG, "level mode out of range (or a structured handle)");
     h->LW.mode = level_mode;
     if (h->factored) {  // the factor's values for the form chosen
       if (int rc = ensure_ranges(h)) return rc;
@@ -1453,17 +1461,10 @@ extern "C" int gbims_set_tuning(gbims_handle *h, int sweep_config, int reduction
     }
   }
   if (sweep_config >= 0) {
-    if (!h->structured || sweep_config >= dia7_num_cfgs())
-      return fail(h, GBIMS_ERR_ARG, "sweep configuration out of range (or not a structured handle)");
     h->D.cfg = sweep_config;
     h->D.cfg_b = -1;
   }
-  if (reduction_blocks > 0) {
-    if (h->nm > 0 || reduction_blocks > h->G_alloc)
-      return fail(h, GBIMS_ERR_ARG, "reduction blocks out of range (or a batch handle)");
-    h->G = reduction_blocks;
-  }
-  drop_graph(h);
+  if (reduction_blocks > 0) h->G = reduction_blocks;
   return GBIMS_OK;
 }
 

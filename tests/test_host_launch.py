@@ -146,3 +146,30 @@ def test_plans_are_sent_on_the_handles_stream(host, level):
     lines = trace(host)
     assert "k_range_fill" in launches(lines)
     assert not [l for l in lines if re.match(r"(memcpy|memset) 0 ", l)]
+
+
+def solve_launches(host, ims, a):
+    n = ims.neq
+    trace(host)
+    ims.imslinear_apply(a.copy(), np.ones(n), np.zeros(n))
+    return trace(host)
+
+
+def test_refused_and_failed_tuning_leave_no_stale_loop(host):
+    """A solve's captured loop sweeps with what the factorisation has just
+    filled, also after a tuning that was refused or that failed half way."""
+    ia, ja, a = band_pattern(3000, [1, 50])
+    ims = ImsLinear(ImsLinearSettings(structure=GENERAL, iter1=1)).imslinear_allocate(3000, ia, ja)
+    first = set(launches(solve_launches(host, ims, a)))
+    assert {"k_range_fill", "k_range_sweep"} <= first
+    # refused for its tiling: nothing of it is taken
+    assert host.gbims_set_tuning(ims._h, 99, 0, 0) == _lib.GBIMS_ERR_ARG
+    assert set(launches(solve_launches(host, ims, a))) == first
+    # a tuning that fails after it has replaced the plans: captured again
+    host.host_fail_copy(4)
+    assert host.gbims_autotune(ims._h, 1, C.byref(_lib.GbimsTuning())) == _lib.GBIMS_ERR_CUDA
+    lines = solve_launches(host, ims, a)
+    assert "capture" in lines and {"k_range_fill", "k_range_sweep"} <= set(launches(lines))
+    assert host.gbims_set_tuning(ims._h, -1, 0, 0) == 0
+    lines = launches(solve_launches(host, ims, a))
+    assert "k_ilu_fwd_level" in lines and not {"k_range_fill", "k_range_sweep"} & set(lines)
