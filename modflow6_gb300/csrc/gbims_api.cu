@@ -139,8 +139,9 @@ static int ensure_ranges(gbims_handle *h) {
   if (h->structured) return GBIMS_OK;
   if (h->LW.mode == 1 && h->plan == 0) {
     const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
-    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, h->st) ||
-        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, h->st)) {
+    const bool spare = h->ipc >= 3;
+    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, spare, h->st) ||
+        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, spare, h->st)) {
       cudaGetLastError();
       h->plan = -1;
     } else {
@@ -1759,13 +1760,17 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
     h->S = Sell();
     GB_CUDA(h, dalloc(&h->D.d_sv, (size_t)7 * neq));
     if (h->mixed) GB_CUDA(h, dalloc(&h->D.f_sv, (size_t)7 * neq));
-    if ((size_t)h->D.slots > h->FW.count) {
+    // the wavefront's factor: a word a slot, no level schedule
+    if ((size_t)h->D.slots != h->FW.count) {
       cudaFree(h->FW.words);
       h->FW.words = nullptr;
       h->FW.count = (size_t)h->D.slots;
       GB_CUDA(h, cudaMalloc(&h->FW.words, 16 * h->FW.count));
       GB_CUDA(h, cudaMemset(h->FW.words, 0, 16 * h->FW.count));
     }
+    cudaFree(h->F.d_rows);
+    cudaFree(h->F.d_slices);
+    h->F = Levels();
     h->D.rows.nchunks = nchunks;
     h->D.rows.n = neq;
     h->D.rows.cm = h->d_bcm;

@@ -362,10 +362,10 @@ void launch_ilu_apply_levels32(int n, const int *d_iapc, const int *d_japc,
 constexpr int kRangeRows = 2048;
 // The plan of one sweep of the pattern iapc/japc in ranges of about `rows`
 // rows (fewer, and slices of fewer rows, where a range would not fit the shared
-// memory), uploaded on st; false when no range size fits or device memory runs
-// out.
+// memory), uploaded on st; spare: with room for another pattern's plan (ILUT).
+// False when no range size fits or device memory runs out.
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                 bool forward, int rows, bool fp32, cudaStream_t st);
+                 bool forward, int rows, bool fp32, bool spare, cudaStream_t st);
 void range_free(RangePlan &P);
 void launch_range_fill(const RangePlan &F, const RangePlan &B, const double *apc, cudaStream_t st);
 void launch_range_fill32(const RangePlan &F, const RangePlan &B, const float *apc, cudaStream_t st);

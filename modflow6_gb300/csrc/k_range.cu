@@ -441,14 +441,14 @@ __global__ void k_range_fill(int nent, const int *__restrict__ src, const int *_
 }
 
 // On the stream of the kernels that read it: work on a non-blocking stream does
-// not wait for copies on the legacy stream.
+// not wait for copies on the legacy stream.  spare: room for the next pattern.
 template <typename V>
-bool upload(const std::vector<V> &h, V **d, size_t *cap, cudaStream_t st) {
+bool upload(const std::vector<V> &h, V **d, size_t *cap, bool spare, cudaStream_t st) {
   if (h.size() > *cap || !*d) {
     if (*d) cudaFree(*d);
     *d = nullptr;
     *cap = 0;
-    const size_t want = std::max<size_t>(1, h.size() + h.size() / 8);
+    const size_t want = std::max<size_t>(1, h.size() + (spare ? h.size() / 8 : 0));
     if (cudaMalloc((void **)d, sizeof(V) * want) != cudaSuccess) return false;
     *cap = want;
   }
@@ -586,7 +586,7 @@ static void level_order(int n, const std::vector<int> &iapc, const std::vector<i
 }
 
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                 bool forward, int rows, bool fp32, cudaStream_t st) {
+                 bool forward, int rows, bool fp32, bool spare, cudaStream_t st) {
   RangeHost &H = P.host;
   std::vector<int> order, lev;
   level_order(n, iapc, japc, forward, order, lev);
@@ -609,10 +609,10 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
   P.maxblock = H.maxblock;
   P.nent = (int)H.src.size();
   const bool sent =
-      upload(H.blk, &P.d_blk, &P.c_blk, st) && upload(H.off, &P.d_off, &P.c_off, st) &&
-      upload(H.rslice, &P.d_rslice, &P.c_rslice, st) && upload(H.src, &P.d_src, &P.c_src, st) &&
-      upload(H.dst, &P.d_dst, &P.c_dst, st) && upload(H.hptr, &P.d_hptr, &P.c_hptr, st) &&
-      upload(H.halo, &P.d_halo, &P.c_halo, st);
+      upload(H.blk, &P.d_blk, &P.c_blk, spare, st) && upload(H.off, &P.d_off, &P.c_off, spare, st) &&
+      upload(H.rslice, &P.d_rslice, &P.c_rslice, spare, st) && upload(H.src, &P.d_src, &P.c_src, spare, st) &&
+      upload(H.dst, &P.d_dst, &P.c_dst, spare, st) && upload(H.hptr, &P.d_hptr, &P.c_hptr, spare, st) &&
+      upload(H.halo, &P.d_halo, &P.c_halo, spare, st);
   // the host arrays may go when this returns
   return cudaStreamSynchronize(st) == cudaSuccess && sent;
 }

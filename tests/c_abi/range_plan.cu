@@ -10,11 +10,14 @@
 namespace {
 
 // What is wrong with a plan: 0 nothing.
-enum { kOk = 0, kNoPlan = 1, kSmem = 2, kSlotEmpty = 3, kSlotTwice = 4, kWordMissing = 5, kBlock = 6 };
+enum { kOk = 0, kNoPlan = 1, kSmem = 2, kSlotEmpty = 3, kSlotTwice = 4, kWordMissing = 5, kBlock = 6, kSpare = 7 };
 
 template <typename T>
 int walk(const gb::RangePlan &P, bool forward, const T *apc, const T *rhs, T *out) {
   const size_t smem = (size_t)P.stages * P.maxblock + sizeof(T) * (size_t)P.maxslots;
+  const gb::RangeHost &H = P.host;
+  const size_t entries = std::max<size_t>(1, H.src.size());
+  if (P.c_blk != H.blk.size() || P.c_src != entries || P.c_dst != entries) return kSpare;
   if (P.stages < gb::kMinStages || P.stages > gb::kMaxStages || smem > gb::kSmemBytes) return kSmem;
   T *vals = reinterpret_cast<T *>(P.d_blk);
   for (int q = 0; q < P.nent; ++q) vals[P.d_dst[q]] = apc[P.d_src[q]];
@@ -82,7 +85,7 @@ extern "C" int range_walk64(int n, const int *iapc, const int *japc, int njapc, 
                             int forward, int rows, const double *rhs, double *out, int *info) {
   gb::RangePlan P;
   std::vector<int> ia(iapc, iapc + n + 1), ja(japc, japc + njapc);
-  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, false, nullptr)) return kNoPlan;
+  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, false, false, nullptr)) return kNoPlan;
   const int v[5] = {P.R, P.nr, P.stages, P.maxblock, (int)P.host.off.size() - 1};
   std::memcpy(info, v, sizeof(v));
   const int rc = walk<double>(P, forward != 0, apc, rhs, out);
@@ -94,7 +97,7 @@ extern "C" int range_walk32(int n, const int *iapc, const int *japc, int njapc, 
                             int forward, int rows, const float *rhs, float *out, int *info) {
   gb::RangePlan P;
   std::vector<int> ia(iapc, iapc + n + 1), ja(japc, japc + njapc);
-  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, true, nullptr)) return kNoPlan;
+  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, true, false, nullptr)) return kNoPlan;
   const int v[5] = {P.R, P.nr, P.stages, P.maxblock, (int)P.host.off.size() - 1};
   std::memcpy(info, v, sizeof(v));
   const int rc = walk<float>(P, forward != 0, apc, rhs, out);

@@ -173,3 +173,21 @@ def test_refused_and_failed_tuning_leave_no_stale_loop(host):
     assert host.gbims_set_tuning(ims._h, -1, 0, 0) == 0
     lines = launches(solve_launches(host, ims, a))
     assert "k_ilu_fwd_level" in lines and not {"k_range_fill", "k_range_sweep"} & set(lines)
+
+
+def test_memory_of_a_batch_of_grids(host):
+    """A batch of one grid holds what a handle of the grid does, besides its
+    chunks' and members' few words: no words by nonzero, no level schedule."""
+    ia, ja, a = grid(4, 64, 96, np.random.default_rng(0))
+    n = ia.size - 1
+    before = host.host_bytes()
+    one = ImsLinear(ImsLinearSettings(structure=(4, 64, 96))).imslinear_allocate(n, ia, ja)
+    single = host.host_bytes() - before
+    before = host.host_bytes()
+    ens = EnsembleLinear(ImsLinearSettings()).allocate(np.array([0, n], np.int32), ia.astype(np.int32),
+                                                       ja.astype(np.int32), [(4, 64, 96)])
+    batch = host.host_bytes() - before
+    assert abs(batch - single) <= 16 * 1024
+    ens.close()
+    one.imslinear_da()
+    assert host.host_bytes() == before - single
