@@ -234,11 +234,11 @@ static void residual64(gbims_handle *h, const Ctl *c, int only_if_north_due) {
 }
 
 // Whether the products are fused with the Krylov steps around them: on
-// systems up to kFuseRows rows whose reductions have a block per 256 rows (no
-// tuned grid), and not where the records' kernel reads P between them.
+// systems up to kFuseRows rows, and not where the records' kernel reads P
+// between them.  Their sums have a block per 256 rows whatever the tuned grid
+// of the other reductions.
 static bool fused(const gbims_handle *h) {
-  return h->nm == 0 && h->n <= kFuseRows && h->G == (h->n + kRedBlock - 1) / kRedBlock &&
-         !(h->rec_cap > 0 && h->rec_nmod > 1);
+  return h->nm == 0 && h->n <= kFuseRows && !(h->rec_cap > 0 && h->rec_nmod > 1);
 }
 
 static void spmv_fin(gbims_handle *h, int op, const void *x, const void *w, void *p0, void *p1, void *y) {
