@@ -196,13 +196,12 @@ int gbims_time_kernels(gbims_handle *h, int reps, gbims_kernel_times *t);
  * on the handle's own factored system it times every wavefront tiling of
  * the structured sweeps (chunk of steps per ring buffer, ring depth,
  * neighbour-word prefetch depth, CTAs per SM), the form and the range size
- * of the sweeps of other patterns, and the thread-block count of the
- * dot/update reductions, and keeps the fastest for the following applies.
- * The tiling does not change any cell's arithmetic; the reduction grid only
- * changes the order in which the partial sums are added (systems of up to
- * 311,296 rows sum the dot products that are fused with a product in blocks of
- * 256 rows whatever the grid).  Batched handles
- * tune the tiling only.  reps: timed applications per candidate. */
+ * of the sweeps of other patterns, and, above 311,296 rows, the thread-block
+ * count of the dot/update reductions, and keeps the fastest for the following
+ * applies.  The tiling does not change any cell's arithmetic; the reduction
+ * grid only changes the order in which the partial sums are added (smaller
+ * systems keep a block per 256 rows, and the tuned solve is the untuned one bit
+ * for bit).  Batched handles tune the tiling only.  reps: timed applications per candidate. */
 typedef struct gbims_tuning {
   int sweep_config;                 /* chosen tiling, -1 when the handle has no wavefront sweeps */
   int sweep_chunk, sweep_ring, sweep_prefetch;

@@ -1372,11 +1372,16 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     out->precond_ms = bt;
   }
   if (h->nm == 0) {
-    // reduction blocks: multiples of the SM count up to the allocated grid
+    // reduction blocks: multiples of the SM count up to the allocated grid.  Up
+    // to kFuseRows rows it stays a block per 256 rows: 152 to 608 blocks take
+    // the same time there (DISV 4 x 250 x 250 587 us an iteration with each),
+    // and every rounding of the untuned solve stays with it.  On 120,000 rows
+    // of XT3D, whose outer closure sits at the inner one, a step took 4 outer
+    // iterations with 152 blocks, 20 with 304 and 6 without tuning.
     int best = h->G;
     double bt = 1e300;
     std::vector<int> cand;
-    for (int g = kNumSM; g < h->G_alloc; g *= 2) cand.push_back(g);
+    for (int g = kNumSM; g < h->G_alloc && n > kFuseRows; g *= 2) cand.push_back(g);
     cand.push_back(h->G_alloc);
     for (int g : cand) {
       const double ms = time_it([&] {
