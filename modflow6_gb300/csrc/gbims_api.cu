@@ -233,12 +233,15 @@ static void residual64(gbims_handle *h, const Ctl *c, int only_if_north_due) {
   else launch_residual64(h->S, h->d_x, h->d_rhs, h->v_d, c, only_if_north_due, h->st);
 }
 
-// Whether the products are fused with the Krylov steps around them: on
-// systems up to kFuseRows rows, and not where the records' kernel reads P
-// between them.  Their sums have a block per 256 rows whatever the tuned grid
-// of the other reductions.
+// Whether the products are fused with the Krylov steps around them: by size
+// (gbims_internal.cuh), and not where the records' kernel reads P between them.
+// Their sums have a block per 256 rows whatever the tuned grid of the other
+// reductions.
+static bool fusible(const gbims_handle *h) {
+  return h->n <= kFuseRows && (h->dia_spmv || h->nja <= kFuseEntries[h->bcgs]);
+}
 static bool fused(const gbims_handle *h) {
-  return h->nm == 0 && h->n <= kFuseRows && !(h->rec_cap > 0 && h->rec_nmod > 1);
+  return h->nm == 0 && fusible(h) && !(h->rec_cap > 0 && h->rec_nmod > 1);
 }
 
 static void spmv_fin(gbims_handle *h, int op, const void *x, const void *w, void *p0, void *p1, void *y) {
@@ -717,7 +720,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, dalloc(&h->v_p, nn));
     GB_CUDA(h, dalloc(&h->v_q, nn));
     GB_CUDA(h, dalloc(&h->v_z, nn));
-    if (!h->bcgs && neq <= kFuseRows) GB_CUDA(h, dalloc(&h->v_p1, nn));
+    if (!h->bcgs && fusible(h)) GB_CUDA(h, dalloc(&h->v_p1, nn));
     if (h->bcgs) {
       GB_CUDA(h, dalloc(&h->v_t, nn)); GB_CUDA(h, dalloc(&h->v_v, nn));
       GB_CUDA(h, dalloc(&h->v_dhat, nn)); GB_CUDA(h, dalloc(&h->v_phat, nn));
@@ -728,7 +731,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
     GB_CUDA(h, dalloc(&h->d_apc32, npc));
     GB_CUDA(h, dalloc(&h->f_d, nn)); GB_CUDA(h, dalloc(&h->f_p, nn));
     GB_CUDA(h, dalloc(&h->f_q, nn)); GB_CUDA(h, dalloc(&h->f_z, nn));
-    if (!h->bcgs && neq <= kFuseRows) GB_CUDA(h, dalloc(&h->f_p1, nn));
+    if (!h->bcgs && fusible(h)) GB_CUDA(h, dalloc(&h->f_p1, nn));
     if (h->bcgs) {
       GB_CUDA(h, dalloc(&h->f_t, nn)); GB_CUDA(h, dalloc(&h->f_v, nn));
       GB_CUDA(h, dalloc(&h->f_dhat, nn)); GB_CUDA(h, dalloc(&h->f_phat, nn));

@@ -15,9 +15,21 @@ namespace gb {
 constexpr int kNumSM = 152;       // GB300: 2 dies x 76 SMs
 constexpr int kRedBlock = 256;    // threads per reduction block
 constexpr int kMaxRedBlocks = 8 * kNumSM;  // grid of reduction kernels: 8 x 256 threads per SM
-// Systems up to this size run their products fused with the Krylov steps
-// around them (k_sparse.cu)
+// Systems of up to kFuseRows rows, and on general patterns of up to kFuseEntries
+// entries (PCG, BiCGSTAB), run their products fused with the Krylov steps around
+// them (k_sparse.cu).  The rows are those of a reduction grid of a block per 256
+// rows: up to there the fused sums are the separate kernels' bit for bit.  An
+// iteration fused / separate, us, FP64 PCG: full DIS grids of 10,000 cells
+// 61.4 / 64.4, 100,000 97.1 / 100.8, 200,000 134.0 / 134.8, 300,000 151.1 /
+// 152.5 (BiCGSTAB 114.3 / 119.1 to 285.1 / 283.4, mixed PCG 55.1 / 59.4 to 129.7
+// / 134.0).  On general patterns the direction is recomputed for each entry:
+// 0.7 million entries 301.7 / 301.7, 1.9 million 794.5 / 793.4, DISV 4 x 250 x
+// 250 with 2.2 million 574 / 563, 5.7 million 1437 / 1387 (mixed 266.0 / 273.6,
+// 617 / 624, -, 1112 / 1106).  BiCGSTAB recomputes nothing: 577.6 / 583.9, 1419 /
+// 1428, XT3D 3 x 200 x 200 with 2.4 million 2650 / 2665 (of several outer
+// iterations), 5.7 million 2574 / 2530.
 constexpr int kFuseRows = kMaxRedBlocks * kRedBlock;
+constexpr int kFuseEntries[2] = {2000000, 3000000};
 // Iterations in one body of the inner loop's graph on those systems: a turn of
 // the WHILE node costs 3 us, an iteration's kernels after the end of the loop
 // about 6.  1x20x30 2.45 -> 2.33 ms a step at 4 and 2.34 at 8, 1x100x100 11.42

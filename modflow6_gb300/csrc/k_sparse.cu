@@ -331,10 +331,11 @@ void launch_residual64(const Sell &S, const double *x, const double *b, double *
 // Products fused with the Krylov steps around them (SpmvFin), for systems
 // where launches and the gaps between them are what an iteration costs: the
 // search direction's update, the product, its dot product and the scalar are
-// one kernel instead of four.  The direction is recomputed at each row's
+// one kernel instead of four.  PCG's direction is recomputed at each row's
 // neighbours, which doubles the product's FP64 instructions: on large systems,
-// where those bound it, the kernels stay apart.  One row a thread, 256 rows a
-// block: the rows, and so the partial sums, of k_dot's blocks.
+// where those bound it, the kernels stay apart (kFuseRows, kFuseEntries, with
+// both sides measured).  One row a thread, 256 rows a block: the rows, and so
+// the partial sums, of k_dot's blocks.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double prod_sum(double a, double b) { return fma(a, b, 0.0); }
 __device__ __forceinline__ double prod_sum(float a, float b) {

@@ -211,3 +211,22 @@ def test_tuned_loop_keeps_its_form(host, precision, accel):
     assert launches(solve_launches(host, ims, a)) == first
     assert host.gbims_set_tuning(ims._h, -1, 17, -1) == 0
     assert launches(solve_launches(host, ims, a)) == first
+
+
+@pytest.mark.parametrize("accel", [1, 2])
+def test_fused_products_by_size(host, accel):
+    """Fused on full grids up to 311,296 rows, and on general patterns up to two
+    million entries (BiCGSTAB three)."""
+    def products(n, ia, ja, a, structure):
+        ims = ImsLinear(ImsLinearSettings(structure=structure, iter1=1, ilinmeth=accel)).imslinear_allocate(n, ia, ja)
+        return {k for k in launches(solve_launches(host, ims, a)) if "spmv" in k}
+    most = 1000000 * (1 + accel)
+    below, above = most // 63, most // 63 + 100  # rows of 63 entries, fewer at both ends
+    for n, offsets, fused in ((32000, [1, 40], True), (below, range(1, 32), True), (above, range(1, 32), False)):
+        ia, ja, a = band_pattern(n, offsets)
+        assert (ja.size <= most) == fused
+        assert ("k_sell_spmv_fin" in products(n, ia, ja, a, GENERAL)) == fused
+    for shape, fused in (((1, 608, 512), True), ((1, 608, 513), False)):
+        ia, ja, a = grid(*shape, np.random.default_rng(0))
+        ia, ja = ia.astype(np.int32), ja.astype(np.int32)
+        assert ("k_dia7_spmv_fin" in products(ia.size - 1, ia, ja, a, shape)) == fused
