@@ -191,7 +191,7 @@ struct SweepArgs {
 template <typename T, int C, int DIR>
 struct Stage;
 // rv: the step's own right-hand side (forward r, backward dinv*y), written
-// by the edge warp; the pre-compute warp folds the layer term into it.
+// by the rhs warp; the pre-compute warp folds the layer term into it.
 template <typename T, int C>
 struct alignas(16) Stage<T, C, 1> {
   T a[C * 32], b[C * 32], x[C * 32];
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(sweep_threads(DIR)) k_dia7_sweep(SweepArgs<T> 
   unsigned long long *full = reinterpret_cast<unsigned long long *>(smem_raw + NS * sizeof(St));
   unsigned long long *empty = full + NS;
   unsigned long long *prep = full + 2 * NS;
-  unsigned long long *rdy = full + 3 * NS;  // rv written (edge warp)
+  unsigned long long *rdy = full + 3 * NS;  // rv written (rhs warp)
   unsigned long long *ofull = full + 4 * NS, *oempty = ofull + 2;  // backward: the out warp's buffers
   OutBuf<T, C> *ob = reinterpret_cast<OutBuf<T, C> *>(smem_raw + NS * sizeof(St) +
                                                       (4 * NS + 4) * sizeof(unsigned long long));
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(sweep_threads(DIR)) k_dia7_sweep(SweepArgs<T> 
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
       mbar_init(&prep[s], 2);  // pre-compute warp + edge warp
-      mbar_init(&rdy[s], 1);   // edge warp
+      mbar_init(&rdy[s], 1);   // rhs warp
     }
     if (DIR < 0)
       for (int q = 0; q < 2; ++q) {

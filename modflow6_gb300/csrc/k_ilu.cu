@@ -1,8 +1,9 @@
-// k_ilu.cu -- ILU0 / MILU0 factorisation of general patterns and the triangular sweeps
-// a level at a time.
+// k_ilu.cu -- ILU0 / MILU0 factorisation of general patterns and the triangular
+// sweeps a level at a time.
 //
 // Factorisation: ims_base_pcilu0 (src/Solution/LinearMethods/ImsLinearBase.f90:928-1042)
-// restated per row, one thread per row, in one launch (see k_ilu0_factor).
+// restated per row in one launch, a lane a row, the lanes of a warp through
+// their lower entries together (see k_ilu0_factor).
 // The row's work vector W is indexed by the row's sorted pattern (IAPC/JAPC
 // from ims_base_pccrs); every update to a W slot and to the dropped-fill sum
 // rs happens in the reference's order, and every operation is rounded
