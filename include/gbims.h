@@ -209,10 +209,12 @@ typedef struct gbims_tuning {
   int reduction_blocks;             /* chosen reduction grid (0: batched handle) */
   int level_mode;                   /* general sweeps (handles without wavefront
                                        sweeps): 0 one launch per level, 1 one launch
-                                       per sweep over ranges of rows; -1 not applicable */
+                                       per sweep (over ranges of rows, or sync-free
+                                       where levels are few); -1 not applicable */
   double level_ms[2];               /* one ILU0 application in each level mode */
   int ncandidates;                  /* tilings timed (general sweeps: ranges of 512,
-                                       1024, 2048, 4096 and 8192 rows) */
+                                       1024, 2048, 4096 and 8192 rows, those that
+                                       fit; then the sync-free form) */
   double candidate_ms[16];          /* one ILU0 application per candidate */
   double precond_ms;                /* of the chosen tilings */
   double vector_ms;                 /* dot + update at the chosen grid */

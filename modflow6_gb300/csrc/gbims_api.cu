@@ -63,7 +63,8 @@ struct gbims_handle {
   bool no_graph = false;   // GBIMS_GRAPH=0: the host drives the loop
   LevelWords LW;           // the general sweeps' result words (unstructured handles)
   RangePlan RF, RB;        // their plans, and the range size asked for (0: the default)
-  int plan = 0;            // the current pattern: not planned yet, planned (1), no plan (-1)
+  int form = 0;            // of mode 1: by the pattern (0), ranges (1), sync-free (2)
+  int plan = 0;            // the current pattern's: not chosen yet (0), ranges, planned (1), sync-free (2)
   int range_rows = 0;
   long long words_nr = 0;  // the grids that the words' epochs count launches of
   bool levels_b = false;   // B (and, for ILUT, F) holds the current factor's levels
@@ -131,28 +132,28 @@ static void ensure_levels(gbims_handle *h) {
 
 // The range sweeps' plans of the current pattern and their words, zeroed
 // before their first use and whenever the grid changes (its tickets number
-// the launches); a handle with wavefront sweeps never needs them.  A pattern
-// that no range size fits is swept level by level.
+// the launches); a handle with wavefront sweeps never needs them.  Patterns of
+// few and wide levels, and those that no range size fits, are swept sync-free.
 static bool by_ranges(const gbims_handle *h) { return h->LW.mode == 1 && h->plan == 1; }
+static bool sync_free(const gbims_handle *h) { return h->LW.mode == 1 && h->plan == 2; }
 
 static int ensure_ranges(gbims_handle *h) {
   if (h->structured) return GBIMS_OK;
   if (h->LW.mode == 1 && h->plan == 0) {
     const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
     const bool spare = h->ipc >= 3;
-    if (!range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, spare, h->st) ||
-        !range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, spare, h->st)) {
-      cudaGetLastError();
-      h->plan = -1;
-    } else {
-      h->plan = 1;
+    h->plan = 2;
+    if (h->form == 1 || (h->form == 0 && ranges_faster(h->n, h->iapc, h->japc, R))) {
+      if (range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, spare, h->st) &&
+          range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, spare, h->st))
+        h->plan = 1;
+      else
+        cudaGetLastError();
     }
     if (h->ipc < 3) h->RF.host = h->RB.host = RangeHost();
   }
-  if (!by_ranges(h)) {
-    ensure_levels(h);
-    return GBIMS_OK;
-  }
+  if (!by_ranges(h)) ensure_levels(h);
+  if (h->LW.mode == 0) return GBIMS_OK;
   const size_t wb = (size_t)h->n * (h->mixed ? 8 : 16);
   if (!h->LW.fwd) {
     GB_CUDA(h, cudaMalloc(&h->LW.fwd, wb));
@@ -161,7 +162,7 @@ static int ensure_ranges(gbims_handle *h) {
     GB_CUDA(h, cudaMalloc((void **)&h->LW.err, sizeof(int)));
     GB_CUDA(h, cudaMemsetAsync(h->LW.err, 0, sizeof(int), h->st));
   }
-  const long long nr = (long long)h->RF.nr << 32 | h->RB.nr;
+  const long long nr = by_ranges(h) ? (long long)h->RF.nr << 32 | h->RB.nr : -1;  // (the other grid is fixed)
   if (h->words_nr != nr) {
     GB_CUDA(h, cudaMemsetAsync(h->LW.fwd, 0, wb, h->st));
     GB_CUDA(h, cudaMemsetAsync(h->LW.bwd, 0, wb, h->st));
@@ -202,6 +203,7 @@ static void precond64(gbims_handle *h, const double *r, double *z) {
     launch_dia7_collect(h->D, h->n, h->D.d_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply64(h->D, r, z, h->d_ctl, h->st);
   else if (by_ranges(h)) launch_range_apply(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else if (sync_free(h)) launch_ilu_apply_sf(h->n, h->d_iapc, h->d_japc, h->d_apc, h->F, h->B, h->LW, r, z, h->d_ctl, h->st);
   else launch_ilu_apply_levels(h->n, h->d_iapc, h->d_japc, h->d_apc, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
@@ -213,6 +215,7 @@ static void precond32(gbims_handle *h, const float *r, float *z) {
     launch_dia7_collect32(h->D, h->n, h->D.f_zfull, z, h->st);
   } else if (h->structured) launch_dia7_apply32(h->D, r, z, h->d_ctl, h->st);
   else if (by_ranges(h)) launch_range_apply32(h->RF, h->RB, h->LW, r, z, h->d_ctl, h->st);
+  else if (sync_free(h)) launch_ilu_apply_sf32(h->n, h->d_iapc, h->d_japc, h->d_apc32, h->F, h->B, h->LW, r, z, h->d_ctl, h->st);
   else launch_ilu_apply_levels32(h->n, h->d_iapc, h->d_japc, h->d_apc32, h->F, h->B, r, z, h->d_ctl, h->st);
 }
 
@@ -1336,10 +1339,10 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
   out->level_mode = -1;
   if (!h->structured) {
     // general sweeps: one launch per level, or one launch per sweep over row
-    // ranges of each size (level_ms[1] is the best of them, candidate_ms the
-    // time at each)
+    // ranges of each size or sync-free (level_ms[1] is the best of them,
+    // candidate_ms the time of each)
     double bt = 1e300;
-    int best = 0, best_rows = 0;
+    int best = 0, best_rows = 0, best_form = h->form;
     auto pre = [&] {
       if (!h->mixed) precond64(h, h->v_p, h->v_z);
       else precond32(h, h->f_p, h->f_z);
@@ -1349,30 +1352,31 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     out->level_ms[0] = time_it(pre);
     bt = out->level_ms[0];
     out->level_ms[1] = 1e300;
-    auto with_rows = [&](int rows) -> int {
+    auto with_rows = [&](int form, int rows) -> int {
       h->LW.mode = 1;
+      h->form = form;
       h->range_rows = rows;
       h->plan = 0;
       if (int rc = ensure_ranges(h)) return rc;
       fill_ranges(h);
       return GBIMS_OK;
     };
-    for (int rows : {512, 1024, 2048, 4096, 8192}) {
-      if (int rc = with_rows(rows)) return rc;
-      if (!by_ranges(h)) break;  // no range size fits the pattern
+    const int rows_before = h->range_rows;
+    for (int rows : {512, 1024, 2048, 4096, 8192, 0}) {  // 0: sync-free
+      if (int rc = with_rows(rows ? 1 : 2, rows ? rows : rows_before)) return rc;
+      if (rows && !by_ranges(h)) continue;  // no range size fits the pattern
       const double ms = time_it(pre);
       out->candidate_ms[out->ncandidates++] = ms;
       out->level_ms[1] = std::min(out->level_ms[1], ms);
       if (ms < bt) {
         bt = ms;
         best = 1;
-        best_rows = rows;
+        best_form = rows ? 1 : 2;
+        best_rows = h->range_rows;
       }
     }
     if (int rc = level_words_error(h)) return rc;
-    if (best == 1) {
-      if (int rc = with_rows(best_rows)) return rc;
-    }
+    if (int rc = with_rows(best_form, best == 1 ? best_rows : rows_before)) return rc;
     h->LW.mode = best;
     out->level_mode = best;
     out->precond_ms = bt;

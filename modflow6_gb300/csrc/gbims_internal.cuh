@@ -186,10 +186,10 @@ struct FactorWords {
 constexpr int kFactorAhead = 4;
 
 // The sweeps of general patterns: mode 0 launches one kernel per level; mode 1
-// runs each sweep as one launch over row ranges (k_range.cu), which hand
-// values to one another in result words tagged with the launch's epoch (fwd,
-// bwd: n words each, 16 bytes in FP64, 8 in FP32, zeroed once; ticket: two
-// counters, 128 bytes apart, zeroed once).
+// runs each sweep as one launch, over row ranges (k_range.cu) or sync-free
+// (k_ilu.cu), which hand values over in result words tagged with the launch's
+// epoch (fwd, bwd: n words each, 16 bytes in FP64, 8 in FP32; ticket: two
+// counters, 128 bytes apart; zeroed whenever the grid changes).
 struct LevelWords {
   int mode = 1;
   void *fwd = nullptr, *bwd = nullptr;
@@ -372,6 +372,13 @@ void launch_ilu_apply_levels32(int n, const int *d_iapc, const int *d_japc,
 // 164 us, XT3D on 15,000 cells 298, 296, 314 and 307 us (5.5, 2.9 and 2.6 ms
 // with a launch per level).
 constexpr int kRangeRows = 2048;
+// One sync-free launch per sweep (k_ilu.cu), rows in level order.
+void launch_ilu_apply_sf(int n, const int *d_iapc, const int *d_japc, const double *d_apc, const Levels &F,
+                         const Levels &B, const LevelWords &W, const double *r, double *d, Ctl *ctl,
+                         cudaStream_t st);
+void launch_ilu_apply_sf32(int n, const int *d_iapc, const int *d_japc, const float *d_apc32, const Levels &F,
+                           const Levels &B, const LevelWords &W, const float *r, float *d, Ctl *ctl,
+                           cudaStream_t st);
 // The plan of one sweep of the pattern iapc/japc in ranges of about `rows`
 // rows (fewer, and slices of fewer rows, where a range would not fit the shared
 // memory), uploaded on st; spare: with room for another pattern's plan (ILUT).
@@ -379,6 +386,9 @@ constexpr int kRangeRows = 2048;
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
                  bool forward, int rows, bool fp32, bool spare, cudaStream_t st);
 void range_free(RangePlan &P);
+// Whether both sweeps of the pattern are estimated to be faster over ranges of
+// about `rows` rows than sync-free.
+bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows);
 void launch_range_fill(const RangePlan &F, const RangePlan &B, const double *apc, cudaStream_t st);
 void launch_range_fill32(const RangePlan &F, const RangePlan &B, const float *apc, cudaStream_t st);
 void launch_range_apply(const RangePlan &F, const RangePlan &B, const LevelWords &W, const double *r,
