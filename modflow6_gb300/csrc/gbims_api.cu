@@ -143,14 +143,19 @@ static int ensure_ranges(gbims_handle *h) {
     const int R = h->range_rows > 0 ? h->range_rows : kRangeRows;
     const bool spare = h->ipc >= 3;
     h->plan = 2;
-    if (h->form == 1 || (h->form == 0 && ranges_faster(h->n, h->iapc, h->japc, R))) {
-      if (range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, spare, h->st) &&
-          range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, spare, h->st))
+    std::vector<int> levels[2];
+    if (h->form == 1 || (h->form == 0 && ranges_faster(h->n, h->iapc, h->japc, R, levels))) {
+      const std::vector<int> *lf = h->form == 0 ? &levels[0] : nullptr, *lb = h->form == 0 ? &levels[1] : nullptr;
+      if (range_build(h->RF, h->n, h->iapc, h->japc, true, R, h->mixed, spare, lf, h->st) &&
+          range_build(h->RB, h->n, h->iapc, h->japc, false, R, h->mixed, spare, lb, h->st))
         h->plan = 1;
       else
         cudaGetLastError();
     }
-    if (h->ipc < 3) h->RF.host = h->RB.host = RangeHost();
+    if (h->ipc < 3) {
+      h->RF.host = RangeHost();
+      h->RB.host = RangeHost();
+    }
   }
   if (!by_ranges(h)) ensure_levels(h);
   if (h->LW.mode == 0) return GBIMS_OK;

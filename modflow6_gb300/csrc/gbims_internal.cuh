@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -199,10 +200,30 @@ struct LevelWords {
 
 // Plan of one range sweep (k_range.cu): rows cut into nr ranges of R; the
 // host arrays while it is built, and their device copies.
+template <typename V>
+class RawArray {  // not initialised; its memory stays for the next plan
+  std::unique_ptr<V[]> p;
+  size_t n = 0, cap = 0;
+
+ public:
+  void need(size_t count) {
+    if (count > cap) {
+      p.reset();
+      cap = 0;
+      p.reset(new V[count]);
+      cap = count;
+    }
+    n = count;
+  }
+  V *data() { return p.get(); }
+  const V *data() const { return p.get(); }
+  size_t size() const { return n; }
+};
 struct RangeHost {
   int R = 0, nr = 0, maxslots = 0, maxblock = 0, stages = 0;
-  std::vector<int> rows, off, rslice, src, dst, hptr, halo;
-  std::vector<unsigned char> blk;
+  std::vector<int> rows, off, rslice, hptr, halo;
+  RawArray<int> src, dst;
+  RawArray<unsigned char> blk;
 };
 struct RangePlan {
   int n = 0, R = 0, nr = 0, maxslots = 0, maxblock = 0, stages = 0, nent = 0;
@@ -381,14 +402,17 @@ void launch_ilu_apply_sf32(int n, const int *d_iapc, const int *d_japc, const fl
                            cudaStream_t st);
 // The plan of one sweep of the pattern iapc/japc in ranges of about `rows`
 // rows (fewer, and slices of fewer rows, where a range would not fit the shared
-// memory), uploaded on st; spare: with room for another pattern's plan (ILUT).
-// False when no range size fits or device memory runs out.
+// memory), uploaded on st; spare: with room for another pattern's plan (ILUT);
+// levels: the rows' levels, if they are known.  False when no range size fits or
+// memory runs out.
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                 bool forward, int rows, bool fp32, bool spare, cudaStream_t st);
+                 bool forward, int rows, bool fp32, bool spare, const std::vector<int> *levels,
+                 cudaStream_t st);
 void range_free(RangePlan &P);
 // Whether both sweeps of the pattern are estimated to be faster over ranges of
-// about `rows` rows than sync-free.
-bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows);
+// about `rows` rows than sync-free; the rows' levels in both sweeps.
+bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows,
+                   std::vector<int> (&levels)[2]);
 void launch_range_fill(const RangePlan &F, const RangePlan &B, const double *apc, cudaStream_t st);
 void launch_range_fill32(const RangePlan &F, const RangePlan &B, const float *apc, cudaStream_t st);
 void launch_range_apply(const RangePlan &F, const RangePlan &B, const LevelWords &W, const double *r,

@@ -51,8 +51,11 @@
 // over through L2): DISV hexagons 4 x 150 x 150 1885 -> 288 us, XT3D 3 x 70 x 70
 // 1668 -> 283 us, ILUT (5, 1e-4) on 6 x 60 x 60 cells 1538 -> 242 us.
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstring>
+#include <memory>
+#include <thread>
 
 #include "gbims_internal.cuh"
 #include "k_llword.cuh"
@@ -442,161 +445,255 @@ __global__ void k_range_fill(int nent, const int *__restrict__ src, const int *_
 
 // On the stream of the kernels that read it: work on a non-blocking stream does
 // not wait for copies on the legacy stream.  spare: room for the next pattern.
-template <typename V>
-bool upload(const std::vector<V> &h, V **d, size_t *cap, bool spare, cudaStream_t st) {
-  if (h.size() > *cap || !*d) {
+template <class H, typename V>
+bool upload(const H &h, V **d, size_t *cap, bool spare, cudaStream_t st) {
+  const size_t n = h.size();
+  if (n > *cap || !*d) {
     if (*d) cudaFree(*d);
     *d = nullptr;
     *cap = 0;
-    const size_t want = std::max<size_t>(1, h.size() + (spare ? h.size() / 8 : 0));
+    const size_t want = std::max<size_t>(1, n + (spare ? n / 8 : 0));
     if (cudaMalloc((void **)d, sizeof(V) * want) != cudaSuccess) return false;
     *cap = want;
   }
-  return h.empty() || cudaMemcpyAsync(*d, h.data(), sizeof(V) * h.size(), cudaMemcpyHostToDevice, st) == cudaSuccess;
+  return n == 0 || cudaMemcpyAsync(*d, h.data(), sizeof(V) * n, cudaMemcpyHostToDevice, st) == cudaSuccess;
+}
+
+// f(i, thread) for i < count on up to `most` threads; false when one returned
+// false or threw.
+constexpr int kPlanThreads = 8;
+template <class F>
+bool parallel(int count, long long work, F f, int most = kPlanThreads) {
+  std::atomic<int> next{0};
+  std::atomic<bool> ok{true};
+  auto run = [&](int thread) {
+    try {
+      for (int i; ok && (i = next.fetch_add(1)) < count;)
+        if (!f(i, thread)) ok = false;
+    } catch (...) {
+      ok = false;
+    }
+  };
+  // a thread costs some 30 us, an entry some 10 ns
+  const int want = (int)std::min<long long>({(long long)most, (long long)count, 1 + work / 20000,
+                                             (long long)std::max(1u, std::thread::hardware_concurrency())});
+  std::vector<std::thread> others;
+  try {
+    for (int t = 1; t < want; ++t) others.emplace_back(run, t);
+  } catch (...) {  // fewer threads, then
+  }
+  run(0);
+  for (std::thread &t : others) t.join();
+  return ok;
 }
 
 }  // namespace
 
 // The plan of one sweep for ranges of R rows, its slices' blocks of at most
 // `block` bytes where they have more than one row; false when a range's slots
-// and the ring exceed the shared memory.  `order`: all rows by level, `lev`
-// their levels.
+// and the ring exceed the shared memory.  `lev`: the rows' levels.  The ranges
+// are laid out side by side: one thread took 8 ms for the 930,000 entries of an
+// ILUT factor of 100,000 rows, at every factorisation, and most of a first solve.
 static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                         bool forward, const std::vector<int> &order, const std::vector<int> &lev,
-                         int R, int block, size_t tsize, RangeHost &P) {
+                         bool forward, const std::vector<int> &lev, int R, int block, size_t tsize,
+                         RangeHost &P) {
   const int nr = (n + R - 1) / R;
+  const long long work = (long long)iapc[n] - iapc[0] + n;
   P.R = R;
   P.nr = nr;
-  // the rows of each range in level order
+  auto first = [&](int r) { return forward ? iapc[r] : japc[r]; };
+  auto last = [&](int r) { return forward ? japc[r] : iapc[r + 1]; };
+  struct Slice {
+    int q, nl, w;
+  };
+  struct Range {
+    std::vector<Slice> slices;
+    std::vector<int> halo;
+    long long bytes = 0, entries = 0;
+    int maxblock = 0;
+  };
+  std::vector<Range> ranges(nr);
   P.rows.resize(n);
-  {
-    std::vector<int> fill(nr);
-    for (int b = 0; b < nr; ++b) fill[b] = b * R;
-    for (int r : order) P.rows[fill[r / R]++] = r;
-  }
   std::vector<int> place(n);  // row -> its slot, when it is its range's own
-  for (int q = 0; q < n; ++q) place[P.rows[q]] = q % R;
-  P.rslice.assign(nr + 1, 0);
-  P.hptr.assign(nr + 1, 0);
-  P.off.assign(1, 0);
-  P.halo.clear();
-  P.blk.clear();
-  P.src.clear();
-  P.dst.clear();
-  P.maxslots = 0;
-  P.maxblock = 0;
-  std::vector<int> mark(n, -1), hidx(n);
-  std::vector<char> read(n, 0);
-  for (int b = 0; b < nr; ++b) {
+  // the rows of each range in level order, cut into slices of up to 32 rows of
+  // one level
+  const bool cut = parallel(nr, work, [&](int b, int) {
+    Range &G = ranges[b];
     const int r0 = b * R, nloc = std::min(R, n - r0);
-    const int h0 = (int)P.halo.size();
-    std::vector<size_t> pads;
-    for (int q0 = r0; q0 < r0 + nloc;) {
-      // a slice: up to 32 rows of one level
+    int lo = INT_MAX, hi = 0;
+    for (int r = r0; r < r0 + nloc; ++r) {
+      lo = std::min(lo, lev[r]);
+      hi = std::max(hi, lev[r]);
+    }
+    int *rows = &P.rows[r0];
+    if (hi - lo < 4 * nloc) {
+      std::vector<int> at(hi - lo + 2, 0);
+      for (int r = r0; r < r0 + nloc; ++r) at[lev[r] - lo + 1]++;
+      for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
+      for (int r = r0; r < r0 + nloc; ++r) rows[at[lev[r] - lo]++] = r;
+    } else {
+      for (int q = 0; q < nloc; ++q) rows[q] = r0 + q;
+      std::stable_sort(rows, rows + nloc, [&](int a, int c) { return lev[a] < lev[c]; });
+    }
+    for (int q = 0; q < nloc; ++q) place[rows[q]] = q;
+    for (int q0 = 0; q0 < nloc;) {
       int q1 = q0, w = 0;
-      const int l0 = lev[P.rows[q0]];
-      for (; q1 < r0 + nloc && q1 < q0 + 32 && lev[P.rows[q1]] == l0; ++q1) {
-        const int r = P.rows[q1];
-        const int wide = std::max(w, forward ? japc[r] - iapc[r] : iapc[r + 1] - japc[r]);
+      const int l0 = lev[rows[q0]];
+      for (; q1 < nloc && q1 < q0 + 32 && lev[rows[q1]] == l0; ++q1) {
+        const int wide = std::max(w, last(rows[q1]) - first(rows[q1]));
         if (q1 > q0 && BlockLayout(q1 + 1 - q0, wide, (int)tsize).bytes > block) break;
         w = wide;
       }
       if (w > 65535) return false;
-      const int nl = q1 - q0;
-      const BlockLayout L(nl, w, (int)tsize);
-      const size_t at = P.blk.size();
-      if ((at + L.bytes) / 16 > (size_t)INT_MAX || (at + L.bytes) / tsize > (size_t)INT_MAX) return false;
-      P.blk.resize(at + L.bytes, 0);
-      const SliceHead head = SliceHead::pack(nl, w, q0 - r0, L);
-      memcpy(&P.blk[at], &head, sizeof(head));
-      memcpy(&P.blk[at + L.rows], &P.rows[q0], sizeof(int) * nl);
-      for (int l = 0; l < nl; ++l) {
-        const int r = P.rows[q0 + l];
-        const int j0 = forward ? iapc[r] : japc[r], j1 = forward ? japc[r] : iapc[r + 1];
-        for (int e = 0; e < w; ++e) {
-          const size_t sp = at + L.slots + 2 * ((size_t)e * nl + l);
-          if (j0 + e >= j1) {
-            pads.push_back(sp);
-            continue;
-          }
-          const int dep = japc[j0 + e];
-          int sl = place[dep];
-          if (dep < r0 || dep >= r0 + nloc) {
-            if (mark[dep] != b) {
-              mark[dep] = b;
-              hidx[dep] = (int)P.halo.size() - h0;
-              P.halo.push_back(dep);
-              read[dep] = 1;
-            }
-            sl = nloc + hidx[dep];
-          }
-          if (sl > 65534) return false;
-          *reinterpret_cast<unsigned short *>(&P.blk[sp]) = (unsigned short)sl;
-          P.src.push_back(j0 + e);
-          P.dst.push_back((int)((at + L.vals) / tsize + (size_t)e * nl + l));
-        }
-        if (!forward) {
-          P.src.push_back(r);
-          P.dst.push_back((int)((at + L.dinv) / tsize + l));
-        }
-      }
-      P.off.push_back((int)(P.blk.size() / 16));
-      P.maxblock = std::max(P.maxblock, L.bytes);
+      const int bytes = BlockLayout(q1 - q0, w, (int)tsize).bytes;
+      G.slices.push_back(Slice{q0, q1 - q0, w});
+      G.bytes += bytes;
+      G.maxblock = std::max(G.maxblock, bytes);
       q0 = q1;
     }
-    P.rslice[b + 1] = (int)P.off.size() - 1;
-    P.hptr[b + 1] = (int)P.halo.size();
-    const int zero = nloc + P.hptr[b + 1] - h0;  // the slot after the halo
-    if (zero > 65535) return false;
-    for (size_t sp : pads) *reinterpret_cast<unsigned short *>(&P.blk[sp]) = (unsigned short)zero;
-    P.maxslots = std::max(P.maxslots, zero + 1);
+    for (int r = r0; r < r0 + nloc; ++r) G.entries += last(r) - first(r);
+    if (!forward) G.entries += nloc;
+    return true;
+  });
+  if (!cut) return false;
+  // where each range's parts start
+  std::vector<long long> byte0(nr + 1, 0), entry0(nr + 1, 0);
+  P.rslice.assign(nr + 1, 0);
+  P.maxblock = 0;
+  for (int b = 0; b < nr; ++b) {
+    byte0[b + 1] = byte0[b] + ranges[b].bytes;
+    entry0[b + 1] = entry0[b] + ranges[b].entries;
+    P.rslice[b + 1] = P.rslice[b] + (int)ranges[b].slices.size();
+    P.maxblock = std::max(P.maxblock, ranges[b].maxblock);
   }
+  if (byte0[nr] / 16 > INT_MAX || byte0[nr] / (long long)tsize > INT_MAX || entry0[nr] > INT_MAX) return false;
   P.stages = (int)std::min<size_t>(kMaxStages, std::max<size_t>(kMinStages, kRingBytes / P.maxblock));
-  if ((size_t)P.stages * P.maxblock + tsize * (size_t)P.maxslots > kSmemBytes) return false;
-  if (P.src.size() > (size_t)INT_MAX) return false;
-  // which rows other ranges read is known now
-  for (size_t s = 0; s + 1 < P.off.size(); ++s) {
-    unsigned char *block = &P.blk[16 * (size_t)P.off[s]];
-    const int nl = reinterpret_cast<const SliceHead *>(block)->rows();
-    int *rows = reinterpret_cast<int *>(block + sizeof(SliceHead));
-    for (int l = 0; l < nl; ++l)
-      if (read[rows[l]]) rows[l] = ~rows[l];
+  P.blk.need((size_t)byte0[nr]);
+  P.src.need((size_t)entry0[nr]);
+  P.dst.need((size_t)entry0[nr]);
+  P.off.resize((size_t)P.rslice[nr] + 1);
+  P.off[P.rslice[nr]] = (int)(byte0[nr] / 16);
+  // the blocks; which rows other ranges read is only known when all are done
+  std::unique_ptr<std::atomic<unsigned char>[]> read(new std::atomic<unsigned char>[(size_t)n]);
+  struct Scratch {
+    std::vector<int> mark, hidx;
+    std::vector<size_t> pads;
+  };
+  // (two words a row and thread: at most 800 MB, or one thread's)
+  const int threads = (int)std::max(1LL, std::min((long long)kPlanThreads, 100000000LL / n));
+  std::vector<Scratch> scratch(threads);
+  const bool filled = parallel(nr, work, [&](int b, int) {
+    const int r0 = b * R, nloc = std::min(R, n - r0);
+    for (int r = r0; r < r0 + nloc; ++r) read[r].store(0, std::memory_order_relaxed);
+    return true;
+  }) && parallel(nr, work, [&](int b, int thread) {
+    Range &G = ranges[b];
+    Scratch &S = scratch[thread];
+    if (S.mark.empty()) {
+      S.mark.assign(n, -1);
+      S.hidx.resize(n);
+    }
+    S.pads.clear();
+    const int r0 = b * R, nloc = std::min(R, n - r0);
+    size_t at = (size_t)byte0[b], en = (size_t)entry0[b];
+    int s = P.rslice[b];
+    unsigned char *blk = P.blk.data();
+    int *src = P.src.data(), *dst = P.dst.data();
+    for (const Slice &sl : G.slices) {
+      const int nl = sl.nl, w = sl.w, *rows = &P.rows[r0 + sl.q];
+      const BlockLayout L(nl, w, (int)tsize);
+      memset(blk + at, 0, L.bytes);
+      const SliceHead head = SliceHead::pack(nl, w, sl.q, L);
+      memcpy(blk + at, &head, sizeof(head));
+      memcpy(blk + at + L.rows, rows, sizeof(int) * nl);
+      unsigned short *slots = reinterpret_cast<unsigned short *>(blk + at + L.slots);
+      const int val0 = (int)((at + L.vals) / tsize), dinv0 = (int)((at + L.dinv) / tsize);
+      for (int l = 0; l < nl; ++l) {
+        const int r = rows[l], j0 = first(r), j1 = last(r);
+        for (int j = j0, e = 0; j < j1; ++j, ++e) {
+          const int dep = japc[j];
+          int slot;
+          if (dep >= r0 && dep - r0 < nloc) {
+            slot = place[dep];
+          } else {
+            if (S.mark[dep] != b) {
+              S.mark[dep] = b;
+              S.hidx[dep] = (int)G.halo.size();
+              G.halo.push_back(dep);
+              read[dep].store(1, std::memory_order_relaxed);
+            }
+            slot = nloc + S.hidx[dep];
+          }
+          if (slot > 65534) return false;
+          slots[e * nl + l] = (unsigned short)slot;
+          src[en] = j;
+          dst[en++] = val0 + e * nl + l;
+        }
+        for (int e = j1 - j0; e < w; ++e) S.pads.push_back(at + L.slots + 2 * ((size_t)e * nl + l));
+        if (!forward) {
+          src[en] = r;
+          dst[en++] = dinv0 + l;
+        }
+      }
+      P.off[s++] = (int)(at / 16);
+      at += L.bytes;
+    }
+    const int zero = nloc + (int)G.halo.size();  // the slot after the halo
+    if (zero > 65535) return false;
+    for (size_t sp : S.pads) *reinterpret_cast<unsigned short *>(blk + sp) = (unsigned short)zero;
+    return true;
+  }, threads);
+  if (!filled) return false;
+  P.hptr.assign(nr + 1, 0);
+  P.halo.clear();
+  P.maxslots = 0;
+  for (int b = 0; b < nr; ++b) {
+    const Range &G = ranges[b];
+    P.halo.insert(P.halo.end(), G.halo.begin(), G.halo.end());
+    P.hptr[b + 1] = (int)P.halo.size();
+    P.maxslots = std::max(P.maxslots, std::min(R, n - b * R) + (int)G.halo.size() + 1);
   }
-  return true;
+  if ((size_t)P.stages * P.maxblock + tsize * (size_t)P.maxslots > kSmemBytes) return false;
+  return parallel(nr, work, [&](int b, int) {
+    for (int s = P.rslice[b]; s < P.rslice[b + 1]; ++s) {
+      unsigned char *bl = P.blk.data() + 16 * (size_t)P.off[s];
+      SliceHead head;
+      memcpy(&head, bl, sizeof(head));
+      int *rows = reinterpret_cast<int *>(bl + sizeof(SliceHead));
+      for (int l = 0; l < head.rows(); ++l)
+        if (read[rows[l]].load(std::memory_order_relaxed)) rows[l] = ~rows[l];
+    }
+    return true;
+  });
 }
 
-// Rows by level: a counting sort of the levels of one sweep.
-static void level_order(int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                        bool forward, std::vector<int> &order, std::vector<int> &lev) {
+// The rows' levels in one sweep.
+static void sweep_levels(int n, const std::vector<int> &iapc, const std::vector<int> &japc,
+                         bool forward, std::vector<int> &lev) {
   lev.assign(n, 0);
-  int nlev = 0;
   for (int q = 0; q < n; ++q) {
     const int r = forward ? q : n - 1 - q;
     const int j0 = forward ? iapc[r] : japc[r], j1 = forward ? japc[r] : iapc[r + 1];
     int l = 0;
     for (int j = j0; j < j1; ++j) l = std::max(l, lev[japc[j]] + 1);
     lev[r] = l;
-    nlev = std::max(nlev, l + 1);
   }
-  std::vector<int> ptr(nlev + 1, 0);
-  for (int r = 0; r < n; ++r) ptr[lev[r] + 1]++;
-  for (int l = 0; l < nlev; ++l) ptr[l + 1] += ptr[l];
-  order.resize(n);
-  for (int r = 0; r < n; ++r) order[ptr[lev[r]]++] = r;
 }
 
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
-                 bool forward, int rows, bool fp32, bool spare, cudaStream_t st) {
+                 bool forward, int rows, bool fp32, bool spare, const std::vector<int> *levels,
+                 cudaStream_t st) {
   RangeHost &H = P.host;
-  std::vector<int> order, lev;
-  level_order(n, iapc, japc, forward, order, lev);
+  std::vector<int> found;
+  if (!levels) sweep_levels(n, iapc, japc, forward, found);
+  const std::vector<int> &lev = levels ? *levels : found;
   // full slices in ranges of at least 256 rows, else narrow ones in any
   const int R0 = std::max(32, (rows + 31) / 32 * 32);
   bool fits = false;
   for (int block : {INT_MAX, kNarrowBlock}) {
     const int least = block == INT_MAX ? 256 : 32;
     for (int R = R0; !fits; R = std::max(least, R / 2)) {
-      fits = range_layout(n, iapc, japc, forward, order, lev, R, block, fp32 ? 4 : 8, H);
+      fits = range_layout(n, iapc, japc, forward, lev, R, block, fp32 ? 4 : 8, H);
       if (R <= least) break;
     }
   }
@@ -626,14 +723,15 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
 // 131, a random graph of 200,000 rows 79 / 128 and 215 / 224, red-black 500 x 500
 // 15 / 16 and 62 / 56, 3000 rows without entries 12 / 9 and 32 / 33, a chain of 7
 // rows 31 / 21 and 14 / 13.
-bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows) {
+bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows,
+                   std::vector<int> (&levels)[2]) {
   const int R = std::max(32, (rows + 31) / 32 * 32);
-  std::vector<int> lev(n), mark(n);
-  std::vector<float> t(n);
-  double free = 0.0, ranges = 0.0;
-  for (int dir = 0; dir < 2; ++dir) {
+  double free[2], ranges[2];
+  const bool ok = parallel(2, (long long)iapc[n] - iapc[0] + n, [&](int dir, int) {
     const bool forward = dir == 0;
-    std::fill(mark.begin(), mark.end(), -1);
+    std::vector<int> &lev = levels[dir], mark(n, -1);
+    std::vector<float> t(n);
+    lev.resize(n);
     int nlev = 0, halo = 0, most = 0, last = -1;
     float longest = 0.f;
     for (int q = 0; q < n; ++q) {
@@ -662,10 +760,11 @@ bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &
       longest = std::max(longest, x);
       most = std::max(most, halo);
     }
-    free += 4.5 + 1.6 * nlev;
-    ranges += 5.5 + 0.0052 * (std::min(n, R) + most) + longest;
-  }
-  return ranges <= free;
+    free[dir] = 4.5 + 1.6 * nlev;
+    ranges[dir] = 5.5 + 0.0052 * (std::min(n, R) + most) + longest;
+    return true;
+  });
+  return ok && ranges[0] + ranges[1] <= free[0] + free[1];
 }
 
 void range_free(RangePlan &P) {

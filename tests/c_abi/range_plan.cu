@@ -85,7 +85,7 @@ extern "C" int range_walk64(int n, const int *iapc, const int *japc, int njapc, 
                             int forward, int rows, const double *rhs, double *out, int *info) {
   gb::RangePlan P;
   std::vector<int> ia(iapc, iapc + n + 1), ja(japc, japc + njapc);
-  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, false, false, nullptr)) return kNoPlan;
+  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, false, false, nullptr, nullptr)) return kNoPlan;
   const int v[5] = {P.R, P.nr, P.stages, P.maxblock, (int)P.host.off.size() - 1};
   std::memcpy(info, v, sizeof(v));
   const int rc = walk<double>(P, forward != 0, apc, rhs, out);
@@ -97,7 +97,7 @@ extern "C" int range_walk32(int n, const int *iapc, const int *japc, int njapc, 
                             int forward, int rows, const float *rhs, float *out, int *info) {
   gb::RangePlan P;
   std::vector<int> ia(iapc, iapc + n + 1), ja(japc, japc + njapc);
-  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, true, false, nullptr)) return kNoPlan;
+  if (!gb::range_build(P, n, ia, ja, forward != 0, rows, true, false, nullptr, nullptr)) return kNoPlan;
   const int v[5] = {P.R, P.nr, P.stages, P.maxblock, (int)P.host.off.size() - 1};
   std::memcpy(info, v, sizeof(v));
   const int rc = walk<float>(P, forward != 0, apc, rhs, out);
