@@ -451,6 +451,10 @@ static bool build_graph(gbims_handle *h) {
 // ---------------------------------------------------------------------------
 // create
 // ---------------------------------------------------------------------------
+// What a handle's creation cleared and copied, on the legacy stream, is there
+// before the handle's stream, which does not wait for that one, reads it.
+static cudaError_t settle() { return cudaStreamSynchronize(nullptr); }
+
 // Wavefront-sweep buffers for members of the given DIS shapes (nlay, nrow,
 // ncol per member) whose rows start at row0.
 static int setup_structured(gbims_handle *h, const std::vector<int> &shapes,
@@ -768,6 +772,7 @@ extern "C" int gbims_create(const gbims_settings *s, int neq, int nja, const int
   GB_CUDA(h, dalloc(&h->d_ctl, 1));
   GB_CUDA(h, cudaMallocHost((void **)&h->h_ctl, sizeof(Ctl)));
   memset(h->h_ctl, 0, sizeof(Ctl));
+  GB_CUDA(h, settle());
   return GBIMS_OK;
 }
 
@@ -1332,7 +1337,7 @@ extern "C" int gbims_autotune(gbims_handle *h, int reps, gbims_tuning *out) {
     int err = 0;
     GB_CUDA(h, cudaMemcpy(&err, h->D.d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (err) {
-      cudaMemset(h->D.d_err, 0, sizeof(int));
+      cudaMemsetAsync(h->D.d_err, 0, sizeof(int), st);
       return fail(h, GBIMS_ERR_CUDA, "structured sweep wait limit reached while tuning");
     }
     out->ncandidates = nc;
@@ -1458,6 +1463,7 @@ extern "C" int gbims_set_dis_nodes(gbims_handle *h, const int *nodeuser) {
     GB_CUDA(h, dalloc(&D.f_zfull, (size_t)nuser + kVecPad));
     GB_CUDA(h, cudaMemset(D.f_rfull, 0, sizeof(float) * ((size_t)nuser + kVecPad)));
   }
+  GB_CUDA(h, settle());
   D.mapped = true;
   drop_graph(h);
   return GBIMS_OK;
@@ -1589,6 +1595,7 @@ extern "C" int gbims_set_inner_records(gbims_handle *h, int nconv, int convnmod,
   GB_CUDA(h, cudaMemcpy(h->d_modstart, ms.data(), sizeof(int) * (convnmod + 1), cudaMemcpyHostToDevice));
   std::vector<long long> none(2 * convnmod, -1);
   GB_CUDA(h, cudaMemcpy(h->d_rec_loc, none.data(), sizeof(long long) * 2 * convnmod, cudaMemcpyHostToDevice));
+  GB_CUDA(h, settle());
   h->rec_cap = nconv;
   return GBIMS_OK;
 }
@@ -1798,6 +1805,7 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
     h->D.rows.geo = h->D.d_geo;
     h->D.rows.mctl = h->d_ctls;
     h->dia_spmv = true;
+    GB_CUDA(h, settle());
     return GBIMS_OK;
   }
   // the products skip the rows of members that are done: per SELL slice its
@@ -1815,6 +1823,7 @@ extern "C" int gbims_batch_create(const gbims_settings *settings, int nmembers,
     h->S.nm = nmembers;
     h->S.mctl = h->d_ctls;
   }
+  GB_CUDA(h, settle());
   return GBIMS_OK;
 }
 

@@ -121,6 +121,8 @@ extern "C" int gbmpnn_create(int nodes, int nja, const int *ia, const int *ja,
   MP_CUDA(h, cudaMemcpy(D.p, p.data(), sizeof(float) * p.size(), cudaMemcpyHostToDevice));
   MP_CUDA(h, cudaMemset(D.m, 0, sizeof(float) * h->np));
   MP_CUDA(h, cudaMemset(D.v, 0, sizeof(float) * h->np));
+  // the handle's stream does not wait for the legacy stream, which these are on
+  MP_CUDA(h, cudaStreamSynchronize(nullptr));
   mpnn_refresh_bf16(D, h->st);
   MP_CUDA(h, cudaStreamSynchronize(h->st));
   MP_CUDA(h, cudaGetLastError());
@@ -229,7 +231,7 @@ extern "C" int gbmpnn_get_params(gbmpnn_handle *h, float *params) {
 
 extern "C" int gbmpnn_set_params(gbmpnn_handle *h, const float *params) {
   if (!h || !params) return GBIMS_ERR_ARG;
-  MP_CUDA(h, cudaMemcpy(h->D.p, params, sizeof(float) * h->np, cudaMemcpyHostToDevice));
+  MP_CUDA(h, cudaMemcpyAsync(h->D.p, params, sizeof(float) * h->np, cudaMemcpyHostToDevice, h->st));
   mpnn_refresh_bf16(h->D, h->st);
   MP_CUDA(h, cudaStreamSynchronize(h->st));
   return GBIMS_OK;

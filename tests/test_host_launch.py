@@ -148,6 +148,58 @@ def test_plans_are_sent_on_the_handles_stream(host, level):
     assert not [l for l in lines if re.match(r"(memcpy|memset) 0 ", l)]
 
 
+def test_creation_is_done_when_it_returns(host):
+    """What the calls that make a handle clear and copy on the legacy stream is
+    waited for before the handle's own stream, which does not wait for it, reads
+    it: zeroed hand-over words above all."""
+    gi, gj, ga = grid(2, 6, 7, np.random.default_rng(0))
+    gi, gj = gi.astype(np.int32), gj.astype(np.int32)
+    bi, bj, ba = band_pattern(84, [1, 7])
+    v = np.zeros(84)
+
+    def check(call):
+        trace(host)
+        call()
+        pending = None
+        for l in trace(host):
+            if re.match(r"(memcpy|memset) 0 ", l):
+                pending = l
+            elif l == "synchronize 0":
+                pending = None
+            else:
+                assert not (pending and l.startswith("launch ")), (pending, l)
+
+    def linear(settings, ia, ja, a, *more):
+        ims = ImsLinear(settings).imslinear_allocate(84, ia, ja)
+        for call in more:
+            assert call(ims._h) == 0
+        assert host.gbims_factor(ims._h, _lib.dptr(a), None) == 0
+        assert host.gbims_precondition(ims._h, _lib.dptr(v), _lib.dptr(v)) == 0
+
+    check(lambda: linear(ImsLinearSettings(structure=GENERAL), bi, bj, ba))
+    check(lambda: linear(ImsLinearSettings(level=3), bi, bj, ba))
+    check(lambda: linear(ImsLinearSettings(structure=(2, 6, 7)), gi, gj, ga))
+    start = np.array([0, 40, 84], np.int32)
+    check(lambda: linear(ImsLinearSettings(structure=GENERAL), bi, bj, ba,
+                         lambda h: host.gbims_set_inner_records(h, 5, 2, _lib.iptr(start))))
+
+    def batch(shapes):
+        ens = EnsembleLinear(ImsLinearSettings()).allocate(np.array([0, 84], np.int32), gi, gj, shapes)
+        assert host.gbims_factor(ens._h, _lib.dptr(ga), None) == 0
+
+    check(lambda: batch(None))
+    check(lambda: batch([(2, 6, 7)]))
+
+    def network():
+        net = C.c_void_p()
+        assert host.gbmpnn_create(84, bj.size, _lib.iptr(bi), _lib.iptr(bj), 1, C.byref(net)) == 0
+        assert host.gbmpnn_set_params(net, f) == 0
+        host.gbmpnn_destroy(net)
+
+    f = np.zeros(200000, np.float32).ctypes.data_as(C.POINTER(C.c_float))
+    check(network)
+
+
 def solve_launches(host, ims, a):
     n = ims.neq
     trace(host)
