@@ -55,6 +55,7 @@
 #include <climits>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <thread>
 
 #include "gbims_internal.cuh"
@@ -682,7 +683,7 @@ static void sweep_levels(int n, const std::vector<int> &iapc, const std::vector<
 
 bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::vector<int> &japc,
                  bool forward, int rows, bool fp32, bool spare, const std::vector<int> *levels,
-                 cudaStream_t st) {
+                 cudaStream_t st) try {
   RangeHost &H = P.host;
   std::vector<int> found;
   if (!levels) sweep_levels(n, iapc, japc, forward, found);
@@ -697,7 +698,10 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
       if (R <= least) break;
     }
   }
-  if (!fits) return false;
+  if (!fits) {
+    H = RangeHost();
+    return false;
+  }
   P.n = n;
   P.R = H.R;
   P.nr = H.nr;
@@ -712,6 +716,9 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
       upload(H.halo, &P.d_halo, &P.c_halo, spare, st);
   // the host arrays may go when this returns
   return cudaStreamSynchronize(st) == cudaSuccess && sent;
+} catch (const std::bad_alloc &) {
+  P.host = RangeHost();
+  return false;
 }
 
 // Both forms' times from the pattern alone, us a sweep.  Sync-free: 4.5 and 1.6 a

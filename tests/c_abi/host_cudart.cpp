@@ -10,12 +10,24 @@
 // whatever its conditions.
 #include <cuda_runtime_api.h>
 
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <new>
 #include <string>
 #include <vector>
+
+// The library's own host allocations of more than `largest` bytes fail.
+static long long largest = LLONG_MAX;
+void *operator new(size_t n) {
+  void *p = (long long)n > largest ? nullptr : std::malloc(n ? n : 1);
+  if (!p) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 struct CUgraph_st {
   std::vector<std::string> lines;  // captured launches
@@ -81,6 +93,7 @@ const char *host_trace() { return trace.c_str(); }
 void host_trace_clear() { trace.clear(); }
 void host_set_device(int d) { device = d; }
 long long host_bytes() { return (long long)held; }
+void host_largest(long long bytes) { largest = bytes; }
 // the next copy of that many bytes fails
 void host_fail_copy(long long bytes) { failing = bytes; }
 

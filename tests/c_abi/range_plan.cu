@@ -3,9 +3,12 @@
 // (host_cudart.cpp), so that no GPU is needed.
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "k_range.cu"
+
+extern "C" void host_largest(long long bytes);  // host_cudart.cpp
 
 namespace {
 
@@ -101,6 +104,23 @@ extern "C" int range_walk32(int n, const int *iapc, const int *japc, int njapc, 
   const int v[5] = {P.R, P.nr, P.stages, P.maxblock, (int)P.host.off.size() - 1};
   std::memcpy(info, v, sizeof(v));
   const int rc = walk<float>(P, forward != 0, apc, rhs, out);
+  gb::range_free(P);
+  return rc;
+}
+
+// A plan where no allocation of more than `bytes` succeeds: kOk or kNoPlan, -1 when
+// an exception gets out.
+extern "C" int range_starved(int n, const int *iapc, const int *japc, int njapc, int forward, int rows,
+                             long long bytes) {
+  gb::RangePlan P;
+  std::vector<int> ia(iapc, iapc + n + 1), ja(japc, japc + njapc);
+  int rc = -1;
+  host_largest(bytes);
+  try {
+    rc = gb::range_build(P, n, ia, ja, forward != 0, rows, false, false, nullptr, nullptr) ? kOk : kNoPlan;
+  } catch (const std::bad_alloc &) {
+  }
+  host_largest(LLONG_MAX);
   gb::range_free(P);
   return rc;
 }

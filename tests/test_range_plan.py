@@ -127,3 +127,15 @@ def test_cut_slices_and_halved_ranges(plans):
     z, info = walk(plans, iapc, japc, apc, v[:3200], 2048)
     np.testing.assert_array_equal(z, oracle.ilu0a(apc, iapc, japc, v[:3200], fma=True))
     assert all(i["slices"] == 100 for i in info)
+
+
+@pytest.mark.parametrize("forward", [1, 0])
+def test_no_memory_is_no_plan(plans, forward):
+    """Where an allocation of the plan fails, there is none, and the caller sweeps
+    without: no exception leaves the library."""
+    n, lower = PATTERNS["grid"]
+    iapc, japc, apc = factor_pattern(n, lower, seed=n)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    results = {plans.range_starved(n, p(iapc), p(japc), japc.size, forward, 2048, C.c_longlong(1 << k))
+               for k in range(2, 28)}
+    assert results == {0, 1}
