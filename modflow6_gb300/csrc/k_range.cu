@@ -460,33 +460,63 @@ bool upload(const H &h, V **d, size_t *cap, bool spare, cudaStream_t st) {
   return n == 0 || cudaMemcpyAsync(*d, h.data(), sizeof(V) * n, cudaMemcpyHostToDevice, st) == cudaSuccess;
 }
 
-// f(i, thread) for i < count on up to `most` threads; false when one returned
-// false or threw.
+// Up to `most` threads that do several jobs together, the calling one among them:
+// started once (a thread costs some 50 us, an entry of a plan some 10 ns) and
+// yielding between jobs, of which there are a few in each millisecond.
 constexpr int kPlanThreads = 8;
-template <class F>
-bool parallel(int count, long long work, F f, int most = kPlanThreads) {
-  std::atomic<int> next{0};
-  std::atomic<bool> ok{true};
-  auto run = [&](int thread) {
+class Team {
+  std::vector<std::thread> others;
+  std::atomic<int> job{0}, left{0}, next{0}, count{0};
+  std::atomic<bool> ok{true}, end{false};
+  bool (*call)(void *, int, int) = nullptr;
+  void *what = nullptr;
+
+  void take(int thread) {
     try {
-      for (int i; ok && (i = next.fetch_add(1)) < count;)
-        if (!f(i, thread)) ok = false;
+      for (int i; ok.load(std::memory_order_relaxed) && (i = next.fetch_add(1)) < count.load();)
+        if (!call(what, i, thread)) ok = false;
     } catch (...) {
       ok = false;
     }
-  };
-  // a thread costs some 30 us, an entry some 10 ns
-  const int want = (int)std::min<long long>({(long long)most, (long long)count, 1 + work / 20000,
-                                             (long long)std::max(1u, std::thread::hardware_concurrency())});
-  std::vector<std::thread> others;
-  try {
-    for (int t = 1; t < want; ++t) others.emplace_back(run, t);
-  } catch (...) {  // fewer threads, then
   }
-  run(0);
-  for (std::thread &t : others) t.join();
-  return ok;
-}
+
+ public:
+  Team(long long work, int most) {
+    const int want = (int)std::min<long long>({(long long)most, 1 + work / 50000,
+                                               (long long)std::max(1u, std::thread::hardware_concurrency())});
+    try {
+      for (int t = 1; t < want; ++t)
+        others.emplace_back([this, t] {
+          for (int seen = 0;;) {
+            while (job.load(std::memory_order_acquire) == seen && !end) std::this_thread::yield();
+            if (end) return;
+            ++seen;
+            take(t);
+            left.fetch_sub(1, std::memory_order_release);
+          }
+        });
+    } catch (...) {  // fewer threads, then
+    }
+  }
+  ~Team() {
+    end = true;
+    for (std::thread &t : others) t.join();
+  }
+  Team(const Team &) = delete;
+  // f(i, thread) for i < n; false when one returned false or threw.
+  template <class F>
+  bool run(int n, F f) {
+    call = [](void *w, int i, int thread) { return (*static_cast<F *>(w))(i, thread); };
+    what = &f;
+    next = 0;
+    count = n;
+    left = (int)others.size();
+    job.fetch_add(1, std::memory_order_release);
+    take(0);
+    while (left.load(std::memory_order_acquire) > 0) std::this_thread::yield();
+    return ok;
+  }
+};
 
 }  // namespace
 
@@ -516,15 +546,25 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
   std::vector<Range> ranges(nr);
   P.rows.resize(n);
   std::vector<int> place(n);  // row -> its slot, when it is its range's own
+  // which rows other ranges read is only known when all blocks are done
+  std::unique_ptr<std::atomic<unsigned char>[]> read(new std::atomic<unsigned char>[(size_t)n]);
+  struct Scratch {
+    std::vector<int> mark, hidx;
+    std::vector<size_t> pads;
+  };
+  // (two words a row and thread: at most 800 MB, or one thread's)
+  std::vector<Scratch> scratch((size_t)std::max(1LL, std::min({(long long)kPlanThreads, 100000000LL / n, (long long)nr})));
+  Team team(work, (int)scratch.size());
   // the rows of each range in level order, cut into slices of up to 32 rows of
   // one level
-  const bool cut = parallel(nr, work, [&](int b, int) {
+  const bool cut = team.run(nr, [&](int b, int) {
     Range &G = ranges[b];
     const int r0 = b * R, nloc = std::min(R, n - r0);
     int lo = INT_MAX, hi = 0;
     for (int r = r0; r < r0 + nloc; ++r) {
       lo = std::min(lo, lev[r]);
       hi = std::max(hi, lev[r]);
+      read[r].store(0, std::memory_order_relaxed);
     }
     int *rows = &P.rows[r0];
     if (hi - lo < 4 * nloc) {
@@ -574,20 +614,7 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
   P.dst.need((size_t)entry0[nr]);
   P.off.resize((size_t)P.rslice[nr] + 1);
   P.off[P.rslice[nr]] = (int)(byte0[nr] / 16);
-  // the blocks; which rows other ranges read is only known when all are done
-  std::unique_ptr<std::atomic<unsigned char>[]> read(new std::atomic<unsigned char>[(size_t)n]);
-  struct Scratch {
-    std::vector<int> mark, hidx;
-    std::vector<size_t> pads;
-  };
-  // (two words a row and thread: at most 800 MB, or one thread's)
-  const int threads = (int)std::max(1LL, std::min((long long)kPlanThreads, 100000000LL / n));
-  std::vector<Scratch> scratch(threads);
-  const bool filled = parallel(nr, work, [&](int b, int) {
-    const int r0 = b * R, nloc = std::min(R, n - r0);
-    for (int r = r0; r < r0 + nloc; ++r) read[r].store(0, std::memory_order_relaxed);
-    return true;
-  }) && parallel(nr, work, [&](int b, int thread) {
+  const bool filled = team.run(nr, [&](int b, int thread) {
     Range &G = ranges[b];
     Scratch &S = scratch[thread];
     if (S.mark.empty()) {
@@ -643,7 +670,7 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
     if (zero > 65535) return false;
     for (size_t sp : S.pads) *reinterpret_cast<unsigned short *>(blk + sp) = (unsigned short)zero;
     return true;
-  }, threads);
+  });
   if (!filled) return false;
   P.hptr.assign(nr + 1, 0);
   P.halo.clear();
@@ -655,7 +682,7 @@ static bool range_layout(int n, const std::vector<int> &iapc, const std::vector<
     P.maxslots = std::max(P.maxslots, std::min(R, n - b * R) + (int)G.halo.size() + 1);
   }
   if ((size_t)P.stages * P.maxblock + tsize * (size_t)P.maxslots > kSmemBytes) return false;
-  return parallel(nr, work, [&](int b, int) {
+  return team.run(nr, [&](int b, int) {
     for (int s = P.rslice[b]; s < P.rslice[b + 1]; ++s) {
       unsigned char *bl = P.blk.data() + 16 * (size_t)P.off[s];
       SliceHead head;
@@ -734,7 +761,8 @@ bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &
                    std::vector<int> (&levels)[2]) {
   const int R = std::max(32, (rows + 31) / 32 * 32);
   double free[2], ranges[2];
-  const bool ok = parallel(2, (long long)iapc[n] - iapc[0] + n, [&](int dir, int) {
+  Team team((long long)iapc[n] - iapc[0] + n, 2);
+  const bool ok = team.run(2, [&](int dir, int) {
     const bool forward = dir == 0;
     std::vector<int> &lev = levels[dir], mark(n, -1);
     std::vector<float> t(n);
