@@ -416,21 +416,27 @@ static void apply_levels(const int *d_iapc, const int *d_japc, const T *d_apc,
   }
 }
 
-// The sync-free sweeps: one launch per sweep, the rows in level order over a
-// resident grid, every value handed over through L2 as a word tagged with the
-// launch's epoch.  Polling is warp-synchronous: in each round every unfinished
-// lane loads all its dependencies' words (up to kDeps in flight at once), and
-// a lane whose words are all of this epoch finishes its row; a lane may wait
-// for one of its own warp, which is seen in the next round.  Rows depend only
-// on rows of lower levels, earlier in the list, and all CTAs are resident, so
-// the lowest unfinished row can always proceed; every wait is bounded besides.
+// The sync-free sweeps: one launch per sweep, a thread a row, the rows in level
+// order, every value handed over through L2 as a word tagged with the launch's
+// epoch.  Polling is warp-synchronous: in each round every unfinished lane loads
+// all its dependencies' words (up to kDeps in flight at once), and a lane whose
+// words are all of this epoch finishes its row; a lane may wait for one of its own
+// warp, which is seen in the next round.  Rows depend only on rows of lower levels,
+// earlier in the list, and a CTA takes the 256 rows of its ticket, in the order in
+// which CTAs start: the lowest unfinished row is always a running CTA's, however
+// many are resident, also beside another handle's sweeps.  Every wait is bounded
+// besides.
 //
-// Bound by the levels, 1.6 us each, where a range sweep pays for its setup, for
-// its halo's way through three warps (5 ns an entry) and for its crossings
-// between ranges: both sweeps of a red-black ordered 500 x 500 grid (2 levels)
-// take 16 us against 56 in ranges, of 300 x 300 cells in random order (16) 58
-// against 131, of a random graph of 200,000 rows (22) 128 against 224; of 1000
-// separate 10 x 10 grids (19) 74 against 37.
+// Bound by the levels, 1.6 us each (more where the rows far ahead of the front are
+// many: their polls slow it), where a range sweep pays for its setup, for its
+// halo's way through three warps (5 ns an entry) and for its crossings between
+// ranges: both sweeps of a red-black ordered 500 x 500 grid (2 levels) take 16 us
+// against 54 in ranges, of 300 x 300 cells in random order (16) 64 against 132, of
+// a random graph of 200,000 rows (22) 142 against 224; of 1000 separate 10 x 10
+// grids (19) 76 against 37.  With fixed strides over a grid of resident CTAs the
+// first three took 15, 61 and 128 and 1500 x 1500 red-black 91 against 108 now, but
+// all CTAs had to be resident: beside another handle's sweeps a warp could wait for
+// a CTA that waited for its place.  Claims by warp took 24, 65, -, 137.
 template <typename T, int DIR>
 __global__ void __launch_bounds__(256) k_ilu_sweep_sf(int n, const int *__restrict__ rows,
                                                       const int *__restrict__ iapc,
@@ -440,97 +446,78 @@ __global__ void __launch_bounds__(256) k_ilu_sweep_sf(int n, const int *__restri
                                                       const LLWord<T> *__restrict__ yin,
                                                       LLWord<T> *out, T *d,
                                                       unsigned long long *ticket, int *err,
-                                                      Ctl *ctl, int active) {
+                                                      Ctl *ctl) {
   __shared__ unsigned s_ep;
+  __shared__ int s_t;
   if (threadIdx.x == 0) {
     // every CTA takes a ticket, so launch e owns tickets [e*grid, (e+1)*grid)
-    const unsigned long long tk = atomicAdd(ticket, 1ULL);
-    s_ep = (unsigned)(tk / gridDim.x) + 1u;
+    const unsigned long long tk = atomicAdd(ticket, 1ULL), launch = tk / gridDim.x;
+    s_ep = (unsigned)launch + 1u;
+    s_t = (int)(tk - launch * gridDim.x);
   }
   __syncthreads();
   if (ctl && ctl->done) return;
-  // the launch always has the same (resident) grid, so that its tickets and
-  // epochs line up with every other launch; CTAs past `active` only take
-  // their ticket
-  if ((int)blockIdx.x >= active) return;
   const unsigned ep = s_ep;
   const int lane = threadIdx.x & 31;
   volatile int *vdone = ctl ? &ctl->done : nullptr;
   constexpr int kDeps = 8;
-  const int stride = active * blockDim.x;
-  for (int q0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); q0 < n; q0 += stride) {
-    const int q = q0 + lane;
-    bool done = q >= n;
-    int row = 0, j0 = 0, j1 = 0;
-    T tv0 = T(0);
-    if (!done) {
-      row = rows[q];
-      if (DIR > 0) {
-        tv0 = r[row];
-        j0 = iapc[row];
-        j1 = japc[row];
-      } else {
-        tv0 = ll_val(yin[row]);
-        j0 = japc[row];
-        j1 = iapc[row + 1];
-      }
-    }
-    const unsigned long long t0 = wclock();
-    while (true) {
-      if (!done) {
-        T tv = tv0;
-        bool ok = true;
-        for (int jb = j0; ok && jb < j1; jb += kDeps) {
-          LLRaw w[kDeps];
-          const int nd = min(kDeps, j1 - jb);
-#pragma unroll
-          for (int q2 = 0; q2 < kDeps; ++q2)
-            if (q2 < nd) ll_issue(out + japc[jb + q2], w[q2]);
-#pragma unroll
-          for (int q2 = 0; q2 < kDeps; ++q2) {
-            if (q2 >= nd || !ok) break;
-            if (!ll_ready<T>(w[q2], ep)) {
-              ok = false;
-            } else {
-              T v;
-              ll_take(w[q2], v);
-              tv = fms<T>(apc[jb + q2], v, tv);
-            }
-          }
-        }
-        if (ok) {
-          if (DIR < 0) {
-            tv = tv * apc[row];
-            d[row] = tv;
-          }
-          ll_put(out + row, tv, ep);
-          done = true;
-        }
-      }
-      if (!__any_sync(0xffffffffu, !done)) break;
-      if (__any_sync(0xffffffffu, (vdone && *vdone) || wclock() - t0 > kWaitCycles)) {
-        if (lane == 0) {
-          atomicExch(err, 1);
-          if (ctl) ctl->done = 1;
-        }
-        return;
-      }
+  const int q = s_t * 256 + (int)threadIdx.x;
+  bool done = q >= n;
+  int row = 0, j0 = 0, j1 = 0;
+  T tv0 = T(0);
+  if (!done) {
+    row = rows[q];
+    if (DIR > 0) {
+      tv0 = r[row];
+      j0 = iapc[row];
+      j1 = japc[row];
+    } else {
+      tv0 = ll_val(yin[row]);
+      j0 = japc[row];
+      j1 = iapc[row + 1];
     }
   }
-}
-
-// Blocks: every CTA that can be resident, always the same (the epochs count
-// launches of that grid); 8 threads per row of the widest level work, the rest
-// return after their ticket.  Threads several levels ahead of the front have
-// their rows' indices and operands loaded by the time it reaches them.
-template <typename T, int DIR>
-static int sf_grid() {
-  static const int per_sm = [] {  // every device is a GB300
-    int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ilu_sweep_sf<T, DIR>, 256, 0);
-    return std::max(1, occ);
-  }();
-  return per_sm * kNumSM;
+  const unsigned long long t0 = wclock();
+  while (true) {
+    if (!done) {
+      T tv = tv0;
+      bool ok = true;
+      for (int jb = j0; ok && jb < j1; jb += kDeps) {
+        LLRaw w[kDeps];
+        const int nd = min(kDeps, j1 - jb);
+#pragma unroll
+        for (int q2 = 0; q2 < kDeps; ++q2)
+          if (q2 < nd) ll_issue(out + japc[jb + q2], w[q2]);
+#pragma unroll
+        for (int q2 = 0; q2 < kDeps; ++q2) {
+          if (q2 >= nd || !ok) break;
+          if (!ll_ready<T>(w[q2], ep)) {
+            ok = false;
+          } else {
+            T v;
+            ll_take(w[q2], v);
+            tv = fms<T>(apc[jb + q2], v, tv);
+          }
+        }
+      }
+      if (ok) {
+        if (DIR < 0) {
+          tv = tv * apc[row];
+          d[row] = tv;
+        }
+        ll_put(out + row, tv, ep);
+        done = true;
+      }
+    }
+    if (!__any_sync(0xffffffffu, !done)) break;
+    if (__any_sync(0xffffffffu, (vdone && *vdone) || wclock() - t0 > kWaitCycles)) {
+      if (lane == 0) {
+        atomicExch(err, 1);
+        if (ctl) ctl->done = 1;
+      }
+      return;
+    }
+  }
 }
 
 template <typename T>
@@ -538,14 +525,11 @@ static void apply_sf(int n, const int *d_iapc, const int *d_japc, const T *d_apc
                      const Levels &B, const LevelWords &W, const T *r, T *d, Ctl *ctl, cudaStream_t st) {
   LLWord<T> *yf = static_cast<LLWord<T> *>(W.fwd);
   LLWord<T> *zb = static_cast<LLWord<T> *>(W.bwd);
-  const int gf = sf_grid<T, 1>(), gb = sf_grid<T, -1>();
-  auto active = [](int grid, int width) {
-    return (int)std::max<long long>(1, std::min<long long>(((long long)width * 8 + 255) / 256, grid));
-  };
-  k_ilu_sweep_sf<T, 1><<<gf, 256, 0, st>>>(n, F.d_rows, d_iapc, d_japc, d_apc, r, nullptr, yf, nullptr, W.ticket,
-                                           W.err, ctl, active(gf, F.maxwidth));
-  k_ilu_sweep_sf<T, -1><<<gb, 256, 0, st>>>(n, B.d_rows, d_iapc, d_japc, d_apc, nullptr, yf, zb, d, W.ticket + 16,
-                                            W.err, ctl, active(gb, B.maxwidth));
+  const int grid = (int)(((long long)n + 255) / 256);
+  k_ilu_sweep_sf<T, 1><<<grid, 256, 0, st>>>(n, F.d_rows, d_iapc, d_japc, d_apc, r, nullptr, yf, nullptr, W.ticket,
+                                             W.err, ctl);
+  k_ilu_sweep_sf<T, -1><<<grid, 256, 0, st>>>(n, B.d_rows, d_iapc, d_japc, d_apc, nullptr, yf, zb, d, W.ticket + 16,
+                                              W.err, ctl);
 }
 
 void launch_ilu_apply_sf(int n, const int *d_iapc, const int *d_japc, const double *d_apc, const Levels &F,

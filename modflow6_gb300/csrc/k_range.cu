@@ -751,12 +751,12 @@ bool range_build(RangePlan &P, int n, const std::vector<int> &iapc, const std::v
 // Both forms' times from the pattern alone, us a sweep.  Sync-free: 4.5 and 1.6 a
 // level.  Over ranges: 5.5, 5 ns for each row and halo entry of the largest
 // range, and the longest chain of dependent rows at 0.2 a link inside a range
-// and 1.5 across.  Estimated / measured, both sweeps: 60 x 60 x 60 cells 579 / 694
-// sync-free and 298 / 373 in ranges, 1000 x 1000 6406 / 6687 and 2110 / 1938, 1000
-// grids of 10 x 10 70 / 74 and 42 / 37, 300 x 300 in random order 60 / 58 and 148 /
-// 131, a random graph of 200,000 rows 79 / 128 and 215 / 224, red-black 500 x 500
-// 15 / 16 and 62 / 56, 3000 rows without entries 12 / 9 and 32 / 33, a chain of 7
-// rows 31 / 21 and 14 / 13.
+// and 1.5 across.  Estimated / measured, both sweeps: 60 x 60 x 60 cells 579 / 1323
+// sync-free and 298 / 372 in ranges, 1000 x 1000 6406 / 10463 and 2110 / 1956, 1000
+// grids of 10 x 10 70 / 76 and 42 / 37, 300 x 300 in random order 60 / 64 and 148 /
+// 132, a random graph of 200,000 rows 79 / 142 and 215 / 224, red-black 500 x 500
+// 15 / 16 and 62 / 54, 3000 rows without entries 12 / 8 and 32 / 33, a chain of 7
+// rows 31 / 19 and 14 / 12.
 bool ranges_faster(int n, const std::vector<int> &iapc, const std::vector<int> &japc, int rows,
                    std::vector<int> (&levels)[2]) {
   const int R = std::max(32, (rows + 31) / 32 * 32);

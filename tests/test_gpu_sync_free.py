@@ -1,8 +1,10 @@
 """The sync-free sweeps of patterns with few levels (k_ilu.cu) against the oracle's
 ilu0a, bit for bit in FP64: no entries, levels of one row and of many, rows of
-many entries, more rows than threads, non-finite right-hand sides; and between
-the forms of the sweeps on one handle."""
+many entries, more rows than threads, non-finite right-hand sides; between the
+forms of the sweeps on one handle; and by several threads on handles of their
+own."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -70,3 +72,33 @@ def test_sync_free_bitexact(gblib, name):
     assert gblib.gbims_factor(m32._h, _lib.dptr(amat), None) == 0
     assert gblib.gbims_precondition(m32._h, _lib.dptr(v), _lib.dptr(z)) == 0
     assert np.max(np.abs(z - zo)) <= 1e-5 * np.max(np.abs(zo))
+
+
+def test_side_by_side(gblib):
+    """Sweeps of several handles at once, each with more blocks than its share of
+    the GPU has places for: none waits for rows that nobody works on."""
+    n = 400000
+    ia, ja, amat = random_pattern(n, 0.4, seed=n)
+    v = np.random.default_rng(2).standard_normal(n)
+    lin = [ImsLinear(ImsLinearSettings(structure=GENERAL)).imslinear_allocate(n, ia, ja) for _ in range(3)]
+    z = np.zeros((len(lin), n))
+    for k, ims in enumerate(lin):
+        assert gblib.gbims_factor(ims._h, _lib.dptr(amat), None) == 0
+        assert gblib.gbims_precondition(ims._h, _lib.dptr(v), _lib.dptr(z[k])) == 0
+    want, wrong = z[0].copy(), []
+    assert np.array_equal(want, z[1])
+
+    def run(k):
+        times = _lib.GbimsKernelTimes()
+        for _ in range(5):
+            if gblib.gbims_time_kernels(lin[k]._h, 40, C.byref(times)) != 0:
+                wrong.append(k)
+            if gblib.gbims_precondition(lin[k]._h, _lib.dptr(v), _lib.dptr(z[k])) != 0 or not np.array_equal(z[k], want):
+                wrong.append(k)
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(len(lin))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not wrong
